@@ -20,12 +20,13 @@
 //     the mbarrier that frees the stage; the epilogue reads the accumulator with tcgen05.ld (lane = tile row)
 //     and writes coalesced NCHW rows;
 //   * stemconv.cu — fp32-pipe kernels for the 3-channel 3x3 first layer.
-// Every wait is bounded.  Input gradients for stride > 1 use a plain gather kernel (no network on the
-// benchmarked path needs them: a strided first layer has no input gradient).
+//   * pwg::gather_gemm_kernel<OP, BN> (conv_gather.cuh) — strided input gradients, one GEMM per stride residue, summed in registers.
+// Every wait is bounded.
 #include "common.cuh"
 #include "stemconv.h"
 
 #include <algorithm>
+#include <vector>
 
 namespace cunn {
 namespace mm {
@@ -546,7 +547,7 @@ add_plane_bias_kernel(float *__restrict__ y, const float *__restrict__ bias, int
         y[i] += __ldg(bias + (int)((i / HW) % Q));
 }
 
-// Input gradient for any stride: gather form, one thread per input pixel (correctness path).
+// Input gradient, gather form, one thread per input pixel: residues of more than 16 rows or columns of taps.
 __global__ void __launch_bounds__(256)
 dgrad_gather_kernel(const float *__restrict__ gy, const float *__restrict__ w, float *__restrict__ gx, int C, int H, int W,
                     int K, int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, int oH, int oW, long long total)
@@ -1293,6 +1294,7 @@ pw_gemm_kernel(const Params p)
 }  // namespace pw
 
 #include "pw_tma.cuh"
+#include "conv_gather.cuh"
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -1541,6 +1543,106 @@ static void pw_wgrad_plan(int N, int C, int K, int HW, int *bn, int *splits, int
     *splits = ceil_div(N, best_ips);
 }
 
+// ---- gathered operand, register accumulation (conv_gather.cuh) -------------------------------------------------------
+typedef void (*GatherKernel)(const pwg::GatherParams);
+template <int OP>
+static GatherKernel gather_pick(int bn)
+{
+    switch (bn) {
+        case 32: return pwg::gather_gemm_kernel<OP, 32>;
+        case 64: return pwg::gather_gemm_kernel<OP, 64>;
+        default: return pwg::gather_gemm_kernel<OP, 128>;
+    }
+}
+static uint32_t magic_of(int d) { return d == 1 ? 0u : (uint32_t)((1ull << 32) / (unsigned)d + 1u); }
+template <int OP>
+static int launch_gather(pwg::GatherParams &p, int bn, cudaStream_t stream)
+{
+    p.n_tiles = ceil_div(p.N_total, bn);
+    p.total_tiles = 0;
+    for (int i = 0; i < p.n_phases; ++i) {
+        pwg::Phase &f = p.ph[i];
+        f.tile0 = p.total_tiles;
+        f.kblocks = ceil_div(f.Kd, BK);
+        f.taps_magic = magic_of(f.taps);
+        f.kW_magic = magic_of(f.kW);
+        p.total_tiles += ceil_div(f.M_total, BM) * p.n_tiles;
+    }
+    const GatherKernel kern = gather_pick<OP>(bn);
+    CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pwg::GSMEM));
+    void *args[] = {(void *)&p};
+    CUNN_CUDA(cudaLaunchKernel((const void *)kern, dim3(std::min(p.total_tiles, sm_count())), dim3(pwg::GTHREADS), args, pwg::GSMEM, stream));
+    return 0;
+}
+
+// One residue of an axis of an input gradient: input positions h0 + i * d (i < n) are reached by taps k0 + t * kstep
+// (t < taps) at output positions o0 + i - t * ostep.
+struct AxisPhase {
+    int h0, n, k0, taps, kstep, o0, ostep;
+};
+static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil)
+{
+    int g = d, r = dil % d;
+    while (r) { const int t = g % r; g = r; r = t; }                       // gcd(d, dil)
+    std::vector<AxisPhase> out;
+    for (int h0 = 0; h0 < std::min(d, H); ++h0) {
+        AxisPhase a{h0, (H - h0 + d - 1) / d, 0, 0, d / g, 0, dil / g};
+        for (int t = 0; t < k; ++t) {
+            const int num = h0 + pad - t * dil;
+            if (num % d) continue;
+            if (!a.taps) { a.k0 = t; a.o0 = num / d; }
+            ++a.taps;
+        }
+        out.push_back(a);
+    }
+    return out;
+}
+// Every phase of every axis within the kernel's sixteen rows and columns of taps.
+static bool phases_fit(const std::vector<AxisPhase> &v)
+{
+    for (const AxisPhase &a : v)
+        if (a.taps > pwg::MAX_KERNEL) return false;
+    return true;
+}
+
+// Input gradient of a convolution with any stride, padding and dilation, plus `bias` per input channel (null: none): the
+// forward pass of a transposed convolution has one.
+static int phased_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
+                             int kH, int kW, int dH, int dW, const std::vector<AxisPhase> &ah, const std::vector<AxisPhase> &aw,
+                             int oH, int oW, cudaStream_t stream)
+{
+    std::vector<pwg::Phase> ph;
+    for (const AxisPhase &a : ah)
+        for (const AxisPhase &b : aw) {
+            pwg::Phase f{};
+            f.HW = a.n * b.n; f.pix_W = b.n; f.M_total = N * f.HW;
+            f.taps = a.taps * b.taps; f.kW = b.taps; f.Kd = K * f.taps;
+            f.dH = f.dW = 1;
+            f.padH = -a.o0; f.padW = -b.o0; f.dilH = -a.ostep; f.dilW = -b.ostep;
+            f.w_base = a.k0 * kW + b.k0; f.w_sH = a.kstep * kW; f.w_sW = b.kstep;
+            f.o_off = a.h0 * W + b.h0; f.o_sH = dH * W; f.o_sW = dW;
+            if (f.taps) {
+                ph.push_back(f);
+                continue;
+            }
+            const long long total = (long long)N * C * f.HW;
+            const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 8));
+            pwg::phase_fill_kernel<<<blocks, 256, 0, stream>>>(gx, bias, C, H * W, f.HW, f.pix_W, f.o_off, f.o_sH, f.o_sW, total);
+            CUNN_LAUNCH_CHECK("convmm grad input (pixels without taps)");
+        }
+    // longest reductions first: the persistent grid deals tiles round-robin, so the last wave is made of the short ones
+    std::stable_sort(ph.begin(), ph.end(), [](const pwg::Phase &a, const pwg::Phase &b) { return a.taps > b.taps; });
+    for (size_t at = 0; at < ph.size(); at += pwg::MAX_PHASES) {
+        pwg::GatherParams q{};
+        q.a = gy; q.b = weight; q.bias = bias; q.out = gx; q.status = device_status_ptr();
+        q.g_C = K; q.g_H = oH; q.g_W = oW; q.N_total = C; q.w_kk = kH * kW; q.o_HW = H * W;
+        q.n_phases = (int)std::min<size_t>(pwg::MAX_PHASES, ph.size() - at);
+        for (int i = 0; i < q.n_phases; ++i) q.ph[i] = ph[at + i];
+        if (launch_gather<OP_DGRAD>(q, pw_bn_for(C), stream)) return 1;
+    }
+    return 0;
+}
+
 }  // namespace mm
 }  // namespace cunn
 
@@ -1605,10 +1707,20 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     return launch(pick_kernel<OP_FWD>(ks_of(kH, kW), bn), p, grid, bn, stream);
 }
 
-static int conv_grad_input(const float *gy, const float *weight, float *gx, int N, int C, int H, int W, int K, int kH, int kW,
-                           int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_)
+// `bias` (null: none) is added to every plane of gx: a transposed convolution's forward pass is this one plus its bias.
+static int conv_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
+                           int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_)
 {
     clear_error();
+    // the stride-1 kernels leave the bias to a pass of its own
+    auto add_bias = [&](int rc) {
+        if (rc || !bias) return rc;
+        const long long total = (long long)N * C * H * W;
+        const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
+        add_plane_bias_kernel<<<blocks, 256, 0, (cudaStream_t)stream_>>>(gx, bias, C, H * W, total);
+        CUNN_LAUNCH_CHECK("full convolution bias");
+        return 0;
+    };
     cudaStream_t stream = (cudaStream_t)stream_;
     int oH, oW;
     if (check(N, C, H, W, K, kH, kW, dH, dW, padH, padW, &oH, &oW, dilH, dilW)) return 1;
@@ -1632,12 +1744,12 @@ static int conv_grad_input(const float *gy, const float *weight, float *gx, int 
             if (make_map(&mb, weight, C, K, 0, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return 1;
             if (q.bulk_out) { if (make_map(&mo, gx, q.HW, C, N, BM, pwt::HALF_STAGE_COLS, CU_TENSOR_MAP_SWIZZLE_NONE)) return 1; }
             else mo = ma;
-            return pw_tma_launch(pw_tma_pick<OP_DGRAD>(bn), q, ma, mb, mo, stream);
+            return add_bias(pw_tma_launch(pw_tma_pick<OP_DGRAD>(bn), q, ma, mb, mo, stream));
         }
         q.vec_a = (q.HW % 4 == 0) && aligned16(gy); q.vec_b = (C % 4 == 0) && aligned16(weight);
         q.bulk_out = (q.HW % 4 == 0) && q.HW >= 8 * BM && aligned16(gx);
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
-        return pw_launch(pw_pick<OP_DGRAD>(bn), q, stream);
+        return add_bias(pw_launch(pw_pick<OP_DGRAD>(bn), q, stream));
     }
     if (dH == 1 && dW == 1 && padH <= dilH * (kH - 1) && padW <= dilW * (kW - 1) && (!dilated || gather_applies(kH, kW))) {
         // stride 1: a convolution of gy with the kernel rotated by 180 degrees and padding dil (k - 1) - pad
@@ -1652,7 +1764,7 @@ static int conv_grad_input(const float *gy, const float *weight, float *gx, int 
             q.vec_a = 0; q.vec_b = 0;
             q.bulk_out = (q.HW % 4 == 0) && q.HW >= 8 * BM && aligned16(gx);
             pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
-            return pw_launch(pw_pick<OP_DGRAD>(bn, gather_ks(kH, kW)), q, stream);
+            return add_bias(pw_launch(pw_pick<OP_DGRAD>(bn, gather_ks(kH, kW)), q, stream));
         }
         GemmParams p{};
         p.a_src = gy; p.b_src = weight; p.bias = nullptr; p.out = gx; p.status = device_status_ptr();
@@ -1661,13 +1773,15 @@ static int conv_grad_input(const float *gy, const float *weight, float *gx, int 
         p.M_total = N * H * W; p.N_total = C; p.Kd = K * kH * kW; p.kblocks = ceil_div(p.Kd, BK); p.out_HW = H * W;
         const int bn = pick_bn_for(C);
         dim3 grid(ceil_div(p.M_total, BM), ceil_div(C, bn), 1);
-        return launch(pick_kernel<OP_DGRAD>(ks_of(kH, kW), bn), p, grid, bn, stream);
+        return add_bias(launch(pick_kernel<OP_DGRAD>(ks_of(kH, kW), bn), p, grid, bn, stream));
     }
+    const std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH), aw = axis_phases(W, kW, dW, padW, dilW);
+    if (phases_fit(ah) && phases_fit(aw)) return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, ah, aw, oH, oW, stream);
     const long long total = (long long)N * C * H * W;
     const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
     dgrad_gather_kernel<<<blocks, 256, 0, stream>>>(gy, weight, gx, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW, total);
     CUNN_LAUNCH_CHECK("convmm grad input (gather)");
-    return 0;
+    return add_bias(0);
 }
 
 static size_t conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW, int padH, int padW,
@@ -1804,7 +1918,7 @@ extern "C" CUNN_API int cunn_b200_convmm_grad_input(const float *gy, const float
                                                     int W, int K, int kH, int kW, int dH, int dW, int padH, int padW,
                                                     cunn_stream_t stream)
 {
-    return conv_grad_input(gy, weight, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1, stream);
+    return conv_grad_input(gy, weight, nullptr, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1, stream);
 }
 
 extern "C" CUNN_API size_t cunn_b200_convmm_acc_grad_workspace(int N, int C, int H, int W, int K, int kH, int kW, int dH,
@@ -1833,7 +1947,7 @@ extern "C" CUNN_API int cunn_b200_dilated_conv_grad_input(const float *gy, const
                                                           int H, int W, int K, int kH, int kW, int dH, int dW, int padH,
                                                           int padW, int dilH, int dilW, cunn_stream_t stream)
 {
-    return conv_grad_input(gy, weight, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, stream);
+    return conv_grad_input(gy, weight, nullptr, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, stream);
 }
 
 extern "C" CUNN_API size_t cunn_b200_dilated_conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH, int kW,
@@ -1889,14 +2003,7 @@ extern "C" CUNN_API int cunn_b200_full_conv_forward(const float *x, const float 
     clear_error();
     int OH, OW;
     if (full_check(N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW, &OH, &OW)) return 1;
-    if (conv_grad_input(x, weight, y, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW, stream_)) return 1;
-    if (bias && N > 0) {
-        const long long total = (long long)N * Q * OH * OW;
-        const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
-        add_plane_bias_kernel<<<blocks, 256, 0, (cudaStream_t)stream_>>>(y, bias, Q, OH * OW, total);
-        CUNN_LAUNCH_CHECK("full convolution bias");
-    }
-    return 0;
+    return conv_grad_input(x, weight, bias, y, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW, stream_);
 }
 
 extern "C" CUNN_API int cunn_b200_full_conv_grad_input(const float *gy, const float *weight, float *gx, int N, int P, int H,

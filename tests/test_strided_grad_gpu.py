@@ -1,0 +1,66 @@
+"""Input gradients of strided convolutions (and the forward pass of transposed ones) on the tensor-core kernel that takes them
+apart into one GEMM per stride residue: sizes at which the phases, tiles and k-blocks end unevenly."""
+import numpy as np
+import pytest
+
+from conftest import assert_parity, norm_err
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.fixture(scope="module")
+def F():
+    from cunn_b200 import functional
+    return functional
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW
+    (2, 128, 14, 14, 64, 3, 3, 2, 2, 1, 1, 1, 1),      # phases of 4, 2, 2 and 1 taps; one column tile of 128
+    (3, 40, 15, 13, 24, 3, 3, 2, 2, 1, 1, 1, 1),       # odd map: phases of different sizes, ragged reduction and columns
+    (1, 5, 9, 7, 3, 2, 2, 3, 3, 0, 0, 1, 1),           # kernel smaller than the stride: residues without taps
+    (2, 70, 8, 8, 33, 1, 1, 2, 2, 0, 0, 1, 1),         # 1x1 stride 2: three of four phases are filled
+    (2, 6, 30, 31, 10, 11, 11, 4, 4, 2, 2, 1, 1),      # sixteen phases of up to 3x3 taps
+    (1, 3, 40, 37, 4, 5, 7, 5, 6, 3, 2, 1, 1),         # thirty phases: two launches
+    (2, 8, 20, 20, 12, 3, 3, 2, 2, 2, 2, 2, 2),        # stride and dilation share a factor: only even residues have taps
+    (2, 8, 21, 19, 12, 3, 3, 2, 3, 3, 3, 3, 2),        # stride and dilation without a common factor
+    (2, 8, 6, 6, 12, 3, 3, 1, 1, 5, 5, 1, 1),          # stride 1, padding beyond the kernel
+    (1, 4, 1, 3, 6, 3, 3, 2, 2, 1, 1, 1, 1),           # fewer rows than the stride
+    (5, 130, 12, 12, 260, 3, 3, 2, 1, 1, 1, 1, 1),     # strides differ; two column tiles, 25 k-blocks
+])
+def test_strided_input_gradient(F, ref64, ref32, shape):
+    N, C, H, W, K, kH, kW, dH, dW, pH, pW, dilH, dilW = shape
+    rng = np.random.default_rng(abs(hash(shape)) % 99991)
+    oH, oW = (H + 2 * pH - dilH * (kH - 1) - 1) // dH + 1, (W + 2 * pW - dilW * (kW - 1) - 1) // dW + 1
+    gy, w = rng.standard_normal((N, K, oH, oW)).astype(np.float32), rng.uniform(-1, 1, (K, C, kH, kW)).astype(np.float32)
+    want = ref64.dilconv_grad_input(gy, w, H, W, dH, dW, pH, pW, dilH, dilW)
+    got = F.dilated_conv_grad_input(dev(gy), dev(w), H, W, dH, dW, pH, pW, dilH, dilW).cpu().numpy()
+    port = ref32.dilconv_grad_input(gy, w, H, W, dH, dW, pH, pW, dilH, dilW)
+    assert_parity("strided gx", got, want, 1e-4, port=port)
+    # a k-block's chain truncates four times at the size of its sum (2^-23 each), the k-blocks are added with rounding (2^-24 each, at
+    # most 56 of them), the split drops 2^-21 of a product: 4e-6 of the largest value holds all of it
+    assert norm_err(got, want) <= 4e-6
+    if dilH == dilW == 1:
+        b = rng.uniform(-1, 1, C).astype(np.float32)
+        adj = (H - ((oH - 1) * dH - 2 * pH + kH), W - ((oW - 1) * dW - 2 * pW + kW))
+        y = F.full_conv_forward(dev(gy), dev(w), dev(b), dH, dW, pH, pW, 1, 1, *adj).cpu().numpy()
+        bias = b[None, :, None, None]
+        assert_parity("transposed y", y, want + bias, 1e-4, port=port + bias)
+        assert norm_err(y, want + bias) <= 4e-6
+
+
+def test_strided_input_gradient_not_finite(F):
+    """Infinities and NaN reach exactly the pixels whose taps read them, with the sign that fp32 arithmetic gives."""
+    import torch
+    N, C, H, W, K = 1, 5, 11, 11, 7
+    gy, w = torch.ones(N, K, 6, 6, device="cuda"), torch.full((K, C, 3, 3), 0.5, device="cuda")
+    gy[0, 3, 2, 2] = float("inf")
+    gy[0, 1, 4, 5] = float("nan")
+    gx = F.convmm_grad_input(gy, w, H, W, 2, 2, 1, 1)
+    want = torch.nn.functional.conv_transpose2d(gy.cpu().double(), w.cpu().double(), None, 2, 1)
+    assert torch.equal(gx.cpu().double(), want) or torch.allclose(gx.cpu().double(), want, rtol=1e-6, equal_nan=True)
