@@ -1,8 +1,9 @@
 // Depthwise convolution for sm_100a: forward, input gradient, parameter gradient.
 //
-// Two families of kernels:
+// Three families of kernels:
 //  * shape-generic kernels (any kernel size, stride, padding, depth multiplier):
 //    one thread per output element / input element, plain coalesced loads;
+//  * staged-plane kernels (dwplane.cuh) for square 3x3, 5x5 and 7x7 kernels of stride 1 or 2;
 //  * the 3x3 / pad 1 / stride 1|2 / multiplier 1 fast path that MobileNet-style
 //    networks use: each CTA owns a group of channels and a range of images, and
 //    streams whole planes (or row bands of one plane) through a ring of shared
@@ -27,6 +28,47 @@ namespace dw {
 // Shape-generic kernels
 // ---------------------------------------------------------------------------
 
+// One output: xp and wp are the channel's input plane and the filter, (ih0, iw0) the window's first pixel.
+__device__ __forceinline__ float fwd_point(const float *__restrict__ xp, const float *__restrict__ wp, float s, int H, int W, int kH, int kW, int ih0,
+                                           int iw0)
+{
+    for (int kh = 0; kh < kH; ++kh) {
+        const int ih = ih0 + kh;
+        if (ih < 0 || ih >= H) continue;
+        for (int kw = 0; kw < kW; ++kw) {
+            const int iw = iw0 + kw;
+            if (iw < 0 || iw >= W) continue;
+            s = fmaf(__ldg(wp + kh * kW + kw), __ldg(xp + ih * W + iw), s);
+        }
+    }
+    return s;
+}
+
+// One input-gradient pixel (h, wi) of channel c of image n.
+__device__ __forceinline__ float dgrad_point(const float *__restrict__ gy, const float *__restrict__ w, long long n, int c, int h, int wi, int C,
+                                             int M, int kH, int kW, int dH, int dW, int padH, int padW, int oH, int oW)
+{
+    float s = 0.f;
+    for (int j = 0; j < M; ++j) {
+        const float *wp = w + ((long long)j * C + c) * kH * kW;
+        const float *gp = gy + ((n * C + c) * M + j) * (long long)oH * oW;
+        for (int kh = 0; kh < kH; ++kh) {
+            const int a = h + padH - kh;
+            if (a < 0 || a % dH) continue;
+            const int oh = a / dH;
+            if (oh >= oH) continue;
+            for (int kw = 0; kw < kW; ++kw) {
+                const int b = wi + padW - kw;
+                if (b < 0 || b % dW) continue;
+                const int ow = b / dW;
+                if (ow >= oW) continue;
+                s = fmaf(__ldg(wp + kh * kW + kw), __ldg(gp + oh * oW + ow), s);
+            }
+        }
+    }
+    return s;
+}
+
 __global__ void __launch_bounds__(256)
 fwd_generic_kernel(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias,
                    float *__restrict__ y, int C, int H, int W, int M, int kH, int kW, int dH, int dW,
@@ -42,20 +84,8 @@ fwd_generic_kernel(const float *__restrict__ x, const float *__restrict__ w, con
         t /= M;
         const int c = (int)(t % C);
         const long long n = t / C;
-        const float *xp = x + (n * C + c) * (long long)H * W;
-        const float *wp = w + ((long long)j * C + c) * kH * kW;
-        float s = bias ? __ldg(bias + (long long)j * C + c) : 0.f;
-        const int ih0 = oh * dH - padH, iw0 = ow * dW - padW;
-        for (int kh = 0; kh < kH; ++kh) {
-            const int ih = ih0 + kh;
-            if (ih < 0 || ih >= H) continue;
-            for (int kw = 0; kw < kW; ++kw) {
-                const int iw = iw0 + kw;
-                if (iw < 0 || iw >= W) continue;
-                s = fmaf(__ldg(wp + kh * kW + kw), __ldg(xp + ih * W + iw), s);
-            }
-        }
-        y[idx] = s;
+        y[idx] = fwd_point(x + (n * C + c) * (long long)H * W, w + ((long long)j * C + c) * kH * kW, bias ? __ldg(bias + (long long)j * C + c) : 0.f,
+                           H, W, kH, kW, oh * dH - padH, ow * dW - padW);
     }
 }
 
@@ -72,25 +102,7 @@ dgrad_generic_kernel(const float *__restrict__ gy, const float *__restrict__ w, 
         t /= H;
         const int c = (int)(t % C);
         const long long n = t / C;
-        float s = 0.f;
-        for (int j = 0; j < M; ++j) {
-            const float *wp = w + ((long long)j * C + c) * kH * kW;
-            const float *gp = gy + ((n * C + c) * M + j) * (long long)oH * oW;
-            for (int kh = 0; kh < kH; ++kh) {
-                const int a = h + padH - kh;
-                if (a < 0 || a % dH) continue;
-                const int oh = a / dH;
-                if (oh >= oH) continue;
-                for (int kw = 0; kw < kW; ++kw) {
-                    const int b = wi + padW - kw;
-                    if (b < 0 || b % dW) continue;
-                    const int ow = b / dW;
-                    if (ow >= oW) continue;
-                    s = fmaf(__ldg(wp + kh * kW + kw), __ldg(gp + oh * oW + ow), s);
-                }
-            }
-        }
-        gx[idx] = s;
+        gx[idx] = dgrad_point(gy, w, n, c, h, wi, C, M, kH, kW, dH, dW, padH, padW, oH, oW);
     }
 }
 
@@ -135,6 +147,8 @@ wgrad_generic_kernel(const float *__restrict__ x, const float *__restrict__ gy, 
         else           gw[((long long)j * C + c) * kk + tap] = (float)((double)gw[((long long)j * C + c) * kk + tap] + (double)scale * s);
     }
 }
+
+#include "dwplane.cuh"
 
 // ---------------------------------------------------------------------------
 // 3x3 fast path
@@ -1274,6 +1288,11 @@ extern "C" int cunn_b200_dwconv_forward(const float *x, const float *weight, con
             return launch_fast(fp, pl, stream, "dwconv forward (3x3)");
         }
     }
+    plane::Params pp;
+    if (plane::plan(pp, plane::FWD, N, C, H, W, M, kH, kW, dH, dW, padH, padW, oH, oW)) {
+        pp.in = x; pp.w = weight; pp.bias = bias; pp.out = y;
+        return plane::launch(pp, plane::FWD, kH, dH, stream);
+    }
     const long long total = (long long)N * C * M * oH * oW;
     fwd_generic_kernel<<<grid_for(total), 256, 0, stream>>>(x, weight, bias, y, C, H, W, M, kH, kW, dH, dW, padH, padW,
                                                            oH, oW, total);
@@ -1310,6 +1329,11 @@ extern "C" int cunn_b200_dwconv_grad_input(const float *gy, const float *weight,
                 return launch_fast(fp, pl, stream, "dwconv grad input (3x3 s2)");
             }
         }
+    }
+    plane::Params pp;
+    if (plane::plan(pp, plane::DGRAD, N, C, H, W, M, kH, kW, dH, dW, padH, padW, oH, oW)) {
+        pp.in = gy; pp.w = weight; pp.out = gx;
+        return plane::launch(pp, plane::DGRAD, kH, dH, stream);
     }
     const long long total = (long long)N * C * H * W;
     dgrad_generic_kernel<<<grid_for(total), 256, 0, stream>>>(gy, weight, gx, C, H, W, M, kH, kW, dH, dW, padH, padW, oH,
@@ -1364,6 +1388,11 @@ extern "C" int cunn_b200_dwconv_acc_grad(const float *x, const float *gy, float 
             fp.partials = (float *)((char *)workspace + wgrad_counter_bytes(C, pl));
             return launch_fast(fp, pl, stream, "dwconv acc grad (3x3)");
         }
+    }
+    plane::Params pp;
+    if (plane::plan(pp, plane::WGRAD, N, C, H, W, M, kH, kW, dH, dW, padH, padW, oH, oW)) {
+        pp.in = x; pp.gy = gy; pp.gw = grad_weight; pp.gb = grad_bias; pp.scale = scale;
+        return plane::launch(pp, plane::WGRAD, kH, dH, stream);
     }
     const int blocks = M * C * (kH * kW + 1);
     wgrad_generic_kernel<<<blocks, 256, 0, stream>>>(x, gy, grad_weight, grad_bias, N, C, H, W, M, kH, kW, dH, dW, padH,

@@ -1,0 +1,440 @@
+// Depthwise convolution by staged planes: square 3x3, 5x5 and 7x7 kernels with stride 1 or 2, any padding, depth multiplier,
+// map size and alignment — what the bulk-copy path (3x3, pad 1, multiplier 1, rows of 16-byte multiples) does not take.
+//
+// The passes move 4 bytes per element of x and y and do k * k multiply-adds per output.  The kernels for any shape read every tap
+// through the cache with a bounds check (25 loads and 50 comparisons per output of a 5x5), and their parameter gradient reads
+// both tensors once per tap.  Here a CTA copies the rows it needs once, asynchronously and with the padding as zeros, into
+// shared memory, and a thread takes strips of TH = 4 outputs of one column: every staged value of the strip's columns is
+// read once (40 reads for 100 multiply-adds of a 5x5 at stride 1, 55 at stride 2), taps and weights are unrolled registers and no
+// bounds are checked.  At stride 2 even and odd columns are staged apart, so that a warp reads consecutive words.
+//   forward      a tile is P consecutive planes of one image, or a band of rows of one plane
+//   input grad   in padded coordinates h + pad = S q + a: gx[S q + a][S r + b] = sum_{t,u} w[a + S t][b + S u] gy[q - t][r - u];
+//                a thread takes TH consecutive q of one r and writes their S * S residues, so no product with a zero is formed
+//   param grad   a cluster of up to eight CTAs per filter shares the images; every thread keeps the k * k + 1 sums of its strips in
+//                registers for at most kChain terms, then they go through fp64: across the warp, the CTA, the cluster and onto the
+//                gradient.  The order is fixed, so results do not depend on timing.
+//
+// Forward / input gradient / parameter gradient on a cold cache, in us: 32 x 96 x 57 x 43, 5x5 stride 2: 671 in all before,
+// 36 / 33 / 57 now (38 MB a pass: 6 us); 12 x 144 x 37 x 29, 3x3 stride 1 (rows of an odd length): 15 / 17 / 34.  What is left is
+// the 4-byte copies and the wait of a CTA for its only tile, which other CTAs of the SM fill.
+#pragma once
+
+namespace plane {
+
+constexpr int TH = 4;                        // outputs (forward, parameter gradient) or q rows (input gradient) per strip
+constexpr int THREADS = 256;
+constexpr int kTileFloats = 6144;            // staged floats per tile to aim at: 24 KB, so that several CTAs share an SM
+constexpr int kMaxFloats = 11264;            // ... and the most a tile may take (44 KB)
+constexpr int kChain = 32;                   // fp32 terms per sum before it goes through fp64
+
+struct Params {
+    const float *in, *gy, *w, *bias;         // forward, parameter gradient: in = x; input gradient: in = gy
+    float *out, *gw, *gb;
+    int N, C, M, H, W, oH, oW, padH, padW;
+    int P, groups;                           // planes of a tile (parameter gradient: images), tiles that cover C (N)
+    int R, bands;                            // strip rows of a band (a multiple of TH), bands
+    int rows, cols, half, ld;                // staged rows and columns per plane; stride 2: columns of one parity; floats per row
+    int base_q, base_r, cols_out;            // input gradient: first q and r; columns of strips
+    int strips;                              // strips per band
+    uint32_t cols_magic, strips_magic;
+    float scale;
+};
+
+__device__ __forceinline__ int mdiv(int k, uint32_t magic) { return magic ? (int)__umulhi((uint32_t)k, magic) : k; }
+__device__ __forceinline__ void copy4(uint32_t dst, const float *src, bool on)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(on ? 4u : 0u) : "memory");
+}
+__device__ __forceinline__ void copies_land()
+{
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+}
+
+// Thread-block clusters: this CTA's rank, their number, a barrier of all their threads, a double in another CTA's shared memory.
+__device__ __forceinline__ int cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
+__device__ __forceinline__ int cluster_size()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return (int)r;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ double cluster_ld(const double *local, int rank)
+{
+    uint32_t a;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// Stages `count` planes (plane i at src + i * step, h x w) from row row0 and column col0 on, zeros outside.
+template <int S>
+__device__ __forceinline__ void stage_planes(const Params &p, float *tile, const float *src, long long step, int count, int h, int w, int row0,
+                                             int col0)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t base = smem_u32(tile);
+    int pl = 0, i = warp;
+    while (i >= p.rows) { i -= p.rows; ++pl; }
+    while (pl < count) {
+        const int row = row0 + i;
+        const bool row_ok = (unsigned)row < (unsigned)h;
+        const float *s = src + pl * step + (long long)row * w;
+        const uint32_t d = base + (uint32_t)((pl * p.rows + i) * p.ld) * 4u;
+        for (int j = lane; j < p.cols; j += 32) {
+            const int col = col0 + j;
+            const bool ok = row_ok && (unsigned)col < (unsigned)w;
+            const int at = S == 1 ? j : (j & 1) * p.half + (j >> 1);
+            copy4(d + (uint32_t)at * 4u, ok ? s + col : src, ok);
+        }
+        i += THREADS / 32;
+        while (i >= p.rows) { i -= p.rows; ++pl; }
+    }
+}
+
+// Weights of `count` channels from c0 on, all M filters of each: slot (p * M + j) * WS; bad[slot]: a weight that is not finite,
+// whose product with a padding zero must not be formed.
+template <int K>
+struct Weights {
+    static constexpr int KK = K * K, WS = (KK + 3) & ~3;
+    __device__ __forceinline__ static void stage(const Params &p, float *wsm, int *bad, int c0, int count)
+    {
+        for (int s = threadIdx.x; s < count * p.M; s += THREADS) bad[s] = 0;
+        __syncthreads();
+        for (int e = threadIdx.x; e < count * p.M * KK; e += THREADS) {
+            const int s = e / KK, i = e - s * KK, pl = s / p.M, j = s - pl * p.M;
+            const float v = __ldg(p.w + ((size_t)j * p.C + c0 + pl) * KK + i);
+            wsm[s * WS + i] = v;
+            if (!(fabsf(v) <= 3.402823466e38f)) bad[s] = 1;
+        }
+    }
+    __device__ __forceinline__ static void load(const float *wsm, int slot, float (&w)[WS])
+    {
+        const float4 *q = reinterpret_cast<const float4 *>(wsm + slot * WS);
+#pragma unroll
+        for (int i = 0; i < WS / 4; ++i) {
+            const float4 v = q[i];
+            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+        }
+    }
+};
+
+template <int K, int S>
+__global__ void __launch_bounds__(THREADS, 3)
+fwd_kernel(const __grid_constant__ Params p)
+{
+    using WT = Weights<K>;
+    extern __shared__ __align__(16) float sm[];
+    float *wsm = sm;                                           // [P * M][WS], then flags, then the tile
+    int *bad = reinterpret_cast<int *>(wsm + p.P * p.M * WT::WS);
+    float *tile = reinterpret_cast<float *>(bad + ((p.P * p.M + 3) & ~3));
+    const int unit = (int)blockIdx.x, band = unit % p.bands, ng = unit / p.bands, g = ng % p.groups, n = ng / p.groups;
+    const int c0 = g * p.P, planes = min(p.P, p.C - c0), r0 = band * p.R;
+    stage_planes<S>(p, tile, p.in + ((long long)n * p.C + c0) * p.H * p.W, (long long)p.H * p.W, planes, p.H, p.W, r0 * S - p.padH, -p.padW);
+    WT::stage(p, wsm, bad, c0, planes);
+    copies_land();
+    const int items = planes * p.M * p.strips * p.oW;
+    for (int it = threadIdx.x; it < items; it += THREADS) {
+        const int t2 = mdiv(it, p.cols_magic), ow = it - t2 * p.oW;
+        const int slot = mdiv(t2, p.strips_magic), t0 = (t2 - slot * p.strips) * TH;
+        const int pl = slot / p.M, j = slot - pl * p.M, c = c0 + pl;
+        const int oh0 = r0 + t0, cnt = min(TH, p.oH - oh0);
+        if (cnt <= 0) continue;
+        const float b = p.bias ? __ldg(p.bias + (size_t)j * p.C + c) : 0.f;
+        float *dst = p.out + (((long long)n * p.C + c) * p.M + j) * p.oH * p.oW + (long long)oh0 * p.oW + ow;
+        if (bad[slot]) {
+            for (int t = 0; t < cnt; ++t)
+                dst[(long long)t * p.oW] = fwd_point(p.in + ((long long)n * p.C + c) * p.H * p.W, p.w + ((size_t)j * p.C + c) * WT::KK, b, p.H, p.W, K, K,
+                                                     (oh0 + t) * S - p.padH, ow * S - p.padW);
+            continue;
+        }
+        float w[WT::WS];
+        WT::load(wsm, slot, w);
+        float acc[TH];
+#pragma unroll
+        for (int t = 0; t < TH; ++t) acc[t] = b;
+        const float *row0 = tile + (pl * p.rows + t0 * S) * p.ld + ow;
+#pragma unroll
+        for (int kw = 0; kw < K; ++kw) {
+            const float *col = row0 + (S == 1 ? kw : (kw & 1) * p.half + (kw >> 1));
+#pragma unroll
+            for (int r = 0; r < (TH - 1) * S + K; ++r) {
+                const float v = col[r * p.ld];
+#pragma unroll
+                for (int t = 0; t < TH; ++t)
+                    if (r - t * S >= 0 && r - t * S < K) acc[t] = fmaf(w[(r - t * S) * K + kw], v, acc[t]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < TH; ++t)
+            if (t < cnt) dst[(long long)t * p.oW] = acc[t];
+    }
+}
+
+template <int K, int S>
+__global__ void __launch_bounds__(THREADS, 3)
+dgrad_kernel(const __grid_constant__ Params p)
+{
+    using WT = Weights<K>;
+    constexpr int T = (K + S - 1) / S;                          // taps of a residue, at most
+    extern __shared__ __align__(16) float sm[];
+    float *wsm = sm;
+    int *bad = reinterpret_cast<int *>(wsm + p.P * p.M * WT::WS);
+    float *tile = reinterpret_cast<float *>(bad + ((p.P * p.M + 3) & ~3));
+    const int unit = (int)blockIdx.x, band = unit % p.bands, ng = unit / p.bands, g = ng % p.groups, n = ng / p.groups;
+    const int c0 = g * p.P, planes = min(p.P, p.C - c0), q0 = p.base_q + band * p.R;
+    stage_planes<1>(p, tile, p.in + ((long long)n * p.C + c0) * p.M * p.oH * p.oW, (long long)p.oH * p.oW, planes * p.M, p.oH, p.oW, q0 - (T - 1),
+                    p.base_r - (T - 1));
+    WT::stage(p, wsm, bad, c0, planes);
+    copies_land();
+    const int items = planes * p.strips * p.cols_out;
+    for (int it = threadIdx.x; it < items; it += THREADS) {
+        const int t2 = mdiv(it, p.cols_magic), ri = it - t2 * p.cols_out;
+        const int pl = mdiv(t2, p.strips_magic), t0 = (t2 - pl * p.strips) * TH;
+        float acc[TH][S][S];
+#pragma unroll
+        for (int t = 0; t < TH; ++t)
+#pragma unroll
+            for (int a = 0; a < S; ++a)
+#pragma unroll
+                for (int b = 0; b < S; ++b) acc[t][a][b] = 0.f;
+        bool any_bad = false;
+        for (int j = 0; j < p.M; ++j) {
+            const int slot = pl * p.M + j;
+            any_bad |= bad[slot] != 0;
+            float w[WT::WS];
+            WT::load(wsm, slot, w);
+            const float *row0 = tile + (slot * p.rows + t0) * p.ld + ri;
+#pragma unroll
+            for (int u = 0; u < T; ++u) {
+#pragma unroll
+                for (int rr = 0; rr < TH + T - 1; ++rr) {
+                    const float v = row0[rr * p.ld + (T - 1 - u)];
+#pragma unroll
+                    for (int t = 0; t < TH; ++t) {
+                        const int tt = t + T - 1 - rr;
+                        if (tt < 0 || tt >= T) continue;
+#pragma unroll
+                        for (int a = 0; a < S; ++a)
+#pragma unroll
+                            for (int b = 0; b < S; ++b)
+                                if (a + S * tt < K && b + S * u < K) acc[t][a][b] = fmaf(w[(a + S * tt) * K + b + S * u], v, acc[t][a][b]);
+                    }
+                }
+            }
+        }
+        const int h0 = (q0 + t0) * S - p.padH, w0 = (p.base_r + ri) * S - p.padW;
+        float *dst = p.out + ((long long)n * p.C + c0 + pl) * p.H * p.W;
+#pragma unroll
+        for (int t = 0; t < TH; ++t)
+#pragma unroll
+            for (int a = 0; a < S; ++a) {
+                const int h = h0 + t * S + a;
+                if ((unsigned)h >= (unsigned)p.H) continue;
+#pragma unroll
+                for (int b = 0; b < S; ++b) {
+                    const int wi = w0 + b;
+                    if ((unsigned)wi >= (unsigned)p.W) continue;
+                    dst[(long long)h * p.W + wi] =
+                        any_bad ? dgrad_point(p.in, p.w, n, c0 + pl, h, wi, p.C, p.M, K, K, S, S, p.padH, p.padW, p.oH, p.oW) : acc[t][a][b];
+                }
+            }
+    }
+}
+
+template <int K, int S>
+__global__ void __launch_bounds__(THREADS, K == 7 ? 2 : 3)
+wgrad_kernel(const __grid_constant__ Params p)
+{
+    constexpr int KK = K * K, SUMS = KK + 1;
+    extern __shared__ __align__(16) float tile[];
+    __shared__ double warp_sums[THREADS / 32][SUMS];
+    __shared__ double cta_sums[SUMS];
+    const int rank = cluster_rank(), ranks = cluster_size();
+    const int jc = (int)blockIdx.x / ranks, j = jc / p.C, c = jc - j * p.C;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < (THREADS / 32) * SUMS; i += THREADS) (&warp_sums[0][0])[i] = 0.0;
+    __syncthreads();
+    float acc[SUMS];
+#pragma unroll
+    for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
+    auto flush = [&]() {
+#pragma unroll
+        for (int i = 0; i < SUMS; ++i) {
+            const double s = warp_sum((double)acc[i]);
+            if (lane == 0) warp_sums[warp][i] += s;
+            acc[i] = 0.f;
+        }
+    };
+    int chain = 0;
+    const long long units = (long long)p.groups * p.bands;                  // (image group, band)
+    const int u_end = (int)(units * (rank + 1) / ranks);
+    for (int u = (int)(units * rank / ranks); u < u_end; ++u) {
+        const int band = u % p.bands, n0 = (u / p.bands) * p.P, imgs = min(p.P, p.N - n0), r0 = band * p.R;
+        stage_planes<S>(p, tile, p.in + ((long long)n0 * p.C + c) * p.H * p.W, (long long)p.C * p.H * p.W, imgs, p.H, p.W, r0 * S - p.padH, -p.padW);
+        copies_land();
+        const int items = imgs * p.strips * p.oW;
+        for (int it0 = 0; it0 < items; it0 += THREADS) {
+            if (chain + TH > kChain) { flush(); chain = 0; }
+            chain += TH;
+            const int it = it0 + (int)threadIdx.x;
+            if (it >= items) continue;
+            const int t2 = mdiv(it, p.cols_magic), ow = it - t2 * p.oW;
+            const int pl = mdiv(t2, p.strips_magic), t0 = (t2 - pl * p.strips) * TH, oh0 = r0 + t0;
+            const float *gp = p.gy + (((long long)(n0 + pl) * p.C + c) * p.M + j) * p.oH * p.oW + (long long)oh0 * p.oW + ow;
+            float gv[TH];
+#pragma unroll
+            for (int t = 0; t < TH; ++t) gv[t] = oh0 + t < p.oH ? __ldg(gp + (long long)t * p.oW) : 0.f;
+#pragma unroll
+            for (int t = 0; t < TH; ++t) acc[KK] += gv[t];
+            const float *row0 = tile + (pl * p.rows + t0 * S) * p.ld + ow;
+#pragma unroll
+            for (int kw = 0; kw < K; ++kw) {
+                const float *col = row0 + (S == 1 ? kw : (kw & 1) * p.half + (kw >> 1));
+#pragma unroll
+                for (int r = 0; r < (TH - 1) * S + K; ++r) {
+                    const float v = col[r * p.ld];
+#pragma unroll
+                    for (int t = 0; t < TH; ++t)
+                        if (r - t * S >= 0 && r - t * S < K) acc[(r - t * S) * K + kw] = fmaf(gv[t], v, acc[(r - t * S) * K + kw]);
+                }
+            }
+        }
+        __syncthreads();                                                    // the tile is read before the next one lands
+    }
+    flush();
+    __syncthreads();
+    for (int i = threadIdx.x; i < SUMS; i += THREADS) {
+        double s = 0.0;
+        for (int w = 0; w < THREADS / 32; ++w) s += warp_sums[w][i];
+        cta_sums[i] = s;
+    }
+    cluster_sync();
+    if (rank == 0) {
+        for (int i = threadIdx.x; i < SUMS; i += THREADS) {
+            double s = 0.0;
+            for (int r = 0; r < ranks; ++r) s += cluster_ld(&cta_sums[i], r);
+            float *dst = i < KK ? p.gw + (size_t)jc * KK + i : (p.gb ? p.gb + jc : nullptr);
+            if (dst) *dst = (float)((double)*dst + (double)p.scale * s);
+        }
+    }
+    cluster_sync();                                                         // shared memory outlives rank 0's reads
+}
+
+static uint32_t magic_of(int d) { return d == 1 ? 0u : (uint32_t)((1ull << 32) / (unsigned)d + 1u); }
+
+enum Pass { FWD, DGRAD, WGRAD };
+
+// Fills the tile plan of a pass; false when the shape is left to the kernels for any shape: other kernel sizes and strides, or
+// rows so long that a strip's do not fit a tile.
+static bool plan(Params &p, Pass pass, int N, int C, int H, int W, int M, int kH, int kW, int dH, int dW, int padH, int padW, int oH, int oW)
+{
+    if (kH != kW || dH != dW || (kH != 3 && kH != 5 && kH != 7) || (dH != 1 && dH != 2)) return false;
+    const int K = kH, S = dH, T = (K + S - 1) / S;
+    p = Params{};
+    p.N = N; p.C = C; p.M = M; p.H = H; p.W = W; p.oH = oH; p.oW = oW; p.padH = padH; p.padW = padW;
+    int rows_out, halo, step;                                   // strip rows of a plane; staged rows = (R - 1) * step + halo
+    if (pass == DGRAD) {
+        p.base_q = padH / S; p.base_r = padW / S;
+        rows_out = (padH + H - 1) / S - p.base_q + 1;
+        p.cols_out = (padW + W - 1) / S - p.base_r + 1;
+        p.cols = p.cols_out + T - 1;
+        p.ld = p.cols;
+        halo = T; step = 1;
+    } else {
+        rows_out = oH;
+        p.cols_out = oW;
+        p.cols = (oW - 1) * S + K;
+        p.half = (p.cols + 1) / 2;
+        p.ld = S == 1 ? p.cols : 2 * p.half;
+        halo = K; step = S;
+    }
+    const int per_plane = pass == DGRAD ? M : 1;                // staged planes per plane of the tile
+    const int wfloats = pass == WGRAD ? 0 : M * (((K * K + 3) & ~3) + 1) + 4;
+    auto floats = [&](long long planes, long long R) { return planes * (per_plane * ((R - 1) * step + halo) * p.ld + wfloats); };
+    const int whole = (rows_out + TH - 1) / TH * TH;
+    if (floats(1, whole) <= kTileFloats) {
+        p.R = whole; p.bands = 1;
+        // enough strips for every thread, as long as the planes fit
+        const int strips = whole / TH, want = (THREADS + strips * p.cols_out * (pass == FWD ? M : 1) - 1) / (strips * p.cols_out * (pass == FWD ? M : 1));
+        const int most = pass == WGRAD ? N : C;
+        p.P = 1;
+        while (p.P < want && p.P < most && floats(p.P + 1, whole) <= kTileFloats) ++p.P;
+    } else {
+        int R = whole;
+        while (R > TH && floats(1, R) > kTileFloats) R -= TH;
+        if (floats(1, R) > kMaxFloats) return false;
+        p.bands = (rows_out + R - 1) / R;
+        p.R = ((rows_out + p.bands - 1) / p.bands + TH - 1) / TH * TH;      // even bands
+        p.bands = (rows_out + p.R - 1) / p.R;
+        p.P = 1;
+    }
+    p.rows = (p.R - 1) * step + halo;
+    p.strips = p.R / TH;
+    p.groups = ((pass == WGRAD ? N : C) + p.P - 1) / p.P;
+    p.cols_magic = magic_of(p.cols_out);
+    p.strips_magic = magic_of(p.strips);
+    const long long items = (long long)p.P * (pass == FWD ? M : 1) * p.strips * p.cols_out;
+    // exact divisions: items * divisor < 2^32 (see magic_of); grids within the launch limits
+    if (items * std::max(p.cols_out, p.strips) >= (1LL << 32) || p.cols_out >= (1 << 16)) return false;
+    if (pass != WGRAD && (long long)N * p.groups * p.bands >= (1LL << 31)) return false;
+    if (pass == WGRAD && (long long)C * M * 8 >= (1LL << 31)) return false;
+    return true;
+}
+static size_t smem_bytes(const Params &p, Pass pass, int K)
+{
+    const size_t t = (size_t)p.P * (pass == DGRAD ? p.M : 1) * p.rows * p.ld;
+    if (pass == WGRAD) return t * 4;
+    const size_t slots = (size_t)p.P * p.M;
+    return (slots * ((K * K + 3) & ~3) + ((slots + 3) & ~(size_t)3) + t) * 4;
+}
+
+typedef void (*Kernel)(const Params);
+template <int K, int S>
+static Kernel pick_pass(Pass pass)
+{
+    return pass == FWD ? fwd_kernel<K, S> : pass == DGRAD ? dgrad_kernel<K, S> : wgrad_kernel<K, S>;
+}
+static Kernel pick(Pass pass, int K, int S)
+{
+    if (K == 3) return S == 1 ? pick_pass<3, 1>(pass) : pick_pass<3, 2>(pass);
+    if (K == 5) return S == 1 ? pick_pass<5, 1>(pass) : pick_pass<5, 2>(pass);
+    return S == 1 ? pick_pass<7, 1>(pass) : pick_pass<7, 2>(pass);
+}
+static int launch(const Params &p, Pass pass, int K, int S, cudaStream_t stream)
+{
+    void *args[] = {(void *)&p};
+    const Kernel kern = pick(pass, K, S);
+    if (pass != WGRAD) {
+        CUNN_CUDA(cudaLaunchKernel((const void *)kern, dim3((unsigned)((long long)p.N * p.groups * p.bands)), dim3(THREADS), args, smem_bytes(p, pass, K), stream));
+        return 0;
+    }
+    int ranks = 1;
+    while (ranks < 8 && (long long)ranks * 2 <= (long long)p.groups * p.bands) ranks *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.C * p.M * ranks));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem_bytes(p, pass, K);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ranks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CUNN_CUDA(cudaLaunchKernelExC(&cfg, (const void *)kern, args));
+    return 0;
+}
+
+}  // namespace plane

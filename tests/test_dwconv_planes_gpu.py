@@ -1,0 +1,83 @@
+"""Depthwise layers on the staged-plane kernels: kernel sizes, strides, paddings, multipliers and maps that the bulk-copy 3x3 path
+does not take, at the edges of strips, bands, channel groups and clusters."""
+import numpy as np
+import pytest
+
+from conftest import assert_parity
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+@pytest.fixture(scope="module")
+def F():
+    from cunn_b200 import functional
+    return functional
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W, M, k, d, padH, padW
+    (3, 10, 57, 43, 1, 5, 2, 2, 2),      # one plane per tile, ragged strips
+    (2, 3, 200, 33, 1, 5, 1, 2, 2),      # several bands
+    (2, 2, 150, 131, 1, 7, 2, 3, 3),     # bands at stride 2, odd rows
+    (17, 6, 7, 7, 1, 7, 1, 3, 3),        # many planes per tile; more images than ranks
+    (5, 7, 14, 14, 2, 5, 1, 2, 2),       # multiplier 2
+    (2, 5, 29, 37, 3, 3, 2, 1, 1),       # multiplier 3 at stride 2
+    (2, 8, 37, 29, 1, 3, 1, 1, 1),       # 3x3 with planes of an odd size
+    (2, 4, 16, 18, 1, 3, 1, 0, 2),       # paddings that differ
+    (2, 4, 11, 9, 1, 5, 2, 4, 0),        # padding of k - 1 and none
+    (2, 3, 12, 12, 1, 3, 2, 3, 3),       # padding of the kernel size: outer outputs see padding only
+    (1, 1, 5, 1200, 1, 7, 1, 3, 3),      # long rows: strips of one band row group
+    (1, 2, 3, 4000, 1, 7, 1, 3, 3),      # rows too long for a tile: the kernels for any shape
+    (1, 3, 1, 1, 1, 5, 2, 2, 2),         # a single pixel
+    (40, 2, 20, 20, 1, 3, 1, 0, 0),      # more terms per thread than one fp32 chain takes
+])
+def test_staged_plane_shapes(F, ref64, ref32, shape):
+    N, C, H, W, M, k, d, pH, pW = shape
+    rng = np.random.default_rng(abs(hash(shape)) % 99991)
+    oH, oW = (H + 2 * pH - k) // d + 1, (W + 2 * pW - k) // d + 1
+    x, gy = rng.standard_normal((N, C, H, W)).astype(np.float32), rng.standard_normal((N, C * M, oH, oW)).astype(np.float32)
+    w, b = rng.uniform(-1, 1, (M, C, k, k)).astype(np.float32), rng.uniform(-1, 1, (M, C)).astype(np.float32)
+    gw0, gb0 = rng.standard_normal((M, C, k, k)).astype(np.float32), rng.standard_normal((M, C)).astype(np.float32)
+    y = F.dwconv_forward(dev(x), dev(w), dev(b), d, d, pH, pW).cpu().numpy()
+    assert_parity("y", y, ref64.dwconv_forward(x, w, b, d, d, pH, pW), 1e-5, port=lambda: ref32.dwconv_forward(x, w, b, d, d, pH, pW))
+    gx = F.dwconv_grad_input(dev(gy), dev(w), H, W, d, d, pH, pW).cpu().numpy()
+    assert_parity("gx", gx, ref64.dwconv_grad_input(gy, w, H, W, d, d, pH, pW), 1e-5, port=lambda: ref32.dwconv_grad_input(gy, w, H, W, d, d, pH, pW))
+    gw, gb = dev(gw0), dev(gb0)
+    F.dwconv_acc_grad(dev(x), dev(gy), gw, gb, d, d, pH, pW, 0.75)
+    want = ref64.dwconv_acc_grad(x, gy, gw0.copy(), gb0.copy(), d, d, pH, pW, 0.75)
+    port = ref32.dwconv_acc_grad(x, gy, gw0.copy(), gb0.copy(), d, d, pH, pW, 0.75)
+    assert_parity("gw", gw.cpu().numpy(), want[0], 1e-5, port=port[0])
+    assert_parity("gb", gb.cpu().numpy(), want[1], 1e-5, port=port[1])
+    # the order of the sums is fixed: the same bits again, without a bias gradient too
+    gw2 = dev(gw0)
+    F.dwconv_acc_grad(dev(x), dev(gy), gw2, None, d, d, pH, pW, 0.75)
+    assert np.array_equal(gw.cpu().numpy(), gw2.cpu().numpy())
+
+
+@pytest.mark.parametrize("d", [1, 2])
+def test_weights_that_are_not_finite_stay_off_the_padding(F, d):
+    import torch
+    x, w = torch.ones(1, 3, 9, 9, device="cuda"), torch.full((1, 3, 5, 5), 0.25, device="cuda")
+    w[0, 1, 0, 2] = float("inf")
+    w[0, 2, 4, 4] = float("nan")
+    y = F.dwconv_forward(x, w, None, d, d, 2, 2)
+    xd, wd = x.cpu().double(), w.cpu().double().view(3, 1, 5, 5)
+    cols = torch.nn.functional.unfold(torch.ones(1, 3, 9, 9).double(), 5, padding=2, stride=d).view(3, 25, -1)     # 0: padding
+    want = torch.where(cols > 0, wd.view(3, 25, 1), torch.zeros(1, dtype=torch.double)).sum(1).view(y.shape)
+    assert torch.allclose(y.cpu().double(), want, equal_nan=True)
+    gx = F.dwconv_grad_input(torch.ones_like(y), w, 9, 9, d, d, 2, 2).cpu()
+    o = y.shape[2]
+    ref = torch.zeros(3, 9, 9, dtype=torch.double)
+    for oh in range(o):
+        for ow in range(o):
+            for kh in range(5):
+                for kw in range(5):
+                    h, q = oh * d - 2 + kh, ow * d - 2 + kw
+                    if 0 <= h < 9 and 0 <= q < 9:
+                        ref[:, h, q] += wd[:, 0, kh, kw]
+    assert torch.allclose(gx[0].double(), ref, equal_nan=True)
