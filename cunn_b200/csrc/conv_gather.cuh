@@ -14,8 +14,9 @@
 // with every k-block that a chain holds (1.1e-6 at 1024 and 2.1e-6 at 2304 products in chains of 11 and 24 k-blocks; a chain of
 // fp32 FMAs, which these passes used before, is 5e-7 off).  Here a chain is ONE k-block: its eight cross-term MMAs come first, while the
 // accumulator is 2^-11 of its final size, then the four hi*hi ones; the 16 producer warps read the finished block back
-// (32 columns each, two TMEM buffers in turn) and add it to fp32 registers with rounding.  The producers' waits already order everything: k-block i is drained before its producer
-// hands over k-block i + 2, which is the next one to use its TMEM buffer, so no further barrier exists.
+// (32 columns each, two TMEM buffers in turn) and add it to fp32 registers with rounding.  The producers' waits already order
+// everything: k-block i is drained before its producer hands over k-block i + 2, which is the next one to use its TMEM buffer, so
+// no further barrier exists.
 //
 // Bound by the producers: 4-byte copies of the gathered operands (128 + up to 128 warp instructions per k-block, those of the weights
 // 9 to 10 cache lines each) and the split; the tensor pipe needs 768 of the 4,700 clocks that a k-block takes.  Input gradient of

@@ -539,6 +539,45 @@ wgrad_bias_reduce_kernel(const float *__restrict__ partial, float *__restrict__ 
     }
 }
 
+// The same for many splits: eight threads share an output, each adds every eighth split, and their sums are added in order.
+__global__ void __launch_bounds__(256)
+wgrad_bias_reduce_wide_kernel(const float *__restrict__ partial, float *__restrict__ gw, long long n, int splits, float scale,
+                              const float *__restrict__ bias_part, float *__restrict__ gb, int K)
+{
+    __shared__ float part_s[8][32];
+    __shared__ double bias_s[8][32];
+    const long long total = n + (bias_part ? K : 0);
+    const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
+    for (long long base = blockIdx.x * 32LL; base < total; base += gridDim.x * 32LL) {
+        const long long i = base + lane;
+        float s = 0.f;
+        double b = 0.0;
+        if (i < n) {
+#pragma unroll 4
+            for (int k = group; k < splits; k += 8) s += __ldg(partial + (size_t)k * n + i);
+        } else if (i < total) {
+            for (int k = group; k < splits; k += 8) b += (double)__ldg(bias_part + (size_t)(i - n) * splits + k);
+        }
+        part_s[group][lane] = s;
+        bias_s[group][lane] = b;
+        __syncthreads();
+        if (group == 0 && i < total) {
+            if (i < n) {
+                float t = 0.f;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) t += part_s[g][lane];
+                gw[i] += scale * t;
+            } else {
+                double t = 0.0;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) t += bias_s[g][lane];
+                gb[i - n] = (float)((double)gb[i - n] + (double)scale * t);
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // y[img][q][pix] += bias[q]: the bias of a transposed convolution, whose product comes out of the input-gradient kernels.
 __global__ void __launch_bounds__(256)
 add_plane_bias_kernel(float *__restrict__ y, const float *__restrict__ bias, int Q, int HW, long long total)
@@ -589,7 +628,7 @@ dgrad_gather_kernel(const float *__restrict__ gy, const float *__restrict__ w, f
 //                                                                        B: 4 channels of one filter = 16 contiguous bytes (K-major)
 //   input grad   D[pixel, c]  = sum_ko gy[img][ko][pix] * W[ko][c]      A: M-major as above;  B: 4 channels c of one ko (N-major)
 //   weight grad  D[ko, c]     = sum_{img,pix} gy[img][ko][pix] * x[img][c][pix]      A, B: 4 pixels of one row (K-major);
-//                                                                        k runs over (image, pixel) of this tile's image range
+//                                                                        k runs over the (image, pixel)s of this tile's split
 //
 // tcgen05.mma takes M/N-major operands through the major bits of the instruction descriptor, so a 16-byte
 // asynchronous copy lands an operand piece in shared memory in its final place, no transposition.  One CTA per SM
@@ -621,7 +660,7 @@ struct Params {
     int M_total, N_total, Kd;
     int n_tiles, tiles_per_split, total_tiles;   // tile = (split * m_tiles + m_tile) * n_tiles + n_tile
     int kblocks;       // k-blocks per tile
-    int n_img, imgs_per_split, splits;
+    int n_img, splits;         // WGRAD: split s sums the k-blocks [s, s + 1) * kblocks of all images
     int vec_a, vec_b;  // 16-byte global loads allowed for A / B
     // kernels larger than 1x1 (KS != 1): the unfolded operand is gathered from a [g_C, g_H, g_W] image tensor, the
     // pixel grid that drives the gather is pix_W wide (HW = its size)
@@ -692,7 +731,7 @@ struct Loader {
     int a_off[4];       // FWD/DGRAD: element offsets of the thread's 4 pixels (channel 0); WGRAD: [0..1] row offsets
     int b_off[2];       // FWD: offsets of the thread's two filter rows (+ chunk); DGRAD: [0] first column; WGRAD: row offsets
     unsigned a_mask, b_mask;
-    int img, pix, img_end;   // WGRAD: image and pixel of the thread's chunk in the current k-block
+    int img, pix;            // WGRAD: image and pixel of the thread's chunk in the current k-block; images >= n_img read as zeros
     unsigned tapmask[4];     // KS != 1, FWD/DGRAD: bit t set when tap t of pixel j lies inside the image
     int img2, pix2;          // KS != 1, WGRAD: image and pixel of this lane's column (k = lane) of the unfolded operand
 
@@ -782,8 +821,9 @@ struct Loader {
                 if (m < p.M_total) a_mask |= 1u << i;
                 if (row < BN && n < p.N_total) b_mask |= 1u << i;
             }
-            img = split * p.imgs_per_split;
-            img_end = min(p.n_img, img + p.imgs_per_split);
+            const int p0 = split * p.kblocks * BK;               // the split's first pixel in the flat (image, pixel) sequence
+            img = p0 / p.HW;
+            pix = p0 - img * p.HW;
             if (KS != 1) {
                 // every producer has issued the copies of the previous tile before the table changes
                 producers_sync();
@@ -801,10 +841,10 @@ struct Loader {
                 }
                 producers_sync();
                 img2 = img;
-                pix2 = lane;
+                pix2 = pix + lane;
                 while (pix2 >= p.HW) { pix2 -= p.HW; ++img2; }
             }
-            pix = (tid & 7) * 4;
+            pix += (tid & 7) * 4;
             while (pix >= p.HW) { pix -= p.HW; ++img; }
         }
     }
@@ -830,7 +870,7 @@ struct Loader {
     __device__ __forceinline__ void row_chunk(const Params &p, uint32_t dst, const float *base, int stride, bool vec, bool on) const
     {
         if (vec) {
-            const bool ok = on && img < img_end;
+            const bool ok = on && img < p.n_img;
             cp_async16(dst, ok ? base + (size_t)img * stride + pix : base, ok);
             return;
         }
@@ -838,7 +878,7 @@ struct Loader {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             while (pj >= p.HW) { pj -= p.HW; ++ij; }
-            const bool ok = on && ij < img_end;
+            const bool ok = on && ij < p.n_img;
             cp_async4(dst + 4 * j, ok ? base + (size_t)ij * stride + pj : base, ok);
             ++pj;
         }
@@ -938,7 +978,7 @@ struct Loader {
                 const int lane = tid & 31;
                 const int oh = pix2 / p.pix_W, ow = pix2 - oh * p.pix_W;
                 const int ih = oh * p.dH - p.padH, iw = ow * p.dW - p.padW;
-                const bool pix_ok = img2 < img_end;
+                const bool pix_ok = img2 < p.n_img;
                 const float *img_base = p.b + (size_t)(pix_ok ? img2 : 0) * p.g_C * p.g_H * p.g_W + (ih * p.g_W + iw);
                 const uint32_t dst0 = sb + (uint32_t)(warp * 128 + (((lane >> 2) ^ (warp & 7)) << 4) + (lane & 3) * 4);
 #pragma unroll
@@ -1403,6 +1443,8 @@ static PwKernel pw_pick(int bn, int ks = 1)
 }
 // Kernels of up to 32 taps run on the same persistent kernel with a gathering loader.
 static bool gather_applies(int kH, int kW) { return kH * kW <= 32; }
+// Kernels of up to 16 x 16 taps: any number of taps on the weight gradient's loader and on conv_gather.cuh.
+static bool small_kernel(int kH, int kW) { return kH <= pwg::MAX_KERNEL && kW <= pwg::MAX_KERNEL; }
 // loader variant of the gathering path: 3x3 has its own instantiation, everything else (a strided or padded 1x1
 // included) the one with run-time kernel sizes
 static int gather_ks(int kH, int kW) { return (kH == 3 && kW == 3) ? 3 : 0; }
@@ -1519,28 +1561,36 @@ static int pw_tma_launch(PwTmaKernel kern, pw::Params &p, CUtensorMap &ma, CUten
     return 0;
 }
 
-// Splits of the image range for the weight gradient on the persistent kernel: every tile takes `imgs_per_split`
-// images.  Candidates are scored by (waves of the persistent grid) x (images per tile) — the time of the slowest
-// CTA — and tiles longer than ~128 k-blocks are avoided when a shorter choice exists (accumulation chains).
-static void pw_wgrad_plan(int N, int C, int K, int HW, int *bn, int *splits, int *imgs_per_split)
+// Splits of the weight gradient's reduction on the persistent kernels: a tile sums `kb_per_split` of the `kb_total` k-blocks of all
+// images.  Candidates fill one to sixteen waves of the persistent grid (and one to four splits, when one already fills it); they are
+// scored by waves x k-blocks per tile — the time of the slowest CTA, plus about six k-blocks for a tile's prologue and its 64 KB of
+// partial sums — and by what the reduction reads; tiles longer than ~128 k-blocks are avoided when a shorter choice exists
+// (accumulation chains).  Splits end anywhere in an image: with whole images per split, 48 of 148 SMs had work at
+// 12 x 144 x 37 x 29 -> 200 and 64 at 32 x 3 x 224 x 224, 7x7.
+static void pw_wgrad_plan(int C, int K, long long kb_total, int *bn, int *splits, int *kb_per_split)
 {
     *bn = pw_bn_for(C);
     const long long tiles_mn = (long long)ceil_div(K, BM) * ceil_div(C, *bn);
     const int grid = sm_count();
-    const long long kb_per_img = ceil_div_ll(HW, BK);
-    int best_ips = 1;
     double best = -1.0;
-    for (int ips = 1; ips <= N; ++ips) {
-        const long long tiles = tiles_mn * ceil_div(N, ips);
-        const long long waves = ceil_div_ll(tiles, grid);
-        // in k-blocks: the tile's own loop + about six more for its prologue, its 64 KB of partial sums and their
-        // share of the final reduction
-        double cost = (double)waves * ((double)ips * kb_per_img + 6.0);
-        if (ips > 1 && (long long)ips * kb_per_img > 128) cost *= 1.0 + 0.25 * (double)((long long)ips * kb_per_img - 128) / 128.0;
-        if (best < 0.0 || cost < best * 0.999) { best = cost; best_ips = ips; }
+    for (int i = 1; i <= 20; ++i) {
+        const long long want = i <= 16 ? (long long)i * grid / tiles_mn : i - 16;
+        const long long kb = ceil_div_ll(kb_total, std::max(1LL, std::min(want, kb_total))), used = ceil_div_ll(kb_total, kb);
+        const long long waves = ceil_div_ll(tiles_mn * used, grid);
+        double cost = (double)waves * ((double)kb + 6.0) + (double)used * K * C * 4.0 / 8e6;     // a k-block lasts as long as 8 MB of L2 reads
+        if (kb > 128) cost *= 1.0 + 0.25 * (double)(kb - 128) / 128.0;
+        if (best < 0.0 || cost < best * 0.999) { best = cost; *splits = (int)used; *kb_per_split = (int)kb; }
     }
-    *imgs_per_split = best_ips;
-    *splits = ceil_div(N, best_ips);
+}
+// k-blocks of a reduction over N images of HW pixels: flat (element copies), or whole groups of 32 per image (tensor maps).
+static long long flat_kblocks(int N, int HW) { return ceil_div_ll((long long)N * HW, BK); }
+static long long group_kblocks(int N, int HW) { return (long long)N * ceil_div(HW, BK); }
+// Workspace for the partial sums of `splits` splits and their bias sums.
+static size_t wgrad_partial_bytes(int C, int K, long long kb_total)
+{
+    int bn, splits, kb;
+    pw_wgrad_plan(C, K, kb_total, &bn, &splits, &kb);
+    return (size_t)splits * K * C * sizeof(float) + (size_t)K * splits * sizeof(float) + 256;
 }
 
 // ---- gathered operand, register accumulation (conv_gather.cuh) -------------------------------------------------------
@@ -1667,7 +1717,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         q.HW = H * W; q.M_total = N * H * W; q.N_total = K; q.Kd = C; q.kblocks = ceil_div(C, BK);
         const int bn = pw_bn_for(K);
         q.n_tiles = ceil_div(K, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
-        q.n_img = N; q.imgs_per_split = N; q.splits = 1;
+        q.n_img = N; q.splits = 1;
         if (tma_applies(x, weight, y, q.HW, C)) {
             alignas(64) CUtensorMap ma, mb, mo;
             q.gpi = ceil_div(q.HW, 32); q.M_total = N * q.gpi * 32; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
@@ -1691,11 +1741,24 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         set_geometry(q, C, H, W, kH, kW, dH, dW, padH, padW, oW, dilH, dilW);
         const int bn = pw_bn_for(K);
         q.n_tiles = ceil_div(K, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
-        q.n_img = N; q.imgs_per_split = N; q.splits = 1;
+        q.n_img = N; q.splits = 1;
         q.vec_a = 0; q.vec_b = (q.Kd % 4 == 0) && aligned16(weight);
         q.bulk_out = (q.HW % 4 == 0) && q.HW >= 8 * BM && aligned16(y);
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
         return pw_launch(pw_pick<OP_FWD>(bn, gather_ks(kH, kW)), q, stream);
+    }
+    if (small_kernel(kH, kW)) {
+        pwg::GatherParams q{};
+        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
+        q.g_C = C; q.g_H = H; q.g_W = W; q.N_total = K; q.w_kk = kH * kW; q.o_HW = oH * oW;
+        q.vec_b = (C * kH * kW) % 4 == 0 && aligned16(weight);
+        q.n_phases = 1;
+        pwg::Phase &f = q.ph[0];
+        f.HW = oH * oW; f.pix_W = oW; f.M_total = N * f.HW;
+        f.taps = kH * kW; f.kW = kW; f.Kd = C * f.taps;
+        f.dH = dH; f.dW = dW; f.padH = padH; f.padW = padW; f.dilH = f.dilW = 1;
+        f.o_sH = oW; f.o_sW = 1;
+        return launch_gather<OP_FWD>(q, pw_bn_for(K), stream);
     }
     GemmParams p{};
     p.a_src = x; p.b_src = weight; p.bias = bias; p.out = y; p.status = device_status_ptr();
@@ -1734,7 +1797,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         q.HW = H * W; q.M_total = N * H * W; q.N_total = C; q.Kd = K; q.kblocks = ceil_div(K, BK);
         const int bn = pw_bn_for(C);
         q.n_tiles = ceil_div(C, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
-        q.n_img = N; q.imgs_per_split = N; q.splits = 1;
+        q.n_img = N; q.splits = 1;
         if (tma_applies(gy, weight, gx, q.HW, C)) {
             alignas(64) CUtensorMap ma, mb, mo;
             q.gpi = ceil_div(q.HW, 32); q.M_total = N * q.gpi * 32; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
@@ -1751,7 +1814,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
         return add_bias(pw_launch(pw_pick<OP_DGRAD>(bn), q, stream));
     }
-    if (dH == 1 && dW == 1 && padH <= dilH * (kH - 1) && padW <= dilW * (kW - 1) && (!dilated || gather_applies(kH, kW))) {
+    if (dH == 1 && dW == 1 && padH <= dilH * (kH - 1) && padW <= dilW * (kW - 1) && (gather_applies(kH, kW) || !small_kernel(kH, kW))) {
         // stride 1: a convolution of gy with the kernel rotated by 180 degrees and padding dil (k - 1) - pad
         if (gather_applies(kH, kW)) {
             pw::Params q{};
@@ -1760,7 +1823,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
             set_geometry(q, K, oH, oW, kH, kW, 1, 1, dilH * (kH - 1) - padH, dilW * (kW - 1) - padW, W, dilH, dilW);
             const int bn = pw_bn_for(C);
             q.n_tiles = ceil_div(C, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
-            q.n_img = N; q.imgs_per_split = N; q.splits = 1;
+            q.n_img = N; q.splits = 1;
             q.vec_a = 0; q.vec_b = 0;
             q.bulk_out = (q.HW % 4 == 0) && q.HW >= 8 * BM && aligned16(gx);
             pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
@@ -1784,6 +1847,21 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
     return add_bias(0);
 }
 
+static int reduce_partials(const float *partial, float *gw, long long n, int splits, float scale, const float *bias_part, float *gb, int K,
+                           cudaStream_t stream)
+{
+    const long long total = n + (bias_part ? K : 0);
+    if (splits >= 16) {
+        const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 32), (long long)sm_count() * 8));
+        wgrad_bias_reduce_wide_kernel<<<blocks, 256, 0, stream>>>(partial, gw, n, splits, scale, bias_part, gb, K);
+    } else {
+        const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 8));
+        wgrad_bias_reduce_kernel<<<blocks, 256, 0, stream>>>(partial, gw, n, splits, scale, bias_part, gb, K);
+    }
+    CUNN_LAUNCH_CHECK("convmm acc grad reduce");
+    return 0;
+}
+
 static size_t conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW, int padH, int padW,
                                       int dilH, int dilW)
 {
@@ -1791,15 +1869,10 @@ static size_t conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH,
     if (check(N, C, H, W, K, kH, kW, dH, dW, padH, padW, &oH, &oW, dilH, dilW) || N == 0) return 0;
     const bool dilated = dilH != 1 || dilW != 1;
     if (!dilated && stem::applies(C, K, kH, kW)) return stem::wgrad_workspace_bytes();
+    if (pw_applies(kH, kW, dH, dW, padH, padW))
+        return std::max(wgrad_partial_bytes(C, K, flat_kblocks(N, H * W)), wgrad_partial_bytes(C, K, group_kblocks(N, H * W)));
+    if (small_kernel(kH, kW)) return wgrad_partial_bytes(C * kH * kW, K, flat_kblocks(N, oH * oW));
     int bn, splits, ips, pb;
-    if (pw_applies(kH, kW, dH, dW, padH, padW)) {
-        pw_wgrad_plan(N, C, K, H * W, &bn, &splits, &ips);
-        return (size_t)splits * K * C * sizeof(float) + (size_t)K * splits * sizeof(float) + 256;
-    }
-    if (gather_applies(kH, kW)) {
-        pw_wgrad_plan(N, C * kH * kW, K, oH * oW, &bn, &splits, &ips);
-        return (size_t)splits * K * C * kH * kW * sizeof(float) + (size_t)K * splits * sizeof(float) + 256;
-    }
     wgrad_plan(N, C, K, kH * kW, oH * oW, &bn, &splits, &ips, &pb);
     const int chunks = std::max(1, std::min(N, ceil_div(sm_count() * 4, K)));
     return (size_t)splits * K * C * kH * kW * sizeof(float) + (size_t)K * chunks * sizeof(float) + 256;
@@ -1821,64 +1894,54 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
     CUNN_CHECK_ARG(workspace && workspace_bytes >= need && ((uintptr_t)workspace & 15) == 0,
                    "convmm acc_grad needs %zu bytes of 16-byte aligned workspace, got %zu", need,
                    workspace ? workspace_bytes : (size_t)0);
-    int bn, splits, ips, pb;
+    int bn, splits, ips, pb, kb;
     const int kk = kH * kW;
     if (!dilated && stem::applies(C, K, kH, kW)) {
         const int ctas = stem::wgrad_ctas();
         const long long n = (long long)K * C * kk;
         float *partial = (float *)workspace, *bias_part = partial + (size_t)ctas * n;
         if (stem::weight_grad_partials(x, gy, partial, grad_bias ? bias_part : nullptr, N, H, W, oH, oW, dH, dW, padH, padW, stream)) return 1;
-        const int rblocks = (int)std::max(1LL, std::min(ceil_div_ll(n + K, 256), (long long)sm_count() * 8));
-        wgrad_bias_reduce_kernel<<<rblocks, 256, 0, stream>>>(partial, grad_weight, n, ctas, scale, grad_bias ? bias_part : nullptr, grad_bias, K);
-        CUNN_LAUNCH_CHECK("convmm acc grad reduce");
-        return 0;
+        return reduce_partials(partial, grad_weight, n, ctas, scale, grad_bias ? bias_part : nullptr, grad_bias, K, stream);
     }
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
-        pw_wgrad_plan(N, C, K, H * W, &bn, &splits, &ips);
+        const bool tma = tma_applies(gy, x, workspace, H * W, 4);
+        pw_wgrad_plan(C, K, tma ? group_kblocks(N, H * W) : flat_kblocks(N, H * W), &bn, &splits, &kb);
         const long long n = (long long)K * C;
         pw::Params q{};
         q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr();
         q.bias_part = grad_bias ? (float *)workspace + (size_t)splits * n : nullptr;
-        q.HW = H * W; q.M_total = K; q.N_total = C; q.Kd = 0;
-        q.kblocks = (int)ceil_div_ll((long long)ips * q.HW, BK);
+        q.HW = H * W; q.M_total = K; q.N_total = C; q.Kd = 0; q.kblocks = kb;
         q.n_tiles = ceil_div(C, bn); q.tiles_per_split = ceil_div(K, BM) * q.n_tiles; q.total_tiles = q.tiles_per_split * splits;
-        q.n_img = N; q.imgs_per_split = ips; q.splits = splits;
+        q.n_img = N; q.splits = splits;
         q.vec_a = (q.HW % 4 == 0) && aligned16(gy); q.vec_b = (q.HW % 4 == 0) && aligned16(x);
-        if (tma_applies(gy, x, workspace, q.HW, 4)) {
+        if (tma) {
             alignas(64) CUtensorMap ma, mb;
-            q.gpi = ceil_div(q.HW, 32); q.kblocks = ips * q.gpi;
+            q.gpi = ceil_div(q.HW, 32);
             tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
             if (make_map(&ma, gy, q.HW, K, N, 32, BM, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
             if (make_map(&mb, x, q.HW, C, N, 32, bn, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
             if (pw_tma_launch(pw_tma_pick<OP_WGRAD>(bn), q, ma, mb, ma, stream)) return 1;
         } else {
-        pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
-        if (pw_launch(pw_pick<OP_WGRAD>(bn), q, stream)) return 1;
+            pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
+            if (pw_launch(pw_pick<OP_WGRAD>(bn), q, stream)) return 1;
         }
-        const int rblocks = (int)std::max(1LL, std::min(ceil_div_ll(n + K, 256), (long long)sm_count() * 8));
-        wgrad_bias_reduce_kernel<<<rblocks, 256, 0, stream>>>((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K);
-        CUNN_LAUNCH_CHECK("convmm acc grad reduce");
-        return 0;
+        return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
-    if (gather_applies(kH, kW)) {
+    if (small_kernel(kH, kW)) {
         const int oHW = oH * oW;
-        pw_wgrad_plan(N, C * kk, K, oHW, &bn, &splits, &ips);
+        pw_wgrad_plan(C * kk, K, flat_kblocks(N, oHW), &bn, &splits, &kb);
         const long long n = (long long)K * C * kk;
         pw::Params q{};
         q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr();
         q.bias_part = grad_bias ? (float *)workspace + (size_t)splits * n : nullptr;
-        q.HW = oHW; q.M_total = K; q.N_total = C * kk; q.Kd = 0;
-        q.kblocks = (int)ceil_div_ll((long long)ips * oHW, BK);
+        q.HW = oHW; q.M_total = K; q.N_total = C * kk; q.Kd = 0; q.kblocks = kb;
         set_geometry(q, C, H, W, kH, kW, dH, dW, padH, padW, oW, dilH, dilW);
         q.n_tiles = ceil_div(C * kk, bn); q.tiles_per_split = ceil_div(K, BM) * q.n_tiles; q.total_tiles = q.tiles_per_split * splits;
-        q.n_img = N; q.imgs_per_split = ips; q.splits = splits;
+        q.n_img = N; q.splits = splits;
         q.vec_a = (oHW % 4 == 0) && aligned16(gy); q.vec_b = 0;
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
         if (pw_launch(pw_pick<OP_WGRAD>(bn, gather_ks(kH, kW)), q, stream)) return 1;
-        const int rblocks = (int)std::max(1LL, std::min(ceil_div_ll(n + K, 256), (long long)sm_count() * 8));
-        wgrad_bias_reduce_kernel<<<rblocks, 256, 0, stream>>>((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K);
-        CUNN_LAUNCH_CHECK("convmm acc grad reduce");
-        return 0;
+        return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
     wgrad_plan(N, C, K, kk, oH * oW, &bn, &splits, &ips, &pb);
     GemmParams p{};

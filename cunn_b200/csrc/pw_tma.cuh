@@ -285,7 +285,7 @@ pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const _
                 } else {
                     const int split = t / p.tiles_per_split, r = t - split * p.tiles_per_split;
                     const int m_tile = r / p.n_tiles, n_tile = r - m_tile * p.n_tiles;
-                    const int im = split * p.imgs_per_split + kb / p.gpi, p0 = (kb % p.gpi) * 32;
+                    const int flat = split * KB + kb, im = flat / p.gpi, p0 = (flat - im * p.gpi) * 32;      // image >= n_img: zero fill
                     tma_load_3d(sa, &map_a, p0, m_tile * BM, im, bar);
                     tma_load_3d(sb, &map_b, p0, n_tile * BN, im, bar);
                 }

@@ -186,3 +186,21 @@ def test_convmm_full_size_adjoint_identities(F, cfg):
     lhs = F.convmm_forward(2 * x - 3 * x2, w, None, 1, 1, pad, pad)
     rhs = 2 * y - 3 * F.convmm_forward(x2, w, None, 1, 1, pad, pad)
     assert float((lhs - rhs).abs().max()) < 1e-4 * float(rhs.abs().max())
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W, K, k, d, pad: weight gradients whose splits end inside an image, and kernels of more than 32 taps
+    (3, 40, 37, 29, 70, 1, 1, 0),        # 1073-pixel planes: element copies, splits at odd pixels
+    (2, 64, 60, 52, 130, 1, 1, 0),       # tensor maps: splits of whole pixel groups
+    (1, 8, 90, 70, 24, 3, 1, 1),         # one image, gathered operand
+    (1, 5, 64, 64, 16, 7, 2, 3),         # 49 taps
+    (2, 3, 71, 53, 40, 11, 4, 2),        # 121 taps, stride 4
+    (2, 6, 19, 23, 33, 9, 1, 4),         # 81 taps at stride 1: all three passes
+    (1, 2, 40, 40, 70, 16, 3, 0),        # 256 taps: the largest kernel of this path
+    (1, 2, 40, 40, 6, 17, 3, 0),         # one row more: the kernel for any size
+    (1, 700, 1, 1, 40, 1, 1, 0),         # a single k-block
+])
+def test_convmm_split_reductions_and_large_kernels(F, ref64, shape):
+    N, C, H, W, K, k, d, pad = shape
+    case = make_case(abs(hash(shape)) % 99991, N, C, H, W, K, k, d, pad, True)
+    check_against_oracle(ref64, F, *case, d, pad, 0.75)
