@@ -1455,6 +1455,15 @@ static void set_geometry(pw::Params &q, int gC, int gH, int gW, int kH, int kW, 
     q.dilH = dilH; q.dilW = dilW;
 }
 static int pw_bn_for(int n_total) { return n_total <= 32 ? 32 : (n_total <= 64 ? 64 : 128); }
+// Column-tile width of a GEMM with `rows` rows: narrower tiles while the wide ones leave half of the SMs without one.  Such a launch
+// lasts as long as one tile, and a tile's k-block costs less the narrower it is (one image through 512 -> 512 at 14 x 14: 8 tiles of
+// 128 columns 18.9 us, 32 of 32 columns 15.5 us).
+static int pw_bn_for(int n_total, long long rows)
+{
+    int bn = pw_bn_for(n_total);
+    while (bn > 32 && ceil_div_ll(rows, BM) * ceil_div(n_total, bn) * 2 <= sm_count()) bn /= 2;
+    return bn;
+}
 
 // Accumulators per tile and accumulator sets: the hi*hi products of the k-blocks are dealt round-robin to `nacc - 1`
 // accumulators to keep the tensor core's truncating accumulation chains short, the cross terms share the last one; two sets (epilogue overlapped with the next tile) when
@@ -1688,7 +1697,9 @@ static int phased_grad_input(const float *gy, const float *weight, const float *
         q.g_C = K; q.g_H = oH; q.g_W = oW; q.N_total = C; q.w_kk = kH * kW; q.o_HW = H * W;
         q.n_phases = (int)std::min<size_t>(pwg::MAX_PHASES, ph.size() - at);
         for (int i = 0; i < q.n_phases; ++i) q.ph[i] = ph[at + i];
-        if (launch_gather<OP_DGRAD>(q, pw_bn_for(C), stream)) return 1;
+        long long rows = 0;
+        for (int i = 0; i < q.n_phases; ++i) rows += q.ph[i].M_total;
+        if (launch_gather<OP_DGRAD>(q, pw_bn_for(C, rows), stream)) return 1;
     }
     return 0;
 }
@@ -1711,11 +1722,26 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     const bool dilated = dilH != 1 || dilW != 1;
     CUNN_CHECK_ARG(!dilated || gather_applies(kH, kW), "dilated kernels of more than 32 taps are not supported");
     if (!dilated && stem::applies(C, K, kH, kW)) return stem::forward(x, weight, bias, y, N, H, W, oH, oW, dH, dW, padH, padW, stream);
+    if (pw_applies(kH, kW, dH, dW, padH, padW) && H * W == 1 && K % 4 == 0 && tma_applies(x, weight, y, C, 4)) {
+        // a fully connected layer: y[n][k] = sum_c x[n][c] W[k][c], two K-major matrices, i.e. the weight gradient's GEMM over one
+        // "image" of C pixels (with element copies of single-pixel planes, 128 x 1024 -> 1000 took 129 us)
+        pw::Params q{};
+        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
+        q.HW = C; q.gpi = ceil_div(C, 32); q.M_total = N; q.N_total = K; q.kblocks = q.gpi;
+        const int bn = pw_bn_for(K, N);
+        q.n_tiles = ceil_div(K, bn); q.tiles_per_split = q.total_tiles = ceil_div(N, BM) * q.n_tiles;
+        q.n_img = 1; q.splits = 1;
+        tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
+        alignas(64) CUtensorMap ma, mb;
+        if (make_map(&ma, x, C, N, 1, 32, BM, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
+        if (make_map(&mb, weight, C, K, 1, 32, bn, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
+        return pw_tma_launch(pw_tma_pick<OP_WGRAD>(bn), q, ma, mb, ma, stream);
+    }
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         pw::Params q{};
         q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
         q.HW = H * W; q.M_total = N * H * W; q.N_total = K; q.Kd = C; q.kblocks = ceil_div(C, BK);
-        const int bn = pw_bn_for(K);
+        const int bn = pw_bn_for(K, q.M_total);
         q.n_tiles = ceil_div(K, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
         q.n_img = N; q.splits = 1;
         if (tma_applies(x, weight, y, q.HW, C)) {
@@ -1739,7 +1765,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
         q.HW = oH * oW; q.M_total = N * oH * oW; q.N_total = K; q.Kd = C * kH * kW; q.kblocks = ceil_div(q.Kd, BK);
         set_geometry(q, C, H, W, kH, kW, dH, dW, padH, padW, oW, dilH, dilW);
-        const int bn = pw_bn_for(K);
+        const int bn = pw_bn_for(K, q.M_total);
         q.n_tiles = ceil_div(K, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
         q.n_img = N; q.splits = 1;
         q.vec_a = 0; q.vec_b = (q.Kd % 4 == 0) && aligned16(weight);
@@ -1758,7 +1784,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         f.taps = kH * kW; f.kW = kW; f.Kd = C * f.taps;
         f.dH = dH; f.dW = dW; f.padH = padH; f.padW = padW; f.dilH = f.dilW = 1;
         f.o_sH = oW; f.o_sW = 1;
-        return launch_gather<OP_FWD>(q, pw_bn_for(K), stream);
+        return launch_gather<OP_FWD>(q, pw_bn_for(K, f.M_total), stream);
     }
     GemmParams p{};
     p.a_src = x; p.b_src = weight; p.bias = bias; p.out = y; p.status = device_status_ptr();
@@ -1791,11 +1817,15 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
     CUNN_CHECK_ARG(gy && weight && gx, "null tensor pointer");
     const bool dilated = dilH != 1 || dilW != 1;
     CUNN_CHECK_ARG(!dilated || gather_applies(kH, kW), "dilated kernels of more than 32 taps are not supported");
+    if (pw_applies(kH, kW, dH, dW, padH, padW) && H * W == 1 && K % 4 == 0 && tma_applies(gy, weight, gx, C, K))
+        // a fully connected layer: gx[n][c] = sum_k gy[n][k] W[k][c] is the 1x1 convolution of the one "image" W (K channels of C
+        // pixels) with the N filters gy
+        return add_bias(conv_forward(weight, gy, nullptr, gx, 1, K, 1, C, N, 1, 1, 1, 1, 0, 0, 1, 1, stream_));
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         pw::Params q{};
         q.a = gy; q.b = weight; q.bias = nullptr; q.out = gx; q.status = device_status_ptr();
         q.HW = H * W; q.M_total = N * H * W; q.N_total = C; q.Kd = K; q.kblocks = ceil_div(K, BK);
-        const int bn = pw_bn_for(C);
+        const int bn = pw_bn_for(C, q.M_total);
         q.n_tiles = ceil_div(C, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
         q.n_img = N; q.splits = 1;
         if (tma_applies(gy, weight, gx, q.HW, C)) {
@@ -1821,7 +1851,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
             q.a = gy; q.b = weight; q.bias = nullptr; q.out = gx; q.status = device_status_ptr();
             q.HW = H * W; q.M_total = N * H * W; q.N_total = C; q.Kd = K * kH * kW; q.kblocks = ceil_div(q.Kd, BK);
             set_geometry(q, K, oH, oW, kH, kW, 1, 1, dilH * (kH - 1) - padH, dilW * (kW - 1) - padW, W, dilH, dilW);
-            const int bn = pw_bn_for(C);
+            const int bn = pw_bn_for(C, q.M_total);
             q.n_tiles = ceil_div(C, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
             q.n_img = N; q.splits = 1;
             q.vec_a = 0; q.vec_b = 0;

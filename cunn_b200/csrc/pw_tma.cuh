@@ -178,7 +178,7 @@ __device__ __forceinline__ void drain_tile(const Params &p, const CUtensorMap &m
             float acc[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j)
-                acc[j] = (OP == OP_FWD && p.bias && n_tile0 + c0 + j < p.N_total) ? __ldg(p.bias + n_tile0 + c0 + j) : 0.f;
+                acc[j] = (OP != OP_DGRAD && p.bias && n_tile0 + c0 + j < p.N_total) ? __ldg(p.bias + n_tile0 + c0 + j) : 0.f;
             gather_acc16<HALVES == 2>(acc, tsrc + (uint32_t)c0, nhi_used, p.nacc, ACC_COLS);
             if (row_ok) {
                 const int n0 = n_tile0 + c0;

@@ -105,6 +105,26 @@ avgpool_fwd_kernel(const float *__restrict__ x, float *__restrict__ y, int H, in
     }
 }
 
+// One window over the whole map (global average pooling): every pixel of a plane gets the plane's gradient over the pixel count.  The
+// tensor is written as one flat array, 16 bytes per thread where it is aligned; 128 x 1024 x 7 x 7 (26 MB written): 71 us with
+// the window walk.
+template <int VEC>
+__global__ void __launch_bounds__(256)
+avgpool_bwd_global_kernel(const float *__restrict__ gy, float *__restrict__ gx, unsigned HW, float divisor, unsigned total)
+{
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < total / VEC; q += gridDim.x * blockDim.x) {
+        unsigned pl = q * VEC / HW, r = q * VEC - pl * HW;
+        float g = 0.f + __ldg(gy + pl) / divisor, out[VEC];
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) {
+            out[j] = g;
+            if (j + 1 < VEC && ++r == HW) { r = 0; g = 0.f + __ldg(gy + ++pl) / divisor; }
+        }
+        if (VEC == 4) reinterpret_cast<float4 *>(gx)[q] = make_float4(out[0], out[1 % VEC], out[2 % VEC], out[3 % VEC]);
+        else gx[q] = out[0];
+    }
+}
+
 __global__ void __launch_bounds__(256)
 avgpool_bwd_kernel(const float *__restrict__ gy, float *__restrict__ gx, int H, int W, int oH, int oW, int kH, int kW,
                    int dH, int dW, int padH, int padW, int include_pad, long long total)
@@ -274,6 +294,14 @@ extern "C" CUNN_API int cunn_b200_avgpool_backward(const float *gy, float *gx, i
     if (N == 0) return 0;
     CUNN_CHECK_ARG(gy && gx, "null tensor pointer");
     const long long total = (long long)N * C * H * W;
+    if (oH == 1 && oW == 1 && kH >= H && kW >= W && padH == 0 && padW == 0 && total < (1LL << 31)) {
+        const bool vec = total % 4 == 0 && ((uintptr_t)gx & 15) == 0;
+        const int blocks = grid_for(vec ? total / 4 : total, 1);
+        if (vec) avgpool_bwd_global_kernel<4><<<blocks, 256, 0, (cudaStream_t)stream>>>(gy, gx, (unsigned)(H * W), (float)(H * W), (unsigned)total);
+        else avgpool_bwd_global_kernel<1><<<blocks, 256, 0, (cudaStream_t)stream>>>(gy, gx, (unsigned)(H * W), (float)(H * W), (unsigned)total);
+        CUNN_LAUNCH_CHECK("average pooling backward");
+        return 0;
+    }
     avgpool_bwd_kernel<<<grid_for(total, 1), 256, 0, (cudaStream_t)stream>>>(gy, gx, H, W, oH, oW, kH, kW, dH, dW, padH, padW,
                                                                             count_include_pad, total);
     CUNN_LAUNCH_CHECK("average pooling backward");

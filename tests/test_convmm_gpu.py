@@ -198,7 +198,13 @@ def test_convmm_full_size_adjoint_identities(F, cfg):
     (2, 6, 19, 23, 33, 9, 1, 4),         # 81 taps at stride 1: all three passes
     (1, 2, 40, 40, 70, 16, 3, 0),        # 256 taps: the largest kernel of this path
     (1, 2, 40, 40, 6, 17, 3, 0),         # one row more: the kernel for any size
-    (1, 700, 1, 1, 40, 1, 1, 0),         # a single k-block
+    (1, 700, 1, 1, 40, 1, 1, 0),         # a single pixel
+    (130, 100, 1, 1, 36, 1, 1, 0),       # fully connected: two row tiles, ragged reduction and columns
+    (1, 32, 1, 1, 4, 1, 1, 0),           # ... one image, one k-block
+    (5, 1024, 1, 1, 1000, 1, 1, 0),      # ... a classifier
+    (5, 64, 1, 1, 6, 1, 1, 0),           # ... outputs whose rows are not 16-byte multiples
+    (1, 512, 14, 14, 512, 1, 1, 0),      # few row tiles: column tiles of 32
+    (1, 96, 14, 14, 200, 3, 1, 1),       # ... gathered operand
 ])
 def test_convmm_split_reductions_and_large_kernels(F, ref64, shape):
     N, C, H, W, K, k, d, pad = shape

@@ -80,3 +80,15 @@ def test_sgd_update(F):
     g = torch.ones(10, device="cuda") * 2
     F.sgd_update(p, g, 0.25)
     assert torch.equal(p.cpu(), torch.arange(10, dtype=torch.float32) - 0.5)
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 7, 7), (2, 4, 8, 8), (1, 3, 5, 1), (1, 1, 1, 1), (7, 3, 3, 2)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_avgpool_global_backward(F, shape, shift):
+    """One window over the map: every pixel gets the plane's gradient over the pixel count, whatever the alignment."""
+    N, C, H, W = shape
+    gy = torch.randn(N, C, 1, 1, device="cuda")
+    buf = torch.full((N * C * H * W + shift + 1,), 7.0, device="cuda")
+    out = buf[shift:shift + N * C * H * W].view(shape)
+    F.avgpool_backward(gy, H, W, H, W, 1, 1, 0, 0, out=out)
+    assert torch.equal(out, (gy / float(H * W)).expand(shape)) and buf[-1] == 7.0
