@@ -164,16 +164,18 @@ fwd_kernel(const __grid_constant__ Params p)
         float acc[TH];
 #pragma unroll
         for (int t = 0; t < TH; ++t) acc[t] = b;
-        const float *row0 = tile + (pl * p.rows + t0 * S) * p.ld + ow;
+        // row by row, so that an output adds its taps in the order of fwd_point: the same bits
+        const float *row = tile + (pl * p.rows + t0 * S) * p.ld + ow;
 #pragma unroll
-        for (int kw = 0; kw < K; ++kw) {
-            const float *col = row0 + (S == 1 ? kw : (kw & 1) * p.half + (kw >> 1));
+        for (int r = 0; r < (TH - 1) * S + K; ++r, row += p.ld) {
+            float v[K];
 #pragma unroll
-            for (int r = 0; r < (TH - 1) * S + K; ++r) {
-                const float v = col[r * p.ld];
+            for (int kw = 0; kw < K; ++kw) v[kw] = row[S == 1 ? kw : (kw & 1) * p.half + (kw >> 1)];
 #pragma unroll
-                for (int t = 0; t < TH; ++t)
-                    if (r - t * S >= 0 && r - t * S < K) acc[t] = fmaf(w[(r - t * S) * K + kw], v, acc[t]);
+            for (int t = 0; t < TH; ++t) {
+                if (r - t * S < 0 || r - t * S >= K) continue;
+#pragma unroll
+                for (int kw = 0; kw < K; ++kw) acc[t] = fmaf(w[(r - t * S) * K + kw], v[kw], acc[t]);
             }
         }
 #pragma unroll

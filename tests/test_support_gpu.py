@@ -91,4 +91,5 @@ def test_avgpool_global_backward(F, shape, shift):
     buf = torch.full((N * C * H * W + shift + 1,), 7.0, device="cuda")
     out = buf[shift:shift + N * C * H * W].view(shape)
     F.avgpool_backward(gy, H, W, H, W, 1, 1, 0, 0, out=out)
-    assert torch.equal(out, (gy / float(H * W)).expand(shape)) and buf[-1] == 7.0
+    want = np.broadcast_to(host(gy) / np.float32(H * W), shape)        # one rounded division
+    assert np.array_equal(host(out), want) and buf[-1] == 7.0
