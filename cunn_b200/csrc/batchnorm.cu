@@ -205,10 +205,10 @@ stats_kernel(const float *__restrict__ x, ChunkStat *__restrict__ part, int N, i
 {
     const int id = (int)blockIdx.x * 8 + ((int)threadIdx.x >> 5);
     if (id >= C * chunks) return;
-    const int c = id / chunks, j = id - c * chunks;
+    const int j = id / C, c = id - j * C;                 // images in ascending order: see launch_apply
     const bool vec = (S % 4 == 0) && (((uintptr_t)x & 15) == 0);
     const ChunkStat s = vec ? chunk_stats<float4, 4>(x, N, C, S, c, chunks, j) : chunk_stats<float, 8>(x, N, C, S, c, chunks, j);
-    if ((threadIdx.x & 31) == 0) part[id] = s;
+    if ((threadIdx.x & 31) == 0) part[(size_t)c * chunks + j] = s;
     if (counters && last_warp_of_channel(counters, c, chunks)) {
         finish_stats_channel_warp(part + (size_t)c * chunks, c, chunks, running_mean, running_var, save_mean, save_std, momentum, eps);
         if ((threadIdx.x & 31) == 0) counters[c] = 0u;
@@ -245,7 +245,8 @@ apply_kernel(const float *__restrict__ x, float *__restrict__ y, const float *__
     const bool vec = (S % 4 == 0) && ((((uintptr_t)x | (uintptr_t)y) & 15) == 0);
     constexpr int PER_CTA = 256 / GROUP;
     const int sub = (int)threadIdx.x / GROUP, t = (int)threadIdx.x % GROUP;
-    for (long long pl = (long long)blockIdx.x * PER_CTA + sub; pl < planes; pl += (long long)gridDim.x * PER_CTA) {
+    for (long long rev = (long long)blockIdx.x * PER_CTA + sub; rev < planes; rev += (long long)gridDim.x * PER_CTA) {
+        const long long pl = planes - 1 - rev;                   // last image first
         const int c = (int)(pl % C);
         const float mean = __ldg(mean_v + c);
         const float invstd = train ? __ldg(std_or_var + c) : 1.f / sqrtf(__ldg(std_or_var + c) + eps);
@@ -312,10 +313,10 @@ apply_flat_kernel(const float *__restrict__ x, float *__restrict__ y, const floa
         float4 v[U];
 #pragma unroll
         for (unsigned u = 0; u < U; ++u)
-            if (q + u * stride < items) v[u] = __ldg(x4 + q + u * stride);
+            if (q + u * stride < items) v[u] = __ldg(x4 + (items - 1 - (q + u * stride)));       // last image first
 #pragma unroll
         for (unsigned u = 0; u < U; ++u)
-            if (q + u * stride < items) item(q + u * stride, v[u]);
+            if (q + u * stride < items) item(items - 1 - (q + u * stride), v[u]);
     }
     if (tid < total - items * 4u) {
         const unsigned e = items * 4u + tid;
@@ -458,7 +459,7 @@ grad_stats_kernel(const float *__restrict__ x, const float *__restrict__ gy, flo
 {
     const int id = (int)blockIdx.x * 8 + ((int)threadIdx.x >> 5);
     if (id >= C * chunks) return;
-    const int c = id / chunks, j = id - c * chunks;
+    const int j = id / C, c = id - j * C;                 // images in ascending order: see launch_apply
     const float mean = __ldg(mean_v + c);
     float invstd = 0.f, gam = 1.f, bet = 0.f;
     if (RELU) {
@@ -469,7 +470,7 @@ grad_stats_kernel(const float *__restrict__ x, const float *__restrict__ gy, flo
     const bool vec = (S % 4 == 0) && ((((uintptr_t)x | (uintptr_t)gy) & 15) == 0);
     const float2 p = vec ? chunk_grad_sums<float4, 4, RELU>(x, gy, N, C, S, c, chunks, j, mean, invstd, gam, bet)
                          : chunk_grad_sums<float, 8, RELU>(x, gy, N, C, S, c, chunks, j, mean, invstd, gam, bet);
-    if ((threadIdx.x & 31) == 0) part[id] = p;
+    if ((threadIdx.x & 31) == 0) part[(size_t)c * chunks + j] = p;
     if (counters && last_warp_of_channel(counters, c, chunks)) {
         finish_grad_channel_warp(part + (size_t)c * chunks, c, chunks, (long long)N * S, weight, bias, mean_v, std_or_var, train, eps_d, scale, grad_weight,
                                  grad_bias, coef);
@@ -486,7 +487,8 @@ grad_apply_kernel(const float *__restrict__ x, const float *__restrict__ gy, flo
     const bool vec = (S % 4 == 0) && ((((uintptr_t)x | (uintptr_t)gy | (uintptr_t)gx) & 15) == 0);
     constexpr int PER_CTA = 256 / GROUP;
     const int sub = (int)threadIdx.x / GROUP, t = (int)threadIdx.x % GROUP;
-    for (long long pl = (long long)blockIdx.x * PER_CTA + sub; pl < planes; pl += (long long)gridDim.x * PER_CTA) {
+    for (long long rev = (long long)blockIdx.x * PER_CTA + sub; rev < planes; rev += (long long)gridDim.x * PER_CTA) {
+        const long long pl = planes - 1 - rev;                   // last image first
         const GradCoef k = coef[pl % C];
         const float *xp = x + pl * S;
         const float *gp = gy + pl * S;
@@ -573,13 +575,14 @@ grad_apply_flat_kernel(const float *__restrict__ x, const float *__restrict__ gy
         for (unsigned u = 0; u < U; ++u) {
             v[u] = zero;
             if (q + u * stride < items) {
-                g[u] = __ldg(g4 + q + u * stride);
-                if (need_x) v[u] = __ldg(x4 + q + u * stride);
+                const unsigned at = items - 1 - (q + u * stride);             // last image first
+                g[u] = __ldg(g4 + at);
+                if (need_x) v[u] = __ldg(x4 + at);
             }
         }
 #pragma unroll
         for (unsigned u = 0; u < U; ++u)
-            if (q + u * stride < items) item(q + u * stride, v[u], g[u]);
+            if (q + u * stride < items) item(items - 1 - (q + u * stride), v[u], g[u]);
     }
     if (tid < total - items * 4u) {
         const unsigned e = items * 4u + tid;
@@ -1113,6 +1116,9 @@ static int flat_grid(unsigned total)
     return (int)std::max(1LL, std::min(ceil_div_ll((long long)(total / 4u), 1024), (long long)sm_count() * 8));
 }
 
+// The sums walk the images in ascending order, so what they read last — up to the 126 MB of L2 — is the end of the tensors: the
+// elementwise passes start there and go backwards (backward pass of 128 x 128 x 56 x 56: 198 -> 187 us, forward 121 -> 118; 128 x 1024 x
+// 7 x 7: 39.0 -> 36.6 us and 35.1 -> 33.3).
 template <bool RELU>
 static void launch_apply(const float *x, float *y, const float *weight, const float *bias, const float *mean_v,
                          const float *std_or_var, int train, float eps, int C, int S, long long planes, cudaStream_t stream)
