@@ -1168,6 +1168,41 @@ static int finalize_plan(Plan &pl)
     return 0;
 }
 
+// The finished plan of a shape on the current device.  Planning scores a few hundred tilings and asks the runtime for the occupancy
+// (about 4 us), as long as a layer of one image runs; a thread keeps its last sixteen plans.  A plan is a function of these numbers alone.
+static bool find_plan(Plan &pl, int mode, int N, int C, int H, int W, int oH, int oW, int S)
+{
+#ifdef CUNN_B200_DEV_HOOKS
+    pl = make_plan(mode, N, C, H, W, oH, oW, S);
+    return pl.ok && finalize_plan(pl) == 0;
+#else
+    struct Entry {
+        int key[9];
+        bool ok;
+        Plan pl;
+    };
+    static thread_local Entry kept[16];
+    static thread_local int used = 0, next = 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    const int key[9] = {mode, N, C, H, W, oH, oW, S, dev};
+    for (int i = 0; i < used; ++i)
+        if (std::equal(key, key + 9, kept[i].key)) {
+            pl = kept[i].pl;
+            return kept[i].ok;
+        }
+    pl = make_plan(mode, N, C, H, W, oH, oW, S);
+    const bool ok = pl.ok && finalize_plan(pl) == 0;
+    Entry &e = kept[next];
+    std::copy(key, key + 9, e.key);
+    e.ok = ok;
+    e.pl = pl;
+    used = std::max(used, next + 1);
+    next = (next + 1) % 16;
+    return ok;
+#endif
+}
+
 static int launch_fast(FastParams &fp, const Plan &pl, cudaStream_t stream, const char *name)
 {
     FastKernel kern = pick_kernel(pl);
@@ -1176,6 +1211,8 @@ static int launch_fast(FastParams &fp, const Plan &pl, cudaStream_t stream, cons
     fp.tiles_base = (int)(pl.tiles / pl.grid);
     fp.tiles_rem = (int)(pl.tiles % pl.grid);
     void *args[] = {(void *)&fp};
+    // another plan of the same kernel may have asked for less since
+    if (pl.smem > 48 * 1024) CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
     // launched as a programmatic dependent of whatever precedes it in the stream: its prologue may overlap
     // the tail of the previous kernel; the kernel itself waits (pdl_wait) before touching global memory
     cudaLaunchConfig_t cfg = {};
@@ -1280,8 +1317,8 @@ extern "C" int cunn_b200_dwconv_forward(const float *x, const float *weight, con
     if (N == 0) return 0;
     CUNN_CHECK_ARG(x && weight && y, "null tensor pointer");
     if (fast_shape(M, kH, kW, dH, dW, padH, padW) && aligned16(x) && aligned16(y)) {
-        Plan pl = make_plan(MODE_FWD, N, C, H, W, oH, oW, dH);
-        if (pl.ok && finalize_plan(pl) == 0) {
+        Plan pl;
+        if (find_plan(pl, MODE_FWD, N, C, H, W, oH, oW, dH)) {
             FastParams fp{};
             fill_params(fp, pl, N, C, H, W, oH, oW);
             fp.in = x; fp.w = weight; fp.bias = bias; fp.out = y;
@@ -1313,16 +1350,16 @@ extern "C" int cunn_b200_dwconv_grad_input(const float *gy, const float *weight,
     if (fast_shape(M, kH, kW, dH, dW, padH, padW) && aligned16(gy) && aligned16(gx)) {
         if (dH == 1) {
             // stride 1: the input gradient is the forward stencil with the kernel rotated by 180 degrees
-            Plan pl = make_plan(MODE_FWD, N, C, oH, oW, H, W, 1);
-            if (pl.ok && finalize_plan(pl) == 0) {
+            Plan pl;
+            if (find_plan(pl, MODE_FWD, N, C, oH, oW, H, W, 1)) {
                 FastParams fp{};
                 fill_params(fp, pl, N, C, oH, oW, H, W);
                 fp.in = gy; fp.w = weight; fp.bias = nullptr; fp.out = gx; fp.flip = 1;
                 return launch_fast(fp, pl, stream, "dwconv grad input (3x3 s1)");
             }
         } else {
-            Plan pl = make_plan(MODE_DGRAD_S2, N, C, H, W, oH, oW, 2);
-            if (pl.ok && finalize_plan(pl) == 0) {
+            Plan pl;
+            if (find_plan(pl, MODE_DGRAD_S2, N, C, H, W, oH, oW, 2)) {
                 FastParams fp{};
                 fill_params(fp, pl, N, C, H, W, oH, oW);
                 fp.in = gy; fp.w = weight; fp.out = gx;
@@ -1351,8 +1388,8 @@ extern "C" size_t cunn_b200_dwconv_acc_grad_workspace(int N, int C, int H, int W
     int oH, oW;
     if (check_common(N, C, H, W, M, kH, kW, dH, dW, padH, padW, &oH, &oW)) return 0;
     if (!fast_shape(M, kH, kW, dH, dW, padH, padW) || N == 0) return 0;
-    Plan pl = make_plan(MODE_WGRAD, N, C, H, W, oH, oW, dH);
-    if (!pl.ok || finalize_plan(pl)) return 0;
+    Plan pl;
+    if (!find_plan(pl, MODE_WGRAD, N, C, H, W, oH, oW, dH)) return 0;
     return wgrad_workspace_bytes(C, pl);
 }
 
@@ -1367,8 +1404,8 @@ extern "C" int cunn_b200_dwconv_acc_grad(const float *x, const float *gy, float 
     if (N == 0) return 0;
     CUNN_CHECK_ARG(x && gy && grad_weight, "null tensor pointer");
     if (fast_shape(M, kH, kW, dH, dW, padH, padW) && aligned16(x) && aligned16(gy)) {
-        Plan pl = make_plan(MODE_WGRAD, N, C, H, W, oH, oW, dH);
-        if (pl.ok && finalize_plan(pl) == 0) {
+        Plan pl;
+        if (find_plan(pl, MODE_WGRAD, N, C, H, W, oH, oW, dH)) {
             FastParams fp{};
             fill_params(fp, pl, N, C, H, W, oH, oW);
             fp.in = x; fp.in2 = gy; fp.w = nullptr; fp.out = nullptr;
@@ -1451,8 +1488,8 @@ extern "C" CUNN_API int cunn_b200_dwconv_acc_grad_static(const float *x, const f
     if (N == 0) return 0;
     CUNN_CHECK_ARG(x && gy && grad_weight, "null tensor pointer");
     if (fast_shape(M, kH, kW, dH, dW, padH, padW) && aligned16(x) && aligned16(gy)) {
-        Plan pl = make_plan(MODE_WGRAD, N, C, H, W, oH, oW, dH);
-        if (pl.ok && finalize_plan(pl) == 0) {
+        Plan pl;
+        if (find_plan(pl, MODE_WGRAD, N, C, H, W, oH, oW, dH)) {
             const size_t need = wgrad_workspace_bytes(C, pl);
             CUNN_CHECK_ARG(need <= kStaticScratchBytes,
                            "dwconv acc_grad (static scratch): this shape needs %zu bytes of scratch, the built-in array "

@@ -4,6 +4,8 @@ Each function mirrors one entry point of include/cunn_b200.h.  torch is used
 for device memory and the current stream only; all arithmetic happens in
 libTHCUNN.so.  Inputs must be contiguous fp32 CUDA tensors.
 """
+import math
+
 import torch
 
 from ._lib import lib, check
@@ -12,7 +14,8 @@ _workspaces = {}
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream (torch.cuda.current_stream().cuda_stream without the Stream object)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _chk(*ts):
@@ -32,7 +35,7 @@ def workspace(nbytes, device, tag="scratch"):
     gradient (tag "dwconv") and batch normalisation (tag "batchnorm") keep ticket counters in their buffers
     that must stay zero between calls, so no other operator may write there; everything else shares the
     "scratch" buffer."""
-    key = (device.index, torch.cuda.current_stream().cuda_stream, tag)
+    key = (device.index, _stream(), tag)
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = torch.zeros(max(int(nbytes), 1 << 20), dtype=torch.uint8, device=device)
@@ -109,11 +112,8 @@ def maxpool_backward(gy, indices, H, W, kH, kW, dH, dW, padH, padW, ceil_mode=Fa
 
 
 def _bn_dims(x):
-    N, C = x.shape[0], x.shape[1]
-    S = 1
-    for d in x.shape[2:]:
-        S *= d
-    return N, C, S
+    N, C, *rest = x.shape
+    return N, C, math.prod(rest)
 
 
 def batchnorm_forward(x, weight, bias, running_mean, running_var, train, momentum=0.1, eps=1e-5, out=None,
@@ -127,10 +127,11 @@ def batchnorm_forward(x, weight, bias, running_mean, running_var, train, momentu
         save_mean = torch.empty(C, dtype=torch.float32, device=x.device)
     if save_std is None:
         save_std = torch.empty(C, dtype=torch.float32, device=x.device)
-    ws = workspace(lib.cunn_b200_batchnorm_workspace(N, C), x.device, "batchnorm")
+    # only the training statistics need scratch memory
+    ws = workspace(lib.cunn_b200_batchnorm_workspace(N, C), x.device, "batchnorm") if train else None
     check(lib.cunn_b200_batchnorm_forward(_ptr(x), _ptr(out), _ptr(weight), _ptr(bias), _ptr(running_mean),
                                           _ptr(running_var), _ptr(save_mean), _ptr(save_std), N, C, S, int(train),
-                                          momentum, eps, _ptr(ws), ws.numel(), _stream()))
+                                          momentum, eps, _ptr(ws), ws.numel() if train else 0, _stream()))
     return out, save_mean, save_std
 
 
@@ -351,10 +352,11 @@ def batchnorm_relu_forward(x, weight, bias, running_mean, running_var, train, mo
         out = torch.empty_like(x)
     save_mean = torch.empty(C, dtype=torch.float32, device=x.device)
     save_std = torch.empty(C, dtype=torch.float32, device=x.device)
-    ws = workspace(lib.cunn_b200_batchnorm_workspace(N, C), x.device, "batchnorm")
+    # only the training statistics need scratch memory
+    ws = workspace(lib.cunn_b200_batchnorm_workspace(N, C), x.device, "batchnorm") if train else None
     check(lib.cunn_b200_batchnorm_relu_forward(_ptr(x), _ptr(out), _ptr(weight), _ptr(bias), _ptr(running_mean),
                                                _ptr(running_var), _ptr(save_mean), _ptr(save_std), N, C, S, int(train),
-                                               momentum, eps, _ptr(ws), ws.numel(), _stream()))
+                                               momentum, eps, _ptr(ws), ws.numel() if train else 0, _stream()))
     return out, save_mean, save_std
 
 
