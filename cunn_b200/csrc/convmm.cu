@@ -777,12 +777,15 @@ struct Loader {
                     a_mask = 15u;
                 }
             } else {
+                // pixels lane + 32 j, as for gathered operands: one copy instruction covers 32 consecutive pixels (four consecutive ones
+                // per lane spread it over 512 bytes, with four-way bank conflicts)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     a_off[j] = 0;
-                    if (m + j < p.M_total) {
-                        const int im = (m + j) / p.HW;
-                        a_off[j] = im * p.Kd * p.HW + (m + j - im * p.HW);
+                    const int mj = m_tile * BM + lane + 32 * j;
+                    if (mj < p.M_total) {
+                        const int im = mj / p.HW;
+                        a_off[j] = im * p.Kd * p.HW + (mj - im * p.HW);
                         a_mask |= 1u << j;
                     }
                 }
@@ -913,7 +916,7 @@ struct Loader {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const bool ok = kok && (a_mask >> j & 1u);
-                        cp_async4(sa + a_so[i] + 4 * j, ok ? p.a + a_off[j] + k * p.HW : p.a, ok);
+                        cp_async4(sa + g_so[i] + MN_ATOM * j, ok ? p.a + a_off[j] + k * p.HW : p.a, ok);
                     }
                 }
             }
@@ -1286,7 +1289,7 @@ pw_gemm_kernel(const Params p)
                 const int j = i - LO_BUFS;
                 if (!mbar_wait(smem_u32(bars + j % RAW_STAGES), (uint32_t)((j / RAW_STAGES) & 1), p.status)) { ok = false; break; }
             }
-            if (KS != 1) __syncwarp();                         // gathered pieces were filled by several lanes of this warp
+            if (KS != 1 || (A_MN && !p.vec_a)) __syncwarp();   // pieces copied element by element were filled by several lanes of this warp
             split_block(rs, lb);
             fence_async_smem();                                // generic-proxy stores -> visible to the tensor core's async proxy
             __syncwarp();
