@@ -92,11 +92,13 @@ __device__ __forceinline__ void stage_planes(const Params &p, float *tile, const
         const bool row_ok = (unsigned)row < (unsigned)h;
         const float *s = src + pl * step + (long long)row * w;
         const uint32_t d = base + (uint32_t)((pl * p.rows + i) * p.ld) * 4u;
-        for (int j = lane; j < p.cols; j += 32) {
-            const int col = col0 + j;
-            const bool ok = row_ok && (unsigned)col < (unsigned)w;
-            const int at = S == 1 ? j : (j & 1) * p.half + (j >> 1);
-            copy4(d + (uint32_t)at * 4u, ok ? s + col : src, ok);
+        // 32 columns further is 32 words further, or 16 of the same parity
+        const float *sj = s + (col0 + lane);
+        uint32_t dj = d + (uint32_t)(S == 1 ? lane : (lane & 1) * p.half + (lane >> 1)) * 4u;
+        unsigned col = (unsigned)(col0 + lane);
+        for (int j = lane; j < p.cols; j += 32, sj += 32, dj += S == 1 ? 128u : 64u, col += 32u) {
+            const bool ok = row_ok && col < (unsigned)w;
+            copy4(dj, ok ? sj : src, ok);
         }
         i += THREADS / 32;
         while (i >= p.rows) { i -= p.rows; ++pl; }
