@@ -1448,6 +1448,8 @@ static PwKernel pw_pick(int bn, int ks = 1)
 static bool gather_applies(int kH, int kW) { return kH * kW <= 32; }
 // Kernels of up to 16 x 16 taps: any number of taps on the weight gradient's loader and on conv_gather.cuh.
 static bool small_kernel(int kH, int kW) { return kH <= pwg::MAX_KERNEL && kW <= pwg::MAX_KERNEL; }
+// The weight gradient's gathering loader takes both kinds.
+static bool gathered_wgrad(int kH, int kW) { return gather_applies(kH, kW) || small_kernel(kH, kW); }
 // loader variant of the gathering path: 3x3 has its own instantiation, everything else (a strided or padded 1x1
 // included) the one with run-time kernel sizes
 static int gather_ks(int kH, int kW) { return (kH == 3 && kW == 3) ? 3 : 0; }
@@ -1906,7 +1908,7 @@ static size_t conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH,
     if (!dilated && stem::applies(C, K, kH, kW)) return stem::wgrad_workspace_bytes();
     if (pw_applies(kH, kW, dH, dW, padH, padW))
         return std::max(wgrad_partial_bytes(C, K, flat_kblocks(N, H * W)), wgrad_partial_bytes(C, K, group_kblocks(N, H * W)));
-    if (small_kernel(kH, kW)) return wgrad_partial_bytes(C * kH * kW, K, flat_kblocks(N, oH * oW));
+    if (gathered_wgrad(kH, kW)) return wgrad_partial_bytes(C * kH * kW, K, flat_kblocks(N, oH * oW));
     int bn, splits, ips, pb;
     wgrad_plan(N, C, K, kH * kW, oH * oW, &bn, &splits, &ips, &pb);
     const int chunks = std::max(1, std::min(N, ceil_div(sm_count() * 4, K)));
@@ -1962,7 +1964,7 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         }
         return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
-    if (small_kernel(kH, kW)) {
+    if (gathered_wgrad(kH, kW)) {
         const int oHW = oH * oW;
         pw_wgrad_plan(C * kk, K, flat_kblocks(N, oHW), &bn, &splits, &kb);
         const long long n = (long long)K * C * kk;

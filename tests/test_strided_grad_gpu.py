@@ -64,3 +64,29 @@ def test_strided_input_gradient_not_finite(F):
     gx = F.convmm_grad_input(gy, w, H, W, 2, 2, 1, 1)
     want = torch.nn.functional.conv_transpose2d(gy.cpu().double(), w.cpu().double(), None, 2, 1)
     assert torch.equal(gx.cpu().double(), want) or torch.allclose(gx.cpu().double(), want, rtol=1e-6, equal_nan=True)
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW: long kernels of up to 32 taps, all passes
+    (2, 3, 5, 60, 7, 1, 32, 1, 1, 0, 5, 1, 1),         # a row of 32 taps
+    (2, 3, 90, 4, 7, 32, 1, 1, 2, 3, 0, 2, 1),         # a dilated column of them, strided across
+    (1, 4, 20, 80, 6, 1, 20, 2, 1, 0, 9, 1, 3),        # a dilated row, more than sixteen columns
+])
+def test_long_kernels(F, ref64, shape):
+    N, C, H, W, K, kH, kW, dH, dW, pH, pW, dilH, dilW = shape
+    rng = np.random.default_rng(abs(hash(shape)) % 99991)
+    oH, oW = (H + 2 * pH - dilH * (kH - 1) - 1) // dH + 1, (W + 2 * pW - dilW * (kW - 1) - 1) // dW + 1
+    x, gy = rng.standard_normal((N, C, H, W)).astype(np.float32), rng.standard_normal((N, K, oH, oW)).astype(np.float32)
+    w, b = rng.uniform(-1, 1, (K, C, kH, kW)).astype(np.float32), rng.uniform(-1, 1, K).astype(np.float32)
+    geo = (dH, dW, pH, pW, dilH, dilW)
+    # the split drops up to 2^-20 of a product and the tensor core truncates its sums: 1e-5 of the largest value, as for the other kernels
+    y = F.dilated_conv_forward(dev(x), dev(w), dev(b), *geo).cpu().numpy()
+    assert norm_err(y, ref64.dilconv_forward(x, w, b, *geo)) <= 1e-5
+    gx = F.dilated_conv_grad_input(dev(gy), dev(w), H, W, *geo).cpu().numpy()
+    assert norm_err(gx, ref64.dilconv_grad_input(gy, w, H, W, *geo)) <= 1e-5
+    gw, gb = np.zeros_like(w), np.zeros(K, np.float32)
+    dgw, dgb = dev(gw), dev(gb)
+    F.dilated_conv_acc_grad(dev(x), dev(gy), dgw, dgb, *geo, 0.75)
+    want = ref64.dilconv_acc_grad(x, gy, gw.copy(), gb.copy(), *geo, 0.75)
+    assert norm_err(dgw.cpu().numpy(), want[0]) <= 1e-5
+    assert norm_err(dgb.cpu().numpy(), want[1]) <= 1e-5
