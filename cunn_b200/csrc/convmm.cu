@@ -14,7 +14,7 @@
 //   * pw::pw_gemm_kernel<OP, BN, KS> — the persistent, warp-specialised kernel (further down): KS = 1 for 1x1
 //     stride-1 convolutions whose operands are plain matrices in memory, KS = 3 / 0 for 3x3 / any kernel of up to
 //     32 taps gathered element by element with asynchronous copies;
-//   * conv_gemm_kernel<OP, KS, BN> (next) — one CTA per 128 x BN tile for kernels of more than 32 taps: all 256
+//   * conv_gemm_kernel<OP, BN> (next) — one CTA per 128 x BN tile for kernels of more than 16 rows or columns: all 256
 //     threads gather operand values (two k-blocks in flight in registers), split them and store 16-byte pieces
 //     into K-major tiles in the 128-byte swizzle; one thread issues the MMAs of the k-block and commits them to
 //     the mbarrier that frees the stage; the epilogue reads the accumulator with tcgen05.ld (lane = tile row)
@@ -159,13 +159,14 @@ __device__ __forceinline__ void store_split(unsigned char *hi_tile, unsigned cha
     *reinterpret_cast<float4 *>(lo_tile + off) = l;
 }
 
-// k index -> (channel, kh, kw).  KS = 1 or 3 makes the divisions compile-time; KS = 0 is generic.
-template <int KS>
+// k index -> (channel, kh, kw).
 __device__ __forceinline__ void split_k(const GemmParams &p, int k, int &c, int &kh, int &kw)
 {
-    if (KS == 1) { c = k; kh = 0; kw = 0; }
-    else if (KS == 3) { c = k / 9; const int r = k - c * 9; kh = r / 3; kw = r - kh * 3; }
-    else { const int kk = p.kH * p.kW; c = k / kk; const int r = k - c * kk; kh = r / p.kW; kw = r - kh * p.kW; }
+    const int kk = p.kH * p.kW;
+    c = k / kk;
+    const int r = k - c * kk;
+    kh = r / p.kW;
+    kw = r - kh * p.kW;
 }
 
 // Row of the gathered image operand: which image, and the top-left corner of its window.
@@ -175,7 +176,6 @@ struct PixRow {
 };
 
 // Four consecutive k values of the gathered operand for one pixel row (zero outside the image / problem).
-template <int KS>
 __device__ __forceinline__ float4 gather_pix_chunk(const GemmParams &p, const PixRow &r, int k0)
 {
     float v[4];
@@ -185,7 +185,7 @@ __device__ __forceinline__ float4 gather_pix_chunk(const GemmParams &p, const Pi
         float x = 0.f;
         if (r.img && k < p.Kd) {
             int c, kh, kw;
-            split_k<KS>(p, k, c, kh, kw);
+            split_k(p, k, c, kh, kw);
             const int ih = r.ih0 + kh, iw = r.iw0 + kw;
             if ((unsigned)ih < (unsigned)p.g_H && (unsigned)iw < (unsigned)p.g_W)
                 x = __ldg(r.img + ((size_t)c * p.g_H + ih) * p.g_W + iw);
@@ -206,7 +206,7 @@ __device__ __forceinline__ float4 rowmajor_chunk(const float *row, int k0, int l
     return make_float4(v[0], v[1], v[2], v[3]);
 }
 
-template <int OP, int KS, int BN>
+template <int OP, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 conv_gemm_kernel(const GemmParams p)
 {
@@ -263,9 +263,7 @@ conv_gemm_kernel(const GemmParams p)
         const int m = m0 + a_row;
         if (m < p.M_total) a_rowptr = p.a_src + (size_t)m * p.pix_HW;   // + img * K * oHW
     }
-    const bool b_vec = (OP == OP_FWD) ? ((p.Kd & 3) == 0 && ((uintptr_t)p.b_src & 15) == 0)
-                                      : (OP == OP_WGRAD && KS == 1 && (p.pix_HW & 3) == 0 && ((uintptr_t)p.b_src & 15) == 0 &&
-                                         p.g_dH == 1 && p.g_dW == 1 && p.g_padH == 0 && p.g_padW == 0);
+    const bool b_vec = OP == OP_FWD && (p.Kd & 3) == 0 && ((uintptr_t)p.b_src & 15) == 0;
     const bool a_vec = OP == OP_WGRAD && (p.pix_HW & 3) == 0 && ((uintptr_t)p.a_src & 15) == 0;
 
     // Loads the pieces of k-block `kb` (CTA-local index) into registers.
@@ -273,7 +271,7 @@ conv_gemm_kernel(const GemmParams p)
         if (OP != OP_WGRAD) {
             const int kbase = kb * BK;
 #pragma unroll
-            for (int i = 0; i < A_PER; ++i) ra[i] = gather_pix_chunk<KS>(p, a_pix, kbase + (a_kc0 + 2 * i) * 4);
+            for (int i = 0; i < A_PER; ++i) ra[i] = gather_pix_chunk(p, a_pix, kbase + (a_kc0 + 2 * i) * 4);
 #pragma unroll
             for (int i = 0; i < B_PER; ++i) {
                 const int q = i * THREADS + tid;
@@ -292,7 +290,7 @@ conv_gemm_kernel(const GemmParams p)
                             float x = 0.f;
                             if (k < p.Kd) {
                                 int ko, kh, kw;
-                                split_k<KS>(p, k, ko, kh, kw);
+                                split_k(p, k, ko, kh, kw);
                                 x = __ldg(p.b_src + (((size_t)ko * p.C + (n0 + row)) * p.kH + (p.kH - 1 - kh)) * p.kW + (p.kW - 1 - kw));
                             }
                             t[j] = x;
@@ -320,25 +318,21 @@ conv_gemm_kernel(const GemmParams p)
                 const int n = n0 + row;
                 if (kc < 8 && n < p.N_total && img_ok) {
                     int c, kh, kw;
-                    split_k<KS>(p, n, c, kh, kw);
+                    split_k(p, n, c, kh, kw);
                     const float *plane = p.b_src + ((size_t)img * p.C + c) * p.g_H * p.g_W;
                     const int k0 = pb * BK + kc * 4;
-                    if (b_vec) {
-                        v = rowmajor_chunk(plane, k0, p.pix_HW, true);
-                    } else {
-                        float t[4];
+                    float t[4];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int pix = k0 + j;
-                            float x = 0.f;
-                            if (pix < p.pix_HW) {
-                                const int ih = pixtab[kb & 1][kc * 4 + j][0] + kh, iw = pixtab[kb & 1][kc * 4 + j][1] + kw;
-                                if ((unsigned)ih < (unsigned)p.g_H && (unsigned)iw < (unsigned)p.g_W) x = __ldg(plane + (size_t)ih * p.g_W + iw);
-                            }
-                            t[j] = x;
+                    for (int j = 0; j < 4; ++j) {
+                        const int pix = k0 + j;
+                        float x = 0.f;
+                        if (pix < p.pix_HW) {
+                            const int ih = pixtab[kb & 1][kc * 4 + j][0] + kh, iw = pixtab[kb & 1][kc * 4 + j][1] + kw;
+                            if ((unsigned)ih < (unsigned)p.g_H && (unsigned)iw < (unsigned)p.g_W) x = __ldg(plane + (size_t)ih * p.g_W + iw);
                         }
-                        v = make_float4(t[0], t[1], t[2], t[3]);
+                        t[j] = x;
                     }
+                    v = make_float4(t[0], t[1], t[2], t[3]);
                 }
                 rb[i] = v;
             }
@@ -1345,22 +1339,14 @@ pw_gemm_kernel(const Params p)
 
 typedef void (*GemmKernel)(const GemmParams);
 
-template <int OP, int KS>
-static GemmKernel pick_bn(int bn)
+template <int OP>
+static GemmKernel pick_kernel(int bn)
 {
     switch (bn) {
-        case 32: return conv_gemm_kernel<OP, KS, 32>;
-        case 64: return conv_gemm_kernel<OP, KS, 64>;
-        case 128: return conv_gemm_kernel<OP, KS, 128>;
-        default: return conv_gemm_kernel<OP, KS, 256>;
+        case 32: return conv_gemm_kernel<OP, 32>;
+        case 64: return conv_gemm_kernel<OP, 64>;
+        default: return conv_gemm_kernel<OP, 128>;
     }
-}
-template <int OP>
-static GemmKernel pick_kernel(int ks, int bn)
-{
-    if (ks == 1) return pick_bn<OP, 1>(bn);
-    if (ks == 3) return pick_bn<OP, 3>(bn);
-    return pick_bn<OP, 0>(bn);
 }
 
 static size_t smem_bytes(int bn)
@@ -1370,13 +1356,7 @@ static size_t smem_bytes(int bn)
     return stage * stages + 1024;   // + alignment slack
 }
 
-static int pick_bn_for(int n_total)
-{
-    if (n_total <= 32) return 32;
-    if (n_total <= 64) return 64;
-    if (n_total <= 128 || n_total % 256 != 0) return 128;
-    return 128;
-}
+static int pick_bn_for(int n_total) { return n_total <= 32 ? 32 : (n_total <= 64 ? 64 : 128); }
 
 static int launch(GemmKernel kern, const GemmParams &p, dim3 grid, int bn, cudaStream_t stream)
 {
@@ -1406,8 +1386,6 @@ static int check(int N, int C, int H, int W, int K, int kH, int kW, int dH, int 
                    "tensors of 2^31 or more elements are not supported");
     return 0;
 }
-
-static int ks_of(int kH, int kW) { return (kH == 1 && kW == 1) ? 1 : (kH == 3 && kW == 3) ? 3 : 0; }
 
 static void wgrad_plan(int N, int C, int K, int kk, int oHW, int *bn, int *splits, int *imgs_per_split, int *pix_blocks)
 {
@@ -1798,7 +1776,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     p.M_total = N * oH * oW; p.N_total = K; p.Kd = C * kH * kW; p.kblocks = ceil_div(p.Kd, BK); p.out_HW = oH * oW;
     const int bn = pick_bn_for(K);
     dim3 grid(ceil_div(p.M_total, BM), ceil_div(K, bn), 1);
-    return launch(pick_kernel<OP_FWD>(ks_of(kH, kW), bn), p, grid, bn, stream);
+    return launch(pick_kernel<OP_FWD>(bn), p, grid, bn, stream);
 }
 
 // `bias` (null: none) is added to every plane of gx: a transposed convolution's forward pass is this one plus its bias.
@@ -1871,7 +1849,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         p.M_total = N * H * W; p.N_total = C; p.Kd = K * kH * kW; p.kblocks = ceil_div(p.Kd, BK); p.out_HW = H * W;
         const int bn = pick_bn_for(C);
         dim3 grid(ceil_div(p.M_total, BM), ceil_div(C, bn), 1);
-        return add_bias(launch(pick_kernel<OP_DGRAD>(ks_of(kH, kW), bn), p, grid, bn, stream));
+        return add_bias(launch(pick_kernel<OP_DGRAD>(bn), p, grid, bn, stream));
     }
     const std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH), aw = axis_phases(W, kW, dW, padW, dilW);
     if (phases_fit(ah) && phases_fit(aw)) return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, ah, aw, oH, oW, stream);
@@ -1988,7 +1966,7 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
     p.M_total = K; p.N_total = C * kk; p.Kd = 0; p.kblocks = ips * pb; p.out_HW = 0;
     p.imgs_per_split = ips; p.pix_blocks = pb;
     dim3 grid(ceil_div(K, BM), ceil_div(C * kk, bn), splits);
-    if (launch(pick_kernel<OP_WGRAD>(ks_of(kH, kW), bn), p, grid, bn, stream)) return 1;
+    if (launch(pick_kernel<OP_WGRAD>(bn), p, grid, bn, stream)) return 1;
     const long long n = (long long)K * C * kk;
     const int rblocks = (int)std::max(1LL, std::min(ceil_div_ll(n, 256), (long long)sm_count() * 8));
     wgrad_reduce_kernel<<<rblocks, 256, 0, stream>>>((const float *)workspace, grad_weight, n, splits, scale);

@@ -198,6 +198,7 @@ def test_convmm_full_size_adjoint_identities(F, cfg):
     (2, 6, 19, 23, 33, 9, 1, 4),         # 81 taps at stride 1: all three passes
     (1, 2, 40, 40, 70, 16, 3, 0),        # 256 taps: the largest kernel of this path
     (1, 2, 40, 40, 6, 17, 3, 0),         # one row more: the kernel for any size
+    (1, 2, 20, 22, 5, 17, 1, 8),         # ... its three passes
     (1, 700, 1, 1, 40, 1, 1, 0),         # a single pixel
     (130, 100, 1, 1, 36, 1, 1, 0),       # fully connected: two row tiles, ragged reduction and columns
     (1, 32, 1, 1, 4, 1, 1, 0),           # ... one image, one k-block
