@@ -416,16 +416,12 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
     if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// Pixels of a phase that no tap reaches: the bias, or zero.
+// Every pixel of every plane: the bias, or zero.
 __global__ void __launch_bounds__(256)
-phase_fill_kernel(float *__restrict__ out, const float *__restrict__ bias, int C, int o_HW, int HW, int pix_W, int o_off, int o_sH,
-                  int o_sW, long long total)
+plane_fill_kernel(float *__restrict__ out, const float *__restrict__ bias, int C, int HW, long long total)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const long long plane = i / HW;
-        const int r = (int)(i - plane * HW), row = r / pix_W, col = r - row * pix_W;
-        out[plane * o_HW + o_off + row * o_sH + col * o_sW] = bias ? __ldg(bias + (int)(plane % C)) : 0.f;
-    }
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
+        out[i] = bias ? __ldg(bias + (int)((i / HW) % C)) : 0.f;
 }
 
 }  // namespace pwg

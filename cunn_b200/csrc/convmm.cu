@@ -26,6 +26,7 @@
 #include "stemconv.h"
 
 #include <algorithm>
+#include <new>
 #include <vector>
 
 namespace cunn {
@@ -1622,7 +1623,8 @@ static int launch_gather(pwg::GatherParams &p, int bn, cudaStream_t stream)
 struct AxisPhase {
     int h0, n, k0, taps, kstep, o0, ostep;
 };
-static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil)
+// Only residues with taps are listed (at most k of them); *gaps is set when there are others.
+static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil, bool *gaps)
 {
     int g = d, r = dil % d;
     while (r) { const int t = g % r; g = r; r = t; }                       // gcd(d, dil)
@@ -1635,7 +1637,8 @@ static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil)
             if (!a.taps) { a.k0 = t; a.o0 = num / d; }
             ++a.taps;
         }
-        out.push_back(a);
+        if (a.taps) out.push_back(a);
+        else *gaps = true;
     }
     return out;
 }
@@ -1650,9 +1653,16 @@ static bool phases_fit(const std::vector<AxisPhase> &v)
 // Input gradient of a convolution with any stride, padding and dilation, plus `bias` per input channel (null: none): the
 // forward pass of a transposed convolution has one.
 static int phased_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
-                             int kH, int kW, int dH, int dW, const std::vector<AxisPhase> &ah, const std::vector<AxisPhase> &aw,
+                             int kH, int kW, int dH, int dW, const std::vector<AxisPhase> &ah, const std::vector<AxisPhase> &aw, bool gaps,
                              int oH, int oW, cudaStream_t stream)
 {
+    if (gaps) {
+        // pixels that no tap reaches: one pass over the tensor however many residues they are
+        const long long total = (long long)N * C * H * W;
+        const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
+        pwg::plane_fill_kernel<<<blocks, 256, 0, stream>>>(gx, bias, C, H * W, total);
+        CUNN_LAUNCH_CHECK("convmm grad input (pixels without taps)");
+    }
     std::vector<pwg::Phase> ph;
     for (const AxisPhase &a : ah)
         for (const AxisPhase &b : aw) {
@@ -1662,15 +1672,8 @@ static int phased_grad_input(const float *gy, const float *weight, const float *
             f.dH = f.dW = 1;
             f.padH = -a.o0; f.padW = -b.o0; f.dilH = -a.ostep; f.dilW = -b.ostep;
             f.w_base = a.k0 * kW + b.k0; f.w_sH = a.kstep * kW; f.w_sW = b.kstep;
-            f.o_off = a.h0 * W + b.h0; f.o_sH = dH * W; f.o_sW = dW;
-            if (f.taps) {
-                ph.push_back(f);
-                continue;
-            }
-            const long long total = (long long)N * C * f.HW;
-            const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 8));
-            pwg::phase_fill_kernel<<<blocks, 256, 0, stream>>>(gx, bias, C, H * W, f.HW, f.pix_W, f.o_off, f.o_sH, f.o_sW, total);
-            CUNN_LAUNCH_CHECK("convmm grad input (pixels without taps)");
+            f.o_off = a.h0 * W + b.h0; f.o_sH = a.n > 1 ? dH * W : 0; f.o_sW = b.n > 1 ? dW : 0;
+            ph.push_back(f);
         }
     // longest reductions first: the persistent grid deals tiles round-robin, so the last wave is made of the short ones
     std::stable_sort(ph.begin(), ph.end(), [](const pwg::Phase &a, const pwg::Phase &b) { return a.taps > b.taps; });
@@ -1851,8 +1854,14 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         dim3 grid(ceil_div(p.M_total, BM), ceil_div(C, bn), 1);
         return add_bias(launch(pick_kernel<OP_DGRAD>(bn), p, grid, bn, stream));
     }
-    const std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH), aw = axis_phases(W, kW, dW, padW, dilW);
-    if (phases_fit(ah) && phases_fit(aw)) return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, ah, aw, oH, oW, stream);
+    try {
+        bool gaps = false;
+        const std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH, &gaps), aw = axis_phases(W, kW, dW, padW, dilW, &gaps);
+        if (phases_fit(ah) && phases_fit(aw))
+            return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, ah, aw, gaps, oH, oW, stream);
+    } catch (const std::bad_alloc &) {
+        return fail("convmm grad input: out of host memory");
+    }
     const long long total = (long long)N * C * H * W;
     const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
     dgrad_gather_kernel<<<blocks, 256, 0, stream>>>(gy, weight, gx, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW, total);

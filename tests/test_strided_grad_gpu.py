@@ -31,6 +31,7 @@ def F():
     (2, 8, 21, 19, 12, 3, 3, 2, 3, 3, 3, 3, 2),        # stride and dilation without a common factor
     (2, 8, 6, 6, 12, 3, 3, 1, 1, 5, 5, 1, 1),          # stride 1, padding beyond the kernel
     (1, 4, 1, 3, 6, 3, 3, 2, 2, 1, 1, 1, 1),           # fewer rows than the stride
+    (1, 5, 90, 70, 6, 1, 2, 40, 33, 0, 0, 1, 1),       # 1320 residues, two of them with taps
     (5, 130, 12, 12, 260, 3, 3, 2, 1, 1, 1, 1, 1),     # strides differ; two column tiles, 25 k-blocks
 ])
 def test_strided_input_gradient(F, ref64, ref32, shape):
