@@ -67,12 +67,16 @@ __device__ __forceinline__ int magic_div(int k, uint32_t magic) { return magic ?
 // 3xTF32 split of a 16-byte piece in place, with rounding: hi = v to 11 bits, lo = v - hi to 11 bits.  Truncating instead (the raw
 // value as hi, as pw::pw_gemm_kernel does it) saves a store, but lo then has the sign of v, and lo * lo and the bits that lo loses add up
 // to -4e-7 of the sum whatever its length; rounded parts lose 2^-24 with either sign.
+// The rounding is an addition to the bits, so it stops short of the values whose bits it would carry over: finite ones within 2^-12 of the
+// largest (they would become infinite), infinities and NaN (0x7fffffff, the NaN that the GPU's own arithmetic makes, would become zero).
+// Those are truncated, and lo of an infinity or a NaN is inf - inf or NaN: every sum that reads one is NaN.
 __device__ __forceinline__ void split_rounded(unsigned char *hi_tile, unsigned char *lo_tile, uint32_t off)
 {
     float4 v = *reinterpret_cast<const float4 *>(hi_tile + off), l;
     auto part = [](float &x, float &lo) {
-        const float h = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
-        lo = __uint_as_float(__float_as_uint(x - h) + 0x1000u);          // the tensor core drops the low 13 bits
+        const uint32_t half = fabsf(x) < 0x1.ffep127f ? 0x1000u : 0u;
+        const float h = __uint_as_float((__float_as_uint(x) + half) & 0xffffe000u);
+        lo = __uint_as_float(__float_as_uint(x - h) + half);             // the tensor core drops the low 13 bits
         x = h;
     };
     part(v.x, l.x); part(v.y, l.y); part(v.z, l.z); part(v.w, l.w);

@@ -91,3 +91,67 @@ def test_long_kernels(F, ref64, shape):
     want = ref64.dilconv_acc_grad(x, gy, gw.copy(), gb.copy(), *geo, 0.75)
     assert norm_err(dgw.cpu().numpy(), want[0]) <= 1e-5
     assert norm_err(dgb.cpu().numpy(), want[1]) <= 1e-5
+
+
+NANS = [0x7fffffff, -1, 0x7fc00000, 0x7f800001]      # what CUDA arithmetic makes of inf - inf, its negative, the host's NaN, the smallest one
+
+
+def with_bits(t, index, bits):
+    import torch
+    t = t.clone()
+    t.view(torch.int32)[index] = bits
+    return t
+
+
+@pytest.mark.parametrize("bits", NANS)
+@pytest.mark.parametrize("where", ["gy", "w"])
+def test_strided_gradient_keeps_every_nan(F, where, bits):
+    """A NaN of any bit pattern reaches the strided input gradient and the transposed forward pass, at the pixels that read it."""
+    import torch
+    rng = torch.Generator(device="cuda").manual_seed(3)
+    gy, w = (torch.randn(*s, device="cuda", generator=rng) for s in ((2, 64, 7, 7), (64, 5, 3, 3)))
+    if where == "gy":
+        gy = with_bits(gy, (1, 40, 2, 3), bits)
+    else:
+        w = with_bits(w, (17, 2, 2, 1), bits)
+    b = torch.randn(5, device="cuda", generator=rng)
+    want = torch.nn.functional.conv_transpose2d(gy.cpu().double(), w.cpu().double(), None, 2, 1)
+    assert int(torch.isnan(want).sum()) > 0 and not torch.isnan(want).all()
+    gx = F.convmm_grad_input(gy, w, 13, 13, 2, 2, 1, 1).cpu().double()
+    assert torch.equal(torch.isnan(gx), torch.isnan(want)) and torch.allclose(gx, want, rtol=1e-4, atol=1e-4, equal_nan=True)
+    y = F.full_conv_forward(gy, w, b, 2, 2, 1, 1).cpu()
+    assert torch.equal(torch.isnan(y), torch.isnan(want))
+
+
+@pytest.mark.parametrize("bits", NANS + [0x7f800000])
+@pytest.mark.parametrize("where", ["x", "w"])
+def test_large_kernel_keeps_what_is_not_finite(F, where, bits):
+    """7x7 forward and stride-1 input gradient: a sum that reads a NaN or an infinity is not finite, every other one is."""
+    import torch
+    rng = torch.Generator(device="cuda").manual_seed(4)
+    x, w = (torch.randn(*s, device="cuda", generator=rng) for s in ((2, 3, 20, 21), (6, 3, 7, 7)))
+    if where == "x":
+        x = with_bits(x, (1, 2, 9, 8), bits)
+    else:
+        w = with_bits(w, (4, 1, 3, 6), bits)
+    want = torch.nn.functional.conv2d(x.cpu().double(), w.cpu().double())
+    y = F.convmm_forward(x, w, None, 1, 1, 0, 0).cpu()
+    assert torch.equal(torch.isfinite(y), torch.isfinite(want)) and not torch.isfinite(y).all()
+    # the same kernel's gradient with every output pixel's taps inside the map: no product that the definition lacks
+    gy = torch.ones(2, 6, 14, 15, device="cuda")
+    if where == "w":
+        want = torch.nn.functional.conv_transpose2d(gy.cpu().double(), w.cpu().double())
+        gx = F.convmm_grad_input(gy, w, 20, 21, 1, 1, 0, 0).cpu().double()
+        assert torch.allclose(gx, want, rtol=1e-4, atol=1e-4, equal_nan=True)
+
+
+def test_largest_finite_values_stay_finite(F):
+    """Rounding the high part of a value next to the largest float must not make it infinite, in either pass."""
+    import torch
+    big = torch.finfo(torch.float32).max
+    x, w = torch.zeros(1, 1, 12, 12, device="cuda"), torch.zeros(1, 1, 7, 7, device="cuda")
+    x[0, 0, 5, 6], w[0, 0, 2, 3] = big, 0.5
+    y = F.convmm_forward(x, w, None, 1, 1, 3, 3)
+    assert y[0, 0, 6, 6].item() == pytest.approx(0.5 * big, rel=2 ** -20) and int((y != 0).sum()) == 1
+    gx = F.convmm_grad_input(x, w, 24, 24, 2, 2, 3, 3)
+    assert gx[0, 0, 9, 12].item() == pytest.approx(0.5 * big, rel=2 ** -20) and int((gx != 0).sum()) == 1
