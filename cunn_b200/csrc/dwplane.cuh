@@ -317,12 +317,49 @@ wgrad_kernel(const __grid_constant__ Params p)
         }
         __syncthreads();                                                    // the tile is read before the next one lands
     }
-    flush();
-    __syncthreads();
-    for (int i = threadIdx.x; i < SUMS; i += THREADS) {
-        double s = 0.0;
-        for (int w = 0; w < THREADS / 32; ++w) s += warp_sums[w][i];
-        cta_sums[i] = s;
+    // The CTA's sums; true if one of the filter's is not finite.
+    auto gather = [&]() {
+        flush();
+        __syncthreads();
+        bool bad = false;
+        for (int i = threadIdx.x; i < SUMS; i += THREADS) {
+            double s = 0.0;
+            for (int w = 0; w < THREADS / 32; ++w) s += warp_sums[w][i];
+            cta_sums[i] = s;
+            bad |= i < KK && !isfinite(s);
+        }
+        return __syncthreads_or(bad) != 0;
+    };
+    if (gather()) {
+        // The staged form also multiplies the padding's zeros by gy and the zeros past the last output by x: an infinity or a NaN there
+        // reaches taps that never read it.  This CTA's share again, product by product.
+        for (int i = threadIdx.x; i < (THREADS / 32) * SUMS; i += THREADS) (&warp_sums[0][0])[i] = 0.0;
+        __syncthreads();
+        chain = 0;
+#pragma unroll 1
+        for (int u = (int)(units * rank / ranks); u < u_end; ++u) {
+            const int band = u % p.bands, n0 = (u / p.bands) * p.P, imgs = min(p.P, p.N - n0), r0 = band * p.R;
+            const int rows = min(p.R, p.oH - r0), items = imgs * rows * p.oW;
+#pragma unroll 1
+            for (int it0 = 0; it0 < items; it0 += THREADS) {
+                if (++chain > kChain) { flush(); chain = 1; }
+                const int it = it0 + (int)threadIdx.x;
+                if (it >= items) continue;
+                const int t2 = it / p.oW, ow = it - t2 * p.oW, pl = t2 / rows, oh = r0 + t2 - pl * rows;
+                const long long n = n0 + pl;
+                const float g = __ldg(p.gy + ((n * p.C + c) * p.M + j) * p.oH * p.oW + (long long)oh * p.oW + ow);
+                const float *xp = p.in + (n * p.C + c) * p.H * p.W;
+                const int ih0 = oh * S - p.padH, iw0 = ow * S - p.padW;
+                acc[KK] += g;
+#pragma unroll
+                for (int kh = 0; kh < K; ++kh)
+#pragma unroll
+                    for (int kw = 0; kw < K; ++kw)
+                        if ((unsigned)(ih0 + kh) < (unsigned)p.H && (unsigned)(iw0 + kw) < (unsigned)p.W)
+                            acc[kh * K + kw] = fmaf(g, __ldg(xp + (long long)(ih0 + kh) * p.W + iw0 + kw), acc[kh * K + kw]);
+            }
+        }
+        gather();
     }
     cluster_sync();
     if (rank == 0) {

@@ -81,3 +81,47 @@ def test_weights_that_are_not_finite_stay_off_the_padding(F, d):
                     if 0 <= h < 9 and 0 <= q < 9:
                         ref[:, h, q] += wd[:, 0, kh, kw]
     assert torch.allclose(gx[0].double(), ref, equal_nan=True)
+
+
+@pytest.mark.parametrize("what", ["inf", "nan", "gpu nan"])
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W, M, k, d, padH, padW
+    (3, 4, 10, 12, 1, 5, 1, 0, 0),       # six rows of outputs: the second strip of four ends in two that do not exist
+    (2, 3, 23, 21, 2, 5, 2, 2, 2),       # rows past the last window, padding on every side
+    (40, 2, 9, 9, 1, 3, 1, 1, 0),        # several ranks
+    (1, 2, 90, 70, 1, 7, 1, 3, 2),       # several bands
+])
+def test_parameter_gradient_not_finite(F, shape, what):
+    """An infinity or a NaN in x or gy reaches exactly the taps whose products read it."""
+    import torch
+    N, C, H, W, M, k, d, pH, pW = shape
+    oH, oW = (H + 2 * pH - k) // d + 1, (W + 2 * pW - k) // d + 1
+    value = {"inf": float("inf"), "nan": float("nan")}.get(what)
+    if value is None:
+        value = torch.full((1,), float("inf"), device="cuda")
+        value = (value - value)[0]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for where in ("x last row", "x inside", "gy corner", "gy inside"):
+        x, gy = torch.randn(N, C, H, W, device="cuda", generator=g), torch.randn(N, C * M, oH, oW, device="cuda", generator=g)
+        if where == "x last row":
+            x[N - 1, C - 1, H - 1, W // 2] = value
+        elif where == "x inside":
+            x[0, 0, H // 2, W // 2] = value
+        elif where == "gy corner":
+            gy[N - 1, C * M - 1, oH - 1, oW - 1] = gy[0, 0, 0, 0] = value
+        else:
+            gy[0, 0, oH // 2, oW // 2] = value
+        gw, gb = torch.zeros(M, C, k, k, device="cuda"), torch.zeros(M, C, device="cuda")
+        F.dwconv_acc_grad(x, gy, gw, gb, d, d, pH, pW)
+        # tap by tap over the windows that are inside the image
+        xd, gd = x.cpu().double(), gy.cpu().double().view(N, C, M, oH, oW)
+        want = torch.zeros(M, C, k, k, dtype=torch.double)
+        for kh in range(k):
+            for kw in range(k):
+                oh = [o for o in range(oH) if 0 <= o * d - pH + kh < H]
+                ow = [o for o in range(oW) if 0 <= o * d - pW + kw < W]
+                if oh and ow:
+                    xs = xd[:, :, [o * d - pH + kh for o in oh]][:, :, :, [o * d - pW + kw for o in ow]]
+                    want[:, :, kh, kw] = (xs[:, :, None] * gd[:, :, :, oh][..., ow]).sum((0, 3, 4)).t()
+        assert torch.allclose(gw.cpu().double(), want, rtol=1e-4, atol=1e-3, equal_nan=True), where
+        assert torch.allclose(gb.cpu().double(), gd.sum((0, 3, 4)).t(), rtol=1e-4, atol=1e-3, equal_nan=True), where
