@@ -223,6 +223,8 @@ __device__ __forceinline__ void drain_block(float (&acc)[COLS], uint32_t taddr, 
 
 // One input-gradient pixel in plain fp32.  The split makes a NaN of an infinity (inf - inf), and 0 * inf of what is left of it, so
 // sums that came out as NaN are taken again this way: what is infinite, and with which sign, then follows from the products.
+// That takes as long as the fp32 form takes (a warp's 32 pixels in step, gy in consecutive words), so it is done after the CTA's last
+// k-block: no warp then waits on a barrier with a limit for this one's arrivals.
 __device__ __forceinline__ float gather_scalar(const GatherParams &p, const Phase &f, int im, int row, int col, int n)
 {
     const int channels = f.Kd / f.taps, kH_n = f.taps / f.kW;
@@ -236,7 +238,7 @@ __device__ __forceinline__ float gather_scalar(const GatherParams &p, const Phas
         for (int tw = 0; tw < f.kW; ++tw) {
             const int iw = col * f.dW - f.padW + tw * f.dilW;
             if ((unsigned)iw >= (unsigned)p.g_W) continue;
-#pragma unroll 1
+#pragma unroll 8
             for (int c = 0; c < channels; ++c)
                 s = fmaf(__ldg(p.b + ((size_t)c * p.N_total + n) * p.w_kk + f.w_base + th * f.w_sH + tw * f.w_sW),
                          __ldg(src + ((size_t)c * p.g_H + ih) * p.g_W + iw), s);
@@ -344,6 +346,17 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
         for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
         int d_tile = (int)blockIdx.x, d_kb = 0, d_phase = 0;                 // the k-block to drain next
         while (d_phase + 1 < p.n_phases && d_tile >= p.ph[d_phase + 1].tile0) ++d_phase;
+        // This lane's pixel of a tile, and the tile's first column for this warp; null: no pixel.
+        auto locate = [&](int tile, const Phase &f, int &n0, int &im, int &row, int &col) -> float * {
+            const int r0 = tile - f.tile0, m_tile = r0 / p.n_tiles, m = m_tile * BM + quarter * 32 + lane;
+            n0 = (r0 - m_tile * p.n_tiles) * BN + cg * COLS;
+            im = m / f.HW;
+            const int r = m - im * f.HW;
+            row = r / f.pix_W;
+            col = r - row * f.pix_W;
+            return m < f.M_total ? p.out + ((size_t)im * p.N_total + n0) * p.o_HW + (f.o_off + row * f.o_sH + col * f.o_sW) : nullptr;
+        };
+        bool nan_seen = false;
         // Adds k-block i's sums (its MMAs are done) to the registers; after a tile's last one, writes the tile.
         auto drain = [&](int i) {
             tc_fence_after();
@@ -351,25 +364,14 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
             tc_fence_before();
             const Phase &f = p.ph[d_phase];
             if (++d_kb < f.kblocks) return;
-            const int r0 = d_tile - f.tile0, m_tile = r0 / p.n_tiles, n0 = (r0 - m_tile * p.n_tiles) * BN + cg * COLS;
-            const int m = m_tile * BM + quarter * 32 + lane;
-            if (m < f.M_total) {
-                const int im = m / f.HW, r = m - im * f.HW, row = r / f.pix_W, col = r - row * f.pix_W;
-                float *dst = p.out + ((size_t)im * p.N_total + n0) * p.o_HW + (f.o_off + row * f.o_sH + col * f.o_sW);
-                bool nan = false;
+            int n0, im, row, col;
+            if (float *dst = locate(d_tile, f, n0, im, row, col)) {
 #pragma unroll
                 for (int j = 0; j < COLS; ++j)
                     if (n0 + j < p.N_total) {
-                        const float v = acc[j] + (p.bias ? __ldg(p.bias + n0 + j) : 0.f);
-                        nan |= v != v;
-                        dst[(size_t)j * p.o_HW] = v;
+                        nan_seen |= acc[j] != acc[j];
+                        dst[(size_t)j * p.o_HW] = acc[j] + (p.bias ? __ldg(p.bias + n0 + j) : 0.f);
                     }
-                if (OP == OP_DGRAD && nan) {
-#pragma unroll 1
-                    for (int j = 0; j < COLS && n0 + j < p.N_total; ++j)
-                        if (isnan(dst[(size_t)j * p.o_HW]))
-                            dst[(size_t)j * p.o_HW] = gather_scalar(p, f, im, row, col, n0 + j) + (p.bias ? __ldg(p.bias + n0 + j) : 0.f);
-                }
             }
             d_kb = 0;
             d_tile += (int)gridDim.x;
@@ -410,10 +412,25 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
             cp_async_commit();
         }
         for (int j = max(0, total_it - LO_BUFS); ok && j < total_it; ++j) {
-            if (!mbar_wait(smem_u32(done + j % RAW_STAGES), (uint32_t)((j / RAW_STAGES) & 1), p.status)) break;
+            if (!mbar_wait(smem_u32(done + j % RAW_STAGES), (uint32_t)((j / RAW_STAGES) & 1), p.status)) { ok = false; break; }
             drain(j);
         }
         cp_async_wait<0>();
+        if (OP == OP_DGRAD && __any_sync(0xffffffffu, ok && nan_seen)) {
+#pragma unroll 1
+            for (int t = (int)blockIdx.x, f_i = 0; t < p.total_tiles; t += (int)gridDim.x) {
+                while (f_i + 1 < p.n_phases && t >= p.ph[f_i + 1].tile0) ++f_i;
+                const Phase &f = p.ph[f_i];
+                int n0, im, row, col;
+                float *dst = locate(t, f, n0, im, row, col);
+                if (!dst) continue;
+#pragma unroll 1
+                for (int j = 0; j < COLS && n0 + j < p.N_total; ++j) {
+                    const float b = p.bias ? __ldg(p.bias + n0 + j) : 0.f;
+                    if (isnan(dst[(size_t)j * p.o_HW]) && !isnan(b)) dst[(size_t)j * p.o_HW] = gather_scalar(p, f, im, row, col, n0 + j) + b;
+                }
+            }
+        }
     }
     tc_fence_before();
     __syncthreads();

@@ -155,3 +155,17 @@ def test_largest_finite_values_stay_finite(F):
     assert y[0, 0, 6, 6].item() == pytest.approx(0.5 * big, rel=2 ** -20) and int((y != 0).sum()) == 1
     gx = F.convmm_grad_input(x, w, 24, 24, 2, 2, 3, 3)
     assert gx[0, 0, 9, 12].item() == pytest.approx(0.5 * big, rel=2 ** -20) and int((gx != 0).sum()) == 1
+
+
+def test_diverged_gradient_of_a_long_reduction(F):
+    """Every sum of a reduction of 73,728 products is infinite or NaN: all are taken again in fp32, outside any wait that has a limit."""
+    import torch
+    from cunn_b200 import device_status
+    K, C, k = 2048, 33, 12
+    gy = torch.full((1, K, 3, 3), float("inf"), device="cuda")
+    w = torch.rand(K, C, k, k, device="cuda") + 0.5
+    w[5, 7, 3, 4] = -1.0                                  # inf - inf for the pixels that read it
+    gx = F.convmm_grad_input(gy, w, 16, 16, 2, 2, 0, 0)
+    want = torch.full((1, C, 16, 16), float("inf"), device="cuda")
+    want[0, 7, 3:9:2, 4:10:2] = float("nan")
+    assert torch.allclose(gx, want, equal_nan=True) and device_status() == 0
