@@ -60,8 +60,8 @@ struct GatherParams {
     Phase ph[MAX_PHASES];
 };
 
-// k / d for k < 2^26 and d <= 256 by multiplication: magic = floor(2^32 / d) + 1, 0 for d = 1.  The error k / 2^32 of the
-// product's fraction stays below 1 / d.
+// k / d for k * d < 2^32 by multiplication: magic = floor(2^32 / d) + 1, 0 for d = 1.  The error k / 2^32 of the product's
+// fraction stays below 1 / d then.  The forward pass has k < 2^24 and d <= 256; input gradients beyond the bound go to phase_fma_kernel.
 __device__ __forceinline__ int magic_div(int k, uint32_t magic) { return magic ? (int)__umulhi((uint32_t)k, magic) : k; }
 
 // 3xTF32 split of a 16-byte piece in place, with rounding: hi = v to 11 bits, lo = v - hi to 11 bits.  Truncating instead (the raw
@@ -435,6 +435,61 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// One residue of an axis of an input gradient: input positions h0 + i * d (i < n) are reached by taps k0 + t * kstep
+// (t < taps) at output positions o0 + i - t * ostep.
+struct AxisPhase {
+    int h0, n, k0, taps, kstep, o0, ostep;
+};
+
+// The same sums in plain fp32, products in the order tap row, tap column, filter: what the tensor-core kernel does not take.
+// blockIdx.y and z are the residues of the rows and columns, blockIdx.x a group of CH channels of blockDim.x of the residue's pixels.
+// A thread reads one value of gy (neighbours in consecutive words) and CH weights (the same ones in a whole warp) for CH products.
+constexpr int CH = 4, MAX_AXIS = 64;
+struct FmaParams {
+    const float *gy, *w, *bias;
+    float *gx;
+    int N, C, H, W, K, kW, kk, dH, dW, oH, oW, groups;
+    AxisPhase rows[MAX_AXIS], cols[MAX_AXIS];
+};
+__global__ void __launch_bounds__(256)
+phase_fma_kernel(const __grid_constant__ FmaParams p)
+{
+    const AxisPhase &a = p.rows[blockIdx.y], &b = p.cols[blockIdx.z];
+    const int part = (int)blockIdx.x / p.groups, n0 = ((int)blockIdx.x - part * p.groups) * CH;
+    const long long m = (long long)part * blockDim.x + threadIdx.x;
+    const int pixels = a.n * b.n;
+    if (m >= (long long)p.N * pixels) return;
+    const int im = (int)(m / pixels), r = (int)(m - (long long)im * pixels), i = r / b.n, j = r - i * b.n;
+    const float *src = p.gy + (size_t)im * p.K * p.oH * p.oW;
+    int plane[CH];                                              // channels past the last repeat it
+#pragma unroll
+    for (int q = 0; q < CH; ++q) plane[q] = min(n0 + q, p.C - 1) * p.kk;
+    float s[CH];
+#pragma unroll
+    for (int q = 0; q < CH; ++q) s[q] = 0.f;
+#pragma unroll 1
+    for (int th = 0; th < a.taps; ++th) {
+        const int oh = a.o0 + i - th * a.ostep;
+        if ((unsigned)oh >= (unsigned)p.oH) continue;
+#pragma unroll 1
+        for (int tw = 0; tw < b.taps; ++tw) {
+            const int ow = b.o0 + j - tw * b.ostep;
+            if ((unsigned)ow >= (unsigned)p.oW) continue;
+            const float *g = src + oh * p.oW + ow, *w = p.w + (a.k0 + th * a.kstep) * p.kW + b.k0 + tw * b.kstep;
+#pragma unroll 4
+            for (int k = 0; k < p.K; ++k, g += p.oH * p.oW, w += (size_t)p.C * p.kk) {
+                const float v = __ldg(g);
+#pragma unroll
+                for (int q = 0; q < CH; ++q) s[q] = fmaf(__ldg(w + plane[q]), v, s[q]);
+            }
+        }
+    }
+    float *dst = p.gx + ((size_t)im * p.C + n0) * p.H * p.W + (size_t)(a.h0 + i * p.dH) * p.W + (b.h0 + j * p.dW);
+#pragma unroll
+    for (int q = 0; q < CH; ++q)
+        if (n0 + q < p.C) dst[(size_t)q * p.H * p.W] = s[q] + (p.bias ? __ldg(p.bias + n0 + q) : 0.f);
 }
 
 // Every pixel of every plane: the bias, or zero.

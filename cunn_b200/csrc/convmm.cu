@@ -581,37 +581,6 @@ add_plane_bias_kernel(float *__restrict__ y, const float *__restrict__ bias, int
         y[i] += __ldg(bias + (int)((i / HW) % Q));
 }
 
-// Input gradient, gather form, one thread per input pixel: residues of more than 16 rows or columns of taps.
-__global__ void __launch_bounds__(256)
-dgrad_gather_kernel(const float *__restrict__ gy, const float *__restrict__ w, float *__restrict__ gx, int C, int H, int W,
-                    int K, int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, int oH, int oW, long long total)
-{
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
-        const int wi = (int)(idx % W);
-        long long t = idx / W;
-        const int h = (int)(t % H);
-        t /= H;
-        const int c = (int)(t % C);
-        const long long n = t / C;
-        float s = 0.f;
-        for (int kh = 0; kh < kH; ++kh) {
-            const int a = h + padH - kh * dilH;
-            if (a < 0 || a % dH) continue;
-            const int oh = a / dH;
-            if (oh >= oH) continue;
-            for (int kw = 0; kw < kW; ++kw) {
-                const int b = wi + padW - kw * dilW;
-                if (b < 0 || b % dW) continue;
-                const int ow = b / dW;
-                if (ow >= oW) continue;
-                for (int k = 0; k < K; ++k)
-                    s = fmaf(__ldg(w + (((size_t)k * C + c) * kH + kh) * kW + kw), __ldg(gy + ((n * K + k) * oH + oh) * (size_t)oW + ow), s);
-            }
-        }
-        gx[idx] = s;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Pointwise convolutions (1x1, stride 1, no padding): persistent kernel
 // ---------------------------------------------------------------------------
@@ -1618,11 +1587,7 @@ static int launch_gather(pwg::GatherParams &p, int bn, cudaStream_t stream)
     return 0;
 }
 
-// One residue of an axis of an input gradient: input positions h0 + i * d (i < n) are reached by taps k0 + t * kstep
-// (t < taps) at output positions o0 + i - t * ostep.
-struct AxisPhase {
-    int h0, n, k0, taps, kstep, o0, ostep;
-};
+using pwg::AxisPhase;
 // Only residues with taps are listed (at most k of them); *gaps is set when there are others.
 static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil, bool *gaps)
 {
@@ -1642,12 +1607,33 @@ static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil,
     }
     return out;
 }
-// Every phase of every axis within the kernel's sixteen rows and columns of taps.
-static bool phases_fit(const std::vector<AxisPhase> &v)
+static int most_taps(const std::vector<AxisPhase> &v)
 {
-    for (const AxisPhase &a : v)
-        if (a.taps > pwg::MAX_KERNEL) return false;
-    return true;
+    int most = 0;
+    for (const AxisPhase &a : v) most = std::max(most, a.taps);
+    return most;
+}
+// The tensor-core kernel's limits: sixteen rows and columns of taps, and a reduction whose index magic_div divides by the taps.
+static bool residue_gemm_takes(int K, int tapsH, int tapsW)
+{
+    const long long taps = (long long)tapsH * tapsW, Kd = ceil_div_ll(K * taps, BK) * BK;
+    return tapsH <= pwg::MAX_KERNEL && tapsW <= pwg::MAX_KERNEL && Kd < (1LL << 31) && Kd * taps < (1LL << 32);
+}
+static int launch_phase_fma(pwg::FmaParams &q, const std::vector<AxisPhase> &ah, const std::vector<AxisPhase> &aw, cudaStream_t stream)
+{
+    q.groups = ceil_div(q.C, pwg::CH);
+    for (size_t at = 0; at < ah.size(); at += pwg::MAX_AXIS)
+        for (size_t bt = 0; bt < aw.size(); bt += pwg::MAX_AXIS) {
+            const int nh = (int)std::min<size_t>(pwg::MAX_AXIS, ah.size() - at), nw = (int)std::min<size_t>(pwg::MAX_AXIS, aw.size() - bt);
+            long long rows = 0, cols = 0;
+            for (int i = 0; i < nh; ++i) { q.rows[i] = ah[at + i]; rows = std::max<long long>(rows, q.rows[i].n); }
+            for (int i = 0; i < nw; ++i) { q.cols[i] = aw[bt + i]; cols = std::max<long long>(cols, q.cols[i].n); }
+            const long long pixels = q.N * rows * cols;
+            const int threads = (int)std::min(256LL, ceil_div_ll(pixels, 32) * 32);
+            pwg::phase_fma_kernel<<<dim3((unsigned)(ceil_div_ll(pixels, threads) * q.groups), nh, nw), threads, 0, stream>>>(q);
+            CUNN_LAUNCH_CHECK("convmm grad input (fp32 residues)");
+        }
+    return 0;
 }
 
 // Input gradient of a convolution with any stride, padding and dilation, plus `bias` per input channel (null: none): the
@@ -1662,6 +1648,12 @@ static int phased_grad_input(const float *gy, const float *weight, const float *
         const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
         pwg::plane_fill_kernel<<<blocks, 256, 0, stream>>>(gx, bias, C, H * W, total);
         CUNN_LAUNCH_CHECK("convmm grad input (pixels without taps)");
+    }
+    if (!residue_gemm_takes(K, most_taps(ah), most_taps(aw))) {
+        pwg::FmaParams q{};
+        q.gy = gy; q.w = weight; q.bias = bias; q.gx = gx;
+        q.N = N; q.C = C; q.H = H; q.W = W; q.K = K; q.kW = kW; q.kk = kH * kW; q.dH = dH; q.dW = dW; q.oH = oH; q.oW = oW;
+        return launch_phase_fma(q, ah, aw, stream);
     }
     std::vector<pwg::Phase> ph;
     for (const AxisPhase &a : ah)
@@ -1857,16 +1849,10 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
     try {
         bool gaps = false;
         const std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH, &gaps), aw = axis_phases(W, kW, dW, padW, dilW, &gaps);
-        if (phases_fit(ah) && phases_fit(aw))
-            return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, ah, aw, gaps, oH, oW, stream);
+        return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, ah, aw, gaps, oH, oW, stream);
     } catch (const std::bad_alloc &) {
         return fail("convmm grad input: out of host memory");
     }
-    const long long total = (long long)N * C * H * W;
-    const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
-    dgrad_gather_kernel<<<blocks, 256, 0, stream>>>(gy, weight, gx, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW, total);
-    CUNN_LAUNCH_CHECK("convmm grad input (gather)");
-    return add_bias(0);
 }
 
 static int reduce_partials(const float *partial, float *gw, long long n, int splits, float scale, const float *bias_part, float *gb, int K,

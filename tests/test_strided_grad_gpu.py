@@ -169,3 +169,30 @@ def test_diverged_gradient_of_a_long_reduction(F):
     want = torch.full((1, C, 16, 16), float("inf"), device="cuda")
     want[0, 7, 3:9:2, 4:10:2] = float("nan")
     assert torch.allclose(gx, want, equal_nan=True) and device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W, K, k, d, pad: reductions and residues that the tensor-core kernel does not take
+    (1, 1, 16, 16, 65540, 16, 1, 0),     # 256 taps of 65,540 filters: an index that cannot be divided by multiplication
+    (2, 5, 40, 37, 6, 35, 2, 3),         # residues of 18 and 17 rows of taps
+    (1, 9, 21, 19, 3, 17, 1, 17),        # stride 1, padding of the kernel size
+    (2, 2, 300, 290, 4, 150, 130, 40),   # more residues than one launch lists, two rows of taps in some
+])
+def test_residues_in_fp32(F, shape):
+    import torch
+    N, C, H, W, K, k, d, p = shape
+    oH, oW = (H + 2 * p - k) // d + 1, (W + 2 * p - k) // d + 1
+    g = torch.Generator().manual_seed(6)
+    gy, w, b = torch.randn(N, K, oH, oW, generator=g), torch.rand(K, C, k, k, generator=g) * 2 - 1, torch.rand(C, generator=g)
+    adj = (H - ((oH - 1) * d - 2 * p + k), W - ((oW - 1) * d - 2 * p + k))
+    want = torch.zeros(N, C, H + 2 * p + k, W + 2 * p + k, dtype=torch.double)
+    for kh in range(k):
+        for kw in range(k):
+            want[:, :, kh:kh + (oH - 1) * d + 1:d, kw:kw + (oW - 1) * d + 1:d] += torch.einsum("nkhw,kc->nchw", gy.double(), w[:, :, kh, kw].double())
+    want = want[:, :, p:p + H, p:p + W]
+    gx = F.convmm_grad_input(dev(gy.numpy()), dev(w.numpy()), H, W, d, d, p, p).cpu().double()
+    # a chain of n fp32 additions of products: n 2^-24 of the sum of magnitudes at most; sqrt(n) 2^-24 of the largest value is met in practice
+    n = K * (-(-k // d)) ** 2
+    assert norm_err(gx.numpy(), want.numpy()) <= 4 * n ** 0.5 * 2.0 ** -24 + 2e-7
+    y = F.full_conv_forward(dev(gy.numpy()), dev(w.numpy()), dev(b.numpy()), d, d, p, p, 1, 1, *adj).cpu()
+    assert torch.equal(y, (gx.float() + b.view(1, -1, 1, 1)))
