@@ -443,7 +443,12 @@ struct AxisPhase {
     int h0, n, k0, taps, kstep, o0, ostep;
 };
 
-// The same sums in plain fp32, products in the order tap row, tap column, filter: what the tensor-core kernel does not take.
+// Sums of fewer products are taken in fp32.  The split and the truncation of a k-block's chain cost 8e-8 to 1.2e-7 of a sum however
+// short it is, a chain of n fp32 FMAs about 1.8e-8 sqrt(n + 1): 7.4e-8 (fp32) and 9.3e-8 (tensor cores) at 16 products, 1.15e-7 and
+// 1.19e-7 at 40, 1.27e-7 and 1.17e-7 at 48, 2.0e-7 and 1.3e-7 at 128 (2-norm, normal gy, weights of either sign).
+constexpr int SHORT_SUM = 48;
+
+// The same sums in plain fp32, products in the order tap row, tap column, filter: short ones, and what the tensor-core kernel does not take.
 // blockIdx.y and z are the residues of the rows and columns, blockIdx.x a group of CH channels of blockDim.x of the residue's pixels.
 // A thread reads one value of gy (neighbours in consecutive words) and CH weights (the same ones in a whole warp) for CH products.
 constexpr int CH = 4, MAX_AXIS = 64;
@@ -451,12 +456,14 @@ struct FmaParams {
     const float *gy, *w, *bias;
     float *gx;
     int N, C, H, W, K, kW, kk, dH, dW, oH, oW, groups;
+    int only_short;                                             // leave residues of SHORT_SUM products or more alone
     AxisPhase rows[MAX_AXIS], cols[MAX_AXIS];
 };
 __global__ void __launch_bounds__(256)
 phase_fma_kernel(const __grid_constant__ FmaParams p)
 {
     const AxisPhase &a = p.rows[blockIdx.y], &b = p.cols[blockIdx.z];
+    if (p.only_short && (long long)p.K * a.taps * b.taps >= SHORT_SUM) return;
     const int part = (int)blockIdx.x / p.groups, n0 = ((int)blockIdx.x - part * p.groups) * CH;
     const long long m = (long long)part * blockDim.x + threadIdx.x;
     const int pixels = a.n * b.n;

@@ -1588,8 +1588,8 @@ static int launch_gather(pwg::GatherParams &p, int bn, cudaStream_t stream)
 }
 
 using pwg::AxisPhase;
-// Only residues with taps are listed (at most k of them); *gaps is set when there are others.
-static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil, bool *gaps)
+// Residues without taps are listed if `all`; *gaps is set when there are any.
+static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil, bool all, bool *gaps)
 {
     int g = d, r = dil % d;
     while (r) { const int t = g % r; g = r; r = t; }                       // gcd(d, dil)
@@ -1602,8 +1602,8 @@ static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil,
             if (!a.taps) { a.k0 = t; a.o0 = num / d; }
             ++a.taps;
         }
-        if (a.taps) out.push_back(a);
-        else *gaps = true;
+        if (a.taps || all) out.push_back(a);
+        if (!a.taps) *gaps = true;
     }
     return out;
 }
@@ -1639,25 +1639,39 @@ static int launch_phase_fma(pwg::FmaParams &q, const std::vector<AxisPhase> &ah,
 // Input gradient of a convolution with any stride, padding and dilation, plus `bias` per input channel (null: none): the
 // forward pass of a transposed convolution has one.
 static int phased_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
-                             int kH, int kW, int dH, int dW, const std::vector<AxisPhase> &ah, const std::vector<AxisPhase> &aw, bool gaps,
-                             int oH, int oW, cudaStream_t stream)
+                             int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, int oH, int oW, cudaStream_t stream)
 {
-    if (gaps) {
+    bool gaps = false;
+    std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH, false, &gaps), aw = axis_phases(W, kW, dW, padW, dilW, false, &gaps);
+    const int mostH = most_taps(ah), mostW = most_taps(aw);
+    // residues whose sums are short are taken in fp32, and all of them where the tensor-core kernel cannot take the longest
+    const bool all_fma = !residue_gemm_takes(K, mostH, mostW) || (long long)K * mostH * mostW < pwg::SHORT_SUM;
+    bool any_fma = all_fma;
+    for (const AxisPhase &a : ah)
+        for (const AxisPhase &b : aw) any_fma |= (long long)K * a.taps * b.taps < pwg::SHORT_SUM;
+    if (gaps && all_fma && std::min(dH, H) <= pwg::MAX_AXIS && std::min(dW, W) <= pwg::MAX_AXIS) {
+        // one launch writes every residue
+        ah = axis_phases(H, kH, dH, padH, dilH, true, &gaps);
+        aw = axis_phases(W, kW, dW, padW, dilW, true, &gaps);
+    } else if (gaps) {
         // pixels that no tap reaches: one pass over the tensor however many residues they are
         const long long total = (long long)N * C * H * W;
         const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
         pwg::plane_fill_kernel<<<blocks, 256, 0, stream>>>(gx, bias, C, H * W, total);
         CUNN_LAUNCH_CHECK("convmm grad input (pixels without taps)");
     }
-    if (!residue_gemm_takes(K, most_taps(ah), most_taps(aw))) {
+    if (any_fma) {
         pwg::FmaParams q{};
         q.gy = gy; q.w = weight; q.bias = bias; q.gx = gx;
         q.N = N; q.C = C; q.H = H; q.W = W; q.K = K; q.kW = kW; q.kk = kH * kW; q.dH = dH; q.dW = dW; q.oH = oH; q.oW = oW;
-        return launch_phase_fma(q, ah, aw, stream);
+        q.only_short = !all_fma;
+        const int rc = launch_phase_fma(q, ah, aw, stream);
+        if (rc || all_fma) return rc;
     }
     std::vector<pwg::Phase> ph;
     for (const AxisPhase &a : ah)
         for (const AxisPhase &b : aw) {
+            if ((long long)K * a.taps * b.taps < pwg::SHORT_SUM) continue;
             pwg::Phase f{};
             f.HW = a.n * b.n; f.pix_W = b.n; f.M_total = N * f.HW;
             f.taps = a.taps * b.taps; f.kW = b.taps; f.Kd = K * f.taps;
@@ -1847,9 +1861,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         return add_bias(launch(pick_kernel<OP_DGRAD>(bn), p, grid, bn, stream));
     }
     try {
-        bool gaps = false;
-        const std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH, &gaps), aw = axis_phases(W, kW, dW, padW, dilW, &gaps);
-        return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, ah, aw, gaps, oH, oW, stream);
+        return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW, stream);
     } catch (const std::bad_alloc &) {
         return fail("convmm grad input: out of host memory");
     }

@@ -196,3 +196,35 @@ def test_residues_in_fp32(F, shape):
     assert norm_err(gx.numpy(), want.numpy()) <= 4 * n ** 0.5 * 2.0 ** -24 + 2e-7
     y = F.full_conv_forward(dev(gy.numpy()), dev(w.numpy()), dev(b.numpy()), d, d, p, p, 1, 1, *adj).cpu()
     assert torch.equal(y, (gx.float() + b.view(1, -1, 1, 1)))
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, K, H, k, d, pad: sums of 1 to 47 products (fp32), of 48 and more (tensor cores), and calls that have both
+    (2, 9, 1, 13, 1, 2, 0), (2, 6, 47, 12, 1, 2, 0), (2, 6, 48, 12, 1, 2, 0), (1, 7, 5, 11, 1, 70, 0), (2, 35, 11, 14, 4, 2, 1), (2, 35, 12, 14, 4, 2, 1),
+    (1, 40, 23, 15, 3, 2, 1), (1, 40, 24, 15, 3, 2, 1), (2, 33, 46, 15, 3, 2, 1), (4, 64, 16, 28, 3, 2, 1),
+])
+def test_short_sums_lose_no_bits(F, shape):
+    """2-norm of the error of strided input gradients against that of a chain of fp32 FMAs, one product after the other."""
+    import torch
+    N, C, K, H, k, d, p = shape
+    o = (H + 2 * p - k) // d + 1
+    g = torch.Generator(device="cuda").manual_seed(K)
+    gy, w = torch.randn(N, K, o, o, device="cuda", generator=g), torch.rand(K, C, k, k, device="cuda", generator=g) * 2 - 1
+    span = (o - 1) * d + k
+    # fma(a, b, c) by rounding the exact 64-bit product and sum: 24 + 24 bits fit, the sum rounds once more at 53
+    chain = torch.zeros(N, C, max(span, H + 2 * p), max(span, H + 2 * p), device="cuda")
+    exact = chain.double()
+    for kh in range(k):
+        for kw in range(k):
+            at = (slice(None), slice(None), slice(kh, kh + (o - 1) * d + 1, d), slice(kw, kw + (o - 1) * d + 1, d))
+            for i in range(K):
+                term = gy[:, i:i + 1].double() * w[i, :, kh, kw].double().view(1, C, 1, 1)
+                exact[at] += term
+                chain[at] = (chain[at].double() + term).float()
+    exact, chain = exact[:, :, p:p + H, p:p + H], chain[:, :, p:p + H, p:p + H]
+    gx = F.convmm_grad_input(gy, w, H, H, d, d, p, p)
+    err = lambda t: float((t.double() - exact).norm() / exact.norm())
+    if K * (-(-k // d)) ** 2 < 48:
+        assert torch.equal(gx, chain)
+    # above the limit the tensor cores' error is the smaller one on average; a tenth covers the scatter of one draw
+    assert err(gx) <= 1.1 * err(chain)
