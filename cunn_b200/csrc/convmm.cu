@@ -26,6 +26,7 @@
 #include "stemconv.h"
 
 #include <algorithm>
+#include <cmath>
 #include <new>
 #include <vector>
 
@@ -1595,12 +1596,15 @@ static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil,
     while (r) { const int t = g % r; g = r; r = t; }                       // gcd(d, dil)
     std::vector<AxisPhase> out;
     for (int h0 = 0; h0 < std::min(d, H); ++h0) {
-        AxisPhase a{h0, (H - h0 + d - 1) / d, 0, 0, d / g, 0, dil / g};
-        for (int t = 0; t < k; ++t) {
-            const int num = h0 + pad - t * dil;
-            if (num % d) continue;
-            if (!a.taps) { a.k0 = t; a.o0 = num / d; }
-            ++a.taps;
+        // the first of its taps is below d / g, the others follow d / g apart
+        const int step = d / g;
+        int first = dil == 1 ? (h0 + pad) % d : 0;
+        while (first < step && first < k && (h0 + pad - first * dil) % d) ++first;
+        AxisPhase a{h0, (H - h0 + d - 1) / d, 0, 0, step, 0, dil / g};
+        if (first < step && first < k) {
+            a.k0 = first;
+            a.taps = (k - first - 1) / step + 1;
+            a.o0 = (h0 + pad - first * dil) / d;
         }
         if (a.taps || all) out.push_back(a);
         if (!a.taps) *gaps = true;
@@ -1636,6 +1640,30 @@ static int launch_phase_fma(pwg::FmaParams &q, const std::vector<AxisPhase> &ah,
     return 0;
 }
 
+// Kernels as long as their stride (patch embeddings) have a residue per tap, with few pixels each: sixteen of them are one launch of the
+// residue GEMM, which lasts as long as its longest tile however few of its 128 rows are pixels, and ones of three channels fill a
+// tenth of the columns.  Estimates in us, from 500 layers of 1 to 64 images: 2.1 per k-block of the longest tile or 2.2 per k-block and SM,
+// and 8 for the rest of a launch; the fp32 kernel takes 2.6 products per ps once it is full.  Input gradient of 3 filters of 64 x 64 on
+// one 64 x 64 image, fp32 residues / residue GEMM / every tap scanned: 5 / 2640 / 125 us; 45 x 3 x 224 x 224, 358 filters of 16 x 16:
+// 0.92 / 2.4 / 40.5 ms; 3 x 61 x 196 x 196, 378 filters of 14 x 14: 0.87 / 0.61 / 43.8 ms.
+static bool fp32_residues_are_faster(int N, int C, int K, const std::vector<AxisPhase> &ah, const std::vector<AxisPhase> &aw)
+{
+    if (ah.size() * aw.size() <= (size_t)pwg::MAX_PHASES) return false;
+    double products = 0, tile_kblocks = 0, longest = 0, rows = 0;
+    for (const AxisPhase &a : ah)
+        for (const AxisPhase &b : aw) {
+            const double m = (double)N * a.n * b.n, kd = (double)K * a.taps * b.taps, kb = std::ceil(kd / BK);
+            products += m * kd * C;
+            tile_kblocks += std::ceil(m / BM) * kb;
+            longest = std::max(longest, kb);
+            rows += m;
+        }
+    const double launches = std::ceil((double)(ah.size() * aw.size()) / pwg::MAX_PHASES);
+    const int bn = pw_bn_for(C, (long long)(rows / launches));
+    const double gemm = launches * (8.0 + std::max(2.1 * longest, tile_kblocks / launches * ceil_div(C, bn) * 2.2 / sm_count()));
+    return 4.0 + products / 2.6e6 < gemm;
+}
+
 // Input gradient of a convolution with any stride, padding and dilation, plus `bias` per input channel (null: none): the
 // forward pass of a transposed convolution has one.
 static int phased_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
@@ -1644,8 +1672,9 @@ static int phased_grad_input(const float *gy, const float *weight, const float *
     bool gaps = false;
     std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH, false, &gaps), aw = axis_phases(W, kW, dW, padW, dilW, false, &gaps);
     const int mostH = most_taps(ah), mostW = most_taps(aw);
-    // residues whose sums are short are taken in fp32, and all of them where the tensor-core kernel cannot take the longest
-    const bool all_fma = !residue_gemm_takes(K, mostH, mostW) || (long long)K * mostH * mostW < pwg::SHORT_SUM;
+    // residues whose sums are short are taken in fp32, and all of them where the tensor-core kernel cannot take the longest or is slower
+    const bool all_fma = !residue_gemm_takes(K, mostH, mostW) || (long long)K * mostH * mostW < pwg::SHORT_SUM ||
+                         fp32_residues_are_faster(N, C, K, ah, aw);
     bool any_fma = all_fma;
     for (const AxisPhase &a : ah)
         for (const AxisPhase &b : aw) any_fma |= (long long)K * a.taps * b.taps < pwg::SHORT_SUM;

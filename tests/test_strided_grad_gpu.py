@@ -177,6 +177,8 @@ def test_diverged_gradient_of_a_long_reduction(F):
     (2, 5, 40, 37, 6, 35, 2, 3),         # residues of 18 and 17 rows of taps
     (1, 9, 21, 19, 3, 17, 1, 17),        # stride 1, padding of the kernel size
     (2, 2, 300, 290, 4, 150, 130, 40),   # more residues than one launch lists, two rows of taps in some
+    (2, 3, 64, 64, 50, 64, 64, 0),       # a residue per tap, two pixels each, on the fp32 side of the rule
+    (3, 61, 196, 196, 90, 14, 14, 0),    # ... and on the tensor cores' side
 ])
 def test_residues_in_fp32(F, shape):
     import torch
