@@ -64,26 +64,6 @@ struct GatherParams {
 // fraction stays below 1 / d then.  The forward pass has k < 2^24 and d <= 256; input gradients beyond the bound go to phase_fma_kernel.
 __device__ __forceinline__ int magic_div(int k, uint32_t magic) { return magic ? (int)__umulhi((uint32_t)k, magic) : k; }
 
-// 3xTF32 split of a 16-byte piece in place, with rounding: hi = v to 11 bits, lo = v - hi to 11 bits.  Truncating instead (the raw
-// value as hi, as pw::pw_gemm_kernel does it) saves a store, but lo then has the sign of v, and lo * lo and the bits that lo loses add up
-// to -4e-7 of the sum whatever its length; rounded parts lose 2^-24 with either sign.
-// The rounding is an addition to the bits, so it stops short of the values whose bits it would carry over: finite ones within 2^-12 of the
-// largest (they would become infinite), infinities and NaN (0x7fffffff, the NaN that the GPU's own arithmetic makes, would become zero).
-// Those are truncated, and lo of an infinity or a NaN is inf - inf or NaN: every sum that reads one is NaN.
-__device__ __forceinline__ void split_rounded(unsigned char *hi_tile, unsigned char *lo_tile, uint32_t off)
-{
-    float4 v = *reinterpret_cast<const float4 *>(hi_tile + off), l;
-    auto part = [](float &x, float &lo) {
-        const uint32_t half = fabsf(x) < 0x1.ffep127f ? 0x1000u : 0u;
-        const float h = __uint_as_float((__float_as_uint(x) + half) & 0xffffe000u);
-        lo = __uint_as_float(__float_as_uint(x - h) + half);             // the tensor core drops the low 13 bits
-        x = h;
-    };
-    part(v.x, l.x); part(v.y, l.y); part(v.z, l.z); part(v.w, l.w);
-    *reinterpret_cast<float4 *>(hi_tile + off) = v;
-    *reinterpret_cast<float4 *>(lo_tile + off) = l;
-}
-
 template <int OP, int BN>
 struct GatherLoader {
     int tile, kb, phase, KB;
@@ -221,8 +201,8 @@ __device__ __forceinline__ void drain_block(float (&acc)[COLS], uint32_t taddr, 
     }
 }
 
-// One input-gradient pixel in plain fp32.  The split makes a NaN of an infinity (inf - inf), and 0 * inf of what is left of it, so
-// sums that came out as NaN are taken again this way: what is infinite, and with which sign, then follows from the products.
+// One input-gradient pixel in plain fp32.  The parts of infinities, and the zeros in place of taps outside gy, form products that are
+// NaN where the definition has none, so sums that came out as NaN are taken again this way.
 // That takes as long as the fp32 form takes (a warp's 32 pixels in step, gy in consecutive words), so it is done after the CTA's last
 // k-block: no warp then waits on a barrier with a limit for this one's arrivals.
 __device__ __forceinline__ float gather_scalar(const GatherParams &p, const Phase &f, int im, int row, int col, int n)
@@ -392,9 +372,9 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
             unsigned char *a_lo = lo_base + (size_t)lb * 2 * TILE, *b_lo = a_lo + TILE;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                split_rounded(a_hi, a_lo, mn_so[h]);
+                split_rounded(a_hi, a_lo, mn_so[h], *reinterpret_cast<const float4 *>(a_hi + mn_so[h]));
                 const bool b_on = B_MN ? lane * 4 < BN : (tid >> 3) + 64 * h < BN;
-                if (b_on) split_rounded(b_hi, b_lo, b_so[h]);
+                if (b_on) split_rounded(b_hi, b_lo, b_so[h], *reinterpret_cast<const float4 *>(b_hi + b_so[h]));
             }
             fence_async_smem();                                // generic-proxy stores -> visible to the tensor core's async proxy
             __syncwarp();

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cmath>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 namespace cunn {
@@ -644,6 +645,26 @@ __device__ __forceinline__ void store_lo_at(unsigned char *lo_tile, uint32_t off
 {
     *reinterpret_cast<float4 *>(lo_tile + off) = make_float4(lo_part(v.x), lo_part(v.y), lo_part(v.z), lo_part(v.w));
 }
+// 3xTF32 split of a 16-byte piece in place, with rounding: hi = v to 11 bits, lo = v - hi to 11 bits.  Truncating instead (the raw
+// value as hi, as store_lo_at does it) saves a store, but lo then has the sign of v, and lo * lo and the bits that lo loses add up
+// to -4e-7 of the sum whatever its length; rounded parts lose 2^-24 with either sign.
+// The rounding is an addition to the bits, so it stops short of the values whose bits it would carry over: finite ones within 2^-12 of the
+// largest (they would become infinite), infinities and NaN (0x7fffffff, the NaN that the GPU's own arithmetic makes, would become zero).
+// A piece that may hold one is truncated; lo of an infinity or a NaN is inf - inf or NaN then, and every sum that reads one is NaN.
+// (cvt.rna.tf32 for both parts, or a branch instead of the select, made a 7x7 layer's forward pass 5 and 6 % slower.)
+__device__ __forceinline__ void split_rounded(unsigned char *hi_tile, unsigned char *lo_tile, uint32_t off, float4 v)
+{
+    const uint32_t half = (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w)) < 0x1.ffep127f ? 0x1000u : 0u;
+    float4 l;
+    auto part = [&](float &x, float &lo) {
+        const float h = __uint_as_float((__float_as_uint(x) + half) & 0xffffe000u);
+        lo = __uint_as_float(__float_as_uint(x - h) + half);             // the tensor core drops the low 13 bits
+        x = h;
+    };
+    part(v.x, l.x); part(v.y, l.y); part(v.z, l.z); part(v.w, l.w);
+    *reinterpret_cast<float4 *>(hi_tile + off) = v;
+    *reinterpret_cast<float4 *>(lo_tile + off) = l;
+}
 __device__ __forceinline__ uint64_t desc_of(uint32_t addr, uint32_t lbo, uint32_t sbo)
 {
     return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
@@ -963,10 +984,12 @@ struct Loader {
     }
 };
 
-template <int OP, int BN, int KS>
+// ROUND (weight gradients): split_rounded instead of the truncating split, bias sums in fp64; see rounds_wgrad.
+template <int OP, int BN, int KS, bool ROUND = false>
 __global__ void __launch_bounds__(THREADS, 1)
 pw_gemm_kernel(const Params p)
 {
+    using BiasSum = typename std::conditional<ROUND, double, float>::type;
     constexpr bool A_MN = OP != OP_WGRAD;     // A is M-major (forward, input gradient)
     constexpr bool B_MN = OP == OP_DGRAD;     // B is N-major (input gradient)
     constexpr int ACC_COLS = BN < 32 ? 32 : BN;
@@ -1025,7 +1048,7 @@ pw_gemm_kernel(const Params p)
         g_so[i] = (uint32_t)((k >> 2) * MN_KATOM + (k & 3) * 128 + (((lane >> 3) ^ (k & 3)) << 5) + (((lane >> 2) & 1) << 4) + (lane & 3) * 4);
     }
 
-    float bsum[2] = {0.f, 0.f};                         // WGRAD: running row sums of gy (bias gradient)
+    BiasSum bsum[2] = {0, 0};                           // WGRAD: running row sums of gy (bias gradient)
     unsigned char *const lo_base = smem + (size_t)RAW_STAGES * 2 * TILE;
     // Splits this thread's own pieces of raw stage `rs` (its copies have landed): the raw tile is the hi tile,
     // lo goes to the same offset of lo buffer `lb`.
@@ -1035,11 +1058,13 @@ pw_gemm_kernel(const Params p)
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float4 va = *reinterpret_cast<const float4 *>(a_hi + a_so[i]);
-            store_lo_at(a_lo, a_so[i], va);
-            if (OP == OP_WGRAD) bsum[i] += (va.x + va.y) + (va.z + va.w);
+            if (ROUND) split_rounded(a_hi, a_lo, a_so[i], va);
+            else store_lo_at(a_lo, a_so[i], va);
+            if (OP == OP_WGRAD) bsum[i] += (BiasSum)((va.x + va.y) + (va.z + va.w));
             if (b_store[i]) {
                 const float4 vb = *reinterpret_cast<const float4 *>(b_hi + b_so[i]);
-                store_lo_at(b_lo, b_so[i], vb);
+                if (ROUND) split_rounded(b_hi, b_lo, b_so[i], vb);
+                else store_lo_at(b_lo, b_so[i], vb);
             }
         }
     };
@@ -1275,15 +1300,15 @@ pw_gemm_kernel(const Params p)
                     // bias gradient: the eight chunk lanes of a row hold its partial sums
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
-                        float sum = bsum[r];
+                        BiasSum sum = bsum[r];
                         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
                         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
                         sum += __shfl_xor_sync(0xffffffffu, sum, 4);
                         const int split = c_tile / p.tiles_per_split, r2 = c_tile - split * p.tiles_per_split;
                         const int m_tile = r2 / p.n_tiles, n_tile = r2 - m_tile * p.n_tiles;
                         const int m = m_tile * BM + (tid >> 3) + 64 * r;
-                        if (p.bias_part && n_tile == 0 && (tid & 7) == 0 && m < p.M_total) p.bias_part[(size_t)m * p.splits + split] = sum;
-                        bsum[r] = 0.f;
+                        if (p.bias_part && n_tile == 0 && (tid & 7) == 0 && m < p.M_total) p.bias_part[(size_t)m * p.splits + split] = (float)sum;
+                        bsum[r] = 0;
                     }
                 }
                 c_kb = 0;
@@ -1377,13 +1402,13 @@ static bool pw_applies(int kH, int kW, int dH, int dW, int padH, int padW)
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 typedef void (*PwKernel)(const pw::Params);
-template <int OP, int KS>
+template <int OP, int KS, bool ROUND = false>
 static PwKernel pw_pick_bn(int bn)
 {
     switch (bn) {
-        case 32: return pw::pw_gemm_kernel<OP, 32, KS>;
-        case 64: return pw::pw_gemm_kernel<OP, 64, KS>;
-        default: return pw::pw_gemm_kernel<OP, 128, KS>;
+        case 32: return pw::pw_gemm_kernel<OP, 32, KS, ROUND>;
+        case 64: return pw::pw_gemm_kernel<OP, 64, KS, ROUND>;
+        default: return pw::pw_gemm_kernel<OP, 128, KS, ROUND>;
     }
 }
 template <int OP>
@@ -1393,6 +1418,8 @@ static PwKernel pw_pick(int bn, int ks = 1)
     if (ks == 3) return pw_pick_bn<OP, 3>(bn);
     return pw_pick_bn<OP, 0>(bn);
 }
+// With rounding, 3x3 kernels take the loader for any size: they are short reductions.
+static PwKernel pw_pick_rounded(int bn, int ks) { return ks == 1 ? pw_pick_bn<OP_WGRAD, 1, true>(bn) : pw_pick_bn<OP_WGRAD, 0, true>(bn); }
 // Kernels of up to 32 taps run on the same persistent kernel with a gathering loader.
 static bool gather_applies(int kH, int kW) { return kH * kW <= 32; }
 // Kernels of up to 16 x 16 taps: any number of taps on the weight gradient's loader and on conv_gather.cuh.
@@ -1422,9 +1449,13 @@ static int pw_bn_for(int n_total, long long rows)
 // Accumulators per tile and accumulator sets: the hi*hi products of the k-blocks are dealt round-robin to `nacc - 1`
 // accumulators to keep the tensor core's truncating accumulation chains short, the cross terms share the last one; two sets (epilogue overlapped with the next tile) when
 // they fit in the 512 TMEM columns.
-static void pw_accumulators(int bn, int kblocks, int *nacc, int *sets, bool wgrad = false)
+static void pw_accumulators(int bn, int kblocks, int *nacc, int *sets, bool wgrad = false, int tiles = 0)
 {
-    if (bn == 128 && wgrad) {
+    if (wgrad && tiles <= sm_count()) {
+        // a CTA's only tile has nothing to overlap with: all columns for short chains
+        *nacc = std::min(8, 512 / std::max(bn, 32));
+        *sets = 1;
+    } else if (bn == 128 && wgrad) {
         // sums over pixels of random-sign products cancel: the weight gradient is the pass most sensitive to the
         // accumulation chains, and its long k loops make the epilogue a small share anyway
         if (kblocks <= 8) { *nacc = 2; *sets = 2; }
@@ -1487,17 +1518,17 @@ static bool tma_applies(const void *a, const void *b, const void *c, int HW, int
     return g_use_tma && HW % 4 == 0 && C % 4 == 0 && aligned16(a) && aligned16(b) && aligned16(c) && encode_tiled() != nullptr;
 }
 // Accumulator plan of the tensor-map kernels: tiles of one or two k-blocks put all products into one accumulator and
-// use up to four accumulator sets, so that the MMA warp runs several tiles ahead of the epilogue warps; longer tiles
-// follow pw_accumulators.
-static void tma_accumulators(int bn, int kblocks, int *nacc, int *sets, bool wgrad = false)
+// use up to four accumulator sets, so that the MMA warp runs several tiles ahead of the epilogue warps; longer tiles, and
+// weight gradients with a tile per CTA, follow pw_accumulators.
+static void tma_accumulators(int bn, int kblocks, int *nacc, int *sets, bool wgrad = false, int tiles = 0)
 {
     const int cols = std::max(bn, 32);
-    if (kblocks <= 2) {
+    if (kblocks <= 2 && !(wgrad && tiles <= sm_count())) {
         *nacc = 1;
         *sets = std::min((int)pwt::MAX_SETS, 512 / cols);
         return;
     }
-    pw_accumulators(bn, kblocks, nacc, sets, wgrad);
+    pw_accumulators(bn, kblocks, nacc, sets, wgrad, tiles);
 }
 typedef void (*PwTmaKernel)(const pw::Params, const CUtensorMap, const CUtensorMap, const CUtensorMap);
 // 4 splitter + 8 epilogue warps for every tile length: measured against 8 + 4 and 16 + 4 on tiles of 8, 16 and 32 k-blocks,
@@ -1545,6 +1576,11 @@ static void pw_wgrad_plan(int C, int K, long long kb_total, int *bn, int *splits
         if (best < 0.0 || cost < best * 0.999) { best = cost; *splits = (int)used; *kb_per_split = (int)kb; }
     }
 }
+// Weight gradients whose operands are split with rounding.  Without it those of kernels of more than 32 taps were 4.2e-7 off for short
+// reductions (1.3e-7 with it; 1.4e-7 on the one-CTA-per-tile kernel they came from), for 8 to 11 % of their time.  Reductions of up to 64
+// k-blocks are split below the image, where the truncating split's error and a chain's add up (fully connected layers 3.8e-7 -> 4.3e-7, 1.2e-7
+// with rounding); their launches wait for memory, and the extra stores cost nothing.
+static bool rounds_wgrad(int kk, long long kb_total) { return kk > 32 || kb_total <= 64; }
 // k-blocks of a reduction over N images of HW pixels: flat (element copies), or whole groups of 32 per image (tensor maps).
 static long long flat_kblocks(int N, int HW) { return ceil_div_ll((long long)N * HW, BK); }
 static long long group_kblocks(int N, int HW) { return (long long)N * ceil_div(HW, BK); }
@@ -1752,7 +1788,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         const int bn = pw_bn_for(K, N);
         q.n_tiles = ceil_div(K, bn); q.tiles_per_split = q.total_tiles = ceil_div(N, BM) * q.n_tiles;
         q.n_img = 1; q.splits = 1;
-        tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
+        tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
         alignas(64) CUtensorMap ma, mb;
         if (make_map(&ma, x, C, N, 1, 32, BM, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
         if (make_map(&mb, weight, C, K, 1, 32, bn, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
@@ -1968,13 +2004,13 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         if (tma) {
             alignas(64) CUtensorMap ma, mb;
             q.gpi = ceil_div(q.HW, 32);
-            tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
+            tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
             if (make_map(&ma, gy, q.HW, K, N, 32, BM, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
             if (make_map(&mb, x, q.HW, C, N, 32, bn, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
             if (pw_tma_launch(pw_tma_pick<OP_WGRAD>(bn), q, ma, mb, ma, stream)) return 1;
         } else {
-            pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
-            if (pw_launch(pw_pick<OP_WGRAD>(bn), q, stream)) return 1;
+            pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
+            if (pw_launch(rounds_wgrad(1, flat_kblocks(N, H * W)) ? pw_pick_rounded(bn, 1) : pw_pick<OP_WGRAD>(bn), q, stream)) return 1;
         }
         return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
@@ -1990,8 +2026,9 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         q.n_tiles = ceil_div(C * kk, bn); q.tiles_per_split = ceil_div(K, BM) * q.n_tiles; q.total_tiles = q.tiles_per_split * splits;
         q.n_img = N; q.splits = splits;
         q.vec_a = (oHW % 4 == 0) && aligned16(gy); q.vec_b = 0;
-        pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true);
-        if (pw_launch(pw_pick<OP_WGRAD>(bn, gather_ks(kH, kW)), q, stream)) return 1;
+        pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
+        const int ks = gather_ks(kH, kW);
+        if (pw_launch(rounds_wgrad(kk, flat_kblocks(N, oHW)) ? pw_pick_rounded(bn, ks) : pw_pick<OP_WGRAD>(bn, ks), q, stream)) return 1;
         return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
     wgrad_plan(N, C, K, kk, oH * oW, &bn, &splits, &ips, &pb);

@@ -211,3 +211,29 @@ def test_convmm_split_reductions_and_large_kernels(F, ref64, shape):
     N, C, H, W, K, k, d, pad = shape
     case = make_case(abs(hash(shape)) % 99991, N, C, H, W, K, k, d, pad, True)
     check_against_oracle(ref64, F, *case, d, pad, 0.75)
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, K, k, d, pad: weight gradients split with rounding
+    (2, 3, 16, 12, 7, 2, 3),             # 49 taps, 128 pixels
+    (13, 3, 16, 18, 11, 4, 5),           # 121 taps
+    (64, 136, 1, 184, 1, 1, 0),          # a fully connected layer
+    (7, 60, 9, 33, 1, 1, 0),             # 567 pixels of unaligned planes
+    (6, 3, 16, 112, 5, 4, 2),            # three k-blocks
+    (5, 20, 13, 40, 3, 1, 1),            # 3x3
+])
+def test_weight_gradient_of_short_reductions(F, shape):
+    import torch
+    N, C, H, K, k, d, p = shape
+    o = (H + 2 * p - k) // d + 1
+    g = torch.Generator(device="cuda").manual_seed(8)
+    x, gy = torch.randn(N, C, H, H, device="cuda", generator=g), torch.randn(N, K, o, o, device="cuda", generator=g)
+    cols = torch.nn.functional.unfold(x.double(), k, padding=p, stride=d)
+    want = torch.einsum("nkp,ncp->kc", gy.double().view(N, K, -1), cols).view(K, C, k, k)
+    gw, gb = torch.zeros(K, C, k, k, device="cuda"), torch.zeros(K, device="cuda")
+    F.convmm_acc_grad(x, gy, gw, gb, d, d, p, p)
+    # 2-norm: 0.76e-7 from parts of 11 rounded bits without lo * lo (normal values), and a chain's truncations of 2^-24 on average, at
+    # most twelve of them at the size of the sum: 2.5e-7 holds both.  Truncated parts alone are 3.5e-7 off.
+    assert float((gw.double() - want).norm() / want.norm()) <= 2.5e-7
+    b = gy.double().sum((0, 2, 3))
+    assert float((gb.double() - b).norm() / b.norm()) <= 2.0 ** -23        # a rounding or two of 32 bits
