@@ -1555,41 +1555,67 @@ static int pw_tma_launch(PwTmaKernel kern, pw::Params &p, CUtensorMap &ma, CUten
     return 0;
 }
 
-// Splits of the weight gradient's reduction on the persistent kernels: a tile sums `kb_per_split` of the `kb_total` k-blocks of all
-// images.  Candidates fill one to sixteen waves of the persistent grid (and one to four splits, when one already fills it); they are
-// scored by waves x k-blocks per tile — the time of the slowest CTA, plus about six k-blocks for a tile's prologue and its 64 KB of
-// partial sums — and by what the reduction reads; tiles longer than ~128 k-blocks are avoided when a shorter choice exists
-// (accumulation chains).  Splits end anywhere in an image: with whole images per split, 48 of 148 SMs had work at
-// 12 x 144 x 37 x 29 -> 200 and 64 at 32 x 3 x 224 x 224, 7x7.
-static void pw_wgrad_plan(int C, int K, long long kb_total, int *bn, int *splits, int *kb_per_split)
+// k-blocks of a reduction over N images of HW pixels: flat (element copies), or whole groups of 32 per image (tensor maps).
+static long long wgrad_kblocks(int N, int HW, bool groups)
 {
-    *bn = pw_bn_for(C);
-    const long long tiles_mn = (long long)ceil_div(K, BM) * ceil_div(C, *bn);
-    const int grid = sm_count();
-    double best = -1.0;
-    for (int i = 1; i <= 20; ++i) {
-        const long long want = i <= 16 ? (long long)i * grid / tiles_mn : i - 16;
-        const long long kb = ceil_div_ll(kb_total, std::max(1LL, std::min(want, kb_total))), used = ceil_div_ll(kb_total, kb);
-        const long long waves = ceil_div_ll(tiles_mn * used, grid);
-        double cost = (double)waves * ((double)kb + 6.0) + (double)used * K * C * 4.0 / 8e6;     // a k-block lasts as long as 8 MB of L2 reads
-        if (kb > 128) cost *= 1.0 + 0.25 * (double)(kb - 128) / 128.0;
-        if (best < 0.0 || cost < best * 0.999) { best = cost; *splits = (int)used; *kb_per_split = (int)kb; }
-    }
+    return groups ? (long long)N * ceil_div(HW, BK) : ceil_div_ll((long long)N * HW, BK);
 }
 // Weight gradients whose operands are split with rounding.  Without it those of kernels of more than 32 taps were 4.2e-7 off for short
 // reductions (1.3e-7 with it; 1.4e-7 on the one-CTA-per-tile kernel they came from), for 8 to 11 % of their time.  Reductions of up to 64
 // k-blocks are split below the image, where the truncating split's error and a chain's add up (fully connected layers 3.8e-7 -> 4.3e-7, 1.2e-7
 // with rounding); their launches wait for memory, and the extra stores cost nothing.
-static bool rounds_wgrad(int kk, long long kb_total) { return kk > 32 || kb_total <= 64; }
-// k-blocks of a reduction over N images of HW pixels: flat (element copies), or whole groups of 32 per image (tensor maps).
-static long long flat_kblocks(int N, int HW) { return ceil_div_ll((long long)N * HW, BK); }
-static long long group_kblocks(int N, int HW) { return (long long)N * ceil_div(HW, BK); }
-// Workspace for the partial sums of `splits` splits and their bias sums.
-static size_t wgrad_partial_bytes(int C, int K, long long kb_total)
+static bool rounds_wgrad(int kk, int N, int HW) { return kk > 32 || wgrad_kblocks(N, HW, false) <= 64; }
+// k-blocks whose large products meet in one accumulator of a tile: the error of a weight gradient grows with them.
+static int wgrad_chain(int bn, long long kb, long long tiles)
+{
+    int nacc, sets;
+    pw_accumulators(bn, (int)kb, &nacc, &sets, true, (int)std::min<long long>(tiles, 1 << 30));
+    return (int)ceil_div_ll(kb, nacc - 1);
+}
+// Splits of the weight gradient's reduction on the persistent kernels: a tile sums `kb_per_split` of the k-blocks of all images.
+// Candidates fill one to sixteen waves of the persistent grid (and one to four splits, when one already fills it); they are
+// scored by waves x k-blocks per tile — the time of the slowest CTA, plus about six k-blocks for a tile's prologue and its 64 KB of
+// partial sums — and by what the reduction reads.  Splits end anywhere in an image: with whole images per split, 48 of 148 SMs had work at
+// 12 x 144 x 37 x 29 -> 200 and 64 at 32 x 3 x 224 x 224, 7x7.
+// The best split into whole images (tiles longer than 128 k-blocks avoided) bounds the accumulation chains: none is longer than its.  Of 4,000
+// layers drawn over 16 to 1024 channels a tenth had longer ones without that bound (37 x 64 x 17 x 17, 4x4: 1.2e-6 off, 7.6e-7 with
+// it), which is worth 0.4 % of the scored time.
+static void pw_wgrad_plan(int C, int K, int kk, int N, int HW, bool groups, int *bn, int *splits, int *kb_per_split)
+{
+    C *= kk;
+    *bn = pw_bn_for(C);
+    const long long tiles_mn = (long long)ceil_div(K, BM) * ceil_div(C, *bn), kb_total = wgrad_kblocks(N, HW, groups);
+    const int grid = sm_count();
+    auto score = [&](long long kb, long long used) {
+        const double cost = (double)ceil_div_ll(tiles_mn * used, grid) * ((double)kb + 6.0);
+        return kb > 128 ? cost * (1.0 + 0.25 * (double)(kb - 128) / 128.0) : cost;
+    };
+    long long whole = kb_total;                                             // k-blocks of a tile of whole images
+    if (!rounds_wgrad(kk, N, HW)) {
+        double best = -1.0;
+        for (int images = 1; images <= N; ++images) {
+            const long long used = ceil_div(N, images);
+            const double cost = score((long long)images * ceil_div(HW, BK), used);
+            if (best < 0.0 || cost < best * 0.999) { best = cost; whole = wgrad_kblocks(images, HW, groups); }
+            if (tiles_mn * used <= grid) break;                             // one wave: more images a tile only make it longer
+        }
+    }
+    const int chain = wgrad_chain(*bn, whole, 1LL << 30);
+    double best = -1.0;
+    for (int i = 0; i <= 20; ++i) {
+        const long long want = i <= 16 ? (long long)i * grid / tiles_mn : i - 16;
+        const long long kb = i ? ceil_div_ll(kb_total, std::max(1LL, std::min(want, kb_total))) : whole, used = ceil_div_ll(kb_total, kb);
+        if (i && !rounds_wgrad(kk, N, HW) && wgrad_chain(*bn, kb, tiles_mn * used) > chain) continue;
+        const double cost = score(kb, used) + (double)used * K * C * 4.0 / 8e6;                   // a k-block lasts as long as 8 MB of L2 reads
+        if (best < 0.0 || cost < best * 0.999) { best = cost; *splits = (int)used; *kb_per_split = (int)kb; }
+    }
+}
+// Workspace for the partial sums of the splits and their bias sums.
+static size_t wgrad_partial_bytes(int C, int K, int kk, int N, int HW, bool groups)
 {
     int bn, splits, kb;
-    pw_wgrad_plan(C, K, kb_total, &bn, &splits, &kb);
-    return (size_t)splits * K * C * sizeof(float) + (size_t)K * splits * sizeof(float) + 256;
+    pw_wgrad_plan(C, K, kk, N, HW, groups, &bn, &splits, &kb);
+    return (size_t)splits * K * C * kk * sizeof(float) + (size_t)K * splits * sizeof(float) + 256;
 }
 
 // ---- gathered operand, register accumulation (conv_gather.cuh) -------------------------------------------------------
@@ -1957,8 +1983,8 @@ static size_t conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH,
     const bool dilated = dilH != 1 || dilW != 1;
     if (!dilated && stem::applies(C, K, kH, kW)) return stem::wgrad_workspace_bytes();
     if (pw_applies(kH, kW, dH, dW, padH, padW))
-        return std::max(wgrad_partial_bytes(C, K, flat_kblocks(N, H * W)), wgrad_partial_bytes(C, K, group_kblocks(N, H * W)));
-    if (gathered_wgrad(kH, kW)) return wgrad_partial_bytes(C * kH * kW, K, flat_kblocks(N, oH * oW));
+        return std::max(wgrad_partial_bytes(C, K, 1, N, H * W, false), wgrad_partial_bytes(C, K, 1, N, H * W, true));
+    if (gathered_wgrad(kH, kW)) return wgrad_partial_bytes(C, K, kH * kW, N, oH * oW, false);
     int bn, splits, ips, pb;
     wgrad_plan(N, C, K, kH * kW, oH * oW, &bn, &splits, &ips, &pb);
     const int chunks = std::max(1, std::min(N, ceil_div(sm_count() * 4, K)));
@@ -1992,7 +2018,7 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
     }
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         const bool tma = tma_applies(gy, x, workspace, H * W, 4);
-        pw_wgrad_plan(C, K, tma ? group_kblocks(N, H * W) : flat_kblocks(N, H * W), &bn, &splits, &kb);
+        pw_wgrad_plan(C, K, 1, N, H * W, tma, &bn, &splits, &kb);
         const long long n = (long long)K * C;
         pw::Params q{};
         q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr();
@@ -2010,13 +2036,13 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
             if (pw_tma_launch(pw_tma_pick<OP_WGRAD>(bn), q, ma, mb, ma, stream)) return 1;
         } else {
             pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
-            if (pw_launch(rounds_wgrad(1, flat_kblocks(N, H * W)) ? pw_pick_rounded(bn, 1) : pw_pick<OP_WGRAD>(bn), q, stream)) return 1;
+            if (pw_launch(rounds_wgrad(1, N, H * W) ? pw_pick_rounded(bn, 1) : pw_pick<OP_WGRAD>(bn), q, stream)) return 1;
         }
         return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
     if (gathered_wgrad(kH, kW)) {
         const int oHW = oH * oW;
-        pw_wgrad_plan(C * kk, K, flat_kblocks(N, oHW), &bn, &splits, &kb);
+        pw_wgrad_plan(C, K, kk, N, oHW, false, &bn, &splits, &kb);
         const long long n = (long long)K * C * kk;
         pw::Params q{};
         q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr();
@@ -2028,7 +2054,7 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         q.vec_a = (oHW % 4 == 0) && aligned16(gy); q.vec_b = 0;
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
         const int ks = gather_ks(kH, kW);
-        if (pw_launch(rounds_wgrad(kk, flat_kblocks(N, oHW)) ? pw_pick_rounded(bn, ks) : pw_pick<OP_WGRAD>(bn, ks), q, stream)) return 1;
+        if (pw_launch(rounds_wgrad(kk, N, oHW) ? pw_pick_rounded(bn, ks) : pw_pick<OP_WGRAD>(bn, ks), q, stream)) return 1;
         return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
     wgrad_plan(N, C, K, kk, oH * oW, &bn, &splits, &ips, &pb);

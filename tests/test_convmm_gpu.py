@@ -237,3 +237,18 @@ def test_weight_gradient_of_short_reductions(F, shape):
     assert float((gw.double() - want).norm() / want.norm()) <= 2.5e-7
     b = gy.double().sum((0, 2, 3))
     assert float((gb.double() - b).norm() / b.norm()) <= 2.0 ** -23        # a rounding or two of 32 bits
+
+
+def test_weight_gradient_chains_stay_short(F):
+    """37 images of 64 x 17 x 17 against 120 x 34 x 34, 4x4 stride 2: 335 k-blocks, split so that an accumulator takes no more of them
+    than with whole images per tile."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x, gy = torch.randn(37, 120, 34, 34, device="cuda", generator=g), torch.randn(37, 64, 17, 17, device="cuda", generator=g)
+    cols = torch.nn.functional.unfold(x.double(), 4, padding=1, stride=2)
+    want = torch.einsum("nkp,ncp->kc", gy.double().view(37, 64, -1), cols).view(64, 120, 4, 4)
+    gw = torch.zeros(64, 120, 4, 4, device="cuda")
+    F.convmm_acc_grad(x, gy, gw, None, 2, 2, 1, 1)
+    # truncated operands 3.5e-7; an accumulator's n truncations of about 2^-24 / 1.4 at two thirds of the sum: 16 a tile of 10 or 19
+    # k-blocks over three accumulators, n = 28 at most -> 8e-7 with half a factor for their growth; one of 38 has n = 52 -> 1.2e-6
+    assert float((gw.double() - want).norm() / want.norm()) <= 1e-6
