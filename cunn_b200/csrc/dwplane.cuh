@@ -10,9 +10,11 @@
 //   forward      a tile is P consecutive planes of one image, or a band of rows of one plane
 //   input grad   in padded coordinates h + pad = S q + a: gx[S q + a][S r + b] = sum_{t,u} w[a + S t][b + S u] gy[q - t][r - u];
 //                a thread takes TH consecutive q of one r and writes their S * S residues, so no product with a zero is formed
-//   param grad   a cluster of up to eight CTAs per filter shares the images; every thread keeps the k * k + 1 sums of its strips in
-//                registers for at most kChain terms, then they go through fp64: across the warp, the CTA, the cluster and onto the
-//                gradient.  The order is fixed, so results do not depend on timing.
+//   param grad   a cluster of up to eight CTAs per filter shares the images; every thread keeps the k * k sums of its strips in
+//                registers for at most kChain terms, then they go through fp64: across the warp (WarpSums), the CTA, the cluster and
+//                onto the gradient; the bias sum is fp64 throughout.  The order is fixed, so results do not depend on timing.  Over 40 layers of
+//                16 to 600 channels the error is that of the kernel for any shape, which has fp64 across threads and images: 3.5e-8 to
+//                6e-8 against 3.5e-8 to 1.2e-7 (2-norm; chains of 32 terms: 4.3e-8 to 1.1e-7).
 //
 // Forward / input gradient / parameter gradient on a cold cache, in us: 32 x 96 x 57 x 43, 5x5 stride 2: 671 in all before,
 // 36 / 33 / 57 now (38 MB a pass: 6 us); 12 x 144 x 37 x 29, 3x3 stride 1 (rows of an odd length): 15 / 17 / 34.  What is left is
@@ -25,7 +27,7 @@ constexpr int TH = 4;                        // outputs (forward, parameter grad
 constexpr int THREADS = 256;
 constexpr int kTileFloats = 6144;            // staged floats per tile to aim at: 24 KB, so that several CTAs share an SM
 constexpr int kMaxFloats = 11264;            // ... and the most a tile may take (44 KB)
-constexpr int kChain = 32;                   // fp32 terms per sum before it goes through fp64
+constexpr int kChain = 8;                    // fp32 terms per sum before it goes through fp64
 
 struct Params {
     const float *in, *gy, *w, *bias;         // forward, parameter gradient: in = x; input gradient: in = gy
@@ -257,30 +259,76 @@ dgrad_kernel(const __grid_constant__ Params p)
     }
 }
 
+// Sums over a warp of SUMS values per lane, added up in fp64.  Each of the five steps halves the values as well as the lanes that they
+// still have to meet: a lane passes on half of its values and keeps the other half, so that SUMS = 25 takes 46 shuffles (250 for a
+// butterfly per value) and every lane ends up with a sum or two of its own.
+template <int SUMS>
+struct WarpSums {
+    static constexpr int P = SUMS <= 16 ? 16 : (SUMS <= 32 ? 32 : 64), KEEP = P > 32 ? 2 : 1;
+    double mine[KEEP];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int q = 0; q < KEEP; ++q) mine[q] = 0.0;
+    }
+    __device__ __forceinline__ void add(float (&acc)[SUMS])
+    {
+        const int lane = threadIdx.x & 31;
+        double v[P / 2];
+#pragma unroll
+        for (int i = 0; i < P / 2; ++i) {
+            const float a = i < SUMS ? acc[i < SUMS ? i : 0] : 0.f, b = i + P / 2 < SUMS ? acc[i + P / 2 < SUMS ? i + P / 2 : 0] : 0.f;
+            v[i] = (double)(lane & 16 ? b : a) + (double)__shfl_xor_sync(0xffffffffu, lane & 16 ? a : b, 16);
+        }
+        int count = P / 2;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) {
+            if (count > KEEP) {
+                count /= 2;
+#pragma unroll
+                for (int i = 0; i < P / 4; ++i)
+                    if (i < count) {
+                        const double a = v[i], b = v[i + count];
+                        v[i] = (lane & o ? b : a) + __shfl_xor_sync(0xffffffffu, lane & o ? a : b, o);
+                    }
+            } else {
+#pragma unroll
+                for (int q = 0; q < KEEP; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < KEEP; ++q) mine[q] += v[q];
+#pragma unroll
+        for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
+    }
+    __device__ __forceinline__ void store(double *dst) const
+    {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int q = 0; q < KEEP; ++q) {
+            const int i = P == 16 ? lane >> 1 : KEEP * lane + q;
+            if (i < SUMS) dst[i] = mine[q];
+        }
+    }
+};
+
 template <int K, int S>
 __global__ void __launch_bounds__(THREADS, K == 7 ? 2 : 3)
 wgrad_kernel(const __grid_constant__ Params p)
 {
-    constexpr int KK = K * K, SUMS = KK + 1;
+    constexpr int KK = K * K, SUMS = KK + 1;                                // the taps and the bias
     extern __shared__ __align__(16) float tile[];
     __shared__ double warp_sums[THREADS / 32][SUMS];
     __shared__ double cta_sums[SUMS];
     const int rank = cluster_rank(), ranks = cluster_size();
     const int jc = (int)blockIdx.x / ranks, j = jc / p.C, c = jc - j * p.C;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < (THREADS / 32) * SUMS; i += THREADS) (&warp_sums[0][0])[i] = 0.0;
-    __syncthreads();
-    float acc[SUMS];
+    const int warp = threadIdx.x >> 5;
+    WarpSums<KK> sums;
+    sums.clear();
+    float acc[KK];
 #pragma unroll
-    for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
-    auto flush = [&]() {
-#pragma unroll
-        for (int i = 0; i < SUMS; ++i) {
-            const double s = warp_sum((double)acc[i]);
-            if (lane == 0) warp_sums[warp][i] += s;
-            acc[i] = 0.f;
-        }
-    };
+    for (int i = 0; i < KK; ++i) acc[i] = 0.f;
+    double bias = 0.0;
     int chain = 0;
     const long long units = (long long)p.groups * p.bands;                  // (image group, band)
     const int u_end = (int)(units * (rank + 1) / ranks);
@@ -290,7 +338,7 @@ wgrad_kernel(const __grid_constant__ Params p)
         copies_land();
         const int items = imgs * p.strips * p.oW;
         for (int it0 = 0; it0 < items; it0 += THREADS) {
-            if (chain + TH > kChain) { flush(); chain = 0; }
+            if (chain + TH > kChain) { sums.add(acc); chain = 0; }
             chain += TH;
             const int it = it0 + (int)threadIdx.x;
             if (it >= items) continue;
@@ -301,7 +349,7 @@ wgrad_kernel(const __grid_constant__ Params p)
 #pragma unroll
             for (int t = 0; t < TH; ++t) gv[t] = oh0 + t < p.oH ? __ldg(gp + (long long)t * p.oW) : 0.f;
 #pragma unroll
-            for (int t = 0; t < TH; ++t) acc[KK] += gv[t];
+            for (int t = 0; t < TH; ++t) bias += (double)gv[t];
             const float *row0 = tile + (pl * p.rows + t0 * S) * p.ld + ow;
 #pragma unroll
             for (int kw = 0; kw < K; ++kw) {
@@ -319,7 +367,10 @@ wgrad_kernel(const __grid_constant__ Params p)
     }
     // The CTA's sums; true if one of the filter's is not finite.
     auto gather = [&]() {
-        flush();
+        sums.add(acc);
+        sums.store(warp_sums[warp]);
+        bias = warp_sum(bias);
+        if ((threadIdx.x & 31) == 0) warp_sums[warp][KK] = bias;
         __syncthreads();
         bool bad = false;
         for (int i = threadIdx.x; i < SUMS; i += THREADS) {
@@ -333,8 +384,8 @@ wgrad_kernel(const __grid_constant__ Params p)
     if (gather()) {
         // The staged form also multiplies the padding's zeros by gy and the zeros past the last output by x: an infinity or a NaN there
         // reaches taps that never read it.  This CTA's share again, product by product.
-        for (int i = threadIdx.x; i < (THREADS / 32) * SUMS; i += THREADS) (&warp_sums[0][0])[i] = 0.0;
-        __syncthreads();
+        sums.clear();
+        bias = 0.0;
         chain = 0;
 #pragma unroll 1
         for (int u = (int)(units * rank / ranks); u < u_end; ++u) {
@@ -342,7 +393,7 @@ wgrad_kernel(const __grid_constant__ Params p)
             const int rows = min(p.R, p.oH - r0), items = imgs * rows * p.oW;
 #pragma unroll 1
             for (int it0 = 0; it0 < items; it0 += THREADS) {
-                if (++chain > kChain) { flush(); chain = 1; }
+                if (++chain > kChain) { sums.add(acc); chain = 1; }
                 const int it = it0 + (int)threadIdx.x;
                 if (it >= items) continue;
                 const int t2 = it / p.oW, ow = it - t2 * p.oW, pl = t2 / rows, oh = r0 + t2 - pl * rows;
@@ -350,7 +401,7 @@ wgrad_kernel(const __grid_constant__ Params p)
                 const float g = __ldg(p.gy + ((n * p.C + c) * p.M + j) * p.oH * p.oW + (long long)oh * p.oW + ow);
                 const float *xp = p.in + (n * p.C + c) * p.H * p.W;
                 const int ih0 = oh * S - p.padH, iw0 = ow * S - p.padW;
-                acc[KK] += g;
+                bias += (double)g;
 #pragma unroll
                 for (int kh = 0; kh < K; ++kh)
 #pragma unroll

@@ -125,3 +125,21 @@ def test_parameter_gradient_not_finite(F, shape, what):
                     want[:, :, kh, kw] = (xs[:, :, None] * gd[:, :, :, oh][..., ow]).sum((0, 3, 4)).t()
         assert torch.allclose(gw.cpu().double(), want, rtol=1e-4, atol=1e-3, equal_nan=True), where
         assert torch.allclose(gb.cpu().double(), gd.sum((0, 3, 4)).t(), rtol=1e-4, atol=1e-3, equal_nan=True), where
+
+
+@pytest.mark.parametrize("shape", [(16, 64, 56, 56, 5, 1), (29, 36, 37, 42, 7, 1), (98, 32, 51, 39, 3, 2)])
+def test_parameter_gradient_sums_in_fp64(F, shape):
+    """2-norm of the error: eight fp32 terms, then fp64, for the taps; fp64 throughout for the bias."""
+    import torch
+    N, C, H, W, k, d = shape
+    p, g = k // 2, torch.Generator(device="cuda").manual_seed(7)
+    oH, oW = (H + 2 * p - k) // d + 1, (W + 2 * p - k) // d + 1
+    x, gy = torch.randn(N, C, H, W, device="cuda", generator=g), torch.randn(N, C, oH, oW, device="cuda", generator=g)
+    cols = torch.nn.functional.unfold(x.double(), k, padding=p, stride=d).view(N, C, k * k, oH * oW)
+    want = torch.einsum("nckp,ncp->ck", cols, gy.double().view(N, C, -1)).view(1, C, k, k)
+    gw, gb = torch.zeros(1, C, k, k, device="cuda"), torch.zeros(1, C, device="cuda")
+    F.dwconv_acc_grad(x, gy, gw, gb, d, d, p, p)
+    # a chain of n FMAs is about 1.8e-8 sqrt(n + 1) off, the result's rounding 3.5e-8: 6.4e-8 for n = 8 (1.1e-7 for 32)
+    assert float((gw.double() - want).norm() / want.norm()) <= 7e-8
+    b = gy.double().sum((0, 2, 3)).view(1, C)
+    assert float((gb.double() - b).abs().max() / b.abs().max()) <= 2.0 ** -24
