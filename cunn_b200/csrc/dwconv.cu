@@ -20,6 +20,7 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace cunn {
 namespace dw {

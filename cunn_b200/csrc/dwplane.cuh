@@ -428,8 +428,40 @@ static uint32_t magic_of(int d) { return d == 1 ? 0u : (uint32_t)((1ull << 32) /
 
 enum Pass { FWD, DGRAD, WGRAD };
 
-// Fills the tile plan of a pass; false when the shape is left to the kernels for any shape: other kernel sizes and strides, or
-// rows so long that a strip's do not fit a tile.
+// Whether a planned pass is faster than the kernel for any shape, by straight lines fitted to 2,970 layers (maps of 3 to 900 columns, 1 to
+// 1024 channels, 1 to 128 images; us on a busy stream).  A few channels, or maps of 7 x 7 to 17 x 17 at stride 2, are over sooner there:
+// staging takes an instruction per row and warp however short the row is, and nothing can be computed before it has landed.
+// Forward of 70 x 560 x 9 x 9, 5x5 stride 2: 26 us for any shape, 66 staged; 32 x 96 x 57 x 43, 5x5 stride 2: 102 and 36 us; input gradient
+// of 12 x 47 x 12 x 9, 3x3 stride 2: 5.0 and 9.8 us; parameter gradient of 1 x 23 x 35 x 35, two 3x3 filters, stride 2: 3.8 and 5.5 us.
+// With the rule 0.2 % of those passes, and 0.5 % of the 3,600 of 1,200 other layers, are more than 7 % slower than for any shape, by 1 to 8 us;
+// 2 % would gain 20 % from the staged form.
+static bool faster_than_any_shape(const Params &p, Pass pass, int K)
+{
+    const double sms = sm_count(), kk = K * K;
+    const double rows_per_warp = (double)p.P * (pass == DGRAD ? p.M : 1) * p.rows * ((p.cols + 31) / 32) / (THREADS / 32);
+    const double strips = std::ceil((double)p.P * (pass == FWD ? p.M : 1) * p.strips * p.cols_out / THREADS);
+    if (pass == WGRAD) {
+        const double ctas = (double)p.C * p.M * (kk + 1) / (sms * 8), loops = std::ceil((double)p.oH * p.oW / 256) * p.N;
+        int ranks = 1;
+        while (ranks < 8 && (long long)ranks * 2 <= (long long)p.groups * p.bands) ranks *= 2;
+        const double units = std::ceil((double)p.groups * p.bands / ranks), waves = std::max(1.0, (double)p.C * p.M * ranks / (sms * 3));
+        return 3.4 + waves * (units * (0.147 * rows_per_warp + 0.015 * strips * kk) + 0.047 * kk) <
+               2.5 + loops * (0.43 + (ctas > 1.0 ? 0.63 * ctas : 0.0));
+    }
+    const double full = (double)p.N * p.groups * p.bands / (sms * 3), weights = (double)p.P * p.M * kk / THREADS;
+    if (pass == FWD) {
+        const double threads = (double)p.N * p.C * p.M * p.oH * p.oW / (sms * 2048);
+        return 2.2 + rows_per_warp * (0.095 + 0.056 * full) + strips * kk * (0.011 + 0.028 * full) + 1.56 * full + 0.37 * weights <
+               0.85 * (2.2 + 0.076 * K + kk * (0.078 + 0.10 * threads + 0.10 * std::max(0.0, threads - 1.0)) + 2.1 * threads);
+    }
+    const double threads = (double)p.N * p.C * p.H * p.W / (sms * 2048);
+    const double staged = 2.6 + 0.10 * K + rows_per_warp * (0.13 + 0.11 * full) + strips * p.M * kk * (0.001 + 0.010 * full) + 2.4 * full + 0.47 * weights;
+    const double any = 1.3 + 0.43 * K * p.M + kk * p.M * (0.16 + 0.46 * threads + 0.02 * std::max(0.0, threads - 1.0));
+    return staged < 0.85 * any || (staged < 4.25 && staged < 1.05 * any);         // the smallest: a launch either way
+}
+
+// Fills the tile plan of a pass; false when the shape is left to the kernels for any shape: other kernel sizes and strides, rows so
+// long that a strip's do not fit a tile, or where they are faster.
 static bool plan(Params &p, Pass pass, int N, int C, int H, int W, int M, int kH, int kW, int dH, int dW, int padH, int padW, int oH, int oW)
 {
     if (kH != kW || dH != dW || (kH != 3 && kH != 5 && kH != 7) || (dH != 1 && dH != 2)) return false;
@@ -482,7 +514,7 @@ static bool plan(Params &p, Pass pass, int N, int C, int H, int W, int M, int kH
     if (items * std::max(p.cols_out, p.strips) >= (1LL << 32) || p.cols_out >= (1 << 16)) return false;
     if (pass != WGRAD && (long long)N * p.groups * p.bands >= (1LL << 31)) return false;
     if (pass == WGRAD && (long long)C * M * 8 >= (1LL << 31)) return false;
-    return true;
+    return faster_than_any_shape(p, pass, K);
 }
 static size_t smem_bytes(const Params &p, Pass pass, int K)
 {

@@ -86,8 +86,9 @@ def test_weights_that_are_not_finite_stay_off_the_padding(F, d):
 @pytest.mark.parametrize("what", ["inf", "nan", "gpu nan"])
 @pytest.mark.parametrize("shape", [
     # N, C, H, W, M, k, d, padH, padW
-    (3, 4, 10, 12, 1, 5, 1, 0, 0),       # six rows of outputs: the second strip of four ends in two that do not exist
-    (2, 3, 23, 21, 2, 5, 2, 2, 2),       # rows past the last window, padding on every side
+    (3, 4, 10, 12, 1, 5, 1, 0, 0),       # the kernel for any shape
+    (20, 40, 10, 12, 1, 5, 1, 0, 0),     # six rows of outputs: the second strip of four ends in two that do not exist
+    (12, 60, 23, 21, 2, 5, 2, 2, 2),     # rows past the last window, padding on every side
     (40, 2, 9, 9, 1, 3, 1, 1, 0),        # several ranks
     (1, 2, 90, 70, 1, 7, 1, 3, 2),       # several bands
 ])
@@ -143,3 +144,16 @@ def test_parameter_gradient_sums_in_fp64(F, shape):
     assert float((gw.double() - want).norm() / want.norm()) <= 7e-8
     b = gy.double().sum((0, 2, 3)).view(1, C)
     assert float((gb.double() - b).abs().max() / b.abs().max()) <= 2.0 ** -24
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W, M, k, d, padH, padW: the same edges with as much work as the staged form is chosen for in every pass
+    (8, 200, 57, 43, 1, 5, 2, 2, 2), (6, 60, 200, 33, 1, 5, 1, 2, 2), (6, 40, 150, 131, 1, 7, 2, 3, 3), (64, 300, 7, 7, 1, 7, 1, 3, 3),
+    (40, 70, 14, 14, 2, 5, 1, 2, 2), (30, 50, 29, 37, 3, 3, 2, 1, 1), (12, 144, 37, 29, 1, 3, 1, 1, 1), (40, 100, 16, 18, 1, 3, 1, 0, 2),
+    (12, 300, 30, 26, 1, 5, 2, 4, 0), (40, 90, 33, 33, 1, 3, 2, 3, 3), (300, 40, 20, 20, 1, 3, 1, 0, 0), (24, 90, 40, 12, 1, 5, 1, 0, 0),
+    (30, 100, 31, 29, 1, 7, 2, 3, 3),
+    # layers that the kernels for any shape take although a tile plan exists
+    (70, 56, 9, 9, 1, 5, 2, 2, 2), (12, 47, 12, 9, 1, 3, 2, 1, 1), (1, 23, 35, 35, 2, 3, 2, 1, 1),
+])
+def test_both_sides_of_the_staging_rule(F, ref64, ref32, shape):
+    test_staged_plane_shapes(F, ref64, ref32, shape)
