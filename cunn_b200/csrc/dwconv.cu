@@ -900,6 +900,8 @@ struct Tuning {
 };
 static thread_local Tuning g_tuning;
 
+constexpr size_t kMaxPlanSmem = 200 * 1024;    // most shared memory of a plan
+
 struct Plan {
     bool ok = false;
     int S = 1, VEC = 1;
@@ -1091,7 +1093,7 @@ static Plan make_plan(int mode, int N, int C, int H, int W, int oH, int oW, int 
                          ((mode == MODE_WGRAD) ? (size_t)pl.items * 10 * 4 : 0);
     const size_t per_stage = (size_t)(pl.stage_floats + pl.stage2_floats) * 4 + 8;
     pl.smem = (size_t)pl.stages * per_stage + fixed;
-    if (pl.smem > 200 * 1024) return pl;
+    if (pl.smem > kMaxPlanSmem) return pl;
     pl.ok = true;
     return pl;
 }
@@ -1144,7 +1146,7 @@ static int finalize_plan(Plan &pl)
     if (occ <= 0) {
         bool asked = false;
         if (pl.smem <= 48 * 1024 ||
-            cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) == cudaSuccess) {
+            cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPlanSmem) == cudaSuccess) {
             int n = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, (const void *)kern, pl.threads, pl.smem) == cudaSuccess && n > 0) {
                 occ = n;
@@ -1158,7 +1160,7 @@ static int finalize_plan(Plan &pl)
         }
         occ = std::min(occ, 8);
     } else if (pl.smem > 48 * 1024) {
-        (void)cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+        (void)cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPlanSmem);
         (void)cudaGetLastError();
     }
     long long grid = (long long)sm_count() * occ;
@@ -1212,8 +1214,8 @@ static int launch_fast(FastParams &fp, const Plan &pl, cudaStream_t stream, cons
     fp.tiles_base = (int)(pl.tiles / pl.grid);
     fp.tiles_rem = (int)(pl.tiles % pl.grid);
     void *args[] = {(void *)&fp};
-    // another plan of the same kernel may have asked for less since
-    if (pl.smem > 48 * 1024) CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+    // the same limit for every plan: with each plan's own, a thread could lower it between another one's call and launch
+    if (pl.smem > 48 * 1024) CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxPlanSmem));
     // launched as a programmatic dependent of whatever precedes it in the stream: its prologue may overlap
     // the tail of the previous kernel; the kernel itself waits (pdl_wait) before touching global memory
     cudaLaunchConfig_t cfg = {};

@@ -222,3 +222,29 @@ def test_dwconv_acc_grad_deterministic_mode(F, ref64):
             assert np.array_equal(first[0], cur[0]) and np.array_equal(first[1], cur[1])
     finally:
         lib.cunn_b200_set_deterministic(0)
+
+
+def test_threads_with_plans_of_different_sizes(F):
+    """Threads on streams of their own whose layers run on the same kernels with different amounts of shared memory."""
+    import threading
+    import torch
+    shapes = [(4, 64, 112, 112), (4, 64, 56, 56), (4, 64, 28, 28), (8, 64, 24, 24), (2, 32, 224, 224), (2, 32, 128, 160), (4, 64, 64, 48), (4, 64, 96, 80)]
+    errors = []
+
+    def work(shape):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                x, w = torch.ones(shape, device="cuda"), torch.ones(1, shape[1], 3, 3, device="cuda")
+                y = torch.empty_like(x)
+                for _ in range(2000):
+                    F.dwconv_forward(x, w, None, 1, 1, 1, 1, out=y)
+                assert torch.all(y[:, :, 1:-1, 1:-1] == 9)
+        except Exception as e:
+            errors.append((shape, str(e)))
+    threads = [threading.Thread(target=work, args=(s,)) for s in shapes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
