@@ -904,6 +904,7 @@ constexpr size_t kMaxPlanSmem = 200 * 1024;    // most shared memory of a plan
 
 struct Plan {
     bool ok = false;
+    bool measured = true;     // the occupancy is the runtime's answer
     int S = 1, VEC = 1;
     bool stage_out = false;
     bool direct = false;      // read rows straight from global memory instead of through the TMA ring
@@ -1153,6 +1154,7 @@ static int finalize_plan(Plan &pl)
                 asked = true;
             }
         }
+        pl.measured = asked;
         if (!asked) {
             (void)cudaGetLastError();
             const int by_smem = (int)((220 * 1024) / (pl.smem + 1024));
@@ -1172,7 +1174,10 @@ static int finalize_plan(Plan &pl)
 }
 
 // The finished plan of a shape on the current device.  Planning scores a few hundred tilings and asks the runtime for the occupancy
-// (about 4 us), as long as a layer of one image runs; a thread keeps its last sixteen plans.  A plan is a function of these numbers alone.
+// (about 4 us), as long as a layer of one image runs.  A thread keeps its last sixteen plans, replaced in order of arrival: enough for
+// inference of a network like MobileNetV1 (nine shapes), while a training step of it that launches layer by layer asks for 22 in turn
+// and plans each anew, as without keeping any.  A plan is a function of these numbers alone; one made while the runtime did not answer
+// (a passing error) is used and not kept.
 static bool find_plan(Plan &pl, int mode, int N, int C, int H, int W, int oH, int oW, int S)
 {
 #ifdef CUNN_B200_DEV_HOOKS
@@ -1187,15 +1192,17 @@ static bool find_plan(Plan &pl, int mode, int N, int C, int H, int W, int oH, in
     static thread_local Entry kept[16];
     static thread_local int used = 0, next = 0;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    const bool known = cudaGetDevice(&dev) == cudaSuccess;
+    if (!known) (void)cudaGetLastError();
     const int key[9] = {mode, N, C, H, W, oH, oW, S, dev};
-    for (int i = 0; i < used; ++i)
+    for (int i = 0; known && i < used; ++i)
         if (std::equal(key, key + 9, kept[i].key)) {
             pl = kept[i].pl;
             return kept[i].ok;
         }
     pl = make_plan(mode, N, C, H, W, oH, oW, S);
     const bool ok = pl.ok && finalize_plan(pl) == 0;
+    if (!known || !pl.measured) return ok;
     Entry &e = kept[next];
     std::copy(key, key + 9, e.key);
     e.ok = ok;
