@@ -1900,9 +1900,10 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
     CUNN_CHECK_ARG(gy && weight && gx, "null tensor pointer");
     const bool dilated = dilH != 1 || dilW != 1;
     CUNN_CHECK_ARG(!dilated || gather_applies(kH, kW), "dilated kernels of more than 32 taps are not supported");
-    if (pw_applies(kH, kW, dH, dW, padH, padW) && H * W == 1 && K % 4 == 0 && tma_applies(gy, weight, gx, C, K))
+    if (pw_applies(kH, kW, dH, dW, padH, padW) && H * W == 1 && K % 4 == 0 && K < (1 << 24) && (long long)K * C < (1LL << 31) &&
+        tma_applies(gy, weight, gx, C, K))
         // a fully connected layer: gx[n][c] = sum_k gy[n][k] W[k][c] is the 1x1 convolution of the one "image" W (K channels of C
-        // pixels) with the N filters gy
+        // pixels) with the N filters gy, within the limits of an image and of a filter
         return add_bias(conv_forward(weight, gy, nullptr, gx, 1, K, 1, C, N, 1, 1, 1, 1, 0, 0, 1, 1, stream_));
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         pw::Params q{};

@@ -252,3 +252,15 @@ def test_weight_gradient_chains_stay_short(F):
     # truncated operands 3.5e-7; an accumulator's n truncations of about 2^-24 / 1.4 at two thirds of the sum: 16 a tile of 10 or 19
     # k-blocks over three accumulators, n = 28 at most -> 8e-7 with half a factor for their growth; one of 38 has n = 52 -> 1.2e-6
     assert float((gw.double() - want).norm() / want.norm()) <= 1e-6
+
+
+def test_fully_connected_gradient_of_2_24_outputs(F):
+    """2^24 outputs: more than the filters of the convolution that stands in for the gradient of a fully connected layer may have taps."""
+    import torch
+    K, C = 1 << 24, 4
+    gy, w = torch.zeros(1, K, 1, 1, device="cuda"), torch.zeros(K, C, 1, 1, device="cuda")
+    at = torch.tensor([0, 5, 8191, K // 2 + 3, K - 1], device="cuda")
+    gy[0, at, 0, 0] = torch.tensor([1.0, 2.0, -3.0, 4.0, 0.5], device="cuda")
+    w[at] = torch.arange(20.0, device="cuda").view(5, 4, 1, 1)
+    gx = F.convmm_grad_input(gy, w, 1, 1, 1, 1, 0, 0)
+    assert torch.equal(gx.view(4), (gy[0, at, 0, 0].view(5, 1) * w[at].view(5, 4)).sum(0))
