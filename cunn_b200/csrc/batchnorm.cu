@@ -24,40 +24,9 @@ struct ChunkStat {
     float n;      // element count
 };
 
-// Merges the chunk statistics of channel c in fp64 (Chan's formula), publishes mean / inverse std and updates
-// the running statistics.
-__device__ __forceinline__ void finish_stats_channel(const ChunkStat *part, int c, int chunks, float *running_mean,
-                                                     float *running_var, float *save_mean, float *save_std,
-                                                     double momentum, double eps)
-{
-    double n = 0.0, mean = 0.0, m2 = 0.0;
-    for (int j = 0; j < chunks; ++j) {
-        const float4 raw = __ldcg(reinterpret_cast<const float4 *>(part + c * chunks + j));   // written by other CTAs
-        const ChunkStat p{raw.x, raw.y, raw.z, raw.w};
-        if (p.n <= 0.f) continue;
-        const double nb = p.n;
-        const double mb = (double)p.k + (double)p.s1 / nb;
-        const double m2b = (double)p.s2 - (double)p.s1 * (double)p.s1 / nb;
-        const double delta = mb - mean, nt = n + nb;
-        mean += delta * nb / nt;
-        m2 += m2b + delta * delta * n * nb / nt;
-        n = nt;
-    }
-    if (m2 < 0.0) m2 = 0.0;
-    // The reference computes in float for float tensors; follow its formulas on the float-rounded mean.
-    const float meanf = (float)mean;
-    const float varN = (float)m2;
-    float invstd = 0.f;
-    if (varN != 0.f || (float)eps != 0.f) invstd = 1.f / sqrtf((float)(m2 / n) + (float)eps);
-    const float unbiased = (float)(m2 / (n - 1.0));
-    save_mean[c] = meanf;
-    save_std[c] = invstd;
-    running_mean[c] = (float)((1.0 - momentum) * (double)running_mean[c] + momentum * (double)meanf);
-    running_var[c] = (float)((1.0 - momentum) * (double)running_var[c] + momentum * (double)unbiased);
-}
-
-// The same by one warp, without a division per partial (they cost 0.3 us each): the mean first, then the squares about it,
-// sum (x - mean)^2 = s2 - 2 d s1 + n d^2 with d = mean - k, in a fixed order.  `part` points at the channel's first partial.
+// Merges the chunk statistics of channel c in fp64, publishes mean / inverse std and updates the running statistics; by one warp, without
+// a division per partial (they cost 0.3 us each): the mean first, then the squares about it, sum (x - mean)^2 = s2 - 2 d s1 + n d^2
+// with d = mean - k, in a fixed order.  `part` points at the channel's first partial.
 __device__ __forceinline__ void finish_stats_channel_warp(const ChunkStat *part, int c, int chunks, float *running_mean,
                                                           float *running_var, float *save_mean, float *save_std,
                                                           double momentum, double eps)
@@ -80,6 +49,7 @@ __device__ __forceinline__ void finish_stats_channel_warp(const ChunkStat *part,
     m2 = warp_sum(m2);
     if (lane != 0) return;
     if (m2 < 0.0) m2 = 0.0;
+    // The reference computes in float for float tensors; follow its formulas on the float-rounded mean.
     const float meanf = (float)mean;
     const float varN = (float)m2;
     float invstd = 0.f;
@@ -168,10 +138,12 @@ __device__ __forceinline__ ChunkStat chunk_stats(const float *x, int N, int C, i
     float first = 0.f, e[V];
     if ((int)(threadIdx.x & 31) < probe) {
         each_of(v[0], e);
-        if constexpr (V == 4) first = (e[0] + e[1]) + (e[2] + e[3]);
+        if constexpr (V == 4) first = ((e[0] + e[1]) + (e[2] + e[3])) * 0.25f;
         else first = e[0];
     }
-    const float k = warp_sum(first) / (float)(probe * V);
+    // no shift where the items hold an infinity or a NaN, or add up to one: x - k would be NaN for items that are neither
+    float k = warp_sum(first) / (float)probe;
+    if (!(fabsf(k) < INFINITY)) k = 0.f;
     float s1[U], s2[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) s1[u] = s2[u] = 0.f;
@@ -221,8 +193,8 @@ stats_finish_kernel(const ChunkStat *__restrict__ part, int C, int chunks, float
                     float *__restrict__ running_var, float *__restrict__ save_mean, float *__restrict__ save_std,
                     double momentum, double eps)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < C) finish_stats_channel(part, c, chunks, running_mean, running_var, save_mean, save_std, momentum, eps);
+    const int c = (int)blockIdx.x * 4 + ((int)threadIdx.x >> 5);
+    if (c < C) finish_stats_channel_warp(part + (size_t)c * chunks, c, chunks, running_mean, running_var, save_mean, save_std, momentum, eps);
 }
 
 // gamma * (x - mean) * invstd + beta with every rounding pinned (no fused multiply-add), so that the backward
@@ -335,37 +307,8 @@ struct GradCoef {
 
 // Backward, pass 2 for channel c: totals the chunk sums in fp64, accumulates gradWeight / gradBias and publishes
 // the coefficients of the input gradient.
-__device__ __forceinline__ void finish_grad_channel(const float2 *part, int c, int chunks, long long count, const float *weight,
-                                                    const float *bias, const float *mean_v, const float *std_or_var,
-                                                    int train, double eps, double scale, float *grad_weight,
-                                                    float *grad_bias, GradCoef *coef)
-{
-    double s = 0.0, d = 0.0;
-    for (int j = 0; j < chunks; ++j) {
-        const float2 p = __ldcg(part + j);                // the channel's partials, written by other CTAs
-        s += (double)p.x;
-        d += (double)p.y;
-    }
-    const float mean = mean_v[c];
-    const float stdv = train ? std_or_var[c] : (float)(1.0 / sqrt((double)std_or_var[c] + eps));
-    const float w = weight ? weight[c] : 1.f;
-    const double norm = 1.0 / (double)count;
-    GradCoef k;
-    k.mean = mean;
-    k.gmean = (float)(s * norm);
-    k.proj = (float)(d * norm * (double)stdv * (double)stdv);
-    k.gscale = stdv * w;
-    k.invstd = train ? std_or_var[c] : 1.f / sqrtf(std_or_var[c] + (float)eps);   // as the forward kernel computes it
-    k.gamma = w;
-    k.beta = bias ? bias[c] : 0.f;
-    k.pad = 0.f;
-    coef[c] = k;
-    if (grad_weight) grad_weight[c] = (float)((double)grad_weight[c] + scale * d * (double)stdv);
-    if (grad_bias) grad_bias[c] = (float)((double)grad_bias[c] + scale * s);
-}
-
-// The same totals by one warp: lanes add strided subsets in fp64 and are then folded in a fixed order, so the
-// result does not depend on timing.  Lane 0 publishes.
+// By one warp: lanes add strided subsets and are then folded in a fixed order, so the result does not depend on timing.
+// Lane 0 publishes.
 __device__ __forceinline__ void finish_grad_channel_warp(const float2 *part, int c, int chunks, long long count, const float *weight,
                                                          const float *bias, const float *mean_v, const float *std_or_var,
                                                          int train, double eps, double scale, float *grad_weight,
@@ -393,7 +336,7 @@ __device__ __forceinline__ void finish_grad_channel_warp(const float2 *part, int
     k.gmean = (float)(s * norm);
     k.proj = (float)(d * norm * (double)stdv * (double)stdv);
     k.gscale = stdv * w;
-    k.invstd = train ? std_or_var[c] : 1.f / sqrtf(std_or_var[c] + (float)eps);
+    k.invstd = train ? std_or_var[c] : 1.f / sqrtf(std_or_var[c] + (float)eps);   // as the forward kernel computes it
     k.gamma = w;
     k.beta = bias ? bias[c] : 0.f;
     k.pad = 0.f;
@@ -408,8 +351,8 @@ grad_finish_kernel(const float2 *__restrict__ part, int C, int chunks, long long
                    const float *__restrict__ std_or_var, int train, double eps, double scale,
                    float *__restrict__ grad_weight, float *__restrict__ grad_bias, GradCoef *__restrict__ coef)
 {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < C) finish_grad_channel(part + (size_t)c * chunks, c, chunks, count, weight, bias, mean_v, std_or_var, train, eps, scale, grad_weight, grad_bias, coef);
+    const int c = (int)blockIdx.x * 4 + ((int)threadIdx.x >> 5);
+    if (c < C) finish_grad_channel_warp(part + (size_t)c * chunks, c, chunks, count, weight, bias, mean_v, std_or_var, train, eps, scale, grad_weight, grad_bias, coef);
 }
 
 // Sums of gy and gy * (x - mean) over one chunk.
@@ -1267,7 +1210,7 @@ static int bn_forward_impl(const float *x, float *y, const float *weight, const 
                                                      save_std, momentum, eps);
         CUNN_LAUNCH_CHECK("batch norm statistics");
         if (!counters) {
-            stats_finish_kernel<<<ceil_div(C, 128), 128, 0, stream>>>(part, C, chunks, running_mean, running_var, save_mean,
+            stats_finish_kernel<<<ceil_div(C, 4), 128, 0, stream>>>(part, C, chunks, running_mean, running_var, save_mean,
                                                                      save_std, momentum, eps);
             CUNN_LAUNCH_CHECK("batch norm statistics finish");
         }
@@ -1353,7 +1296,7 @@ static int bn_backward_impl(const float *x, const float *gy, bool relu, const fl
         CUNN_CUDA(cudaMemsetAsync(part, 0, (size_t)C * chunks * sizeof(float2), stream));
     }
     if (!need_sums || !counters) {
-        grad_finish_kernel<<<ceil_div(C, 128), 128, 0, stream>>>(part, C, chunks, (long long)N * S, weight, bias, mean_v, sv, train,
+        grad_finish_kernel<<<ceil_div(C, 4), 128, 0, stream>>>(part, C, chunks, (long long)N * S, weight, bias, mean_v, sv, train,
                                                                 eps, scale, grad_weight, grad_bias, coef);
         CUNN_LAUNCH_CHECK("batch norm gradient finish");
     }

@@ -44,3 +44,27 @@ def test_bn_constant_channel_has_no_variance(F, shape, value):     # noqa: F811
     rm, rv = torch.zeros(shape[1], device="cuda"), torch.ones(shape[1], device="cuda")
     y, sm, ss = F.batchnorm_forward(x, None, None, rm, rv, True, 0.1, 0.0)
     assert torch.equal(sm, torch.full_like(sm, value)) and torch.all(ss == 0) and torch.all(y == 0)
+
+
+@pytest.mark.parametrize("shape", [(3, 4, 20, 20), (40, 3, 31, 29), (2, 5000, 5, 7), (9, 2, 96, 100)])
+def test_bn_statistics_of_what_is_not_finite(F, shape):     # noqa: F811
+    """The mean is a sum: infinite where one sign of infinity is among the values, wherever it stands, NaN for both or a NaN."""
+    inf = float("inf")
+    for first in (True, False):
+        x = torch.randn(shape, device="cuda")
+        at = (0, slice(None), 0, 0) if first else (shape[0] - 1, slice(None), shape[2] - 1, shape[3] - 1)
+        bad = torch.zeros(shape[1], device="cuda")
+        bad[0], bad[1], bad[2 % shape[1]] = inf, -inf, float("nan")
+        x[at] += bad
+        rm, rv = torch.zeros(shape[1], device="cuda"), torch.ones(shape[1], device="cuda")
+        _, sm, ss = F.batchnorm_forward(x, None, None, rm, rv, True, 0.1, 1e-5)
+        want = x.double().mean((0, 2, 3)).float()
+        assert torch.allclose(sm, want, rtol=1e-5, atol=1e-6, equal_nan=True) and torch.allclose(rm, 0.1 * want, rtol=1e-5, atol=1e-6, equal_nan=True)
+        assert torch.equal(torch.isnan(ss), ~torch.isfinite(want)) and torch.equal(torch.isnan(rv), ~torch.isfinite(want))
+
+
+def test_bn_constant_channel_of_large_values(F):     # noqa: F811
+    x = torch.full((2, 3, 16, 16), 5e36, device="cuda")
+    rm, rv = torch.zeros(3, device="cuda"), torch.ones(3, device="cuda")
+    y, sm, _ = F.batchnorm_forward(x, None, None, rm, rv, True, 0.1, 1e-5)
+    assert torch.equal(sm, torch.full_like(sm, 5e36)) and torch.all(y == 0)
