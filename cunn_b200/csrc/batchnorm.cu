@@ -119,6 +119,7 @@ __device__ __forceinline__ bool last_warp_of_channel(unsigned int *counters, int
         last = atomicAdd(counters + c, 1u) == (unsigned int)(chunks - 1);
     }
     last = __shfl_sync(0xffffffffu, last, 0);
+    __syncwarp();                                          // a shuffle orders no memory: the other lanes read after lane 0's ticket
     if (last) __threadfence();                            // the other warps' partials are visible after their tickets
     return last != 0;
 }
