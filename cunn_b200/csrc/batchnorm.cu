@@ -34,6 +34,7 @@ __device__ __forceinline__ void finish_stats_channel_warp(const ChunkStat *part,
     const int lane = threadIdx.x & 31;
     const float4 *raw = reinterpret_cast<const float4 *>(part);                 // k, s1, s2, n
     double n = 0.0, sum = 0.0, m2 = 0.0;
+#pragma unroll 4
     for (int j = lane; j < chunks; j += 32) {
         const float4 p = __ldcg(raw + j);
         n += (double)p.w;
@@ -41,6 +42,7 @@ __device__ __forceinline__ void finish_stats_channel_warp(const ChunkStat *part,
     }
     n = warp_sum(n);
     const double mean = warp_sum(sum) / n;
+#pragma unroll 4
     for (int j = lane; j < chunks; j += 32) {
         const float4 p = __ldcg(raw + j);
         const double d = mean - (double)p.x;
@@ -75,17 +77,16 @@ struct ChunkWalk {
         constexpr int V = (int)(sizeof(T) / sizeof(float));
         const int lane = threadIdx.x & 31;
         L = S / V;
-        const long long total = (long long)N * L;
-        const long long q0 = total * j / chunks, items = total * (j + 1) / chunks - q0;
-        const long long q = q0 + lane;
-        const int n = (int)(q / L);
-        i = (int)(q - (long long)n * L);
-        left = items > lane ? (int)((items - lane + 31) / 32) : 0;
+        const int total = N * L, each = total / chunks, more = total - each * chunks;      // the first `more` chunks have one item more
+        const int q = j * each + min(j, more) + lane, items = each + (j < more ? 1 : 0);
+        const int n = q / L;
+        i = q - n * L;
+        left = items > lane ? (items - lane + 31) / 32 : 0;
         off = ((unsigned)n * (unsigned)C + (unsigned)c) * (unsigned)S + (unsigned)i * V;
         rstep = 32 % L;
         step = (unsigned)(32 / L) * (unsigned)C * (unsigned)S + (unsigned)rstep * V;
         wrap = (unsigned)(C - 1) * (unsigned)S;
-        return (int)items * V;        // elements of the chunk
+        return items * V;             // elements of the chunk
     }
     // The next U items of x (and of y); returns how many this lane has.
     template <int U, bool TWO>
@@ -317,6 +318,7 @@ __device__ __forceinline__ void finish_grad_channel_warp(const float2 *part, int
 {
     const int lane = threadIdx.x & 31;
     double s = 0.0, d = 0.0;
+#pragma unroll 4
     for (int j = lane; j < chunks; j += 32) {
         const float2 p = __ldcg(part + j);
         s += (double)p.x;
@@ -1029,14 +1031,19 @@ constexpr int kMaxCounterChannels = 4096;
 constexpr int kCounterArrays = 6;
 constexpr size_t kCounterBytes = (size_t)kCounterArrays * kMaxCounterChannels * sizeof(unsigned int);
 
-// Chunks per channel: 48 warps per SM, at least kMinChunk elements each where the channel has them.  One batch of loads per lane: small
-// tensors are over soonest when every load is in flight at once (forward / backward of 12 x 144 x 37 x 29: 22.2 / 24.5 us with chunks
-// of 2048, 17.3 / 18.5 with 512; 128 x 1024 x 7 x 7 prefers the longer ones, 32.8 / 35.0 and 35.1 / 39.0).
-constexpr int kMinChunk = 512;
+// Chunks per channel: 48 warps per SM at most, and chunks of at least kMinChunk elements.  One batch of loads per lane: small tensors are
+// over soonest when every load is in flight at once (forward / backward of 12 x 144 x 37 x 29: 22.2 / 24.5 us with chunks of 2048, 17.3
+// / 18.5 with 512; 128 x 1024 x 7 x 7 prefers the longer ones, 32.8 / 35.0 and 35.1 / 39.0).  Beyond kFewChunks of them chunks are
+// longer, since the channel's last warp reads them all: 19 x 22 x 94 x 94 17.7 / 17.0 us with 322 chunks, 12.9 / 12.7 with 128 (13.8 / 13.0
+// with CTAs per image, as before the warps); 189 x 8 x 109 x 183 87 / 109 us with 888 chunks, 142 / 171 with 128.
+constexpr int kMinChunk = 512, kFewChunks = 128, kLongChunk = 2048;
 static int most_chunks(int C) { return std::max(1, ceil_div(sm_count() * 48, C)); }
 static int pick_chunks(int N, int C, int S)
 {
-    return (int)std::max(1LL, std::min<long long>(most_chunks(C), (long long)N * S / kMinChunk));
+    const long long count = (long long)N * S;
+    const int least = S % 4 != 0 && C * count <= (1 << 19) ? kMinChunk / 2 : kMinChunk;          // a lane's batch is eight floats, or four float4
+    const long long wanted = std::max(std::min<long long>(count / least, kFewChunks), count / kLongChunk);
+    return (int)std::max(1LL, std::min<long long>(most_chunks(C), wanted));
 }
 
 // Planes of up to 1024 elements are handled by one warp each, larger ones by a whole CTA.
