@@ -13,9 +13,17 @@ from ._lib import lib, check
 _workspaces = {}
 
 
-def _stream():
-    """Handle of the current device's current stream (torch.cuda.current_stream().cuda_stream without the Stream object)."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+try:
+    # 0.2 us a layer instead of the 3.3 us of torch.cuda.current_stream().cuda_stream; not a public interface of torch
+    _raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+    def _stream():
+        """Handle of the current device's current stream."""
+        return _raw_stream(_device())
+except AttributeError:
+    def _stream():
+        """Handle of the current device's current stream."""
+        return torch.cuda.current_stream().cuda_stream
 
 
 def _chk(*ts):
