@@ -1560,11 +1560,13 @@ static long long wgrad_kblocks(int N, int HW, bool groups)
 {
     return groups ? (long long)N * ceil_div(HW, BK) : ceil_div_ll((long long)N * HW, BK);
 }
-// Weight gradients whose operands are split with rounding.  Without it those of kernels of more than 32 taps were 4.2e-7 off for short
-// reductions (1.3e-7 with it; 1.4e-7 on the one-CTA-per-tile kernel they came from), for 8 to 11 % of their time.  Reductions of up to 64
-// k-blocks are split below the image, where the truncating split's error and a chain's add up (fully connected layers 3.8e-7 -> 4.3e-7, 1.2e-7
-// with rounding); their launches wait for memory, and the extra stores cost nothing.
-static bool rounds_wgrad(int kk, int N, int HW) { return kk > 32 || wgrad_kblocks(N, HW, false) <= 64; }
+// Weight gradients whose operands are split with rounding, for 8 to 11 % of their time.  Kernels of more than 32 taps came from a kernel that
+// rounds and sums each image apart, with an error that grows with the image: 1.4e-7 to 4.6e-7 for up to 16 x 16 outputs, where truncated
+// operands alone are 4.2e-7 off (rounded ones and their chains 1.3e-7 to 2.6e-7), but 1.35e-6 at 28 x 28 against 0.6e-6 to 1.1e-6 with
+// truncated ones, and 2.2e-5 against 2.4e-6 at 112 x 112.  Reductions of up to 64 k-blocks are split below the image, where the truncating
+// split's error and a chain's add up (fully connected layers 3.8e-7 -> 4.3e-7, 1.2e-7 with rounding); their launches wait for memory, and the
+// extra stores cost nothing.
+static bool rounds_wgrad(int kk, int N, int HW) { return kk > 32 ? HW < 784 : wgrad_kblocks(N, HW, false) <= 64; }
 // k-blocks whose large products meet in one accumulator of a tile: the error of a weight gradient grows with them.
 static int wgrad_chain(int bn, long long kb, long long tiles)
 {
@@ -1591,7 +1593,8 @@ static void pw_wgrad_plan(int C, int K, int kk, int N, int HW, bool groups, int 
         return kb > 128 ? cost * (1.0 + 0.25 * (double)(kb - 128) / 128.0) : cost;
     };
     long long whole = kb_total;                                             // k-blocks of a tile of whole images
-    if (!rounds_wgrad(kk, N, HW)) {
+    const bool bounded = kk <= 32 && !rounds_wgrad(kk, N, HW);
+    if (bounded) {
         double best = -1.0;
         for (int images = 1; images <= N; ++images) {
             const long long used = ceil_div(N, images);
@@ -1602,10 +1605,10 @@ static void pw_wgrad_plan(int C, int K, int kk, int N, int HW, bool groups, int 
     }
     const int chain = wgrad_chain(*bn, whole, 1LL << 30);
     double best = -1.0;
-    for (int i = 0; i <= 20; ++i) {
+    for (int i = bounded ? 0 : 1; i <= 20; ++i) {
         const long long want = i <= 16 ? (long long)i * grid / tiles_mn : i - 16;
         const long long kb = i ? ceil_div_ll(kb_total, std::max(1LL, std::min(want, kb_total))) : whole, used = ceil_div_ll(kb_total, kb);
-        if (i && !rounds_wgrad(kk, N, HW) && wgrad_chain(*bn, kb, tiles_mn * used) > chain) continue;
+        if (i && bounded && wgrad_chain(*bn, kb, tiles_mn * used) > chain) continue;
         const double cost = score(kb, used) + (double)used * K * C * 4.0 / 8e6;                   // a k-block lasts as long as 8 MB of L2 reads
         if (best < 0.0 || cost < best * 0.999) { best = cost; *splits = (int)used; *kb_per_split = (int)kb; }
     }
