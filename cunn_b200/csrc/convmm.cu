@@ -1060,7 +1060,7 @@ pw_gemm_kernel(const Params p)
             const float4 va = *reinterpret_cast<const float4 *>(a_hi + a_so[i]);
             if (ROUND) split_rounded(a_hi, a_lo, a_so[i], va);
             else store_lo_at(a_lo, a_so[i], va);
-            if (OP == OP_WGRAD) bsum[i] += (BiasSum)((va.x + va.y) + (va.z + va.w));
+            if (OP == OP_WGRAD) bsum[i] += ((BiasSum)va.x + (BiasSum)va.y) + ((BiasSum)va.z + (BiasSum)va.w);
             if (b_store[i]) {
                 const float4 vb = *reinterpret_cast<const float4 *>(b_hi + b_so[i]);
                 if (ROUND) split_rounded(b_hi, b_lo, b_so[i], vb);
