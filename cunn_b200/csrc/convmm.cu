@@ -1519,11 +1519,11 @@ static bool tma_applies(const void *a, const void *b, const void *c, int HW, int
 }
 // Accumulator plan of the tensor-map kernels: tiles of one or two k-blocks put all products into one accumulator and
 // use up to four accumulator sets, so that the MMA warp runs several tiles ahead of the epilogue warps; longer tiles, and
-// weight gradients with a tile per CTA, follow pw_accumulators.
-static void tma_accumulators(int bn, int kblocks, int *nacc, int *sets, bool wgrad = false, int tiles = 0)
+// launches with a tile per CTA, follow pw_accumulators, which keeps the small products apart from the large ones.
+static void tma_accumulators(int bn, int kblocks, int *nacc, int *sets, bool wgrad, int tiles)
 {
     const int cols = std::max(bn, 32);
-    if (kblocks <= 2 && !(wgrad && tiles <= sm_count())) {
+    if (kblocks <= 2 && tiles > sm_count()) {
         *nacc = 1;
         *sets = std::min((int)pwt::MAX_SETS, 512 / cols);
         return;
@@ -1834,7 +1834,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
             alignas(64) CUtensorMap ma, mb, mo;
             q.gpi = ceil_div(q.HW, 32); q.M_total = N * q.gpi * 32; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
             q.bulk_out = (q.HW % 32 == 0) && q.HW >= 8 * BM;
-            tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
+            tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, false, q.total_tiles);
             if (make_map(&ma, x, q.HW, C, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return 1;
             if (make_map(&mb, weight, C, K, 0, 32, bn, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
             if (q.bulk_out) { if (make_map(&mo, y, q.HW, K, N, BM, pwt::HALF_STAGE_COLS, CU_TENSOR_MAP_SWIZZLE_NONE)) return 1; }
@@ -1919,7 +1919,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
             alignas(64) CUtensorMap ma, mb, mo;
             q.gpi = ceil_div(q.HW, 32); q.M_total = N * q.gpi * 32; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
             q.bulk_out = (q.HW % 32 == 0) && q.HW >= 8 * BM;
-            tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
+            tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, false, q.total_tiles);
             if (make_map(&ma, gy, q.HW, K, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return 1;
             if (make_map(&mb, weight, C, K, 0, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return 1;
             if (q.bulk_out) { if (make_map(&mo, gx, q.HW, C, N, BM, pwt::HALF_STAGE_COLS, CU_TENSOR_MAP_SWIZZLE_NONE)) return 1; }

@@ -264,3 +264,17 @@ def test_fully_connected_gradient_of_2_24_outputs(F):
     w[at] = torch.arange(20.0, device="cuda").view(5, 4, 1, 1)
     gx = F.convmm_grad_input(gy, w, 1, 1, 1, 1, 0, 0)
     assert torch.equal(gx.view(4), (gy[0, at, 0, 0].view(5, 1) * w[at].view(5, 4)).sum(0))
+
+
+@pytest.mark.parametrize("shape", [(64, 8, 60), (3, 152, 4), (130, 64, 64), (64, 60, 8)])
+def test_fully_connected_layers_of_one_or_two_k_blocks(F, shape):
+    """Forward and input gradient keep the large products' accumulator apart from the small ones'."""
+    import torch
+    N, C, K = shape
+    g = torch.Generator(device="cuda").manual_seed(10)
+    x, w, gy = (torch.randn(*s, 1, 1, device="cuda", generator=g) for s in ((N, C), (K, C), (N, K)))
+    y, gx = F.convmm_forward(x, w, None, 1, 1, 0, 0).view(N, K), F.convmm_grad_input(gy, w, 1, 1, 1, 1, 0, 0).view(N, C)
+    xd, wd, gd = (t.double().flatten(1) for t in (x, w, gy))
+    # truncated operands 3.5e-7; two chains of four and eight truncations, the longer one at 2^-10 of the sum: 2e-7
+    for got, want in ((y, xd @ wd.t()), (gx, gd @ wd)):
+        assert float((got.double() - want).norm() / want.norm()) <= 5.5e-7
