@@ -67,7 +67,7 @@ __device__ __forceinline__ void finish_stats_channel_warp(const ChunkStat *part,
 // (16-byte pieces where planes allow it, else elements) in (image, plane) order, and a warp walks it 32 items at a time, U loads in flight
 // and U independent sums per lane.  Nothing waits for another warp, so chunks can be short and the GPU evenly full whatever N, C and
 // S are.  CTAs that reduced whole images of a channel spent more on probing the shift, two block reductions and their ticket than on
-// data: 128 x 512 x 14 x 14 (51 MB), cold cache: forward sums 24.3 us, gradient sums 28.7 us (103 MB).
+// data: 128 x 512 x 14 x 14, cold cache: forward sums (51 MB) 25.8 us with them, 20.4 us with warps; gradient sums (103 MB) 34.6 and 27.9 us.
 template <typename T>
 struct ChunkWalk {
     int i, L, rstep, left;            // item in the plane, items per plane, 32 mod L, items of this lane still to come
@@ -1116,9 +1116,10 @@ static const bool g_group_bytes_from_env = [] {
 }();
 #endif
 
-// 0: never use the grouped kernels; 1 (default): where measurements show they win — the training forward pass with
-// channel slabs of at least 6 MB (below that the per-group hand-offs cost more than the saved pass; the backward
-// kernel moves the algorithmic 3 passes but is instruction-bound and 10-20 % slower than the two-launch path);
+// 0: never use the grouped kernels; 1 (default): the training forward pass with channel slabs of at least 6 MB — two launches / grouped,
+// in us: 128 x 64 x 112 x 112 (6.4 MB) 221 / 212, 256 x 64 x 112 x 112 (12.8) 423 / 416, 1024 x 64 x 56 x 56 (12.8) 459 / 415, 1024 x 128 x
+// 56 x 56 (12.8) 895 / 825, 1024 x 32 x 112 x 112 (51.4) 831 / 833, but 512 x 32 x 112 x 112 (25.7) 419 / 450; below, the plan has too little
+// work per group.  The backward kernel moves the algorithmic 3 passes but is instruction-bound and 10-20 % slower than two launches;
 // 2: wherever they apply.
 static int g_grouped_mode = 1;
 static const size_t kGroupedMinSlab = (size_t)6 << 20;

@@ -7,7 +7,8 @@
 // A strided input gradient is taken apart into dH x dW phases: the input pixels with (h + padH) mod dH = a and
 // (w + padW) mod dW = b are reached by the taps of that residue only, and for them the sum is a stride-1 convolution of gy
 // with those taps.  A phase is therefore an ordinary GEMM whose rows are the phase's pixels and whose reduction runs over
-// (ko, the phase's taps); no product with a zero is formed.  All phases are tiles of one launch, longest reduction first.
+// (ko, the phase's taps); no product with a zero is formed.  All phases are tiles of one launch, longest reduction first, but for those
+// whose sums are short, or which fill too little of a tile: phase_fma_kernel takes them in fp32.
 //
 // Tiles, split (3xTF32), descriptors and the copies' ring are those of pw::pw_gemm_kernel.  What differs is the
 // accumulation: the tensor core truncates when it adds to an accumulator, and an error of about 1e-7 of the result grows
@@ -19,11 +20,11 @@
 // no further barrier exists.
 //
 // Bound by the producers: 4-byte copies of the gathered operands (128 + up to 128 warp instructions per k-block, those of the weights
-// 9 to 10 cache lines each) and the split; the tensor pipe needs 768 of the 4,700 clocks that a k-block takes.  Input gradient of
-// 64 x 128 x 56 x 56, 256 filters 3x3 stride 2: 44.9 ms with a thread per pixel, 0.47 ms here (63 TFLOP/s); forward of the transposed
-// 64 x 256 x 14 x 14 -> 128 x 28 x 28, 4x4: 26.9 ms and 0.27 ms (95 TFLOP/s).
-// Relative error (2-norm) of those two: 4.7e-7 and 5.6e-7 before, 1.5e-7 and 1.6e-7 now; over reductions of 16 to 9000 products 1.2e-7 to
-// 9.4e-7 before and 1.3e-7 to 2.1e-7 now.
+// 9 to 10 cache lines each) and the split; the tensor pipe needs 768 of the 4,400 clocks that a k-block takes.  Input gradient of
+// 64 x 128 x 56 x 56, 256 filters 3x3 stride 2: 44.9 ms with a thread per pixel, 0.43 ms here (69 TFLOP/s); forward of the transposed
+// 64 x 256 x 14 x 14 -> 128 x 28 x 28, 4x4: 26.9 ms and 0.245 ms (54 TFLOP/s).
+// Relative error (2-norm) of those two: 4.7e-7 and 5.6e-7 before, 1.6e-7 and 1.7e-7 now; over sums of 48 to 9216 products 1.3e-7 to
+// 1.6e-6 before and 1.2e-7 to 3.3e-7 now; shorter ones are the same sums as before.
 #pragma once
 
 namespace pwg {

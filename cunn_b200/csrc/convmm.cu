@@ -8,19 +8,21 @@
 //
 //   forward      D[pixel, k_out]        = sum_{c,kh,kw}  x(pixel; c,kh,kw)   * W[k_out][c,kh,kw]
 //   input grad   D[pixel, c]            = sum_{k,kh,kw}  gy(pixel; k,kh,kw)  * W[k][c][flipped kh,kw]   (stride 1)
-//   weight grad  D[k_out, (c,kh,kw)]    = sum_{img,pix}  gy[img][k_out][pix] * x(pix; c,kh,kw)          (split over images)
+//   weight grad  D[k_out, (c,kh,kw)]    = sum_{img,pix}  gy[img][k_out][pix] * x(pix; c,kh,kw)          (split over pixels)
 //
-// Three kernel families share these roles:
-//   * pw::pw_gemm_kernel<OP, BN, KS> — the persistent, warp-specialised kernel (further down): KS = 1 for 1x1
-//     stride-1 convolutions whose operands are plain matrices in memory, KS = 3 / 0 for 3x3 / any kernel of up to
-//     32 taps gathered element by element with asynchronous copies;
+// Five kernel families share these roles:
+//   * pwt::pw_tma_kernel<OP, BN, ...> (pw_tma.cuh) — 1x1 stride-1 convolutions on aligned tensors, and fully connected layers;
+//   * pw::pw_gemm_kernel<OP, BN, KS> — the persistent, warp-specialised kernel (further down): KS = 1 for the other 1x1
+//     stride-1 convolutions, whose operands are plain matrices in memory, KS = 3 / 0 for 3x3 / any other kernel gathered element
+//     by element with asynchronous copies: of up to 32 taps, in the weight gradient of up to 16 rows and columns (256 taps);
 //   * conv_gemm_kernel<OP, BN> (next) — one CTA per 128 x BN tile for kernels of more than 16 rows or columns: all 256
 //     threads gather operand values (two k-blocks in flight in registers), split them and store 16-byte pieces
 //     into K-major tiles in the 128-byte swizzle; one thread issues the MMAs of the k-block and commits them to
 //     the mbarrier that frees the stage; the epilogue reads the accumulator with tcgen05.ld (lane = tile row)
 //     and writes coalesced NCHW rows;
-//   * stemconv.cu — fp32-pipe kernels for the 3-channel 3x3 first layer.
-//   * pwg::gather_gemm_kernel<OP, BN> (conv_gather.cuh) — strided input gradients, one GEMM per stride residue, summed in registers.
+//   * stemconv.cu — fp32-pipe kernels for the 3-channel 3x3 first layer;
+//   * pwg::gather_gemm_kernel<OP, BN> (conv_gather.cuh) — strided input gradients, one GEMM per stride residue, summed in registers, and
+//     both passes of kernels of more than 32 taps; pwg::phase_fma_kernel for the residues that are better off in fp32.
 // Every wait is bounded.
 #include "common.cuh"
 #include "stemconv.h"
@@ -709,7 +711,7 @@ __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;"
 
 // Where the operand loads of one thread stand: tile, k-block and the thread's element offsets inside that tile.
 // M/N-major pieces: lane = group of 4 rows, k = warp + 16 i.  K-major pieces: chunk kc = tid & 7, rows (tid >> 3) + 64 i.
-// KS = 1: pointwise.  KS = 3 / 0: 3x3 / any kernel of up to 32 taps, any stride and padding: the same tiles, but
+// KS = 1: pointwise.  KS = 3 / 0: 3x3 / any kernel of up to 32 taps (weight gradient: 256), any stride and padding: the same tiles, but
 // the unfolded operand is gathered with 4-byte copies (zero-filled outside the image).
 template <int OP, int BN, int KS>
 struct Loader {

@@ -17,7 +17,7 @@
 //                6e-8 against 3.5e-8 to 1.2e-7 (2-norm; chains of 32 terms: 4.3e-8 to 1.1e-7).
 //
 // Forward / input gradient / parameter gradient on a cold cache, in us: 32 x 96 x 57 x 43, 5x5 stride 2: 671 in all before,
-// 36 / 33 / 57 now (38 MB a pass: 6 us); 12 x 144 x 37 x 29, 3x3 stride 1 (rows of an odd length): 15 / 17 / 34.  What is left is
+// 35 / 30 / 54 now (38 MB a pass: 6 us); 12 x 144 x 37 x 29, 3x3 stride 1 (rows of an odd length): 13 / 16 / 33.  What is left is
 // the 4-byte copies and the wait of a CTA for its only tile, which other CTAs of the SM fill.
 #pragma once
 

@@ -230,3 +230,21 @@ def test_short_sums_lose_no_bits(F, shape):
         assert torch.equal(gx, chain)
     # above the limit the tensor cores' error is the smaller one on average; a tenth covers the scatter of one draw
     assert err(gx) <= 1.1 * err(chain)
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, K, H, k, d, pad: sums of 64 to 9216 products on the tensor cores
+    (2, 40, 64, 26, 1, 2, 0), (4, 128, 256, 28, 3, 2, 1), (1, 96, 1024, 15, 3, 2, 1), (1, 40, 1024, 14, 6, 2, 2), (8, 128, 256, 28, 4, 2, 1),
+])
+def test_long_sums_do_not_drift(F, shape):
+    import torch
+    N, C, K, H, k, d, p = shape
+    o = (H + 2 * p - k) // d + 1
+    g = torch.Generator(device="cuda").manual_seed(11)
+    gy, w = torch.randn(N, K, o, o, device="cuda", generator=g), torch.rand(K, C, k, k, device="cuda", generator=g) * 2 - 1
+    want = torch.nn.grad.conv2d_input((N, C, H, H), w.double(), gy.double(), d, p)
+    gx = F.convmm_grad_input(gy, w, H, H, d, d, p, p)
+    # 2-norm: 0.8e-7 from parts of 11 rounded bits without lo * lo and 1e-7 from a k-block's truncations at the size of its own sum, which do
+    # not grow with the blocks' number b; its additions round a growing sum, 2^-24 / sqrt(12) of sqrt(i / b) each: 1.8e-8 sqrt(b / 2)
+    blocks = -(-K * (-(-k // d)) ** 2 // 32)
+    assert float((gx.double() - want).norm() / want.norm()) <= 1.7e-7 + 1.8e-8 * (blocks / 2) ** 0.5
