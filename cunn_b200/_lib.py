@@ -49,6 +49,12 @@ _decl("cunn_b200_full_conv_forward", c_int, [c_void_p] * 4 + _FCONV + [c_void_p]
 _decl("cunn_b200_full_conv_grad_input", c_int, [c_void_p] * 3 + _FCONV + [c_void_p])
 _decl("cunn_b200_full_conv_acc_grad_workspace", c_size_t, _FCONV)
 _decl("cunn_b200_full_conv_acc_grad", c_int, [c_void_p] * 4 + _FCONV + [c_float, c_void_p, c_size_t, c_void_p])
+_decl("cunn_b200_conv_scratch", c_size_t, [c_int] + _DCONV)
+_decl("cunn_b200_conv_forward_scratch", c_int, [c_void_p] * 4 + _DCONV + [c_void_p, c_size_t, c_void_p])
+_decl("cunn_b200_conv_grad_input_scratch", c_int, [c_void_p] * 3 + _DCONV + [c_void_p, c_size_t, c_void_p])
+_decl("cunn_b200_full_conv_scratch", c_size_t, [c_int] + _FCONV)
+_decl("cunn_b200_full_conv_forward_scratch", c_int, [c_void_p] * 4 + _FCONV + [c_void_p, c_size_t, c_void_p])
+_decl("cunn_b200_full_conv_grad_input_scratch", c_int, [c_void_p] * 3 + _FCONV + [c_void_p, c_size_t, c_void_p])
 _LCONV = _CONV + [c_int, c_int]  # ... oH oW
 _decl("cunn_b200_local_conv_forward", c_int, [c_void_p] * 4 + _LCONV + [c_void_p])
 _decl("cunn_b200_local_conv_grad_input", c_int, [c_void_p] * 3 + _LCONV + [c_void_p])

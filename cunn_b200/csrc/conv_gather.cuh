@@ -418,12 +418,6 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
     if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
-// One residue of an axis of an input gradient: input positions h0 + i * d (i < n) are reached by taps k0 + t * kstep
-// (t < taps) at output positions o0 + i - t * ostep.
-struct AxisPhase {
-    int h0, n, k0, taps, kstep, o0, ostep;
-};
-
 // Sums of fewer products are taken in fp32.  The split and the truncation of a k-block's chain cost 8e-8 to 1.2e-7 of a sum however
 // short it is, a chain of n fp32 FMAs about 1.8e-8 sqrt(n + 1): 7.4e-8 (fp32) and 9.3e-8 (tensor cores) at 16 products, 1.15e-7 and
 // 1.19e-7 at 40, 1.27e-7 and 1.17e-7 at 48, 2.0e-7 and 1.3e-7 at 128 (2-norm, normal gy, weights of either sign).

@@ -1,0 +1,1249 @@
+// Convolutions of more than one tap on operands that are split once.
+//
+// The kernels of convmm.cu gather every operand value for every tap and split it on the way: for a 3x3 layer each input value is
+// copied with 4-byte copies, and split, nine times per column tile, and the warps that do so are what the layer waits for.  Here a
+// first pass over the tensors writes every value once, as two fp16 parts in pixel-major order (channels contiguous), and the matrix
+// kernel fetches its tiles with im2col tensor-map copies: 128 consecutive output pixels x 32 channels of one tap are one copy, zeros
+// outside the image included, in the layout that the tensor core reads.  No thread touches an operand again.
+//
+// Split.  v = (hi + lo) * 2^e with hi, lo of 11 bits each, products hi*hi + hi*lo + lo*hi: the same bits as the 3xTF32 split with
+// rounding (tf32 and fp16 have 11-bit significands), at twice the rate of tf32 and half its bytes.  fp16 has five exponent bits, so
+// values are scaled by powers of two, which is exact:
+//   * activations of the forward pass and of input gradients: one exponent per pixel and group of 64 channels, that of its largest
+//     finite value.  It varies along the reduction, so the tensor core sums one block of 64 channels at a time and the block's sum
+//     is scaled when it is added to fp32 registers.
+//   * weights: one exponent per filter (input gradient: per input channel), applied when the result is written.
+//   * weight gradients reduce over pixels: one exponent per channel of x and of gy, found by a pass over both.
+// A value is kept to max(2^-23 |v|, 2^-40 of the largest in its group).  Infinities and NaN stay what they are (lo = 0) and do not
+// count for the exponent.
+//
+// Accumulation: the tensor core truncates when it adds, so a chain is one block, 64 channels (or pixels) of 12 additions, the eight of
+// the cross terms first, while the accumulator is small; blocks are added in registers with rounding (two TMEM buffers in turn).
+//
+// Forward / input gradient / parameter gradient in us, gathering kernels before and now: 3x3 256 -> 256 on 128 x 14 x 14 270 / 313 / 354 and
+// 102 / 100 / 160 (87 TFLOP/s and 290 in the first two); 3x3 stride 2 128 -> 256 on 64 x 56 x 56 312 / 427 / 360 and 139 / 181 / 248; 4x4
+// stride 2 transposed 256 -> 128 on 64 x 14 x 14 240 / 193 / 172 and 77 / 62 / 95.  2-norm errors of the first 9.7e-7 / 2.1e-6 / 2.7e-6 and 0.8e-7 /
+// 1.6e-7 / 1.9e-7.  Of 102 us of a pass the split takes 15.  The matrix kernel needs 1,130 clocks per 128 x 256 x 32 block, where the tensor
+// pipe needs 768 and reading its operands from shared memory, and filling them, 940.
+//
+// Work: 128 x BN tiles of the persistent grid; the tiles of a last wave that would leave SMs idle are cut along the reduction, and the
+// CTA that finishes a tile last adds its parts in their order (a counter per tile; nobody waits).
+#include "axis_phases.h"
+#include "conv_split.h"
+#include "umma.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <new>
+
+namespace cunn {
+namespace split {
+
+using namespace mm;
+
+constexpr int BM = 128;                  // tile rows (TMEM lanes)
+constexpr int BK = 32;                   // reduction values per stage
+constexpr int GROUP = 64;                // channels that share an exponent; M/N-major operands: values per 128-byte row
+constexpr int EPI_WARPS = 8;
+constexpr int MMA_WARP = EPI_WARPS + 3;            // two warpgroups that sum, then three warps that issue copies and one for the MMAs
+constexpr int THREADS = (MMA_WARP + 1) * 32;
+// Registers: the block is launched with 168 a thread (65,536 / 384); 2 x 224 + 56 = 3 x 168.
+constexpr int SUM_REGS = 224, ISSUE_REGS = 56;
+constexpr int MAX_PHASES = 4;            // stride 2
+constexpr size_t RING_BYTES = 192 * 1024;
+constexpr size_t SMEM = RING_BYTES + EPI_WARPS * 4096;
+constexpr int SCALED_MAX = 14;           // the largest value of a group lies in [2^14, 2^15) after scaling
+
+
+// ---- exponents ----------------------------------------------------------------------------------------------------------------
+// Exponent of a group from the bits of its largest finite magnitude; 2^(SCALED_MAX - e) is a normal number.
+__device__ __forceinline__ int group_exp(uint32_t max_bits) { return max((int)(max_bits >> 23) - 127, -112); }
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }      // -126 <= e <= 127
+// s * 2^e, |e| <= 252, in two steps that neither overflow nor lose bits unless the result does
+__device__ __forceinline__ float scale_by(float s, int e)
+{
+    const int h = e / 2;
+    return s * pow2(h) * pow2(e - h);
+}
+__device__ __forceinline__ bool finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ float finite_abs(float v) { return finite(v) ? fabsf(v) : 0.f; }
+// The two parts of v * s; lo of what is not finite is zero.
+__device__ __forceinline__ void parts(float v, float s, __half &hi, __half &lo)
+{
+    const float t = v * s;
+    hi = __float2half_rn(t);
+    lo = finite(v) ? __float2half_rn(t - __half2float(hi)) : __float2half_rn(0.f);
+}
+
+// ---- splitting --------------------------------------------------------------------------------------------------------------------
+struct Act {                     // [images][C][HW] fp32 -> hi, lo: [2][images * HW][Cp] fp16
+    const float *src;
+    __half *dst;
+    int8_t *exps;                // per pixel and group: exponent; null: exponents come from chmax
+    const uint32_t *chmax;       // per channel: bits of the largest finite magnitude
+    double *bias_part;           // [blocks of 64 pixels][C] sums of src, or null
+    int C, Cp, HW, groups, blocks;
+    int vec;                     // planes of a multiple of four values, 16-byte aligned
+    uint32_t pixels;
+};
+struct PrepParams {
+    Act act[2];
+    int n_act;
+    // weights, one block per row (filter, or input channel of an input gradient): value (row, c, tap) at row * w_row + c * w_c + tap
+    const float *w;
+    __half *w_dst;               // [2][taps][rows][Cp]
+    int *w_exp;                  // [rows]: exponent
+    int rows, w_C, w_Cp, taps;
+    long long w_row, w_c;
+    int *tickets;
+    int n_tickets;
+};
+
+__device__ __forceinline__ void prep_weights(const PrepParams &p, int row)
+{
+    __shared__ uint32_t red[8];
+    const float *w = p.w + (long long)row * p.w_row;
+    const int n = p.w_C * p.taps;
+    float m = 0.f;
+    for (int i = threadIdx.x; i < n; i += 256) {
+        const int c = i / p.taps, t = i - c * p.taps;
+        m = fmaxf(m, finite_abs(__ldg(w + c * p.w_c + t)));
+    }
+    uint32_t b = __float_as_uint(m);
+    b = __reduce_max_sync(0xffffffffu, b);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = b;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) b = max(b, red[i]);
+    const int e = group_exp(b);
+    if (threadIdx.x == 0) p.w_exp[row] = e;
+    const float s = pow2(SCALED_MAX - e);
+    const size_t part = (size_t)p.taps * p.rows * p.w_Cp;
+    for (int i = threadIdx.x; i < p.w_Cp * p.taps; i += 256) {
+        const int t = i / p.w_Cp, c = i - t * p.w_Cp;
+        __half hi, lo;
+        parts(c < p.w_C ? __ldg(w + c * p.w_c + t) : 0.f, s, hi, lo);
+        __half *d = p.w_dst + ((size_t)t * p.rows + row) * p.w_Cp + c;
+        d[0] = hi;
+        d[part] = lo;
+    }
+}
+
+// One block: 64 pixels (of the flat pixel sequence) x 64 channels, through shared memory: read along the pixels, written along the
+// channels, a warp four pixels of 128 bytes at a time (16 bytes of each of 32 pixels per instruction took twice as long).
+template <bool PER_CHANNEL>
+__device__ __forceinline__ void prep_act(const Act &a, int block)
+{
+    __shared__ float tile[GROUP][65];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int pb = block / a.groups, g = block - pb * a.groups;
+    const uint32_t p0 = (uint32_t)pb * 64u;
+    double sums[8];
+    if (a.vec) {
+        // four consecutive pixels of a channel: lanes 0-15 of one, 16-31 of the next
+        const uint32_t px = p0 + (lane & 15) * 4, im = px / (uint32_t)a.HW;
+        const bool ok = px < a.pixels;                                    // pixels is a multiple of four
+        const float *src = a.src + (ok ? (size_t)im * a.C * a.HW + (px - im * a.HW) : 0);
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = g * GROUP + warp * 8 + i * 2 + (lane >> 4);
+            v[i] = ok && c < a.C ? __ldg(reinterpret_cast<const float4 *>(src + (size_t)c * a.HW)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float *t = &tile[warp * 8 + i * 2 + (lane >> 4)][(lane & 15) * 4];
+            t[0] = v[i].x; t[1] = v[i].y; t[2] = v[i].z; t[3] = v[i].w;
+            sums[i] = ((double)v[i].x + (double)v[i].y) + ((double)v[i].z + (double)v[i].w);
+        }
+    } else {
+        const float *src[2];
+        bool ok[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t px = p0 + h * 32 + lane, im = px / (uint32_t)a.HW;
+            ok[h] = px < a.pixels;
+            src[h] = a.src + (ok[h] ? (size_t)im * a.C * a.HW + (px - im * a.HW) : 0);
+        }
+        float v[8][2];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = g * GROUP + warp * 8 + i;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) v[i][h] = ok[h] && c < a.C ? __ldg(src[h] + (size_t)c * a.HW) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) tile[warp * 8 + i][h * 32 + lane] = v[i][h];
+            sums[i] = (double)v[i][0] + (double)v[i][1];
+        }
+    }
+    if (a.bias_part) {
+        const int channels = a.vec ? 4 : 8, top = a.vec ? 8 : 16;          // lanes that share a channel: 16 or all
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i >= channels) break;
+            double s = sums[i];
+            for (int o = top; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const int c = g * GROUP + warp * 8 + (a.vec ? i * 2 + (lane >> 4) : i);
+            if ((lane & (a.vec ? 15 : 31)) == 0 && c < a.C) a.bias_part[(size_t)pb * a.C + c] = s;
+        }
+    }
+    const int piece = lane & 7, c0 = g * GROUP + piece * 8;               // eight channels of a pixel
+    float f[8];
+    if (PER_CHANNEL) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = pow2(SCALED_MAX - group_exp(c0 + i < a.C ? __ldg(a.chmax + c0 + i) : 0u));
+    }
+    __syncthreads();
+    const size_t part = (size_t)a.pixels * a.Cp;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int col = warp * 8 + h * 4 + (lane >> 3);
+        const uint32_t px = p0 + col;
+        float r[8], m = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = tile[piece * 8 + i][col];
+        if (!PER_CHANNEL) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) m = fmaxf(m, finite_abs(r[i]));
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            const int e = group_exp(__float_as_uint(m));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = pow2(SCALED_MAX - e);
+            if (piece == 0 && px < a.pixels) a.exps[(size_t)px * a.groups + g] = (int8_t)e;
+        }
+        if (px < a.pixels && c0 < a.Cp) {
+            __align__(16) __half hi[8];
+            __align__(16) __half lo[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) parts(r[i], f[i], hi[i], lo[i]);
+            __half *d = a.dst + (size_t)px * a.Cp + c0;
+            *reinterpret_cast<uint4 *>(d) = *reinterpret_cast<const uint4 *>(hi);
+            *reinterpret_cast<uint4 *>(d + part) = *reinterpret_cast<const uint4 *>(lo);
+        }
+    }
+}
+
+template <bool PER_CHANNEL>
+__global__ void __launch_bounds__(256)
+prep_kernel(const __grid_constant__ PrepParams p)
+{
+    pdl_wait();
+    pdl_launch_dependents();
+    int b = (int)blockIdx.x;
+    if (b == 0)
+        for (int i = threadIdx.x; i < p.n_tickets; i += 256) p.tickets[i] = 0;
+    if (b < p.rows) {
+        prep_weights(p, b);
+        return;
+    }
+    b -= p.rows;
+    if (b < p.act[0].blocks) prep_act<PER_CHANNEL>(p.act[0], b);
+    else if (p.n_act > 1) prep_act<PER_CHANNEL>(p.act[1], b - p.act[0].blocks);
+}
+
+// Largest finite magnitude of every channel: block = (channel, chunk of images), a warp per plane.
+struct MaxParams {
+    const float *src[2];
+    uint32_t *chmax[2];
+    int C[2], HW[2], chunks[2], vec[2], images;       // vec: planes of a multiple of four values, 16-byte aligned
+};
+__global__ void __launch_bounds__(256)
+channel_max_kernel(const __grid_constant__ MaxParams p)
+{
+    pdl_launch_dependents();
+    __shared__ uint32_t red[8];
+    int b = (int)blockIdx.x, t = 0;
+    if (b >= p.C[0] * p.chunks[0]) { b -= p.C[0] * p.chunks[0]; t = 1; }
+    const int chunk = b / p.C[t], c = b - chunk * p.C[t], HW = p.HW[t], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = (int)((long long)p.images * chunk / p.chunks[t]), n1 = (int)((long long)p.images * (chunk + 1) / p.chunks[t]);
+    const size_t step = (size_t)p.C[t] * HW;
+    const float *src = p.src[t] + (size_t)c * HW;
+    float m = 0.f;
+    for (int n = n0 + warp; n < n1; n += 32) {                             // four planes at a time; those past the last repeat the first
+        const float *s[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[j] = src + (size_t)(n + 8 * j < n1 ? n + 8 * j : n) * step;
+        if (p.vec[t]) {
+#pragma unroll 2
+            for (int i = lane; i < HW / 4; i += 32) {
+                float4 v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const float4 *>(s[j]) + i);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    m = fmaxf(m, fmaxf(fmaxf(finite_abs(v[j].x), finite_abs(v[j].y)), fmaxf(finite_abs(v[j].z), finite_abs(v[j].w))));
+            }
+        } else {
+#pragma unroll 2
+            for (int i = lane; i < HW; i += 32) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) m = fmaxf(m, finite_abs(__ldg(s[j] + i)));
+            }
+        }
+    }
+    uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if (lane == 0) red[warp] = bits;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 1; i < 8; ++i) bits = max(bits, red[i]);
+        atomicMax(p.chmax[t] + c, bits);
+    }
+}
+
+// ---- matrix kernel ------------------------------------------------------------------------------------------------------------------
+// One sub-problem of the forward pass or an input gradient (a stride residue): output pixels (r / pix_W, r % pix_W) read the gathered
+// tensor at (row * stH + lH + th * dlH, col * stW + lW + tw * dlW) with the weight of tap w_base + th * w_sH + tw * w_sW, and are written
+// at o_off + row * o_sH + col * o_sW of an output plane.
+struct Phase {
+    int tile0, HW, pix_W, M_total;
+    int taps, kW, blocks;                    // blocks of the reduction: taps * Params::groups
+    int lH, lW, stH, stW, dlH, dlW;
+    int w_base, w_sH, w_sW;
+    int o_off, o_sH, o_sW;
+};
+struct Params {
+    const int8_t *exps;                      // exponent per (pixel, group) of the gathered tensor
+    const int *w_exp;                        // ... per column
+    const float *bias;                       // or null
+    float *out, *partial;
+    int *tickets, *status;
+    const float *raw_a, *raw_w;              // the operands in fp32, for sums that came out as NaN; null: left as they are
+    int images, g_C, g_H, g_W, groups;
+    int w_kk, o_HW, N_total, n_tiles, width; // columns in all, column tiles and a tile's columns
+    int n_phases, full, splits, items;       // items [0, full) are whole tiles, then `splits` parts of each further tile
+    // weight gradient: rows = output channels, columns = (tap, group of 64 input channels) pairs, reduction over pixels
+    int m_tiles, tiles, blocks, per_split, col_groups, kW, pix_HW, pix_W;
+    int lH, lW, stH, stW, dlH, dlW;
+    Phase ph[MAX_PHASES];
+};
+struct Maps {
+    CUtensorMap a[MAX_PHASES];               // weight gradient: [0] gy
+    CUtensorMap b;
+};
+
+__device__ __forceinline__ void load_im2col(uint32_t dst, const CUtensorMap *map, int c, int w, int h, int n, int ow, int oh, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6], {%7, %8};"
+                 ::"r"(dst), "l"((uint64_t)map), "r"(c), "r"(w), "r"(h), "r"(n), "r"(bar), "h"((uint16_t)ow), "h"((uint16_t)oh) : "memory");
+}
+__device__ __forceinline__ void load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_f16_acc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
+{
+    asm volatile("tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, 1;" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc) : "memory");
+}
+
+// What item i of the work list is.
+struct Item {
+    int phase, m_tile, n_tile, part, tail, begin, end;       // tail: index among the tiles that are cut, -1: a whole tile
+};
+template <bool WG>
+__device__ __forceinline__ Item item_of(const Params &p, int i)
+{
+    Item it;
+    it.phase = 0;
+    if (WG) {
+        it.part = i / p.tiles;
+        const int t = i - it.part * p.tiles;
+        it.m_tile = t / p.n_tiles;
+        it.n_tile = t - it.m_tile * p.n_tiles;
+        it.tail = 0;
+        it.begin = it.part * p.per_split;
+        it.end = min(it.begin + p.per_split, p.blocks);
+        return it;
+    }
+    int t = i;
+    it.part = 0;
+    it.tail = -1;
+    if (i >= p.full) {
+        const int j = i - p.full;
+        it.tail = j / p.splits;
+        it.part = j - it.tail * p.splits;
+        t = p.full + it.tail;
+        if (p.splits == 1) it.tail = -1;
+    }
+    while (it.phase + 1 < p.n_phases && t >= p.ph[it.phase + 1].tile0) ++it.phase;
+    const Phase &f = p.ph[it.phase];
+    const int r = t - f.tile0;
+    it.m_tile = r / p.n_tiles;
+    it.n_tile = r - it.m_tile * p.n_tiles;
+    it.begin = 0;
+    it.end = f.blocks;
+    if (it.tail >= 0) {
+        it.begin = (int)((long long)f.blocks * it.part / p.splits);
+        it.end = (int)((long long)f.blocks * (it.part + 1) / p.splits);
+    }
+    return it;
+}
+
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+          "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+// The wait names the registers, so that nothing reads them before it.
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                   "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]),
+                   "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]),
+                   "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); }
+
+// One input-gradient value in plain fp32: products with the zeros in place of taps outside gy, or of an infinity's parts, can make a
+// NaN that the definition does not have.
+__device__ float plain_sum(const Params &p, const Phase &f, int im, int row, int col, int n)
+{
+    const float *src = p.raw_a + (size_t)im * p.g_C * p.g_H * p.g_W;
+    float s = 0.f;
+#pragma unroll 1
+    for (int th = 0; th < f.taps / f.kW; ++th) {
+        const int ih = row * f.stH + f.lH + th * f.dlH;
+        if ((unsigned)ih >= (unsigned)p.g_H) continue;
+#pragma unroll 1
+        for (int tw = 0; tw < f.kW; ++tw) {
+            const int iw = col * f.stW + f.lW + tw * f.dlW;
+            if ((unsigned)iw >= (unsigned)p.g_W) continue;
+#pragma unroll 8
+            for (int c = 0; c < p.g_C; ++c)
+                s = fmaf(__ldg(p.raw_w + ((size_t)c * p.N_total + n) * p.w_kk + f.w_base + th * f.w_sH + tw * f.w_sW),
+                         __ldg(src + ((size_t)c * p.g_H + ih) * p.g_W + iw), s);
+        }
+    }
+    return s;
+}
+
+// Exponents below every group's: of pixels outside the tensor, and of a row before its first block.
+constexpr int NO_EXP = -120;
+// 2^(e - top) for e <= top; what lies 2^126 below the row's largest block is nothing.
+__device__ __forceinline__ float step(int e, int top) { return top - e > 126 ? 0.f : pow2(e - top); }
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) { return (uint64_t)__float_as_uint(hi) << 32 | __float_as_uint(lo); }
+// two fp32 operations, each rounded as the scalar one
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+template <int N>
+__device__ __forceinline__ void raise(uint64_t (&acc2)[N], int &top, int to)
+{
+    const float f = step(top, to);
+    const uint64_t f2 = pack2(f, f);
+#pragma unroll
+    for (int j = 0; j < N; ++j) acc2[j] = mul2(acc2[j], f2);
+    top = to;
+}
+
+// Warps 0-7: sums (TMEM -> registers -> memory), two per TMEM lane quarter, each half of the columns; warps 8-10: copies; warp 11: MMAs.
+template <int BN, bool WG>
+__global__ void __launch_bounds__(THREADS, 1)
+split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps)
+{
+    constexpr int STAGE = 2 * BK * 2 * (BM + BN), NS = (int)(RING_BYTES / STAGE);
+    constexpr int A_PART = BM * BK * 2, B_PART = BN * BK * 2, A_LO = A_PART, B_HI = 2 * A_PART, B_LO = B_HI + B_PART;
+    constexpr int HALF_COLS = BN / 2;
+    constexpr uint32_t TMEM_COLS = 2 * BN;
+    constexpr size_t PART = BN * BM + BM;             // partial sums of a cut tile and their rows' exponents
+
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ uint64_t full[NS], empty[NS];          // stage landed; its MMAs are done
+    __shared__ uint64_t ready[2], drained[2];         // a block's sums are in TMEM buffer b; they have been read
+    __shared__ uint32_t tmem_base_s;
+    __shared__ int last_s;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < NS; ++s) { mbar_init(smem_u32(full + s), 1); mbar_init(smem_u32(empty + s), 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(ready + b), 1); mbar_init(smem_u32(drained + b), EPI_WARPS); }
+        mbar_fence_init();
+    }
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_base_s), TMEM_COLS);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_s;
+    pdl_wait();
+    pdl_launch_dependents();
+
+    if (warp >= EPI_WARPS) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ISSUE_REGS));
+      if (warp < MMA_WARP) {
+        // A thread's copies start about 100 clocks apart and 4 or 8 KB each take 60 to 180, so three warps share them.
+        const int part_of = warp - EPI_WARPS;
+        if (lane == 0) {
+            int rs = 0;
+            uint32_t parity = 1;                      // the first round finds the stages empty
+            bool ok = true;
+            for (int i = (int)blockIdx.x; ok && i < p.items; i += (int)gridDim.x) {
+                const Item it = item_of<WG>(p, i);
+                if (!WG) {
+                    const Phase &f = p.ph[it.phase];
+                    const int m0 = it.m_tile * BM, im = m0 / f.HW, r = m0 - im * f.HW, row = r / f.pix_W, col = r - row * f.pix_W;
+                    const int h0 = row * f.stH + f.lH, w0 = col * f.stW + f.lW, n0 = it.n_tile * p.width;
+                    const int tap = it.begin / p.groups;
+                    int c = (it.begin - tap * p.groups) * GROUP, th = tap / f.kW, tw = tap - th * f.kW;
+                    const CUtensorMap *ma = &maps.a[it.phase];
+                    for (int q = it.begin; q < it.end;) {
+                        if (!mbar_wait(smem_u32(empty + rs), parity, p.status)) { ok = false; break; }
+                        const uint32_t bar = smem_u32(full + rs), s = smem_u32(smem) + (uint32_t)(rs * STAGE);
+                        if (part_of == 0) mbar_arrive_expect_tx(bar, STAGE);
+                        if (part_of < 2) {
+                            load_im2col(s + (uint32_t)(part_of * A_LO), ma, c, w0, h0, im + part_of * p.images, tw * f.dlW, th * f.dlH, bar);
+                        } else {
+                            const int wt = f.w_base + th * f.w_sH + tw * f.w_sW;
+                            load_3d(s + B_HI, &maps.b, c, n0, wt, bar);
+                            load_3d(s + B_LO, &maps.b, c, n0, wt + p.w_kk, bar);
+                        }
+                        c += BK;
+                        if (c >= p.g_C) { c = 0; if (++tw == f.kW) { tw = 0; ++th; } }
+                        if ((c & (GROUP - 1)) == 0) ++q;                           // the group's last stage
+                        if (++rs == NS) { rs = 0; parity ^= 1u; }
+                    }
+                } else {
+                    const int g0 = it.n_tile * (BN / GROUP), ng = min(BN / GROUP, p.col_groups - g0);
+                    for (int q = 2 * it.begin; q < 2 * it.end; ++q) {
+                        if (!mbar_wait(smem_u32(empty + rs), parity, p.status)) { ok = false; break; }
+                        const uint32_t bar = smem_u32(full + rs), s = smem_u32(smem) + (uint32_t)(rs * STAGE);
+                        if (part_of == 0) mbar_arrive_expect_tx(bar, (uint32_t)(2 * A_PART + 2 * ng * GROUP * BK * 2));
+                        const int p0 = q * BK, im = p0 / p.pix_HW, r = p0 - im * p.pix_HW, row = r / p.pix_W, col = r - row * p.pix_W;
+                        const int h0 = row * p.stH + p.lH, w0 = col * p.stW + p.lW;
+                        for (int l = part_of; l < 2 * (BM / GROUP + ng); l += 3) {
+                            const int part = l & 1, j = (l >> 1) - BM / GROUP;
+                            if (j < 0) {
+                                load_3d(s + (uint32_t)(part * A_PART + (l >> 1) * GROUP * BK * 2), &maps.a[0], it.m_tile * BM + (l >> 1) * GROUP, p0, part, bar);
+                            } else {
+                                const int tap = (g0 + j) / p.groups, g = g0 + j - tap * p.groups, th = tap / p.kW, tw = tap - th * p.kW;
+                                load_im2col(s + (uint32_t)(B_HI + part * B_PART + j * GROUP * BK * 2), &maps.b, g * GROUP, w0, h0,
+                                            im + part * p.images, tw * p.dlW, th * p.dlH, bar);
+                            }
+                        }
+                        if (++rs == NS) { rs = 0; parity ^= 1u; }
+                    }
+                }
+            }
+        }
+      } else {
+        if (lane == 0) {
+            // descriptors: K-major tiles of 64-byte rows in the 64-byte swizzle (groups of 8 rows 512 bytes apart); M/N-major ones of
+            // 128-byte rows in the 128-byte swizzle (8 k values 1024 bytes, 64 values of M or N 4096 bytes apart)
+            constexpr uint32_t LOW = WG ? (uint32_t)(GROUP * BK * 2 >> 4) << 16 : 1u << 16;
+            constexpr uint32_t HIGH = (uint32_t)((WG ? 1024 : 512) >> 4) | (1u << 14) | ((WG ? 2u : 4u) << 29);
+            constexpr uint32_t STEP = WG ? 2048u >> 4 : 2u;                        // 16 k values
+            auto desc = [](uint32_t low) { return ((uint64_t)HIGH << 32) | low; };
+            const uint32_t ring = (smem_u32(smem) >> 4) & 0x3fffu;
+            int rs = 0, buf = 0;
+            uint32_t parity = 0, free_parity = 1;
+            bool ok = true;
+            for (int i = (int)blockIdx.x; ok && i < p.items; i += (int)gridDim.x) {
+                const Item it = item_of<WG>(p, i);
+                const int cols = WG ? min(BN, (p.col_groups - it.n_tile * (BN / GROUP)) * GROUP)
+                                    : min(p.width, ((p.N_total - it.n_tile * p.width) + 15) & ~15);
+                const uint32_t idesc = (1u << 4) | ((WG ? 1u : 0u) << 15) | ((WG ? 1u : 0u) << 16) | ((uint32_t)(cols >> 3) << 17) |
+                                       ((uint32_t)(BM >> 4) << 24);
+                int c = WG ? 0 : it.begin % p.groups * GROUP;
+                for (int q = it.begin; q < it.end; ++q) {
+                    if (!mbar_wait(smem_u32(drained + buf), free_parity, p.status)) { ok = false; break; }
+                    const uint32_t d = tmem_base + (uint32_t)(buf * BN);
+                    // 16-channel steps of the group that hold channels, two per stage
+                    const int steps = WG ? 4 : min(4, (p.g_C - c + 15) >> 4);
+                    // the small products first, while the accumulator is small: both stages' cross terms, then their hi*hi
+                    uint32_t st[2];
+                    const int first = rs;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (2 * h >= steps) break;
+                        if (!mbar_wait(smem_u32(full + rs), parity, p.status)) { ok = false; break; }
+                        tc_fence_after();
+                        st[h] = ring + (uint32_t)(rs * STAGE >> 4);
+                        const uint32_t ah = st[h] | LOW, al = (st[h] + (A_LO >> 4)) | LOW, bh = (st[h] + (B_HI >> 4)) | LOW, bl = (st[h] + (B_LO >> 4)) | LOW;
+                        umma_f16(d, desc(al), desc(bh), idesc, h ? 1u : 0u);       // a block's first one overwrites the buffer
+                        umma_f16_acc(d, desc(ah), desc(bl), idesc);
+                        if (2 * h + 1 < steps) {
+                            umma_f16_acc(d, desc(al + STEP), desc(bh + STEP), idesc);
+                            umma_f16_acc(d, desc(ah + STEP), desc(bl + STEP), idesc);
+                        }
+                        if (++rs == NS) { rs = 0; parity ^= 1u; }
+                    }
+                    if (!ok) break;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if (2 * h >= steps) break;
+                        const uint32_t ah = st[h] | LOW, bh = (st[h] + (B_HI >> 4)) | LOW;
+                        umma_f16_acc(d, desc(ah), desc(bh), idesc);
+                        if (2 * h + 1 < steps) umma_f16_acc(d, desc(ah + STEP), desc(bh + STEP), idesc);
+                        umma_commit(smem_u32(empty + (h == 0 ? first : first + 1 == NS ? 0 : first + 1)));
+                    }
+                    umma_commit(smem_u32(ready + buf));
+                    c += GROUP;
+                    if (c >= p.g_C) c = 0;
+                    if (buf ^= 1) {} else free_parity ^= 1u;
+                }
+            }
+        }
+      }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SUM_REGS));
+        const int quarter = warp & 3, col0 = (warp >> 2) * HALF_COLS, row_in = quarter * 32 + lane;
+        const uint32_t tsrc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
+        int buf = 0;
+        uint32_t parity = 0;
+        bool ok = true, nan_seen = false, tail_done = false;
+        // this lane's pixel of a tile
+        auto locate = [&](const Item &it, const Phase &f, int &im, int &row, int &col) {
+            const int m = it.m_tile * BM + row_in;
+            im = m / f.HW;
+            const int r = m - im * f.HW;
+            row = r / f.pix_W;
+            col = r - row * f.pix_W;
+            return m < f.M_total;
+        };
+        for (int i = (int)blockIdx.x; ok && i < p.items; i += (int)gridDim.x) {
+            const Item it = item_of<WG>(p, i);
+            const Phase &f = p.ph[it.phase];
+            uint64_t acc2[HALF_COLS / 2];                                          // columns 2 j and 2 j + 1
+#pragma unroll
+            for (int j = 0; j < HALF_COLS / 2; ++j) acc2[j] = 0;
+            const int cols = WG ? min(BN, (p.col_groups - it.n_tile * (BN / GROUP)) * GROUP) : min(p.width, p.N_total - it.n_tile * p.width);
+            const int my_cols = cols - col0;                                       // may be zero or negative
+            int im = 0, row = 0, col = 0;
+            bool row_ok = true;
+            if (!WG) row_ok = locate(it, f, im, row, col);
+            // exponents of the blocks, one ahead; the registers hold the row's sums / 2^top, which is raised before a block would exceed it
+            int g = 0, th = 0, tw = 0;
+            if (!WG) { const int tap = it.begin / p.groups; g = it.begin - tap * p.groups; th = tap / f.kW; tw = tap - th * f.kW; }
+            const int ih0 = row * f.stH + f.lH, iw0 = col * f.stW + f.lW;
+            auto exp_at = [&]() -> int {
+                const int ih = ih0 + th * f.dlH, iw = iw0 + tw * f.dlW;
+                return row_ok && (unsigned)ih < (unsigned)p.g_H && (unsigned)iw < (unsigned)p.g_W
+                           ? (int)__ldg(p.exps + (((size_t)im * p.g_H + ih) * p.g_W + iw) * p.groups + g) : NO_EXP;
+            };
+            int next = WG ? 0 : exp_at(), top = NO_EXP;
+            for (int q = it.begin; q < it.end; ++q) {
+                const int e = next;
+                if (!WG && q + 1 < it.end) {
+                    if (++g == p.groups) { g = 0; if (++tw == f.kW) { tw = 0; ++th; } }
+                    next = exp_at();
+                }
+                float s = 1.f;
+                if (!WG) {
+                    if (__any_sync(0xffffffffu, e > top)) raise(acc2, top, max(e + 4, top));
+                    s = step(e, top);
+                }
+                if (!mbar_wait(smem_u32(ready + buf), parity, p.status)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t t0 = tsrc + (uint32_t)(buf * BN);
+                const uint64_t s2 = pack2(s, s);
+                uint32_t r[2][32];
+                tmem_ld32_issue(t0, r[0]);
+#pragma unroll
+                for (int c = 0; c < HALF_COLS; c += 32) {                          // columns past the tile's hold anything and are not used
+                    tmem_wait_ld(r[(c / 32) & 1]);
+                    if (c + 32 < HALF_COLS) tmem_ld32_issue(t0 + (uint32_t)(c + 32), r[(c / 32 + 1) & 1]);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        const uint64_t v = (uint64_t)r[(c / 32) & 1][j + 1] << 32 | r[(c / 32) & 1][j];
+                        uint64_t &a = acc2[(c + j) / 2];
+                        a = WG ? add2(a, v) : fma2(v, s2, a);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(drained + buf));
+                if (buf ^= 1) {} else parity ^= 1u;
+            }
+            if (!ok) break;
+            float acc[HALF_COLS];
+#pragma unroll
+            for (int j = 0; j < HALF_COLS; j += 2) {
+                acc[j] = __uint_as_float((uint32_t)acc2[j / 2]);
+                acc[j + 1] = __uint_as_float((uint32_t)(acc2[j / 2] >> 32));
+            }
+            if (WG) {
+                // [split][column][row]: a warp writes 128 consecutive bytes of a column
+                float *dst = p.partial + ((size_t)it.part * p.n_tiles * BN + (size_t)it.n_tile * BN + col0) * (p.m_tiles * BM) + it.m_tile * BM + row_in;
+                const int stride = p.m_tiles * BM;
+#pragma unroll
+                for (int j = 0; j < HALF_COLS; ++j, dst += stride) *dst = acc[j];
+                continue;
+            }
+            if (it.tail >= 0) {
+                float *mine = p.partial + (size_t)(it.tail * p.splits + it.part) * PART + (size_t)col0 * BM + row_in;
+                int *my_top = reinterpret_cast<int *>(p.partial + (size_t)(it.tail * p.splits + it.part) * PART + BN * BM) + row_in;
+                if (col0 == 0) __stcg(my_top, top);
+#pragma unroll
+                for (int j = 0; j < HALF_COLS; ++j) __stcg(mine + j * BM, acc[j]);
+                __threadfence();
+                epilogue_sync();
+                if (tid == 0) last_s = atomicAdd(p.tickets + it.tail, 1) == p.splits - 1;
+                epilogue_sync();
+                if (!last_s) continue;
+                __threadfence();
+                const float *first = p.partial + (size_t)it.tail * p.splits * PART + row_in;
+                auto top_of = [&](int s) { return __ldcg(reinterpret_cast<const int *>(first + (size_t)s * PART + BN * BM)); };
+                top = NO_EXP;
+                for (int s = 0; s < p.splits; ++s) top = max(top, top_of(s));
+#pragma unroll
+                for (int j = 0; j < HALF_COLS; ++j) acc[j] = 0.f;
+#pragma unroll 1
+                for (int s = 0; s < p.splits; ++s) {
+                    const float w = step(top_of(s), top);
+                    const float *src = first + (size_t)s * PART + (size_t)col0 * BM;
+#pragma unroll
+                    for (int j = 0; j < HALF_COLS; ++j) acc[j] = fmaf(__ldcg(src + j * BM), w, acc[j]);
+                }
+                tail_done = true;
+            }
+            // Through shared memory, 32 columns at a time, so that the columns can be a loop: as straight code over registers, run once a
+            // tile, it is fetched from memory and took 20 us of a layer.
+            const int n0 = it.n_tile * p.width + col0;
+            float *dst = p.out + ((size_t)im * p.N_total + n0) * p.o_HW + (f.o_off + row * f.o_sH + col * f.o_sW);
+            float *stage = reinterpret_cast<float *>(smem + RING_BYTES) + warp * 1024 + lane;     // a lane reads what it wrote itself
+#pragma unroll
+            for (int c = 0; c < HALF_COLS; c += 32) {
+                if (c >= my_cols) break;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) stage[j * 32] = acc[c + j];
+                if (!row_ok) continue;
+                const int last = min(32, my_cols - c);
+#pragma unroll 4
+                for (int j = 0; j < last; ++j) {
+                    const float v = stage[j * 32];
+                    nan_seen |= v != v;
+                    dst[(size_t)(c + j) * p.o_HW] = scale_by(v, __ldg(p.w_exp + n0 + c + j) + top - 2 * SCALED_MAX) +
+                                                    (p.bias ? __ldg(p.bias + n0 + c + j) : 0.f);
+                }
+            }
+        }
+        if (!WG && p.raw_a && __any_sync(0xffffffffu, ok && nan_seen)) {
+            // outside the pipeline: no wait with a limit depends on how long this takes
+#pragma unroll 1
+            for (int i = (int)blockIdx.x; i < p.items; i += (int)gridDim.x) {
+                const Item it = item_of<WG>(p, i);
+                if (it.tail >= 0 && !tail_done) continue;
+                const Phase &f = p.ph[it.phase];
+                int im, row, col;
+                if (!locate(it, f, im, row, col)) continue;
+                const int n0 = it.n_tile * p.width + col0, my_cols = min(p.width, p.N_total - it.n_tile * p.width) - col0;
+                float *dst = p.out + ((size_t)im * p.N_total + n0) * p.o_HW + (f.o_off + row * f.o_sH + col * f.o_sW);
+#pragma unroll 1
+                for (int j = 0; j < HALF_COLS && j < my_cols; ++j) {
+                    const float b = p.bias ? __ldg(p.bias + n0 + j) : 0.f;
+                    if (isnan(dst[(size_t)j * p.o_HW]) && !isnan(b)) dst[(size_t)j * p.o_HW] = plain_sum(p, f, im, row, col, n0 + j) + b;
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// gw[ko][c][tap] += scale * the sum of the splits in their order, scaled back; further blocks: the bias gradient from its partial sums.
+// A block takes 32 output channels x 32 consecutive (c, tap): partial sums are contiguous along the output channels, gw along (c, tap).
+struct ReduceParams {
+    const float *partial;
+    float *gw, *gb;
+    const uint32_t *gy_max, *x_max;
+    const double *bias_part;
+    int K, C, kk, groups, splits, cols, rows, gw_blocks, bias_blocks;
+    float scale;
+};
+__global__ void __launch_bounds__(256)
+reduce_kernel(const __grid_constant__ ReduceParams p)
+{
+    pdl_wait();
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if ((int)blockIdx.x >= p.gw_blocks) {
+        const int k = ((int)blockIdx.x - p.gw_blocks) * 8 + warp;
+        if (k >= p.K) return;
+        double s = 0.0;
+        for (int i = lane; i < p.bias_blocks; i += 32) s += p.bias_part[(size_t)i * p.K + k];
+        s = warp_sum(s);
+        if (lane == 0) p.gb[k] = (float)((double)p.gb[k] + (double)p.scale * s);
+        return;
+    }
+    __shared__ float tile[32][33];
+    const int n = p.C * p.kk, o_blocks = (n + 31) / 32;
+    const int kb = (int)blockIdx.x / o_blocks, ob = (int)blockIdx.x - kb * o_blocks;
+    const int ko = kb * 32 + lane;
+    const size_t split_step = (size_t)p.cols * p.rows;
+    const float *src[4];
+    int c[4];
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int o = min(ob * 32 + warp + 8 * i, n - 1);
+        c[i] = o / p.kk;
+        src[i] = p.partial + (size_t)(((o - c[i] * p.kk) * p.groups + (c[i] >> 6)) * GROUP + (c[i] & 63)) * p.rows + ko;      // ko < rows
+    }
+#pragma unroll 4
+    for (int k = 0; k < p.splits; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[i] += __ldg(src[i] + k * split_step);
+    const int eg = ko < p.K ? group_exp(__ldg(p.gy_max + ko)) : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tile[warp + 8 * i][lane] = scale_by(sum[i], eg + group_exp(__ldg(p.x_max + c[i])) - 2 * SCALED_MAX);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int k = kb * 32 + warp + 8 * i, o = ob * 32 + lane;
+        if (k < p.K && o < n) p.gw[(size_t)k * n + o] += p.scale * tile[lane][warp + 8 * i];
+    }
+}
+
+// ---- host ---------------------------------------------------------------------------------------------------------------------------
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+typedef CUresult (*EncodeIm2colFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                   const int *, const int *, cuuint32_t, cuuint32_t, const cuuint32_t *, CUtensorMapInterleave,
+                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static void *driver_entry(const char *name)
+{
+    void *ptr = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &ptr, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) ptr = nullptr;
+    return ptr;
+}
+static EncodeTiledFn encode_tiled()
+{
+    static EncodeTiledFn fn = (EncodeTiledFn)driver_entry("cuTensorMapEncodeTiled");
+    return fn;
+}
+static EncodeIm2colFn encode_im2col()
+{
+    static EncodeIm2colFn fn = (EncodeIm2colFn)driver_entry("cuTensorMapEncodeIm2col");
+    return fn;
+}
+
+static bool can_vec(const float *src, int HW) { return HW % 4 == 0 && ((uintptr_t)src & 15) == 0; }
+static int round8(int c) { return (c + 7) & ~7; }
+static size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+// fp16 [d2][d1][d0], boxes of box0 x box1 x 1.
+static int map_3d(CUtensorMap *m, const __half *base, long long d0, long long d1, long long d2, int box0, int box1, CUtensorMapSwizzle swz)
+{
+    cuuint64_t dims[3] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2};
+    cuuint64_t strides[2] = {(cuuint64_t)d0 * 2, (cuuint64_t)d0 * (cuuint64_t)d1 * 2};
+    cuuint32_t box[3] = {(cuuint32_t)box0, (cuuint32_t)box1, 1}, estr[3] = {1, 1, 1};
+    const CUresult r = encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void *)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : fail("cuTensorMapEncodeTiled failed with code %d", (int)r);
+}
+// An axis of an im2col walk: positions low, low + step, ... (n of them) of an axis of `size`, plus a tap's offset of up to (taps - 1) * dil.
+struct Walk {
+    int size, low, n, step, taps, dil;
+    int upper() const { return low + (n - 1) * step - (size - 1); }
+    // the map's fields: corners of 8 bits with sign, offsets of 8 bits, steps of up to 8
+    bool fits() const { return low >= -128 && low <= 127 && upper() >= -128 && upper() <= 127 && (taps - 1) * dil <= 255 && step <= 8; }
+};
+// fp16 [images2][H][W][Cp] (both parts' images), boxes of `pixels` consecutive pixels of the walk x `channels`.
+static int map_im2col(CUtensorMap *m, const __half *base, int Cp, int images2, const Walk &h, const Walk &w, int channels, int pixels,
+                      CUtensorMapSwizzle swz)
+{
+    cuuint64_t dims[4] = {(cuuint64_t)Cp, (cuuint64_t)w.size, (cuuint64_t)h.size, (cuuint64_t)images2};
+    cuuint64_t strides[3] = {(cuuint64_t)Cp * 2, (cuuint64_t)Cp * 2 * w.size, (cuuint64_t)Cp * 2 * w.size * h.size};
+    const int lower[2] = {w.low, h.low}, upper[2] = {w.upper(), h.upper()};
+    cuuint32_t estr[4] = {1, (cuuint32_t)w.step, (cuuint32_t)h.step, 1};
+    const CUresult r = encode_im2col()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, (void *)base, dims, strides, lower, upper, (cuuint32_t)channels,
+                                       (cuuint32_t)pixels, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : fail("cuTensorMapEncodeIm2col failed with code %d", (int)r);
+}
+
+template <class... Args>
+static int launch(const char *name, const void *kern, int grid, int threads, size_t smem, cudaStream_t stream, bool dependent, Args &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    if (smem) CUNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    void *ptrs[] = {(void *)&args...};
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, kern, ptrs);
+    return e == cudaSuccess ? 0 : fail("launch of %s failed: %s", name, cudaGetErrorString(e));
+}
+
+// Images per round: the parts of one round's images take about as much memory as the images and are bounded.
+constexpr size_t ROUND_BYTES = (size_t)512 << 20;
+static int images_per_round(int N, size_t image_bytes)
+{
+    const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)N, ROUND_BYTES / std::max<size_t>(1, image_bytes)));
+    return ceil_div(N, ceil_div(N, most));             // rounds of one size
+}
+// Tensor maps of less memory than this are left alone: some drivers encode smaller im2col maps for walks that they do not do.
+constexpr size_t MIN_MAP_BYTES = 131072;
+
+// ---- forward pass and input gradients -------------------------------------------------------------------------------------------
+struct Plan {
+    Params p;
+    Walk wh[MAX_PHASES], ww[MAX_PHASES];
+    int images, Cp, bn;                    // images per round, channels of the gathered tensor padded to 8, column tile of the kernel
+    int rows, taps;                        // weight rows (columns of the product) and taps
+    size_t off_w, off_exps, off_exp, off_tickets, off_partial, bytes;
+};
+
+// The tiles of `images` images: their number, which of them are cut, and into how many parts.
+static void plan_tiles(Params &p, int images)
+{
+    p.images = images;
+    int tiles = 0, blocks = 1 << 30;
+    for (int i = 0; i < p.n_phases; ++i) {
+        Phase &f = p.ph[i];
+        f.tile0 = tiles;
+        f.M_total = images * f.HW;
+        f.blocks = f.taps * p.groups;
+        tiles += ceil_div(f.M_total, BM) * p.n_tiles;
+        blocks = std::min(blocks, f.blocks);
+    }
+    const int grid = sm_count(), rest = tiles % grid;
+    p.full = tiles - rest;
+    p.splits = rest ? std::max(1, std::min(std::min(grid / rest, blocks / 4), 16)) : 1;
+    p.items = p.full + rest * p.splits;
+}
+
+// `gathered`: channels, rows and columns of the tensor that is read; `columns`: channels of the tensor that is written.
+static bool finish_plan(Plan &pl, int N, int gC, int gH, int gW, int columns, int kk, int oHW)
+{
+    Params &p = pl.p;
+    p.g_C = gC; p.g_H = gH; p.g_W = gW;
+    p.groups = ceil_div(gC, GROUP);
+    p.w_kk = kk; p.o_HW = oHW; p.N_total = columns;
+    pl.bn = columns <= 128 ? 128 : 256;
+    p.n_tiles = ceil_div(columns, pl.bn);
+    p.width = (ceil_div(columns, p.n_tiles) + 15) & ~15;
+    pl.Cp = round8(gC);
+    pl.rows = columns; pl.taps = kk;
+    const size_t image_bytes = (size_t)gH * gW * pl.Cp * 4;
+    pl.images = images_per_round(N, image_bytes);
+    if (pl.images * image_bytes < MIN_MAP_BYTES) return false;
+    for (int i = 0; i < p.n_phases; ++i)
+        if (!pl.wh[i].fits() || !pl.ww[i].fits()) return false;
+    plan_tiles(p, pl.images);
+    size_t at = round256(pl.images * image_bytes);
+    pl.off_w = at; at += round256((size_t)2 * kk * columns * pl.Cp * 2);
+    pl.off_exps = at; at += round256((size_t)pl.images * gH * gW * p.groups);
+    pl.off_exp = at; at += round256((size_t)columns * 4);
+    pl.off_tickets = at; at += round256((size_t)sm_count() * 4);
+    pl.off_partial = at; at += round256((size_t)sm_count() * (pl.bn + 1) * BM * 4);
+    pl.bytes = at + 256;
+    return true;
+}
+
+// Column tile of the element-copy kernels: narrower ones while the wide ones leave half of the SMs without a tile.
+static int element_copy_columns(int columns, long long rows)
+{
+    int bn = columns <= 32 ? 32 : columns <= 64 ? 64 : 128;
+    while (bn > 32 && ceil_div_ll(rows, BM) * ceil_div(columns, bn) * 2 <= sm_count()) bn /= 2;
+    return bn;
+}
+// Whether the forward pass is over sooner here than on the gathering kernel: the split reads and writes the whole input, so short sums
+// that read it once or twice (few channels, strides) are better off there.  Estimates in us fitted to 195 layers of 3x3 to 5x5 drawn from
+// 16 to 1024 channels and maps of 7 to 112 (within 0.8 to 1.2 of the times of nine in ten): 17.1 ms for all of them, 17.1 ms by the rule,
+// 16.8 ms with the better one each time, 36.1 ms on the gathering kernel; the rule's losses are 6 of 195, the worst 1.17 times.
+static bool forward_is_faster(const Plan &pl, const Geometry &g)
+{
+    if (g.kH * g.kW > 32) return true;                      // those sum fp32 blocks there: 2.2 us a k-block
+    const Params &p = pl.p;
+    const int grid = sm_count(), tiles = p.full + (p.items - p.full) / p.splits, rest = tiles - p.full, blocks = p.ph[0].blocks;
+    const double in = (double)g.N * g.C * g.H * g.W / 1e6, out = (double)g.N * g.K * g.oH * g.oW / 1e6, weights = (double)g.K * g.C * g.kH * g.kW / 1e6;
+    const double waves = p.full / grid + (rest ? 1 : 0), longest = blocks * (p.full / grid + (rest ? 1.0 / p.splits : 0.0));
+    const double here = 12.2 + 2.4 * waves + (pl.bn == 256 ? 1.18 : 0.75) * longest + 2.0 * in + 1.34 * out + (p.splits > 1 ? 5.1 : 0.0) + 11.8 * weights;
+    const long long rows = (long long)g.N * g.oH * g.oW;
+    const int bn = element_copy_columns(g.K, rows);
+    const double there_waves = (double)ceil_div_ll(ceil_div_ll(rows, BM) * ceil_div(g.K, bn), grid);
+    const double there = 9.2 + there_waves * (0.84 + (bn == 128 ? 1.36 : bn == 64 ? 1.1 : 1.01) * ceil_div(g.C * g.kH * g.kW, BK)) + 1.12 * out;
+    return here < there;
+}
+
+static bool plan_forward(Plan &pl, const Geometry &g)
+{
+    pl = Plan{};
+    if (g.C < 16 || g.K < 16 || g.kH * g.kW == 1 || (long long)g.C * g.kH * g.kW < 128) return false;
+    Phase &f = pl.p.ph[0];
+    f.HW = g.oH * g.oW; f.pix_W = g.oW; f.taps = g.kH * g.kW; f.kW = g.kW;
+    f.lH = -g.padH; f.lW = -g.padW; f.stH = g.dH; f.stW = g.dW; f.dlH = g.dilH; f.dlW = g.dilW;
+    f.w_sH = g.kW; f.w_sW = 1; f.o_sH = g.oW; f.o_sW = 1;
+    pl.p.n_phases = 1;
+    pl.wh[0] = Walk{g.H, f.lH, g.oH, g.dH, g.kH, g.dilH};
+    pl.ww[0] = Walk{g.W, f.lW, g.oW, g.dW, g.kW, g.dilW};
+    return finish_plan(pl, g.N, g.C, g.H, g.W, g.K, g.kH * g.kW, f.HW) && forward_is_faster(pl, g);
+}
+
+// No rule on times: of 123 drawn layers one took longer than on the other kernels, by 4 %.  Residues of fewer than 48 products belong to
+// phase_fma_kernel, which loses no bits of them.
+static bool plan_grad_input(Plan &pl, const Geometry &g)
+{
+    pl = Plan{};
+    if (g.C < 16 || g.K < 64 || g.kH * g.kW == 1 || g.dH > 2 || g.dW > 2) return false;
+    bool gaps = false;
+    const std::vector<AxisPhase> ah = axis_phases(g.H, g.kH, g.dH, g.padH, g.dilH, false, &gaps), aw = axis_phases(g.W, g.kW, g.dW, g.padW, g.dilW, false, &gaps);
+    if (gaps || ah.empty() || aw.empty()) return false;
+    Params &p = pl.p;
+    struct Pair { const AxisPhase *a, *b; } order[MAX_PHASES];
+    for (const AxisPhase &a : ah)
+        for (const AxisPhase &b : aw) order[p.n_phases++] = Pair{&a, &b};
+    // longest reductions first: the tiles that are cut, and the last wave, are the short ones
+    std::stable_sort(order, order + p.n_phases, [](const Pair &u, const Pair &v) { return u.a->taps * u.b->taps > v.a->taps * v.b->taps; });
+    for (int i = 0; i < p.n_phases; ++i) {
+        const AxisPhase &a = *order[i].a, &b = *order[i].b;
+        Phase &f = p.ph[i];
+        f.HW = a.n * b.n; f.pix_W = b.n; f.taps = a.taps * b.taps; f.kW = b.taps;
+        // taps in ascending order of position: the last tap of the residue reads the first one
+        f.lH = a.o0 - (a.taps - 1) * a.ostep; f.lW = b.o0 - (b.taps - 1) * b.ostep;
+        f.stH = f.stW = 1; f.dlH = a.ostep; f.dlW = b.ostep;
+        f.w_base = (a.k0 + (a.taps - 1) * a.kstep) * g.kW + b.k0 + (b.taps - 1) * b.kstep;
+        f.w_sH = -a.kstep * g.kW; f.w_sW = -b.kstep;
+        f.o_off = a.h0 * g.W + b.h0; f.o_sH = g.dH * g.W; f.o_sW = g.dW;
+        pl.wh[i] = Walk{g.oH, f.lH, a.n, 1, a.taps, a.ostep};
+        pl.ww[i] = Walk{g.oW, f.lW, b.n, 1, b.taps, b.ostep};
+    }
+    return finish_plan(pl, g.N, g.K, g.oH, g.oW, g.C, g.kH * g.kW, g.H * g.W);
+}
+
+// src: the gathered tensor; weights of (row, channel, tap) at row * w_row + channel * w_c + tap.
+static int run_plan(Plan &pl, int N, const float *src, const float *weight, long long w_row, long long w_c, const float *bias, float *out, bool redo_nan,
+                    void *scratch, cudaStream_t stream)
+{
+    Params &p = pl.p;
+    char *ws = (char *)scratch;
+    __half *a = (__half *)ws, *w = (__half *)(ws + pl.off_w);
+    p.exps = (const int8_t *)(ws + pl.off_exps); p.w_exp = (int *)(ws + pl.off_exp); p.tickets = (int *)(ws + pl.off_tickets);
+    p.partial = (float *)(ws + pl.off_partial); p.bias = bias; p.status = device_status_ptr();
+    const int g_HW = p.g_H * p.g_W;
+    alignas(64) Maps maps;
+    if (map_3d(&maps.b, w, pl.Cp, pl.rows, 2 * pl.taps, BK, pl.bn, CU_TENSOR_MAP_SWIZZLE_64B)) return 1;
+    for (int at = 0; at < N; at += pl.images) {
+        const int n = std::min(pl.images, N - at);
+        plan_tiles(p, n);
+        const float *from = src + (size_t)at * p.g_C * g_HW;
+        p.out = out + (size_t)at * p.N_total * p.o_HW;
+        p.raw_a = redo_nan ? from : nullptr;
+        p.raw_w = weight;
+        for (int i = 0; i < p.n_phases; ++i)
+            if (map_im2col(&maps.a[i], a, pl.Cp, 2 * n, pl.wh[i], pl.ww[i], BK, BM, CU_TENSOR_MAP_SWIZZLE_64B)) return 1;
+        PrepParams q{};
+        Act &act = q.act[0];
+        act.src = from; act.dst = a; act.exps = const_cast<int8_t *>(p.exps); act.C = p.g_C; act.Cp = pl.Cp; act.HW = g_HW;
+        act.groups = p.groups; act.pixels = (uint32_t)n * g_HW; act.blocks = (int)ceil_div_ll((long long)act.pixels, 64) * p.groups;
+        act.vec = can_vec(from, g_HW);
+        q.n_act = 1;
+        q.w = weight; q.w_dst = w; q.w_exp = const_cast<int *>(p.w_exp); q.rows = at ? 0 : pl.rows; q.w_C = p.g_C; q.w_Cp = pl.Cp; q.taps = pl.taps;
+        q.w_row = w_row; q.w_c = w_c; q.tickets = p.tickets; q.n_tickets = sm_count();
+        if (launch("convolution operand split", (const void *)prep_kernel<false>, q.rows + act.blocks, 256, 0, stream, false, q)) return 1;
+        const void *kern = pl.bn == 128 ? (const void *)split_gemm_kernel<128, false> : (const void *)split_gemm_kernel<256, false>;
+        if (launch("convolution of split operands", kern, std::min(p.items, sm_count()), THREADS, SMEM, stream, true, p, maps)) return 1;
+    }
+    return 0;
+}
+
+size_t forward_scratch(const Geometry &g)
+{
+    Plan pl;
+    return plan_forward(pl, g) ? pl.bytes : 0;
+}
+size_t grad_input_scratch(const Geometry &g)
+{
+    Plan pl;
+    return plan_grad_input(pl, g) ? pl.bytes : 0;
+}
+int forward(const Geometry &g, const float *x, const float *weight, const float *bias, float *y, void *scratch, cudaStream_t stream)
+{
+    Plan pl;
+    if (!plan_forward(pl, g)) return fail("convolution forward: no plan for split operands");
+    const int kk = g.kH * g.kW;
+    return run_plan(pl, g.N, x, weight, (long long)g.C * kk, kk, bias, y, false, scratch, stream);
+}
+int grad_input(const Geometry &g, const float *gy, const float *weight, const float *bias, float *gx, void *scratch, cudaStream_t stream)
+{
+    Plan pl;
+    if (!plan_grad_input(pl, g)) return fail("convolution input gradient: no plan for split operands");
+    const int kk = g.kH * g.kW;
+    return run_plan(pl, g.N, gy, weight, kk, (long long)g.C * kk, bias, gx, g.dH > 1 || g.dW > 1, scratch, stream);
+}
+
+// ---- weight gradients ---------------------------------------------------------------------------------------------------------------
+struct WgradPlan {
+    Params p;
+    Walk wh, ww;
+    int images, Cp, Kp, bn;
+    size_t off_gy, off_max, off_bias, off_partial, bytes;
+};
+static void plan_splits(WgradPlan &pl, int images)
+{
+    Params &p = pl.p;
+    p.images = images;
+    p.blocks = (int)ceil_div_ll((long long)images * p.pix_HW, 2 * BK);
+    const int grid = sm_count();
+    double best = -1.0;
+    for (int waves = 1; waves <= 8; ++waves) {
+        const int want = std::max(1, std::min(p.blocks, waves * grid / p.tiles));
+        const int per = ceil_div(p.blocks, want), splits = ceil_div(p.blocks, per);
+        // a tile's partial sums cost about four blocks, and the reduction reads all of them
+        const double cost = (double)ceil_div_ll((long long)p.tiles * splits, grid) * (per + 4.0) + (double)splits * p.tiles * 4.0 / grid;
+        if (best < 0.0 || cost < best * 0.999) { best = cost; p.per_split = per; p.splits = splits; }
+    }
+    p.items = p.tiles * p.splits;
+}
+// As forward_is_faster: the two passes over both tensors cost more than the gathering kernel where sums are many but products few.
+// Fitted to 221 layers: 37.6 ms on the gathering kernel, 26.3 ms here, 23.7 ms by the rule, 23.5 ms with the better one each time; 3 of
+// 221 lose, the worst 1.34 times.
+static bool grad_weight_is_faster(const WgradPlan &pl, const Geometry &g)
+{
+    if (g.kH * g.kW > 32) return true;
+    const Params &p = pl.p;
+    const int grid = sm_count();
+    const double weights = (double)g.K * g.C * g.kH * g.kW / 1e6, in = (double)g.N * g.H * g.W * p.groups * GROUP / 1e6;
+    const double out = (double)g.N * p.pix_HW * ceil_div(g.K, GROUP) * GROUP / 1e6;
+    const double here = 14.2 + 2.05 * ceil_div(p.items, grid) * p.per_split + 2.85 * (double)p.items * pl.bn * BM / 1e6 + 3.05 * (in + out) + 3.2 * weights;
+    const double tiles = (double)ceil_div(g.K, BM) * ceil_div(g.C * g.kH * g.kW, BM), blocks = (double)ceil_div_ll((long long)g.N * p.pix_HW, BK);
+    const double there = 14.7 + 1.82 * tiles * blocks / grid + 6.85 * weights + (tiles * blocks > grid ? 1.16 : 0.0) +
+                         0.143 * std::min(blocks, std::ceil(tiles * blocks / grid));
+    return here < there;
+}
+static bool plan_grad_weight(WgradPlan &pl, const Geometry &g)
+{
+    pl = WgradPlan{};
+    Params &p = pl.p;
+    if (g.C < 16 || g.K < 16 || g.kH * g.kW == 1) return false;
+    const int kk = g.kH * g.kW;
+    p.groups = ceil_div(g.C, GROUP);
+    p.col_groups = kk * p.groups;
+    pl.bn = p.col_groups <= 2 ? 128 : 256;
+    p.n_tiles = ceil_div(p.col_groups, pl.bn / GROUP);
+    p.m_tiles = ceil_div(g.K, BM);
+    p.tiles = p.n_tiles * p.m_tiles;
+    p.kW = g.kW; p.pix_HW = g.oH * g.oW; p.pix_W = g.oW;
+    p.lH = -g.padH; p.lW = -g.padW; p.stH = g.dH; p.stW = g.dW; p.dlH = g.dilH; p.dlW = g.dilW;
+    pl.wh = Walk{g.H, p.lH, g.oH, g.dH, g.kH, g.dilH};
+    pl.ww = Walk{g.W, p.lW, g.oW, g.dW, g.kW, g.dilW};
+    if (!pl.wh.fits() || !pl.ww.fits()) return false;
+    pl.Cp = round8(g.C); pl.Kp = round8(g.K);
+    const size_t x_bytes = (size_t)g.H * g.W * pl.Cp * 4, gy_bytes = (size_t)p.pix_HW * pl.Kp * 4;
+    pl.images = images_per_round(g.N, std::max(x_bytes, gy_bytes));
+    if (pl.images * x_bytes < MIN_MAP_BYTES) return false;
+    plan_splits(pl, pl.images);
+    if (!grad_weight_is_faster(pl, g)) return false;
+    size_t at = round256(pl.images * x_bytes);
+    pl.off_gy = at; at += round256(pl.images * gy_bytes);
+    pl.off_max = at; at += round256((size_t)(g.C + g.K) * 4);
+    pl.off_bias = at; at += round256((size_t)ceil_div_ll((long long)pl.images * p.pix_HW, 64) * g.K * 8);
+    // a round of fewer images may be cut into a few more parts than a whole one
+    pl.off_partial = at; at += round256((size_t)(p.splits + 1) * p.n_tiles * pl.bn * p.m_tiles * BM * 4);
+    pl.bytes = at + 256;
+    return true;
+}
+size_t grad_weight_scratch(const Geometry &g)
+{
+    WgradPlan pl;
+    return plan_grad_weight(pl, g) ? pl.bytes : 0;
+}
+int grad_weight(const Geometry &g, const float *x, const float *gy, float *grad_weight, float *grad_bias, float scale, void *scratch,
+                cudaStream_t stream)
+{
+    WgradPlan pl;
+    if (!plan_grad_weight(pl, g)) return fail("convolution parameter gradient: no plan for split operands");
+    Params &p = pl.p;
+    char *ws = (char *)scratch;
+    __half *xs = (__half *)ws, *gs = (__half *)(ws + pl.off_gy);
+    uint32_t *gy_max = (uint32_t *)(ws + pl.off_max), *x_max = gy_max + g.K;
+    double *bias_part = (double *)(ws + pl.off_bias);
+    p.partial = (float *)(ws + pl.off_partial);
+    p.status = device_status_ptr();
+    const int kk = g.kH * g.kW, x_HW = g.H * g.W;
+    const int most = p.splits + 1;
+    for (int at = 0; at < g.N; at += pl.images) {
+        const int n = std::min(pl.images, g.N - at);
+        plan_splits(pl, n);
+        if (p.splits > most) { p.per_split = ceil_div(p.blocks, most); p.splits = ceil_div(p.blocks, p.per_split); p.items = p.tiles * p.splits; }
+        const float *xr = x + (size_t)at * g.C * x_HW, *gr = gy + (size_t)at * g.K * p.pix_HW;
+        alignas(64) Maps maps;
+        if (map_3d(&maps.a[0], gs, pl.Kp, (long long)n * p.pix_HW, 2, GROUP, BK, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
+        if (map_im2col(&maps.b, xs, pl.Cp, 2 * n, pl.wh, pl.ww, GROUP, BK, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
+        CUNN_CUDA(cudaMemsetAsync(gy_max, 0, (size_t)(g.C + g.K) * 4, stream));
+        MaxParams m{};
+        m.src[0] = gr; m.src[1] = xr; m.chmax[0] = gy_max; m.chmax[1] = x_max; m.C[0] = g.K; m.C[1] = g.C; m.HW[0] = p.pix_HW; m.HW[1] = x_HW;
+        m.images = n;
+        for (int t = 0; t < 2; ++t) {
+            m.chunks[t] = std::max(1, std::min(ceil_div(n, 8), ceil_div(sm_count() * 8, m.C[t])));
+            m.vec[t] = can_vec(m.src[t], m.HW[t]);
+        }
+        if (launch("convolution channel maxima", (const void *)channel_max_kernel, m.C[0] * m.chunks[0] + m.C[1] * m.chunks[1], 256, 0, stream, false, m)) return 1;
+        PrepParams q{};
+        for (int t = 0; t < 2; ++t) {
+            Act &act = q.act[t];
+            act.src = t ? xr : gr; act.dst = t ? xs : gs; act.chmax = t ? x_max : gy_max; act.bias_part = !t && grad_bias ? bias_part : nullptr;
+            act.C = t ? g.C : g.K; act.Cp = t ? pl.Cp : pl.Kp; act.HW = t ? x_HW : p.pix_HW; act.groups = ceil_div(act.C, GROUP);
+            act.vec = can_vec(act.src, act.HW);
+            act.pixels = (uint32_t)n * act.HW; act.blocks = (int)ceil_div_ll((long long)act.pixels, 64) * act.groups;
+        }
+        q.n_act = 2;
+        if (launch("convolution operand split", (const void *)prep_kernel<true>, q.act[0].blocks + q.act[1].blocks, 256, 0, stream, true, q)) return 1;
+        const void *kern = pl.bn == 128 ? (const void *)split_gemm_kernel<128, true> : (const void *)split_gemm_kernel<256, true>;
+        if (launch("convolution parameter gradient of split operands", kern, std::min(p.items, sm_count()), THREADS, SMEM, stream, true, p, maps)) return 1;
+        ReduceParams r{};
+        r.partial = p.partial; r.gw = grad_weight; r.gb = grad_bias; r.gy_max = gy_max; r.x_max = x_max; r.bias_part = bias_part;
+        r.K = g.K; r.C = g.C; r.kk = kk; r.groups = p.groups; r.splits = p.splits; r.cols = p.n_tiles * pl.bn; r.rows = p.m_tiles * BM;
+        r.gw_blocks = ceil_div(g.K, 32) * ceil_div(g.C * kk, 32);
+        r.bias_blocks = (int)ceil_div_ll((long long)n * p.pix_HW, 64);
+        r.scale = scale;
+        if (launch("convolution parameter gradient sums", (const void *)reduce_kernel, r.gw_blocks + (grad_bias ? ceil_div(g.K, 8) : 0), 256, 0, stream,
+                   true, r)) return 1;
+    }
+    return 0;
+}
+
+}  // namespace split
+}  // namespace cunn

@@ -25,7 +25,10 @@
 //     both passes of kernels of more than 32 taps; pwg::phase_fma_kernel for the residues that are better off in fp32.
 // Every wait is bounded.
 #include "common.cuh"
+#include "axis_phases.h"
+#include "conv_split.h"
 #include "stemconv.h"
+#include "umma.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -64,68 +67,6 @@ struct GemmParams {
     // WGRAD
     int imgs_per_split, pix_blocks;  // images per split, k-blocks per image
 };
-
-// ---- tcgen05 wrappers ---------------------------------------------------------------------------
-__device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols)
-{
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// The same with accumulation always on: no predicate to set up.
-__device__ __forceinline__ void umma_tf32_acc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
-{
-    asm volatile("tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, 1;" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc) : "memory");
-}
-// Arrives on the mbarrier once every MMA issued so far by this thread has finished reading shared memory
-// and writing TMEM.
-__device__ __forceinline__ void umma_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 // Shared-memory matrix descriptor: K-major tile in the 128-byte swizzle (row r holds its eight 16-byte chunks
 // at positions chunk ^ (r & 7); groups of 8 rows are 1024 bytes apart).  The tensor core reads this form without
@@ -1655,29 +1596,6 @@ static int launch_gather(pwg::GatherParams &p, int bn, cudaStream_t stream)
     return 0;
 }
 
-using pwg::AxisPhase;
-// Residues without taps are listed if `all`; *gaps is set when there are any.
-static std::vector<AxisPhase> axis_phases(int H, int k, int d, int pad, int dil, bool all, bool *gaps)
-{
-    int g = d, r = dil % d;
-    while (r) { const int t = g % r; g = r; r = t; }                       // gcd(d, dil)
-    std::vector<AxisPhase> out;
-    for (int h0 = 0; h0 < std::min(d, H); ++h0) {
-        // the first of its taps is below d / g, the others follow d / g apart
-        const int step = d / g;
-        int first = dil == 1 ? (h0 + pad) % d : 0;
-        while (first < step && first < k && (h0 + pad - first * dil) % d) ++first;
-        AxisPhase a{h0, (H - h0 + d - 1) / d, 0, 0, step, 0, dil / g};
-        if (first < step && first < k) {
-            a.k0 = first;
-            a.taps = (k - first - 1) / step + 1;
-            a.o0 = (h0 + pad - first * dil) / d;
-        }
-        if (a.taps || all) out.push_back(a);
-        if (!a.taps) *gaps = true;
-    }
-    return out;
-}
 static int most_taps(const std::vector<AxisPhase> &v)
 {
     int most = 0;
@@ -1798,8 +1716,22 @@ static int phased_grad_input(const float *gy, const float *weight, const float *
 using namespace cunn;
 using namespace cunn::mm;
 
+// Scratch memory of the kernels in conv_split.cu, or 0 where they do not take the pass.
+enum Pass : int { PASS_FORWARD = 0, PASS_GRAD_INPUT = 1, PASS_GRAD_WEIGHT = 2 };
+static size_t split_scratch(int pass, const split::Geometry &g)
+{
+    if (!g_use_tma || g.N == 0) return 0;
+    return pass == PASS_FORWARD ? split::forward_scratch(g) : pass == PASS_GRAD_INPUT ? split::grad_input_scratch(g) : split::grad_weight_scratch(g);
+}
+static bool split_applies(int pass, const split::Geometry &g, const void *scratch, size_t scratch_bytes)
+{
+    const size_t need = scratch && aligned16(scratch) ? split_scratch(pass, g) : 0;
+    return need && scratch_bytes >= need;
+}
+
 static int conv_forward(const float *x, const float *weight, const float *bias, float *y, int N, int C, int H, int W, int K,
-                        int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_)
+                        int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_,
+                        void *scratch = nullptr, size_t scratch_bytes = 0)
 {
     clear_error();
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -1848,6 +1780,8 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
         return pw_launch(pw_pick<OP_FWD>(bn), q, stream);
     }
+    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
+    if (split_applies(PASS_FORWARD, geo, scratch, scratch_bytes)) return split::forward(geo, x, weight, bias, y, scratch, stream);
     if (gather_applies(kH, kW)) {
         pw::Params q{};
         q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
@@ -1886,7 +1820,8 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
 
 // `bias` (null: none) is added to every plane of gx: a transposed convolution's forward pass is this one plus its bias.
 static int conv_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
-                           int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_)
+                           int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_,
+                           void *scratch = nullptr, size_t scratch_bytes = 0)
 {
     clear_error();
     // the stride-1 kernels leave the bias to a pass of its own
@@ -1932,6 +1867,12 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         q.bulk_out = (q.HW % 4 == 0) && q.HW >= 8 * BM && aligned16(gx);
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
         return add_bias(pw_launch(pw_pick<OP_DGRAD>(bn), q, stream));
+    }
+    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
+    try {
+        if (split_applies(PASS_GRAD_INPUT, geo, scratch, scratch_bytes)) return split::grad_input(geo, gy, weight, bias, gx, scratch, stream);
+    } catch (const std::bad_alloc &) {
+        return fail("convmm grad input: out of host memory");
     }
     if (dH == 1 && dW == 1 && padH <= dilH * (kH - 1) && padW <= dilW * (kW - 1) && (gather_applies(kH, kW) || !small_kernel(kH, kW))) {
         // stride 1: a convolution of gy with the kernel rotated by 180 degrees and padding dil (k - 1) - pad
@@ -2046,6 +1987,8 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         }
         return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
+    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
+    if (split_applies(PASS_GRAD_WEIGHT, geo, workspace, workspace_bytes)) return split::grad_weight(geo, x, gy, grad_weight, grad_bias, scale, workspace, stream);
     if (gathered_wgrad(kH, kW)) {
         const int oHW = oH * oW;
         pw_wgrad_plan(C, K, kk, N, oHW, false, &bn, &splits, &kb);
@@ -2119,6 +2062,35 @@ extern "C" CUNN_API int cunn_b200_convmm_acc_grad(const float *x, const float *g
                          workspace_bytes, stream);
 }
 
+extern "C" CUNN_API size_t cunn_b200_conv_scratch(int pass, int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW, int padH,
+                                                  int padW, int dilH, int dilW)
+{
+    int oH, oW;
+    if (pass < PASS_FORWARD || pass > PASS_GRAD_WEIGHT || check(N, C, H, W, K, kH, kW, dH, dW, padH, padW, &oH, &oW, dilH, dilW)) {
+        clear_error();
+        return 0;
+    }
+    try {
+        return split_scratch(pass, split::Geometry{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW});
+    } catch (const std::bad_alloc &) {
+        return 0;
+    }
+}
+
+extern "C" CUNN_API int cunn_b200_conv_forward_scratch(const float *x, const float *weight, const float *bias, float *y, int N, int C, int H,
+                                                       int W, int K, int kH, int kW, int dH, int dW, int padH, int padW, int dilH,
+                                                       int dilW, void *scratch, size_t scratch_bytes, cunn_stream_t stream)
+{
+    return conv_forward(x, weight, bias, y, N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, stream, scratch, scratch_bytes);
+}
+
+extern "C" CUNN_API int cunn_b200_conv_grad_input_scratch(const float *gy, const float *weight, float *gx, int N, int C, int H, int W, int K,
+                                                          int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW,
+                                                          void *scratch, size_t scratch_bytes, cunn_stream_t stream)
+{
+    return conv_grad_input(gy, weight, nullptr, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, stream, scratch, scratch_bytes);
+}
+
 extern "C" CUNN_API int cunn_b200_dilated_conv_forward(const float *x, const float *weight, const float *bias, float *y, int N,
                                                        int C, int H, int W, int K, int kH, int kW, int dH, int dW, int padH,
                                                        int padW, int dilH, int dilW, cunn_stream_t stream)
@@ -2178,6 +2150,9 @@ static int full_check(int N, int P, int H, int W, int Q, int kH, int kW, int dH,
 }
 
 static int bias_chunks(int N, int Q) { return std::max(1, std::min(N, ceil_div(sm_count() * 4, Q))); }
+static size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
+// The transposed convolution's bias sums, at the head of its parameter gradient's workspace.
+static size_t full_bias_bytes(int N, int Q) { return round256((size_t)Q * bias_chunks(N, Q) * sizeof(float)); }
 
 extern "C" CUNN_API int cunn_b200_full_conv_forward(const float *x, const float *weight, const float *bias, float *y, int N,
                                                     int P, int H, int W, int Q, int kH, int kW, int dH, int dW, int padH,
@@ -2199,7 +2174,42 @@ extern "C" CUNN_API int cunn_b200_full_conv_grad_input(const float *gy, const fl
     return conv_forward(gy, weight, nullptr, gx, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW, stream_);
 }
 
-static size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
+extern "C" CUNN_API size_t cunn_b200_full_conv_scratch(int pass, int N, int P, int H, int W, int Q, int kH, int kW, int dH, int dW, int padH,
+                                                       int padW, int dilH, int dilW, int adjH, int adjW)
+{
+    int OH, OW;
+    if (pass < PASS_FORWARD || pass > PASS_GRAD_WEIGHT ||
+        full_check(N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW, &OH, &OW)) {
+        clear_error();
+        return 0;
+    }
+    // the adjoint convolution: its input gradient is this forward pass
+    const int of = pass == PASS_FORWARD ? PASS_GRAD_INPUT : pass == PASS_GRAD_INPUT ? PASS_FORWARD : PASS_GRAD_WEIGHT;
+    const size_t bytes = cunn_b200_conv_scratch(of, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW);
+    return bytes && of == PASS_GRAD_WEIGHT ? full_bias_bytes(N, Q) + bytes : bytes;
+}
+
+extern "C" CUNN_API int cunn_b200_full_conv_forward_scratch(const float *x, const float *weight, const float *bias, float *y, int N, int P, int H,
+                                                            int W, int Q, int kH, int kW, int dH, int dW, int padH, int padW, int dilH,
+                                                            int dilW, int adjH, int adjW, void *scratch, size_t scratch_bytes,
+                                                            cunn_stream_t stream)
+{
+    clear_error();
+    int OH, OW;
+    if (full_check(N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW, &OH, &OW)) return 1;
+    return conv_grad_input(x, weight, bias, y, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW, stream, scratch, scratch_bytes);
+}
+
+extern "C" CUNN_API int cunn_b200_full_conv_grad_input_scratch(const float *gy, const float *weight, float *gx, int N, int P, int H, int W,
+                                                               int Q, int kH, int kW, int dH, int dW, int padH, int padW, int dilH,
+                                                               int dilW, int adjH, int adjW, void *scratch, size_t scratch_bytes,
+                                                               cunn_stream_t stream)
+{
+    clear_error();
+    int OH, OW;
+    if (full_check(N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW, &OH, &OW)) return 1;
+    return conv_forward(gy, weight, nullptr, gx, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW, stream, scratch, scratch_bytes);
+}
 
 extern "C" CUNN_API size_t cunn_b200_full_conv_acc_grad_workspace(int N, int P, int H, int W, int Q, int kH, int kW, int dH,
                                                                   int dW, int padH, int padW, int dilH, int dilW, int adjH,
@@ -2207,8 +2217,7 @@ extern "C" CUNN_API size_t cunn_b200_full_conv_acc_grad_workspace(int N, int P, 
 {
     int OH, OW;
     if (full_check(N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW, &OH, &OW) || N == 0) return 0;
-    return round256(conv_acc_grad_workspace(N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW)) +
-           (size_t)Q * bias_chunks(N, Q) * sizeof(float) + 256;
+    return full_bias_bytes(N, Q) + round256(conv_acc_grad_workspace(N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW)) + 256;
 }
 
 extern "C" CUNN_API int cunn_b200_full_conv_acc_grad(const float *x, const float *gy, float *grad_weight, float *grad_bias,
@@ -2220,19 +2229,18 @@ extern "C" CUNN_API int cunn_b200_full_conv_acc_grad(const float *x, const float
     int OH, OW;
     if (full_check(N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW, &OH, &OW)) return 1;
     if (N == 0) return 0;
-    const size_t conv_ws = round256(conv_acc_grad_workspace(N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW));
     const int chunks = bias_chunks(N, Q);
-    const size_t need = conv_ws + (size_t)Q * chunks * sizeof(float) + 256;
+    const size_t head = full_bias_bytes(N, Q), need = cunn_b200_full_conv_acc_grad_workspace(N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW);
     CUNN_CHECK_ARG(workspace && workspace_bytes >= need && ((uintptr_t)workspace & 15) == 0,
                    "full convolution acc_grad needs %zu bytes of 16-byte aligned workspace, got %zu", need,
                    workspace ? workspace_bytes : (size_t)0);
     // the adjoint convolution's "input" is gy and its "output gradient" is x
-    if (conv_acc_grad(gy, x, grad_weight, nullptr, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW, scale, workspace,
-                      conv_ws, stream_))
+    if (conv_acc_grad(gy, x, grad_weight, nullptr, N, Q, OH, OW, P, kH, kW, dH, dW, padH, padW, dilH, dilW, scale,
+                      (char *)workspace + head, workspace_bytes - head, stream_))
         return 1;
     if (grad_bias) {
         cudaStream_t stream = (cudaStream_t)stream_;
-        float *part = (float *)((char *)workspace + conv_ws);
+        float *part = (float *)workspace;
         bias_partial_kernel<<<Q * chunks, 256, 0, stream>>>(gy, part, N, Q, OH * OW, chunks);
         CUNN_LAUNCH_CHECK("full convolution bias gradient");
         bias_finish_kernel<<<ceil_div(Q, 128), 128, 0, stream>>>(part, grad_bias, Q, chunks, scale);

@@ -6,6 +6,9 @@
 #include "common.cuh"
 #include "../../include/THCUNN_b200.h"   // with CUNN_B200_USE_REAL_THC this pulls in cutorch's <THC/THC.h>
 
+#include <list>
+#include <mutex>
+#include <new>
 #include <stdlib.h>
 #include <string.h>
 #include <string>
@@ -27,6 +30,91 @@ extern "C" void thcunn_b200_not_implemented(THCState *state, const char *name)
     else fprintf(stderr, "THCUNN error: %s is not implemented in this build\n", name);
 }
 
+// ---- scratch of the convolutions -------------------------------------------------------------------------
+// The fast kernels of a convolution want scratch memory, which the passes did without before: what goes wrong with it must not
+// show.  A call has its buffer to itself until its kernels are queued, and gets one that only its own stream has used, so calls of
+// several threads and streams stay independent; where none can be had (no memory; a stream under capture, whose graph would keep the
+// address) it gets `least` bytes as ever, or none, and the other kernels.
+struct ScratchBuffer {
+    int device;
+    cudaStream_t stream;
+    void *ptr;
+    size_t bytes;
+    bool busy;
+};
+static std::mutex g_conv_scratch_mutex;
+static std::list<ScratchBuffer> g_conv_scratch;                            // used longest ago first
+
+struct ConvScratch {
+    void *ptr = nullptr;
+    size_t bytes = 0;
+    ScratchBuffer *owner = nullptr;
+    ConvScratch(THCState *s, size_t want, size_t least = 0)
+    {
+        if (want > least && take(state_stream(s), want)) return;
+        if (!least) return;
+        ptr = state_scratch(s, 0, least);
+        bytes = ptr ? state_scratch_bytes(s, 0) : 0;
+    }
+    ConvScratch(const ConvScratch &) = delete;
+    ConvScratch &operator=(const ConvScratch &) = delete;
+    ~ConvScratch()
+    {
+        if (!owner) return;
+        std::lock_guard<std::mutex> lock(g_conv_scratch_mutex);
+        owner->busy = false;
+    }
+
+private:
+    bool take(cudaStream_t stream, size_t want)
+    {
+        constexpr size_t KEPT = 4;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        int dev = 0;
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        std::lock_guard<std::mutex> lock(g_conv_scratch_mutex);
+        auto &pool = g_conv_scratch;
+        auto it = pool.begin();
+        while (it != pool.end() && (it->busy || it->device != dev || it->stream != stream)) ++it;
+        if (it != pool.end() && it->bytes >= want) {
+            pool.splice(pool.end(), pool, it);
+        } else {
+            // a larger one in its place, or in that of the one used longest ago when enough are kept; cudaFree waits for the device,
+            // so no kernel reads what goes
+            if (it == pool.end() && pool.size() >= KEPT) {
+                it = pool.begin();
+                while (it != pool.end() && it->busy) ++it;
+            }
+            if (it != pool.end()) {
+                if (cudaFree(it->ptr) != cudaSuccess) {
+                    cudaGetLastError();
+                    return false;
+                }
+                pool.erase(it);
+            }
+            void *p = nullptr;
+            if (cudaMalloc(&p, want) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            try {
+                pool.push_back(ScratchBuffer{dev, stream, p, want, false});
+            } catch (const std::bad_alloc &) {
+                cudaFree(p);
+                return false;
+            }
+        }
+        owner = &pool.back();
+        owner->busy = true;
+        ptr = owner->ptr;
+        bytes = owner->bytes;
+        return true;
+    }
+};
+
 // ---- element types of the hot path ---------------------------------------------------------------------
 // The reference instantiates every entry point for float and double (THCGenerateFloatTypes.h); here the hot-path
 // wrappers below are templates over one of these two descriptions: element type, `accreal` of the binding
@@ -39,8 +127,22 @@ struct RealFloat {
     static constexpr auto dwconv_grad_input = &cunn_b200_dwconv_grad_input;
     static constexpr auto dwconv_acc_grad_workspace = &cunn_b200_dwconv_acc_grad_workspace;
     static constexpr auto dwconv_acc_grad = &cunn_b200_dwconv_acc_grad;
-    static constexpr auto convmm_forward = &cunn_b200_convmm_forward;
-    static constexpr auto convmm_grad_input = &cunn_b200_convmm_grad_input;
+    static int convmm_forward(THCState *s, const float *x, const float *w, const float *b, float *y, int N, int C, int H, int W, int K, int kH,
+                              int kW, int dH, int dW, int padH, int padW)
+    {
+        const ConvScratch ws(s, kH * kW > 1 ? cunn_b200_conv_scratch(0, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1) : 0);
+        return cunn_b200_conv_forward_scratch(x, w, b, y, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1, ws.ptr, ws.bytes, state_stream(s));
+    }
+    static int convmm_grad_input(THCState *s, const float *gy, const float *w, float *gx, int N, int C, int H, int W, int K, int kH, int kW,
+                                 int dH, int dW, int padH, int padW)
+    {
+        const ConvScratch ws(s, kH * kW > 1 ? cunn_b200_conv_scratch(1, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1) : 0);
+        return cunn_b200_conv_grad_input_scratch(gy, w, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1, ws.ptr, ws.bytes, state_stream(s));
+    }
+    static size_t convmm_acc_grad_scratch(int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW, int padH, int padW)
+    {
+        return kH * kW > 1 ? cunn_b200_conv_scratch(2, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1) : 0;
+    }
     static constexpr auto convmm_acc_grad_workspace = &cunn_b200_convmm_acc_grad_workspace;
     static constexpr auto convmm_acc_grad = &cunn_b200_convmm_acc_grad;
     static constexpr auto batchnorm_workspace = &cunn_b200_batchnorm_workspace;
@@ -57,8 +159,17 @@ struct RealDouble {
     static constexpr auto dwconv_grad_input = &cunn_b200_double_dwconv_grad_input;
     static constexpr auto dwconv_acc_grad_workspace = &cunn_b200_double_dwconv_acc_grad_workspace;
     static constexpr auto dwconv_acc_grad = &cunn_b200_double_dwconv_acc_grad;
-    static constexpr auto convmm_forward = &cunn_b200_double_convmm_forward;
-    static constexpr auto convmm_grad_input = &cunn_b200_double_convmm_grad_input;
+    static int convmm_forward(THCState *s, const double *x, const double *w, const double *b, double *y, int N, int C, int H, int W, int K,
+                              int kH, int kW, int dH, int dW, int padH, int padW)
+    {
+        return cunn_b200_double_convmm_forward(x, w, b, y, N, C, H, W, K, kH, kW, dH, dW, padH, padW, state_stream(s));
+    }
+    static int convmm_grad_input(THCState *s, const double *gy, const double *w, double *gx, int N, int C, int H, int W, int K, int kH, int kW,
+                                 int dH, int dW, int padH, int padW)
+    {
+        return cunn_b200_double_convmm_grad_input(gy, w, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, state_stream(s));
+    }
+    static size_t convmm_acc_grad_scratch(int, int, int, int, int, int, int, int, int, int, int) { return 0; }
     static constexpr auto convmm_acc_grad_workspace = &cunn_b200_double_convmm_acc_grad_workspace;
     static constexpr auto convmm_acc_grad = &cunn_b200_double_convmm_acc_grad;
     static constexpr auto batchnorm_workspace = &cunn_b200_double_batchnorm_workspace;
@@ -211,8 +322,8 @@ static void hot_SpatialConvolutionMM_updateOutput(
     if (x) {
         const long sz4[4] = {N, K, oH, oW};
         if (tensor_resize(s, output, 4, sz4, (int)sizeof(typename R::real))) {
-            TH_CALL(s, R::convmm_forward(tdata<typename R::real>(x), tdata<typename R::real>(weight), bias ? tdata<typename R::real>(bias) : nullptr, tdata<typename R::real>(output),
-                                                (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW, state_stream(s)));
+            TH_CALL(s, R::convmm_forward(s, tdata<typename R::real>(x), tdata<typename R::real>(weight), bias ? tdata<typename R::real>(bias) : nullptr, tdata<typename R::real>(output),
+                                                (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW));
             if (input->nDimension == 3) tensor_resize(s, output, 3, sz4 + 1, (int)sizeof(typename R::real));
         }
     }
@@ -231,8 +342,8 @@ static void hot_SpatialConvolutionMM_updateGradInput(
     if (gy) {
         const long sz4[4] = {N, C, H, W};
         if (tensor_resize(s, gradInput, 4, sz4, (int)sizeof(typename R::real))) {
-            TH_CALL(s, R::convmm_grad_input(tdata<typename R::real>(gy), tdata<typename R::real>(weight), tdata<typename R::real>(gradInput), (int)N, (int)C, (int)H,
-                                                   (int)W, (int)K, kH, kW, dH, dW, padH, padW, state_stream(s)));
+            TH_CALL(s, R::convmm_grad_input(s, tdata<typename R::real>(gy), tdata<typename R::real>(weight), tdata<typename R::real>(gradInput), (int)N, (int)C, (int)H,
+                                                   (int)W, (int)K, kH, kW, dH, dW, padH, padW));
             if (input->nDimension == 3) tensor_resize(s, gradInput, 3, sz4 + 1, (int)sizeof(typename R::real));
         }
     }
@@ -250,11 +361,11 @@ static void hot_SpatialConvolutionMM_accGradParameters(
     typename R::tensor *x = new_contiguous(s, input, (int)sizeof(typename R::real)), *gy = new_contiguous(s, gradOutput, (int)sizeof(typename R::real));
     if (x && gy) {
         const size_t need = R::convmm_acc_grad_workspace((int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW);
-        void *ws = need ? state_scratch(s, 0, need) : nullptr;
-        if (!need || ws)
+        const ConvScratch ws(s, R::convmm_acc_grad_scratch((int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW), need);
+        if (!need || ws.ptr)
             TH_CALL(s, R::convmm_acc_grad(tdata<typename R::real>(x), tdata<typename R::real>(gy), tdata<typename R::real>(gradWeight), gradBias ? tdata<typename R::real>(gradBias) : nullptr,
-                                                 (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW, scale, ws,
-                                                 state_scratch_bytes(s, 0), state_stream(s)));
+                                                 (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW, scale, ws.ptr, ws.bytes,
+                                                 state_stream(s)));
     }
 done:
     tensor_free(s, x); tensor_free(s, gy);
@@ -272,9 +383,11 @@ extern "C" CUNN_API void THNN_CudaSpatialDilatedConvolution_updateOutput(
     if (x) {
         const long sz4[4] = {N, K, oH, oW};
         if (tensor_resize(s, output, 4, sz4, 4)) {
-            TH_CALL(s, cunn_b200_dilated_conv_forward(tdata<float>(x), tdata<float>(weight), bias ? tdata<float>(bias) : nullptr,
+            const ConvScratch ws(s, cunn_b200_conv_scratch(0, (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW,
+                                                                          dilationH, dilationW));
+            TH_CALL(s, cunn_b200_conv_forward_scratch(tdata<float>(x), tdata<float>(weight), bias ? tdata<float>(bias) : nullptr,
                                                       tdata<float>(output), (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW,
-                                                      padH, padW, dilationH, dilationW, state_stream(s)));
+                                                      padH, padW, dilationH, dilationW, ws.ptr, ws.bytes, state_stream(s)));
             if (input->nDimension == 3) tensor_resize(s, output, 3, sz4 + 1, 4);
         }
     }
@@ -292,9 +405,11 @@ extern "C" CUNN_API void THNN_CudaSpatialDilatedConvolution_updateGradInput(
     if (gy) {
         const long sz4[4] = {N, C, H, W};
         if (tensor_resize(s, gradInput, 4, sz4, 4)) {
-            TH_CALL(s, cunn_b200_dilated_conv_grad_input(tdata<float>(gy), tdata<float>(weight), tdata<float>(gradInput), (int)N, (int)C,
+            const ConvScratch ws(s, cunn_b200_conv_scratch(1, (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW,
+                                                                          dilationH, dilationW));
+            TH_CALL(s, cunn_b200_conv_grad_input_scratch(tdata<float>(gy), tdata<float>(weight), tdata<float>(gradInput), (int)N, (int)C,
                                                          (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW, dilationH, dilationW,
-                                                         state_stream(s)));
+                                                         ws.ptr, ws.bytes, state_stream(s)));
             if (input->nDimension == 3) tensor_resize(s, gradInput, 3, sz4 + 1, 4);
         }
     }
@@ -313,11 +428,12 @@ extern "C" CUNN_API void THNN_CudaSpatialDilatedConvolution_accGradParameters(
     if (x && gy) {
         const size_t need = cunn_b200_dilated_conv_acc_grad_workspace((int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW,
                                                                        dilationH, dilationW);
-        void *ws = need ? state_scratch(s, 0, need) : nullptr;
-        if (!need || ws)
+        const ConvScratch ws(s, cunn_b200_conv_scratch(2, (int)N, (int)C, (int)H, (int)W, (int)K, kH, kW, dH, dW, padH, padW,
+                                                                      dilationH, dilationW), need);
+        if (!need || ws.ptr)
             TH_CALL(s, cunn_b200_dilated_conv_acc_grad(tdata<float>(x), tdata<float>(gy), tdata<float>(gradWeight),
                                                        gradBias ? tdata<float>(gradBias) : nullptr, (int)N, (int)C, (int)H, (int)W, (int)K,
-                                                       kH, kW, dH, dW, padH, padW, dilationH, dilationW, scale, ws, need, state_stream(s)));
+                                                       kH, kW, dH, dW, padH, padW, dilationH, dilationW, scale, ws.ptr, ws.bytes, state_stream(s)));
     }
 done:
     tensor_free(s, x);
@@ -371,9 +487,11 @@ extern "C" CUNN_API void THNN_CudaSpatialFullDilatedConvolution_updateOutput(
     if (x) {
         const long sz4[4] = {N, Q, OH, OW};
         if (tensor_resize(s, output, 4, sz4, 4)) {
-            TH_CALL(s, cunn_b200_full_conv_forward(tdata<float>(x), tdata<float>(weight), bias ? tdata<float>(bias) : nullptr,
+            const ConvScratch ws(s, cunn_b200_full_conv_scratch(0, (int)N, (int)P, (int)H, (int)W, (int)Q, kH, kW, dH, dW, padH,
+                                                                               padW, dilationH, dilationW, adjH, adjW));
+            TH_CALL(s, cunn_b200_full_conv_forward_scratch(tdata<float>(x), tdata<float>(weight), bias ? tdata<float>(bias) : nullptr,
                                                    tdata<float>(output), (int)N, (int)P, (int)H, (int)W, (int)Q, kH, kW, dH, dW, padH,
-                                                   padW, dilationH, dilationW, adjH, adjW, state_stream(s)));
+                                                   padW, dilationH, dilationW, adjH, adjW, ws.ptr, ws.bytes, state_stream(s)));
             if (input->nDimension == 3) tensor_resize(s, output, 3, sz4 + 1, 4);
         }
     }
@@ -391,9 +509,11 @@ extern "C" CUNN_API void THNN_CudaSpatialFullDilatedConvolution_updateGradInput(
     if (gy) {
         const long sz4[4] = {N, P, H, W};
         if (tensor_resize(s, gradInput, 4, sz4, 4)) {
-            TH_CALL(s, cunn_b200_full_conv_grad_input(tdata<float>(gy), tdata<float>(weight), tdata<float>(gradInput), (int)N, (int)P,
+            const ConvScratch ws(s, cunn_b200_full_conv_scratch(1, (int)N, (int)P, (int)H, (int)W, (int)Q, kH, kW, dH, dW, padH,
+                                                                               padW, dilationH, dilationW, adjH, adjW));
+            TH_CALL(s, cunn_b200_full_conv_grad_input_scratch(tdata<float>(gy), tdata<float>(weight), tdata<float>(gradInput), (int)N, (int)P,
                                                       (int)H, (int)W, (int)Q, kH, kW, dH, dW, padH, padW, dilationH, dilationW, adjH,
-                                                      adjW, state_stream(s)));
+                                                      adjW, ws.ptr, ws.bytes, state_stream(s)));
             if (input->nDimension == 3) tensor_resize(s, gradInput, 3, sz4 + 1, 4);
         }
     }
@@ -412,11 +532,12 @@ extern "C" CUNN_API void THNN_CudaSpatialFullDilatedConvolution_accGradParameter
     if (x && gy) {
         const size_t need = cunn_b200_full_conv_acc_grad_workspace((int)N, (int)P, (int)H, (int)W, (int)Q, kH, kW, dH, dW, padH, padW,
                                                                     dilationH, dilationW, adjH, adjW);
-        void *ws = need ? state_scratch(s, 0, need) : nullptr;
-        if (!need || ws)
+        const ConvScratch ws(s, cunn_b200_full_conv_scratch(2, (int)N, (int)P, (int)H, (int)W, (int)Q, kH, kW, dH, dW, padH, padW,
+                                                                           dilationH, dilationW, adjH, adjW), need);
+        if (!need || ws.ptr)
             TH_CALL(s, cunn_b200_full_conv_acc_grad(tdata<float>(x), tdata<float>(gy), tdata<float>(gradWeight),
                                                     gradBias ? tdata<float>(gradBias) : nullptr, (int)N, (int)P, (int)H, (int)W, (int)Q,
-                                                    kH, kW, dH, dW, padH, padW, dilationH, dilationW, adjH, adjW, scale, ws, need,
+                                                    kH, kW, dH, dW, padH, padW, dilationH, dilationW, adjH, adjW, scale, ws.ptr, ws.bytes,
                                                     state_stream(s)));
     }
 done:

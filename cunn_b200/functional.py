@@ -158,6 +158,26 @@ def batchnorm_backward(x, gy, weight, running_mean, running_var, save_mean, save
     return out if want_gx else None
 
 
+_LARGE = 16 << 20
+
+
+def _conv_scratch(size_fn, which, geo, device, least=0):
+    """(tensor, pointer, bytes) of the scratch memory that a pass of a convolution takes: 0 forward, 1 input gradient, 2 parameter
+    gradient, which cannot do without `least` bytes.  Large buffers are the allocator's again when the call has been queued; none are
+    shared between streams or with a graph under capture."""
+    need = size_fn(which, *geo)
+    if need > least:
+        try:
+            ws = torch.empty(need, dtype=torch.uint8, device=device)
+            return ws, _ptr(ws), need
+        except torch.cuda.OutOfMemoryError:
+            pass                                           # the kernels without scratch
+    if not least:
+        return None, None, 0
+    ws = workspace(least, device) if least <= _LARGE else torch.empty(least, dtype=torch.uint8, device=device)
+    return ws, _ptr(ws), ws.numel()
+
+
 def convmm_forward(x, weight, bias, dH, dW, padH, padW, out=None):
     """weight: [K, C, kH, kW] contiguous (the reference's [K, C*kH*kW] view of the same memory)."""
     _chk(x, weight, bias)
@@ -166,6 +186,12 @@ def convmm_forward(x, weight, bias, dH, dW, padH, padW, out=None):
     oH, oW = conv_out(H, kH, dH, padH), conv_out(W, kW, dW, padW)
     if out is None:
         out = torch.empty((N, K, max(oH, 0), max(oW, 0)), dtype=torch.float32, device=x.device)
+    if kH * kW > 1:
+        geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
+        ws = _conv_scratch(lib.cunn_b200_conv_scratch, 0, geo, x.device)
+        check(lib.cunn_b200_conv_forward_scratch(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), *geo,
+                                                 ws[1], ws[2], _stream()))
+        return out
     check(lib.cunn_b200_convmm_forward(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), N, C, H, W, K, kH, kW,
                                        dH, dW, padH, padW, _stream()))
     return out
@@ -177,6 +203,12 @@ def convmm_grad_input(gy, weight, H, W, dH, dW, padH, padW, out=None):
     N = gy.shape[0]
     if out is None:
         out = torch.empty((N, C, H, W), dtype=torch.float32, device=gy.device)
+    if kH * kW > 1:
+        geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
+        ws = _conv_scratch(lib.cunn_b200_conv_scratch, 1, geo, gy.device)
+        check(lib.cunn_b200_conv_grad_input_scratch(_ptr(gy), _ptr(weight), _ptr(out), *geo,
+                                                    ws[1], ws[2], _stream()))
+        return out
     check(lib.cunn_b200_convmm_grad_input(_ptr(gy), _ptr(weight), _ptr(out), N, C, H, W, K, kH, kW,
                                           dH, dW, padH, padW, _stream()))
     return out
@@ -188,9 +220,13 @@ def convmm_acc_grad(x, gy, grad_weight, grad_bias, dH, dW, padH, padW, scale=1.0
     N, C, H, W = x.shape
     K, _, kH, kW = grad_weight.shape
     need = lib.cunn_b200_convmm_acc_grad_workspace(N, C, H, W, K, kH, kW, dH, dW, padH, padW)
-    ws = workspace(need, x.device)
+    if kH * kW > 1 and need:
+        ws, at, size = _conv_scratch(lib.cunn_b200_conv_scratch, 2, (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1), x.device, need)
+    else:
+        ws = workspace(need, x.device)
+        at, size = _ptr(ws), ws.numel()
     check(lib.cunn_b200_convmm_acc_grad(_ptr(x), _ptr(gy), _ptr(grad_weight), _ptr(grad_bias), N, C, H, W, K, kH, kW,
-                                        dH, dW, padH, padW, scale, _ptr(ws), ws.numel(), _stream()))
+                                        dH, dW, padH, padW, scale, at, size, _stream()))
     return grad_weight, grad_bias
 
 
@@ -206,8 +242,10 @@ def dilated_conv_forward(x, weight, bias, dH, dW, padH, padW, dilH, dilW, out=No
     oH, oW = dilated_conv_out(H, kH, dH, padH, dilH), dilated_conv_out(W, kW, dW, padW, dilW)
     if out is None:
         out = torch.empty((N, K, max(oH, 0), max(oW, 0)), dtype=torch.float32, device=x.device)
-    check(lib.cunn_b200_dilated_conv_forward(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), N, C, H, W, K, kH, kW,
-                                             dH, dW, padH, padW, dilH, dilW, _stream()))
+    geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW)
+    ws = _conv_scratch(lib.cunn_b200_conv_scratch, 0, geo, x.device)
+    check(lib.cunn_b200_conv_forward_scratch(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), *geo,
+                                             ws[1], ws[2], _stream()))
     return out
 
 
@@ -217,8 +255,10 @@ def dilated_conv_grad_input(gy, weight, H, W, dH, dW, padH, padW, dilH, dilW, ou
     N = gy.shape[0]
     if out is None:
         out = torch.empty((N, C, H, W), dtype=torch.float32, device=gy.device)
-    check(lib.cunn_b200_dilated_conv_grad_input(_ptr(gy), _ptr(weight), _ptr(out), N, C, H, W, K, kH, kW,
-                                                dH, dW, padH, padW, dilH, dilW, _stream()))
+    geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW)
+    ws = _conv_scratch(lib.cunn_b200_conv_scratch, 1, geo, gy.device)
+    check(lib.cunn_b200_conv_grad_input_scratch(_ptr(gy), _ptr(weight), _ptr(out), *geo,
+                                                ws[1], ws[2], _stream()))
     return out
 
 
@@ -227,10 +267,9 @@ def dilated_conv_acc_grad(x, gy, grad_weight, grad_bias, dH, dW, padH, padW, dil
     _chk(x, gy, grad_weight, grad_bias)
     N, C, H, W = x.shape
     K, _, kH, kW = grad_weight.shape
-    need = lib.cunn_b200_dilated_conv_acc_grad_workspace(N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW)
-    ws = workspace(need, x.device)
-    check(lib.cunn_b200_dilated_conv_acc_grad(_ptr(x), _ptr(gy), _ptr(grad_weight), _ptr(grad_bias), N, C, H, W, K, kH, kW,
-                                              dH, dW, padH, padW, dilH, dilW, scale, _ptr(ws), ws.numel(), _stream()))
+    geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW)
+    ws = _conv_scratch(lib.cunn_b200_conv_scratch, 2, geo, x.device, max(lib.cunn_b200_dilated_conv_acc_grad_workspace(*geo), 1))
+    check(lib.cunn_b200_dilated_conv_acc_grad(_ptr(x), _ptr(gy), _ptr(grad_weight), _ptr(grad_bias), *geo, scale, ws[1], ws[2], _stream()))
     return grad_weight, grad_bias
 
 
@@ -246,8 +285,10 @@ def full_conv_forward(x, weight, bias, dH, dW, padH, padW, dilH=1, dilW=1, adjH=
     OH, OW = full_conv_out(H, kH, dH, padH, dilH, adjH), full_conv_out(W, kW, dW, padW, dilW, adjW)
     if out is None:
         out = torch.empty((N, Q, max(OH, 0), max(OW, 0)), dtype=torch.float32, device=x.device)
-    check(lib.cunn_b200_full_conv_forward(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), N, P, H, W, Q, kH, kW,
-                                          dH, dW, padH, padW, dilH, dilW, adjH, adjW, _stream()))
+    geo = (N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW)
+    ws = _conv_scratch(lib.cunn_b200_full_conv_scratch, 0, geo, x.device)
+    check(lib.cunn_b200_full_conv_forward_scratch(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), *geo,
+                                                  ws[1], ws[2], _stream()))
     return out
 
 
@@ -257,8 +298,10 @@ def full_conv_grad_input(gy, weight, H, W, dH, dW, padH, padW, dilH=1, dilW=1, a
     N = gy.shape[0]
     if out is None:
         out = torch.empty((N, P, H, W), dtype=torch.float32, device=gy.device)
-    check(lib.cunn_b200_full_conv_grad_input(_ptr(gy), _ptr(weight), _ptr(out), N, P, H, W, Q, kH, kW,
-                                             dH, dW, padH, padW, dilH, dilW, adjH, adjW, _stream()))
+    geo = (N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW)
+    ws = _conv_scratch(lib.cunn_b200_full_conv_scratch, 1, geo, gy.device)
+    check(lib.cunn_b200_full_conv_grad_input_scratch(_ptr(gy), _ptr(weight), _ptr(out), *geo,
+                                                     ws[1], ws[2], _stream()))
     return out
 
 
@@ -268,9 +311,8 @@ def full_conv_acc_grad(x, gy, grad_weight, grad_bias, dH, dW, padH, padW, dilH=1
     N, P, H, W = x.shape
     _, Q, kH, kW = grad_weight.shape
     geo = (N, P, H, W, Q, kH, kW, dH, dW, padH, padW, dilH, dilW, adjH, adjW)
-    ws = workspace(lib.cunn_b200_full_conv_acc_grad_workspace(*geo), x.device)
-    check(lib.cunn_b200_full_conv_acc_grad(_ptr(x), _ptr(gy), _ptr(grad_weight), _ptr(grad_bias), *geo, scale,
-                                           _ptr(ws), ws.numel(), _stream()))
+    ws = _conv_scratch(lib.cunn_b200_full_conv_scratch, 2, geo, x.device, max(lib.cunn_b200_full_conv_acc_grad_workspace(*geo), 1))
+    check(lib.cunn_b200_full_conv_acc_grad(_ptr(x), _ptr(gy), _ptr(grad_weight), _ptr(grad_bias), *geo, scale, ws[1], ws[2], _stream()))
     return grad_weight, grad_bias
 
 

@@ -123,12 +123,28 @@ CUNN_API int cunn_b200_convmm_acc_grad(const float *x, const float *gy, float *g
                                        int dH, int dW, int padH, int padW, float scale,
                                        void *workspace, size_t workspace_bytes, cunn_stream_t stream);
 
-/* 1x1 stride-1 convolutions on 16-byte aligned tensors with H*W and C multiples of 4 fetch their operand tiles with
- * tensor-map (TMA) copies; everything else, and every shape after cunn_b200_convmm_set_tma(0), uses the element-copy
- * loader.  Results are identical; the switch exists so that both loaders can be tested and timed.  No reference
- * counterpart. */
+/* Tensor-map (TMA) copies fetch the operand tiles of 1x1 stride-1 convolutions on 16-byte aligned tensors with H*W and C
+ * multiples of 4, and of the kernels that take scratch memory (next); everything else, and every shape after
+ * cunn_b200_convmm_set_tma(0), uses the element-copy loaders.  Results agree to rounding; the switch exists so that both
+ * loaders can be tested and timed.  No reference counterpart. */
 CUNN_API void cunn_b200_convmm_set_tma(int on);
 CUNN_API int cunn_b200_convmm_get_tma(void);
+
+/* Forward pass (pass 0) and input gradient (pass 1) of a convolution with scratch memory: kernels of more than one tap then
+ * run on operands that a first pass splits once, two to five times faster.  cunn_b200_conv_scratch(...) gives the bytes
+ * (16-byte aligned, contents arbitrary, at most about the size of the tensor that the pass reads, bounded by 0.5 GiB
+ * and one image's, plus that of the weights); 0: the pass has no use for scratch.  With less, or NULL, the calls are those
+ * without scratch.  No reference counterpart: the reference's `columns` buffer is scratch of the same kind. */
+CUNN_API size_t cunn_b200_conv_scratch(int pass, int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW,
+                                       int padH, int padW, int dilH, int dilW);
+CUNN_API int cunn_b200_conv_forward_scratch(const float *x, const float *weight, const float *bias, float *y,
+                                            int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW,
+                                            int padH, int padW, int dilH, int dilW, void *scratch, size_t scratch_bytes,
+                                            cunn_stream_t stream);
+CUNN_API int cunn_b200_conv_grad_input_scratch(const float *gy, const float *weight, float *gx,
+                                               int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW,
+                                               int padH, int padW, int dilH, int dilW, void *scratch, size_t scratch_bytes,
+                                               cunn_stream_t stream);
 
 /* ---- SpatialDilatedConvolution -------------------------------------------------
  * The same three passes with the kernel taps dilH x dilW apart: output size
@@ -167,6 +183,17 @@ CUNN_API int cunn_b200_full_conv_grad_input(const float *gy, const float *weight
                                             int N, int P, int H, int W, int Q, int kH, int kW, int dH, int dW,
                                             int padH, int padW, int dilH, int dilW, int adjH, int adjW,
                                             cunn_stream_t stream);
+/* The first two with scratch memory, as for cunn_b200_conv_forward_scratch. */
+CUNN_API size_t cunn_b200_full_conv_scratch(int pass, int N, int P, int H, int W, int Q, int kH, int kW, int dH, int dW,
+                                            int padH, int padW, int dilH, int dilW, int adjH, int adjW);
+CUNN_API int cunn_b200_full_conv_forward_scratch(const float *x, const float *weight, const float *bias, float *y,
+                                                 int N, int P, int H, int W, int Q, int kH, int kW, int dH, int dW,
+                                                 int padH, int padW, int dilH, int dilW, int adjH, int adjW, void *scratch,
+                                                 size_t scratch_bytes, cunn_stream_t stream);
+CUNN_API int cunn_b200_full_conv_grad_input_scratch(const float *gy, const float *weight, float *gx,
+                                                    int N, int P, int H, int W, int Q, int kH, int kW, int dH, int dW,
+                                                    int padH, int padW, int dilH, int dilW, int adjH, int adjW,
+                                                    void *scratch, size_t scratch_bytes, cunn_stream_t stream);
 CUNN_API size_t cunn_b200_full_conv_acc_grad_workspace(int N, int P, int H, int W, int Q, int kH, int kW,
                                                        int dH, int dW, int padH, int padW, int dilH, int dilW,
                                                        int adjH, int adjW);
