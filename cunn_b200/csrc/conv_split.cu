@@ -20,11 +20,12 @@
 // Accumulation: the tensor core truncates when it adds, so a chain is one block, 64 channels (or pixels) of 12 additions, the eight of
 // the cross terms first, while the accumulator is small; blocks are added in registers with rounding (two TMEM buffers in turn).
 //
-// Forward / input gradient / parameter gradient in us, gathering kernels before and now: 3x3 256 -> 256 on 128 x 14 x 14 270 / 313 / 354 and
-// 102 / 100 / 160 (87 TFLOP/s and 290 in the first two); 3x3 stride 2 128 -> 256 on 64 x 56 x 56 312 / 427 / 360 and 139 / 181 / 248; 4x4
-// stride 2 transposed 256 -> 128 on 64 x 14 x 14 240 / 193 / 172 and 77 / 62 / 95.  2-norm errors of the first 9.7e-7 / 2.1e-6 / 2.7e-6 and 0.8e-7 /
-// 1.6e-7 / 1.9e-7.  Of 102 us of a pass the split takes 15.  The matrix kernel needs 1,130 clocks per 128 x 256 x 32 block, where the tensor
-// pipe needs 768 and reading its operands from shared memory, and filling them, 940.
+// Forward / input gradient / parameter gradient in us, gathering kernels and here: 3x3 256 -> 256 on 128 x 14 x 14 270 / 313 / 354 and
+// 101 / 99 / 124; 3x3 stride 2 128 -> 256 on 64 x 56 x 56 312 / 427 / 360 and 134 / 172 / 189; 4x4 stride 2 transposed 256 -> 128 on
+// 64 x 14 x 14 240 / 193 / 172 and 72 / 61 / 80; 7x7 stride 2, 3 -> 64 on 32 x 224 x 224 234 / - / 316 and 130 / - / 196.  2-norm errors of the
+// first 9.7e-7 / 2.1e-6 / 2.7e-6 and 0.8e-7 / 1.6e-7 / 1.9e-7.  The split takes 14 of the 101 us, in a parameter gradient the maxima 18 and
+// the split 19 of 124.  The matrix kernel needs 1,100 to 1,200 clocks per 128 x 256 x 32 values, where the tensor pipe needs 768 and reading
+// its operands from shared memory, and filling them, 940.
 //
 // Work: 128 x BN tiles of the persistent grid; the tiles of a last wave that would leave SMs idle are cut along the reduction, and the
 // CTA that finishes a tile last adds its parts in their order (a counter per tile; nobody waits).
@@ -53,7 +54,8 @@ constexpr int THREADS = (MMA_WARP + 1) * 32;
 constexpr int SUM_REGS = 224, ISSUE_REGS = 56;
 constexpr int MAX_PHASES = 4;            // stride 2
 constexpr size_t RING_BYTES = 192 * 1024;
-constexpr size_t SMEM = RING_BYTES + EPI_WARPS * 4096;
+constexpr int STORE_COLS = 16, STORE_BYTES = STORE_COLS * (128 + 16);     // columns that a summing warp stores at a time, and its room for them
+constexpr size_t SMEM = RING_BYTES + EPI_WARPS * STORE_BYTES;
 constexpr int SCALED_MAX = 14;           // the largest value of a group lies in [2^14, 2^15) after scaling
 
 
@@ -78,38 +80,51 @@ __device__ __forceinline__ void parts(float v, float s, __half &hi, __half &lo)
 }
 
 // ---- splitting --------------------------------------------------------------------------------------------------------------------
+constexpr int TILE_PITCH = 65, TILE_VALUES = GROUP * TILE_PITCH;          // shared memory of a splitting block, in fp32 values
+
+// Few input channels: a convolution of kH x kW taps and C channels is one of kH x 1 taps and kW * C channels on the tensor of row windows
+// x'[n][h][ow][kw * C + c] = x[n][c][h][ow * dW - padW + kw].  C = 0: the tensor as it is.
+struct Window {
+    int C, kW, dW, padW, W, oW;
+    // values of one row of the image, in pixel-major order with its padding, that the windows of the row cut out
+    __host__ __device__ int row_values() const { return ((oW - 1) * dW + kW) * C; }
+    __host__ __device__ int block_rows() const { return row_values() <= TILE_VALUES / 4 ? 4 : row_values() <= TILE_VALUES / 2 ? 2 : 1; }
+};
 struct Act {                     // [images][C][HW] fp32 -> hi, lo: [2][images * HW][Cp] fp16
     const float *src;
     __half *dst;
     int8_t *exps;                // per pixel and group: exponent; null: exponents come from chmax
     const uint32_t *chmax;       // per channel: bits of the largest finite magnitude
-    double *bias_part;           // [blocks of 64 pixels][C] sums of src, or null
-    int C, Cp, HW, groups, blocks;
+    int C, Cp, HW, groups, blocks, ctas;      // tiles (row windows: rows), and the blocks that take them
     int vec;                     // planes of a multiple of four values, 16-byte aligned
+    Window win;
     uint32_t pixels;
 };
 struct PrepParams {
     Act act[2];
-    int n_act;
-    // weights, one block per row (filter, or input channel of an input gradient): value (row, c, tap) at row * w_row + c * w_c + tap
+    // weights, a block per row (filter, or input channel of an input gradient): value (row, c, tap) at row * w_row + c * w_c + tap
     const float *w;
     __half *w_dst;               // [2][taps][rows][Cp]
     int *w_exp;                  // [rows]: exponent
     int rows, w_C, w_Cp, taps;
     long long w_row, w_c;
+    int win_C, win_kW;           // Window's: value (row, kw * C + c, th) at row * w_row + c * w_c + th * kW + kw; 0: none
     int *tickets;
     int n_tickets;
 };
 
-__device__ __forceinline__ void prep_weights(const PrepParams &p, int row)
+__device__ __forceinline__ void prep_weights(const PrepParams &p, int row, float *tile)
 {
     __shared__ uint32_t red[8];
     const float *w = p.w + (long long)row * p.w_row;
-    const int n = p.w_C * p.taps;
+    const int C = p.win_C ? p.win_C : p.w_C, per = p.win_C ? p.taps * p.win_kW : p.taps, n = p.w_C * p.taps;      // channels, taps of each, values
     float m = 0.f;
+#pragma unroll 8
     for (int i = threadIdx.x; i < n; i += 256) {
-        const int c = i / p.taps, t = i - c * p.taps;
-        m = fmaxf(m, finite_abs(__ldg(w + c * p.w_c + t)));
+        const int c = i / per;
+        const float v = __ldg(w + c * p.w_c + (i - c * per));
+        if (i < TILE_VALUES) tile[i] = v;
+        m = fmaxf(m, finite_abs(v));
     }
     uint32_t b = __float_as_uint(m);
     b = __reduce_max_sync(0xffffffffu, b);
@@ -121,10 +136,16 @@ __device__ __forceinline__ void prep_weights(const PrepParams &p, int row)
     if (threadIdx.x == 0) p.w_exp[row] = e;
     const float s = pow2(SCALED_MAX - e);
     const size_t part = (size_t)p.taps * p.rows * p.w_Cp;
+#pragma unroll 4
     for (int i = threadIdx.x; i < p.w_Cp * p.taps; i += 256) {
         const int t = i / p.w_Cp, c = i - t * p.w_Cp;
+        float v = 0.f;
+        if (c < p.w_C) {
+            const int kw = p.win_C ? c / C : 0, ch = c - kw * C, at = p.win_C ? t * p.win_kW + kw : t, flat = ch * per + at;
+            v = flat < TILE_VALUES ? tile[flat] : __ldg(w + ch * p.w_c + at);
+        }
         __half hi, lo;
-        parts(c < p.w_C ? __ldg(w + c * p.w_c + t) : 0.f, s, hi, lo);
+        parts(v, s, hi, lo);
         __half *d = p.w_dst + ((size_t)t * p.rows + row) * p.w_Cp + c;
         d[0] = hi;
         d[part] = lo;
@@ -134,13 +155,12 @@ __device__ __forceinline__ void prep_weights(const PrepParams &p, int row)
 // One block: 64 pixels (of the flat pixel sequence) x 64 channels, through shared memory: read along the pixels, written along the
 // channels, a warp four pixels of 128 bytes at a time (16 bytes of each of 32 pixels per instruction took twice as long).
 template <bool PER_CHANNEL>
-__device__ __forceinline__ void prep_act(const Act &a, int block)
+__device__ __forceinline__ void prep_act(const Act &a, int block, float *tile_)
 {
-    __shared__ float tile[GROUP][65];
+    float(*tile)[TILE_PITCH] = reinterpret_cast<float(*)[TILE_PITCH]>(tile_);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int pb = block / a.groups, g = block - pb * a.groups;
     const uint32_t p0 = (uint32_t)pb * 64u;
-    double sums[8];
     if (a.vec) {
         // four consecutive pixels of a channel: lanes 0-15 of one, 16-31 of the next
         const uint32_t px = p0 + (lane & 15) * 4, im = px / (uint32_t)a.HW;
@@ -156,7 +176,6 @@ __device__ __forceinline__ void prep_act(const Act &a, int block)
         for (int i = 0; i < 4; ++i) {
             float *t = &tile[warp * 8 + i * 2 + (lane >> 4)][(lane & 15) * 4];
             t[0] = v[i].x; t[1] = v[i].y; t[2] = v[i].z; t[3] = v[i].w;
-            sums[i] = ((double)v[i].x + (double)v[i].y) + ((double)v[i].z + (double)v[i].w);
         }
     } else {
         const float *src[2];
@@ -178,18 +197,6 @@ __device__ __forceinline__ void prep_act(const Act &a, int block)
         for (int i = 0; i < 8; ++i) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) tile[warp * 8 + i][h * 32 + lane] = v[i][h];
-            sums[i] = (double)v[i][0] + (double)v[i][1];
-        }
-    }
-    if (a.bias_part) {
-        const int channels = a.vec ? 4 : 8, top = a.vec ? 8 : 16;          // lanes that share a channel: 16 or all
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (i >= channels) break;
-            double s = sums[i];
-            for (int o = top; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            const int c = g * GROUP + warp * 8 + (a.vec ? i * 2 + (lane >> 4) : i);
-            if ((lane & (a.vec ? 15 : 31)) == 0 && c < a.C) a.bias_part[(size_t)pb * a.C + c] = s;
         }
     }
     const int piece = lane & 7, c0 = g * GROUP + piece * 8;               // eight channels of a pixel
@@ -229,71 +236,165 @@ __device__ __forceinline__ void prep_act(const Act &a, int block)
     }
 }
 
+// Row windows: a block takes up to four rows of the images.  A row's values are split once, into shared memory in pixel-major order; a
+// window is a run of them.  (Split where they are written, 3.5 times each for 7x7 stride 2, 32 x 3 x 224 x 224 took 59 us; with a block
+// per row 45.)  One exponent per row.
 template <bool PER_CHANNEL>
+__device__ __forceinline__ void prep_window(const Act &a, int block, float *tile)
+{
+    __shared__ uint32_t red[8];
+    const Window &w = a.win;
+    const int n = w.row_values(), R = w.block_rows(), T = 256 / R, slot = threadIdx.x / T, tid = threadIdx.x - slot * T;
+    const int rows = a.HW / w.oW, row = block * R + slot, cols = n / w.C;
+    const bool ok = row < a.blocks;
+    const int im = ok ? row / rows : 0, h = ok ? row - im * rows : 0;
+    const size_t plane = (size_t)rows * w.W;
+    const float *src = a.src + (size_t)im * w.C * plane + (size_t)h * w.W;
+    __half *hi = reinterpret_cast<__half *>(tile) + slot * (2 * TILE_VALUES / R), *lo = hi + n;
+    float s = 0.f;
+    if (!PER_CHANNEL) {
+        float m = 0.f;
+        for (int c = 0; c < w.C; ++c) {
+#pragma unroll 4
+            for (int i = tid; i < w.W; i += T) m = fmaxf(m, finite_abs(__ldg(src + c * plane + i)));
+        }
+        uint32_t b = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = b;
+        __syncthreads();
+        for (int i = 0; i < 8 / R; ++i) b = max(b, red[slot * (8 / R) + i]);
+        const int e = group_exp(b);
+        s = pow2(SCALED_MAX - e);
+        if (ok)
+            for (int i = tid; i < w.oW; i += T) a.exps[(size_t)row * w.oW + i] = (int8_t)e;
+    }
+    for (int c = 0; c < w.C; ++c) {
+        if (PER_CHANNEL) s = pow2(SCALED_MAX - group_exp(__ldg(a.chmax + c)));
+#pragma unroll 4
+        for (int i = tid; i < cols; i += T) {
+            const int at = i - w.padW;
+            parts((unsigned)at < (unsigned)w.W ? __ldg(src + c * plane + at) : 0.f, s, hi[i * w.C + c], lo[i * w.C + c]);
+        }
+    }
+    __syncthreads();
+    if (!ok) return;
+    // 16-byte pieces of the windows; those past a window's last value are zeros
+    const int pieces = a.Cp / 8, step = w.dW * w.C;
+    const size_t part = (size_t)a.pixels * a.Cp;
+    __half *dst = a.dst + (size_t)row * w.oW * a.Cp;
+    for (int i = tid; i < w.oW * pieces; i += T) {
+        const int ow = i / pieces, c0 = (i - ow * pieces) * 8, at = ow * step + c0, left = a.C - c0;
+        __align__(16) __half ph[8];
+        __align__(16) __half pl[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            ph[k] = k < left ? hi[at + k] : __ushort_as_half(0);
+            pl[k] = k < left ? lo[at + k] : __ushort_as_half(0);
+        }
+        *reinterpret_cast<uint4 *>(dst + (size_t)i * 8) = *reinterpret_cast<const uint4 *>(ph);
+        *reinterpret_cast<uint4 *>(dst + part + (size_t)i * 8) = *reinterpret_cast<const uint4 *>(pl);
+    }
+}
+
+// WINDOW: the last tensor is one of row windows.
+template <bool PER_CHANNEL, bool WINDOW>
 __global__ void __launch_bounds__(256)
 prep_kernel(const __grid_constant__ PrepParams p)
 {
+    __shared__ float tile[TILE_VALUES];
     pdl_wait();
     pdl_launch_dependents();
     int b = (int)blockIdx.x;
     if (b == 0)
         for (int i = threadIdx.x; i < p.n_tickets; i += 256) p.tickets[i] = 0;
     if (b < p.rows) {
-        prep_weights(p, b);
+        prep_weights(p, b, tile);
         return;
     }
     b -= p.rows;
-    if (b < p.act[0].blocks) prep_act<PER_CHANNEL>(p.act[0], b);
-    else if (p.n_act > 1) prep_act<PER_CHANNEL>(p.act[1], b - p.act[0].blocks);
+    const Act &act = p.act[PER_CHANNEL && b >= p.act[0].ctas ? 1 : 0];
+    if (PER_CHANNEL && b >= p.act[0].ctas) b -= p.act[0].ctas;
+    if (WINDOW && act.win.C) prep_window<PER_CHANNEL>(act, b, tile);
+    else prep_act<PER_CHANNEL>(act, b, tile);
 }
 
-// Largest finite magnitude of every channel: block = (channel, chunk of images), a warp per plane.
+// Largest finite magnitude of every channel, and the sums of the first tensor's channels (the bias gradient): block = (channel, chunk of
+// the channel's pieces), a warp per piece of a plane.
+constexpr int PIECE = 2048;              // values of a plane that a warp takes, at most
 struct MaxParams {
     const float *src[2];
     uint32_t *chmax[2];
-    int C[2], HW[2], chunks[2], vec[2], images;       // vec: planes of a multiple of four values, 16-byte aligned
+    double *sums;                                                // [chunks][C] of the first tensor, or null
+    int C[2], HW[2], pieces[2], chunks[2], vec[2], images;       // pieces of a plane; vec: planes of a multiple of four values, 16-byte aligned
 };
 __global__ void __launch_bounds__(256)
 channel_max_kernel(const __grid_constant__ MaxParams p)
 {
     pdl_launch_dependents();
+    __shared__ double part[8];
     __shared__ uint32_t red[8];
     int b = (int)blockIdx.x, t = 0;
     if (b >= p.C[0] * p.chunks[0]) { b -= p.C[0] * p.chunks[0]; t = 1; }
-    const int chunk = b / p.C[t], c = b - chunk * p.C[t], HW = p.HW[t], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n0 = (int)((long long)p.images * chunk / p.chunks[t]), n1 = (int)((long long)p.images * (chunk + 1) / p.chunks[t]);
-    const size_t step = (size_t)p.C[t] * HW;
+    const int chunk = b / p.C[t], c = b - chunk * p.C[t], HW = p.HW[t], per = p.pieces[t], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long total = (long long)p.images * per;
+    const int n0 = (int)(total * chunk / p.chunks[t]), n1 = (int)(total * (chunk + 1) / p.chunks[t]);
+    const int unit = p.vec[t] ? HW / 4 : HW, len = (unit + per - 1) / per;           // (per - 1) * len < unit
     const float *src = p.src[t] + (size_t)c * HW;
+    const bool add = p.sums && t == 0;
     float m = 0.f;
-    for (int n = n0 + warp; n < n1; n += 32) {                             // four planes at a time; those past the last repeat the first
+    double sum = 0.0;
+    for (int n = n0 + warp; n < n1; n += 32) {                             // four pieces at a time
         const float *s[4];
+        int left[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) s[j] = src + (size_t)(n + 8 * j < n1 ? n + 8 * j : n) * step;
+        for (int j = 0; j < 4; ++j) {
+            // a piece past the last, or a value past a piece's last, repeats another one: loads without conditions
+            const int k = n + 8 * j < n1 ? n + 8 * j : n, im = per == 1 ? k : k / per, from = (k - im * per) * len;
+            s[j] = src + (size_t)im * p.C[t] * HW + (size_t)from * (p.vec[t] ? 4 : 1);
+            left[j] = min(len, unit - from) - 1;
+        }
         if (p.vec[t]) {
 #pragma unroll 2
-            for (int i = lane; i < HW / 4; i += 32) {
+            for (int i = lane; i < len; i += 32) {
                 float4 v[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const float4 *>(s[j]) + i);
+                for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const float4 *>(s[j]) + min(i, left[j]));
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                     m = fmaxf(m, fmaxf(fmaxf(finite_abs(v[j].x), finite_abs(v[j].y)), fmaxf(finite_abs(v[j].z), finite_abs(v[j].w))));
+                if (add) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (i <= left[j] && n + 8 * j < n1) sum += ((double)v[j].x + (double)v[j].y) + ((double)v[j].z + (double)v[j].w);
+                }
             }
         } else {
 #pragma unroll 2
-            for (int i = lane; i < HW; i += 32) {
+            for (int i = lane; i < len; i += 32) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) m = fmaxf(m, finite_abs(__ldg(s[j] + i)));
+                for (int j = 0; j < 4; ++j) {
+                    const float v = __ldg(s[j] + min(i, left[j]));
+                    m = fmaxf(m, finite_abs(v));
+                    if (add && i <= left[j] && n + 8 * j < n1) sum += (double)v;
+                }
             }
         }
     }
     uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
     if (lane == 0) red[warp] = bits;
+    if (add) {
+        sum = warp_sum(sum);
+        if (lane == 0) part[warp] = sum;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int i = 1; i < 8; ++i) bits = max(bits, red[i]);
         atomicMax(p.chmax[t] + c, bits);
+        if (add) {
+#pragma unroll
+            for (int i = 1; i < 8; ++i) sum += part[i];
+            p.sums[(size_t)chunk * p.C[0] + c] = sum;
+        }
     }
 }
 
@@ -420,7 +521,14 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&r)[32])
                  :
                  : "memory");
 }
-__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory"); }
+// Barrier of the warps that share a tile.
+template <int SETS>
+__device__ __forceinline__ void sums_sync(int set)
+{
+    if (SETS == 1) asm volatile("bar.sync 1, 256;" ::: "memory");
+    else if (set == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+    else asm volatile("bar.sync 2, 128;" ::: "memory");
+}
 
 // One input-gradient value in plain fp32: products with the zeros in place of taps outside gy, or of an infinity's parts, can make a
 // NaN that the definition does not have.
@@ -480,29 +588,35 @@ __device__ __forceinline__ void raise(uint64_t (&acc2)[N], int &top, int to)
 }
 
 // Warps 0-7: sums (TMEM -> registers -> memory), two per TMEM lane quarter, each half of the columns; warps 8-10: copies; warp 11: MMAs.
-template <int BN, bool WG>
+// BG (weight gradient): values per row of the gathered operand, 64 or, for tensors of up to 32 channels, 32.
+template <int BN, bool WG, int BG = GROUP>
 __global__ void __launch_bounds__(THREADS, 1)
 split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps maps)
 {
     constexpr int STAGE = 2 * BK * 2 * (BM + BN), NS = (int)(RING_BYTES / STAGE);
     constexpr int A_PART = BM * BK * 2, B_PART = BN * BK * 2, A_LO = A_PART, B_HI = 2 * A_PART, B_LO = B_HI + B_PART;
-    constexpr int HALF_COLS = BN / 2;
-    constexpr uint32_t TMEM_COLS = 2 * BN;
+    // The two summing warpgroups take half of the columns of a tile each; or, where a thread can hold a whole row, they work on a tile
+    // each, with half of the stages and of TMEM and an issuing warp of its own (ALT).  A block of 64 channels costs its issuing thread
+    // 250 clocks of waits, 180 of commits and 70 per MMA, which is more than the MMAs of narrow tiles take, and one group writes its tile
+    // while the other one sums (7x7 on 3 channels has seven blocks a tile).
+    constexpr bool ALT = !WG && BN <= 128;
+    constexpr int HALF_COLS = ALT ? BN : BN / 2, SETS = ALT ? 2 : 1, BUFS = 512 / BN / SETS;      // TMEM buffers per set
+    constexpr int RING = NS / SETS;                                                                // stages per set
     constexpr size_t PART = BN * BM + BM;             // partial sums of a cut tile and their rows' exponents
 
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t full[NS], empty[NS];          // stage landed; its MMAs are done
-    __shared__ uint64_t ready[2], drained[2];         // a block's sums are in TMEM buffer b; they have been read
+    __shared__ uint64_t ready[SETS * BUFS], drained[SETS * BUFS];         // a block's sums are in TMEM buffer b; they have been read
     __shared__ uint32_t tmem_base_s;
-    __shared__ int last_s;
+    __shared__ int last_s[2];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(smem_u32(full + s), 1); mbar_init(smem_u32(empty + s), 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(smem_u32(ready + b), 1); mbar_init(smem_u32(drained + b), EPI_WARPS); }
+        for (int b = 0; b < SETS * BUFS; ++b) { mbar_init(smem_u32(ready + b), 1); mbar_init(smem_u32(drained + b), EPI_WARPS / SETS); }
         mbar_fence_init();
     }
-    if (warp == 0) tmem_alloc(smem_u32(&tmem_base_s), TMEM_COLS);
+    if (warp == 0) tmem_alloc(smem_u32(&tmem_base_s), 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -512,14 +626,17 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
 
     if (warp >= EPI_WARPS) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ISSUE_REGS));
-      if (warp < MMA_WARP) {
-        // A thread's copies start about 100 clocks apart and 4 or 8 KB each take 60 to 180, so three warps share them.
-        const int part_of = warp - EPI_WARPS;
+      const int set = ALT ? warp & 1 : 0, first_item = (int)blockIdx.x + set * (int)gridDim.x, item_step = SETS * (int)gridDim.x;
+      uint64_t *const my_full = full + set * RING, *const my_empty = empty + set * RING;
+      unsigned char *const my_smem = smem + (size_t)set * RING * STAGE;
+      if (warp < (ALT ? MMA_WARP - 1 : MMA_WARP)) {
+        // A thread's copies start about 100 clocks apart and 4 or 8 KB each take 60 to 180: three warps share them, or one has a set's.
+        const int part_of = ALT ? 0 : warp - EPI_WARPS;
         if (lane == 0) {
             int rs = 0;
             uint32_t parity = 1;                      // the first round finds the stages empty
             bool ok = true;
-            for (int i = (int)blockIdx.x; ok && i < p.items; i += (int)gridDim.x) {
+            for (int i = first_item; ok && i < p.items; i += item_step) {
                 const Item it = item_of<WG>(p, i);
                 if (!WG) {
                     const Phase &f = p.ph[it.phase];
@@ -529,38 +646,48 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                     int c = (it.begin - tap * p.groups) * GROUP, th = tap / f.kW, tw = tap - th * f.kW;
                     const CUtensorMap *ma = &maps.a[it.phase];
                     for (int q = it.begin; q < it.end;) {
-                        if (!mbar_wait(smem_u32(empty + rs), parity, p.status)) { ok = false; break; }
-                        const uint32_t bar = smem_u32(full + rs), s = smem_u32(smem) + (uint32_t)(rs * STAGE);
+                        if (!mbar_wait(smem_u32(my_empty + rs), parity, p.status)) { ok = false; break; }
+                        const uint32_t bar = smem_u32(my_full + rs), s = smem_u32(my_smem) + (uint32_t)(rs * STAGE);
                         if (part_of == 0) mbar_arrive_expect_tx(bar, STAGE);
-                        if (part_of < 2) {
+                        if (ALT || part_of < 2)
                             load_im2col(s + (uint32_t)(part_of * A_LO), ma, c, w0, h0, im + part_of * p.images, tw * f.dlW, th * f.dlH, bar);
-                        } else {
+                        if (ALT || part_of == 2) {
                             const int wt = f.w_base + th * f.w_sH + tw * f.w_sW;
                             load_3d(s + B_HI, &maps.b, c, n0, wt, bar);
+                            if (ALT) load_im2col(s + A_LO, ma, c, w0, h0, im + p.images, tw * f.dlW, th * f.dlH, bar);
                             load_3d(s + B_LO, &maps.b, c, n0, wt + p.w_kk, bar);
                         }
                         c += BK;
                         if (c >= p.g_C) { c = 0; if (++tw == f.kW) { tw = 0; ++th; } }
                         if ((c & (GROUP - 1)) == 0) ++q;                           // the group's last stage
-                        if (++rs == NS) { rs = 0; parity ^= 1u; }
+                        if (++rs == RING) { rs = 0; parity ^= 1u; }
                     }
                 } else {
-                    const int g0 = it.n_tile * (BN / GROUP), ng = min(BN / GROUP, p.col_groups - g0);
+                    const int g0 = it.n_tile * (BN / BG), ng = min(BN / BG, p.col_groups - g0);
+                    const int mg = min(BM / GROUP, (p.N_total - it.m_tile * BM + GROUP - 1) / GROUP);      // rows past the last are left as they are
+                    // this warp's copies of the gathered operand: l = part_of + 3 k -> part l & 1 of group l >> 1
+                    constexpr int PER_WARP = (2 * (BN / BG) + 2) / 3;
+                    int chan[PER_WARP], offs[PER_WARP];
+#pragma unroll
+                    for (int k = 0; k < PER_WARP; ++k) {
+                        const int j = (part_of + 3 * k) >> 1, tap = (g0 + j) / p.groups, th = tap / p.kW, tw = tap - th * p.kW;
+                        chan[k] = (g0 + j - tap * p.groups) * BG;
+                        offs[k] = tw * p.dlW | th * p.dlH << 16;
+                    }
                     for (int q = 2 * it.begin; q < 2 * it.end; ++q) {
                         if (!mbar_wait(smem_u32(empty + rs), parity, p.status)) { ok = false; break; }
                         const uint32_t bar = smem_u32(full + rs), s = smem_u32(smem) + (uint32_t)(rs * STAGE);
-                        if (part_of == 0) mbar_arrive_expect_tx(bar, (uint32_t)(2 * A_PART + 2 * ng * GROUP * BK * 2));
+                        if (part_of == 0) mbar_arrive_expect_tx(bar, (uint32_t)((2 * mg * GROUP + 2 * ng * BG) * BK * 2));
                         const int p0 = q * BK, im = p0 / p.pix_HW, r = p0 - im * p.pix_HW, row = r / p.pix_W, col = r - row * p.pix_W;
                         const int h0 = row * p.stH + p.lH, w0 = col * p.stW + p.lW;
-                        for (int l = part_of; l < 2 * (BM / GROUP + ng); l += 3) {
-                            const int part = l & 1, j = (l >> 1) - BM / GROUP;
-                            if (j < 0) {
-                                load_3d(s + (uint32_t)(part * A_PART + (l >> 1) * GROUP * BK * 2), &maps.a[0], it.m_tile * BM + (l >> 1) * GROUP, p0, part, bar);
-                            } else {
-                                const int tap = (g0 + j) / p.groups, g = g0 + j - tap * p.groups, th = tap / p.kW, tw = tap - th * p.kW;
-                                load_im2col(s + (uint32_t)(B_HI + part * B_PART + j * GROUP * BK * 2), &maps.b, g * GROUP, w0, h0,
-                                            im + part * p.images, tw * p.dlW, th * p.dlH, bar);
-                            }
+                        for (int l = part_of; l < 2 * mg; l += 3)
+                            load_3d(s + (uint32_t)((l & 1) * A_PART + (l >> 1) * GROUP * BK * 2), &maps.a[0], it.m_tile * BM + (l >> 1) * GROUP, p0, l & 1, bar);
+#pragma unroll
+                        for (int k = 0; k < PER_WARP; ++k) {
+                            const int l = part_of + 3 * k, part = l & 1, j = l >> 1;
+                            if (j < ng)
+                                load_im2col(s + (uint32_t)(B_HI + part * B_PART + j * BG * BK * 2), &maps.b, chan[k], w0, h0, im + part * p.images,
+                                            offs[k] & 0xffff, offs[k] >> 16, bar);
                         }
                         if (++rs == NS) { rs = 0; parity ^= 1u; }
                     }
@@ -570,25 +697,29 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
       } else {
         if (lane == 0) {
             // descriptors: K-major tiles of 64-byte rows in the 64-byte swizzle (groups of 8 rows 512 bytes apart); M/N-major ones of
-            // 128-byte rows in the 128-byte swizzle (8 k values 1024 bytes, 64 values of M or N 4096 bytes apart)
-            constexpr uint32_t LOW = WG ? (uint32_t)(GROUP * BK * 2 >> 4) << 16 : 1u << 16;
-            constexpr uint32_t HIGH = (uint32_t)((WG ? 1024 : 512) >> 4) | (1u << 14) | ((WG ? 2u : 4u) << 29);
-            constexpr uint32_t STEP = WG ? 2048u >> 4 : 2u;                        // 16 k values
-            auto desc = [](uint32_t low) { return ((uint64_t)HIGH << 32) | low; };
-            const uint32_t ring = (smem_u32(smem) >> 4) & 0x3fffu;
+            // 128-byte rows in the 128-byte swizzle (8 k values 1024 bytes, 64 values of M or N 4096 bytes apart), or of 64-byte rows
+            constexpr bool NARROW = WG && BG == 32;
+            constexpr uint32_t A_LOW = WG ? (uint32_t)(GROUP * BK * 2 >> 4) << 16 : 1u << 16, B_LOW = NARROW ? (uint32_t)(BG * BK * 2 >> 4) << 16 : A_LOW;
+            constexpr uint32_t A_HIGH = (uint32_t)((WG ? 1024 : 512) >> 4) | (1u << 14) | ((WG ? 2u : 4u) << 29);
+            constexpr uint32_t B_HIGH = NARROW ? (uint32_t)(512 >> 4) | (1u << 14) | (4u << 29) : A_HIGH;
+            constexpr uint32_t A_STEP = WG ? 2048u >> 4 : 2u, B_STEP = NARROW ? 1024u >> 4 : A_STEP;       // 16 k values
+            auto da = [](uint32_t low) { return ((uint64_t)A_HIGH << 32) | low; };
+            auto db = [](uint32_t low) { return ((uint64_t)B_HIGH << 32) | low; };
+            const uint32_t ring = (smem_u32(my_smem) >> 4) & 0x3fffu;
             int rs = 0, buf = 0;
-            uint32_t parity = 0, free_parity = 1;
+            uint32_t parity = 0, freed = 1;
             bool ok = true;
-            for (int i = (int)blockIdx.x; ok && i < p.items; i += (int)gridDim.x) {
+            for (int i = first_item; ok && i < p.items; i += item_step) {
                 const Item it = item_of<WG>(p, i);
-                const int cols = WG ? min(BN, (p.col_groups - it.n_tile * (BN / GROUP)) * GROUP)
+                const int cols = WG ? min(BN, (p.col_groups - it.n_tile * (BN / BG)) * BG)
                                     : min(p.width, ((p.N_total - it.n_tile * p.width) + 15) & ~15);
                 const uint32_t idesc = (1u << 4) | ((WG ? 1u : 0u) << 15) | ((WG ? 1u : 0u) << 16) | ((uint32_t)(cols >> 3) << 17) |
                                        ((uint32_t)(BM >> 4) << 24);
                 int c = WG ? 0 : it.begin % p.groups * GROUP;
                 for (int q = it.begin; q < it.end; ++q) {
-                    if (!mbar_wait(smem_u32(drained + buf), free_parity, p.status)) { ok = false; break; }
-                    const uint32_t d = tmem_base + (uint32_t)(buf * BN);
+                    const int slot = set * BUFS + buf;
+                    if (!mbar_wait(smem_u32(drained + slot), freed, p.status)) { ok = false; break; }
+                    const uint32_t d = tmem_base + (uint32_t)(slot * BN);
                     // 16-channel steps of the group that hold channels, two per stage
                     const int steps = WG ? 4 : min(4, (p.g_C - c + 15) >> 4);
                     // the small products first, while the accumulator is small: both stages' cross terms, then their hi*hi
@@ -597,39 +728,42 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         if (2 * h >= steps) break;
-                        if (!mbar_wait(smem_u32(full + rs), parity, p.status)) { ok = false; break; }
+                        if (!mbar_wait(smem_u32(my_full + rs), parity, p.status)) { ok = false; break; }
                         tc_fence_after();
                         st[h] = ring + (uint32_t)(rs * STAGE >> 4);
-                        const uint32_t ah = st[h] | LOW, al = (st[h] + (A_LO >> 4)) | LOW, bh = (st[h] + (B_HI >> 4)) | LOW, bl = (st[h] + (B_LO >> 4)) | LOW;
-                        umma_f16(d, desc(al), desc(bh), idesc, h ? 1u : 0u);       // a block's first one overwrites the buffer
-                        umma_f16_acc(d, desc(ah), desc(bl), idesc);
+                        const uint32_t ah = st[h] | A_LOW, al = (st[h] + (A_LO >> 4)) | A_LOW;
+                        const uint32_t bh = (st[h] + (B_HI >> 4)) | B_LOW, bl = (st[h] + (B_LO >> 4)) | B_LOW;
+                        umma_f16(d, da(al), db(bh), idesc, h ? 1u : 0u);           // a block's first one overwrites the buffer
+                        umma_f16_acc(d, da(ah), db(bl), idesc);
                         if (2 * h + 1 < steps) {
-                            umma_f16_acc(d, desc(al + STEP), desc(bh + STEP), idesc);
-                            umma_f16_acc(d, desc(ah + STEP), desc(bl + STEP), idesc);
+                            umma_f16_acc(d, da(al + A_STEP), db(bh + B_STEP), idesc);
+                            umma_f16_acc(d, da(ah + A_STEP), db(bl + B_STEP), idesc);
                         }
-                        if (++rs == NS) { rs = 0; parity ^= 1u; }
+                        if (++rs == RING) { rs = 0; parity ^= 1u; }
                     }
                     if (!ok) break;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         if (2 * h >= steps) break;
-                        const uint32_t ah = st[h] | LOW, bh = (st[h] + (B_HI >> 4)) | LOW;
-                        umma_f16_acc(d, desc(ah), desc(bh), idesc);
-                        if (2 * h + 1 < steps) umma_f16_acc(d, desc(ah + STEP), desc(bh + STEP), idesc);
-                        umma_commit(smem_u32(empty + (h == 0 ? first : first + 1 == NS ? 0 : first + 1)));
+                        const uint32_t ah = st[h] | A_LOW, bh = (st[h] + (B_HI >> 4)) | B_LOW;
+                        umma_f16_acc(d, da(ah), db(bh), idesc);
+                        if (2 * h + 1 < steps) umma_f16_acc(d, da(ah + A_STEP), db(bh + B_STEP), idesc);
+                        umma_commit(smem_u32(my_empty + (h == 0 ? first : first + 1 == RING ? 0 : first + 1)));
                     }
-                    umma_commit(smem_u32(ready + buf));
+                    umma_commit(smem_u32(ready + slot));
                     c += GROUP;
                     if (c >= p.g_C) c = 0;
-                    if (buf ^= 1) {} else free_parity ^= 1u;
+                    if (++buf == BUFS) { buf = 0; freed ^= 1u; }
                 }
             }
         }
       }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SUM_REGS));
-        const int quarter = warp & 3, col0 = (warp >> 2) * HALF_COLS, row_in = quarter * 32 + lane;
-        const uint32_t tsrc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
+        const int quarter = warp & 3, half = warp >> 2, col0 = ALT ? 0 : half * HALF_COLS, row_in = quarter * 32 + lane;
+        const uint32_t tsrc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ALT ? half * BUFS * BN : col0);
+        const int first_item = (int)blockIdx.x + (ALT ? half * (int)gridDim.x : 0), item_step = SETS * (int)gridDim.x;
+        uint64_t *const my_ready = ready + (ALT ? half * BUFS : 0), *const my_drained = drained + (ALT ? half * BUFS : 0);
         int buf = 0;
         uint32_t parity = 0;
         bool ok = true, nan_seen = false, tail_done = false;
@@ -642,13 +776,13 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
             col = r - row * f.pix_W;
             return m < f.M_total;
         };
-        for (int i = (int)blockIdx.x; ok && i < p.items; i += (int)gridDim.x) {
+        for (int i = first_item; ok && i < p.items; i += item_step) {
             const Item it = item_of<WG>(p, i);
             const Phase &f = p.ph[it.phase];
             uint64_t acc2[HALF_COLS / 2];                                          // columns 2 j and 2 j + 1
 #pragma unroll
             for (int j = 0; j < HALF_COLS / 2; ++j) acc2[j] = 0;
-            const int cols = WG ? min(BN, (p.col_groups - it.n_tile * (BN / GROUP)) * GROUP) : min(p.width, p.N_total - it.n_tile * p.width);
+            const int cols = WG ? min(BN, (p.col_groups - it.n_tile * (BN / BG)) * BG) : min(p.width, p.N_total - it.n_tile * p.width);
             const int my_cols = cols - col0;                                       // may be zero or negative
             int im = 0, row = 0, col = 0;
             bool row_ok = true;
@@ -674,7 +808,7 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                     if (__any_sync(0xffffffffu, e > top)) raise(acc2, top, max(e + 4, top));
                     s = step(e, top);
                 }
-                if (!mbar_wait(smem_u32(ready + buf), parity, p.status)) { ok = false; break; }
+                if (!mbar_wait(smem_u32(my_ready + buf), parity, p.status)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t t0 = tsrc + (uint32_t)(buf * BN);
                 const uint64_t s2 = pack2(s, s);
@@ -693,8 +827,8 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(drained + buf));
-                if (buf ^= 1) {} else parity ^= 1u;
+                if (lane == 0) mbar_arrive(smem_u32(my_drained + buf));
+                if (++buf == BUFS) { buf = 0; parity ^= 1u; }
             }
             if (!ok) break;
             float acc[HALF_COLS];
@@ -714,14 +848,14 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
             if (it.tail >= 0) {
                 float *mine = p.partial + (size_t)(it.tail * p.splits + it.part) * PART + (size_t)col0 * BM + row_in;
                 int *my_top = reinterpret_cast<int *>(p.partial + (size_t)(it.tail * p.splits + it.part) * PART + BN * BM) + row_in;
-                if (col0 == 0) __stcg(my_top, top);
+                if (ALT || half == 0) __stcg(my_top, top);
 #pragma unroll
                 for (int j = 0; j < HALF_COLS; ++j) __stcg(mine + j * BM, acc[j]);
                 __threadfence();
-                epilogue_sync();
-                if (tid == 0) last_s = atomicAdd(p.tickets + it.tail, 1) == p.splits - 1;
-                epilogue_sync();
-                if (!last_s) continue;
+                sums_sync<SETS>(half);
+                if ((tid & (ALT ? 127 : 255)) == 0) last_s[half] = atomicAdd(p.tickets + it.tail, 1) == p.splits - 1;
+                sums_sync<SETS>(half);
+                if (!last_s[ALT ? half : 0]) continue;
                 __threadfence();
                 const float *first = p.partial + (size_t)it.tail * p.splits * PART + row_in;
                 auto top_of = [&](int s) { return __ldcg(reinterpret_cast<const int *>(first + (size_t)s * PART + BN * BM)); };
@@ -738,31 +872,49 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                 }
                 tail_done = true;
             }
-            // Through shared memory, 32 columns at a time, so that the columns can be a loop: as straight code over registers, run once a
-            // tile, it is fetched from memory and took 20 us of a layer.
-            const int n0 = it.n_tile * p.width + col0;
+            // Through shared memory, 16 columns at a time, so that the columns can be a loop: as straight code over registers, run once a
+            // tile, it is fetched from memory and took 20 us of a layer.  2^(row + column exponent) goes on in two halves, see scale_by;
+            // a lane fetches a column's halves and bias for all (from memory in the loop: 160 clocks a column; by shuffles 90).
+            const int n0 = it.n_tile * p.width + col0, he = (top - 2 * SCALED_MAX) / 2;
+            const float ra = pow2(he), rb = pow2(top - 2 * SCALED_MAX - he);
             float *dst = p.out + ((size_t)im * p.N_total + n0) * p.o_HW + (f.o_off + row * f.o_sH + col * f.o_sW);
-            float *stage = reinterpret_cast<float *>(smem + RING_BYTES) + warp * 1024 + lane;     // a lane reads what it wrote itself
+            float *stage = reinterpret_cast<float *>(smem + RING_BYTES + warp * STORE_BYTES) + lane;        // a lane reads what it wrote itself
+            float4 *column = reinterpret_cast<float4 *>(smem + RING_BYTES + warp * STORE_BYTES + STORE_COLS * 128);
 #pragma unroll
-            for (int c = 0; c < HALF_COLS; c += 32) {
+            for (int c = 0; c < HALF_COLS; c += STORE_COLS) {
                 if (c >= my_cols) break;
+                const int last = min(STORE_COLS, my_cols - c);
+                __syncwarp();
+                if (lane < STORE_COLS) {
+                    const int ec = lane < last ? __ldg(p.w_exp + n0 + c + lane) : 0, hc = ec / 2;
+                    column[lane] = make_float4(pow2(hc), pow2(ec - hc), p.bias && lane < last ? __ldg(p.bias + n0 + c + lane) : 0.f, 0.f);
+                }
 #pragma unroll
-                for (int j = 0; j < 32; ++j) stage[j * 32] = acc[c + j];
-                if (!row_ok) continue;
-                const int last = min(32, my_cols - c);
-#pragma unroll 4
-                for (int j = 0; j < last; ++j) {
-                    const float v = stage[j * 32];
-                    nan_seen |= v != v;
-                    dst[(size_t)(c + j) * p.o_HW] = scale_by(v, __ldg(p.w_exp + n0 + c + j) + top - 2 * SCALED_MAX) +
-                                                    (p.bias ? __ldg(p.bias + n0 + c + j) : 0.f);
+                for (int j = 0; j < STORE_COLS; ++j) stage[j * 32] = acc[c + j];
+                __syncwarp();
+                const int count = row_ok ? last : 0;
+                float *to = dst + (size_t)c * p.o_HW;
+#pragma unroll 1
+                for (int j = 0; j < last; j += 8) {                // eight columns in step: one after the other they take 130 clocks each
+                    float v[8];
+                    float4 k[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { v[i] = stage[(j + i) * 32]; k[i] = column[j + i]; }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        nan_seen |= v[i] != v[i];
+                        v[i] = v[i] * (ra * k[i].x) * (rb * k[i].y) + k[i].z;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i, to += p.o_HW)
+                        if (j + i < count) *to = v[i];
                 }
             }
         }
-        if (!WG && p.raw_a && __any_sync(0xffffffffu, ok && nan_seen)) {
+        if (!WG && p.raw_a && __any_sync(0xffffffffu, ok && nan_seen)) {          // rows past the last may have seen some: they write nothing
             // outside the pipeline: no wait with a limit depends on how long this takes
 #pragma unroll 1
-            for (int i = (int)blockIdx.x; i < p.items; i += (int)gridDim.x) {
+            for (int i = first_item; i < p.items; i += item_step) {
                 const Item it = item_of<WG>(p, i);
                 if (it.tail >= 0 && !tail_done) continue;
                 const Phase &f = p.ph[it.phase];
@@ -780,17 +932,19 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
+    if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
 // gw[ko][c][tap] += scale * the sum of the splits in their order, scaled back; further blocks: the bias gradient from its partial sums.
-// A block takes 32 output channels x 32 consecutive (c, tap): partial sums are contiguous along the output channels, gw along (c, tap).
+// Partial sums are contiguous along the output channels, gw along (c, tap).
 struct ReduceParams {
     const float *partial;
     float *gw, *gb;
     const uint32_t *gy_max, *x_max;
     const double *bias_part;
-    int K, C, kk, groups, splits, cols, rows, gw_blocks, bias_blocks;
+    int K, C, kk, groups, bg, splits, cols, rows, gw_blocks, bias_blocks;
+    int shares;                              // warps that share an output's splits: 1, 2, 4 or 8
+    int win_kW;                              // Window's kernel columns, or 0
     float scale;
 };
 __global__ void __launch_bounds__(256)
@@ -808,32 +962,44 @@ reduce_kernel(const __grid_constant__ ReduceParams p)
         if (lane == 0) p.gb[k] = (float)((double)p.gb[k] + (double)p.scale * s);
         return;
     }
-    __shared__ float tile[32][33];
-    const int n = p.C * p.kk, o_blocks = (n + 31) / 32;
+    // a warp: 32 output channels x 4 consecutive (c, tap) x every `shares`-th split
+    __shared__ float tile[8][4][33];
+    const int n = p.C * p.kk, per = 32 / p.shares, o_blocks = (n + per - 1) / per;
     const int kb = (int)blockIdx.x / o_blocks, ob = (int)blockIdx.x - kb * o_blocks;
-    const int ko = kb * 32 + lane;
-    const size_t split_step = (size_t)p.cols * p.rows;
+    const int ko = kb * 32 + lane, share = warp & (p.shares - 1), o0 = ob * per + warp / p.shares * 4;
+    const size_t split_step = (size_t)p.cols * p.rows * p.shares;
     const float *src[4];
     int c[4];
     float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int o = min(ob * 32 + warp + 8 * i, n - 1);
+        const int o = min(o0 + i, n - 1);
         c[i] = o / p.kk;
-        src[i] = p.partial + (size_t)(((o - c[i] * p.kk) * p.groups + (c[i] >> 6)) * GROUP + (c[i] & 63)) * p.rows + ko;      // ko < rows
+        int t = o - c[i] * p.kk, at = c[i];
+        if (p.win_kW) {
+            const int th = t / p.win_kW;
+            at += (t - th * p.win_kW) * p.C;
+            t = th;
+        }
+        src[i] = p.partial + ((size_t)share * p.cols + (t * p.groups + at / p.bg) * p.bg + at % p.bg) * p.rows + ko;             // ko < rows
     }
 #pragma unroll 4
-    for (int k = 0; k < p.splits; ++k)
+    for (int k = share; k < p.splits; k += p.shares)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sum[i] += __ldg(src[i] + k * split_step);
+        for (int i = 0; i < 4; ++i) {
+            sum[i] += __ldg(src[i]);
+            src[i] += split_step;
+        }
     const int eg = ko < p.K ? group_exp(__ldg(p.gy_max + ko)) : 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) tile[warp + 8 * i][lane] = scale_by(sum[i], eg + group_exp(__ldg(p.x_max + c[i])) - 2 * SCALED_MAX);
+    for (int i = 0; i < 4; ++i) tile[warp][i][lane] = scale_by(sum[i], eg + group_exp(__ldg(p.x_max + c[i])) - 2 * SCALED_MAX);
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int k = kb * 32 + warp + 8 * i, o = ob * 32 + lane;
-        if (k < p.K && o < n) p.gw[(size_t)k * n + o] += p.scale * tile[lane][warp + 8 * i];
+    for (int i = tid; i < 32 * per; i += 256) {
+        const int k = i / per, o = i - k * per;
+        if (kb * 32 + k >= p.K || ob * per + o >= n) continue;
+        float s = 0.f;
+        for (int j = 0; j < p.shares; ++j) s += tile[(o >> 2) * p.shares + j][o & 3][k];
+        p.gw[(size_t)(kb * 32 + k) * n + ob * per + o] += p.scale * s;
     }
 }
 
@@ -863,7 +1029,21 @@ static EncodeIm2colFn encode_im2col()
 }
 
 static bool can_vec(const float *src, int HW) { return HW % 4 == 0 && ((uintptr_t)src & 15) == 0; }
-static int round8(int c) { return (c + 7) & ~7; }
+// Blocks of a splitting launch.
+static int prep_grid(PrepParams &q, int tensors)
+{
+    int grid = q.rows;
+    for (int i = 0; i < tensors; ++i) {
+        Act &a = q.act[i];
+        a.blocks = a.win.C ? (int)(a.pixels / (uint32_t)a.win.oW) : (int)ceil_div_ll((long long)a.pixels, 64) * a.groups;
+        a.ctas = a.win.C ? ceil_div(a.blocks, a.win.block_rows()) : a.blocks;
+        grid += a.ctas;
+    }
+    return grid;
+}
+// Channels of a split tensor, padded with zeros: pixels start on 32 or 64 bytes.  A copy's rows of 64 bytes that begin anywhere else
+// take three times as long (pixels of 48 bytes: 3.3 clocks a row).
+static int padded(int c) { return c < 64 ? (c + 15) & ~15 : (c + 31) & ~31; }
 static size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 // fp16 [d2][d1][d0], boxes of box0 x box1 x 1.
@@ -927,8 +1107,21 @@ static int images_per_round(int N, size_t image_bytes)
 constexpr size_t MIN_MAP_BYTES = 131072;
 
 // ---- forward pass and input gradients -------------------------------------------------------------------------------------------
+// Few input channels: the geometry of the same convolution on the tensor of row windows.
+static bool windowed(const Geometry &g, Geometry &v, Window &win)
+{
+    v = g;
+    win = Window{};
+    if (g.C >= 16) return true;
+    win = Window{g.C, g.kW, g.dW, g.padW, g.W, g.oW};
+    if (g.C * g.kW > GROUP || g.dilW != 1 || win.row_values() > TILE_VALUES) return false;
+    v.C = g.C * g.kW; v.W = g.oW; v.kW = v.dW = v.dilW = 1; v.padW = 0;
+    return true;
+}
+
 struct Plan {
     Params p;
+    Window win;
     Walk wh[MAX_PHASES], ww[MAX_PHASES];
     int images, Cp, bn;                    // images per round, channels of the gathered tensor padded to 8, column tile of the kernel
     int rows, taps;                        // weight rows (columns of the product) and taps
@@ -961,10 +1154,10 @@ static bool finish_plan(Plan &pl, int N, int gC, int gH, int gW, int columns, in
     p.g_C = gC; p.g_H = gH; p.g_W = gW;
     p.groups = ceil_div(gC, GROUP);
     p.w_kk = kk; p.o_HW = oHW; p.N_total = columns;
-    pl.bn = columns <= 128 ? 128 : 256;
+    pl.bn = columns <= 64 ? 64 : columns <= 128 ? 128 : 256;
     p.n_tiles = ceil_div(columns, pl.bn);
     p.width = (ceil_div(columns, p.n_tiles) + 15) & ~15;
-    pl.Cp = round8(gC);
+    pl.Cp = padded(gC);
     pl.rows = columns; pl.taps = kk;
     const size_t image_bytes = (size_t)gH * gW * pl.Cp * 4;
     pl.images = images_per_round(N, image_bytes);
@@ -989,29 +1182,61 @@ static int element_copy_columns(int columns, long long rows)
     while (bn > 32 && ceil_div_ll(rows, BM) * ceil_div(columns, bn) * 2 <= sm_count()) bn /= 2;
     return bn;
 }
-// Whether the forward pass is over sooner here than on the gathering kernel: the split reads and writes the whole input, so short sums
-// that read it once or twice (few channels, strides) are better off there.  Estimates in us fitted to 195 layers of 3x3 to 5x5 drawn from
-// 16 to 1024 channels and maps of 7 to 112 (within 0.8 to 1.2 of the times of nine in ten): 17.1 ms for all of them, 17.1 ms by the rule,
-// 16.8 ms with the better one each time, 36.1 ms on the gathering kernel; the rule's losses are 6 of 195, the worst 1.17 times.
-static bool forward_is_faster(const Plan &pl, const Geometry &g)
+// Whether a pass is over sooner here than on the gathering kernels (convmm.cu): the split reads and writes the whole tensor, so short sums
+// that read it once or twice (few channels, strides, small images) are better off there.  Both times are estimated, in us: here from
+// the column tile's blocks that the busiest SM sums, the values that the split reads and writes, what is written, and whether tiles are
+// cut; there from the k-blocks of the busiest SM and what is written.  The coefficients were fitted to 859 layers drawn over 16 to
+// 1024 channels (few-channel layers: 3), kernels of 2x2 to 11x11 and maps of 7 to 224; nine in ten estimates lie within 0.72 to 1.24 of
+// the time.  Sums of the times in ms, there / here / by the rule / with the better one each time, and the rule's losses of more than 3 %:
+//   forward               53.0 / 21.9 / 21.9 / 21.7    5 of 314, the worst 1.17
+//   few channels          7.08 / 5.21 / 4.68 / 4.65    0 of 110   (kernels of up to 32 taps)
+//                         4.64 / 3.48 / 3.39 / 3.38    1 of 88, 1.03
+//   strided gradients     22.3 / 9.06 / 9.02 / 9.00    1 of 129, 1.06   (stride 1: 29.3 / 8.0, never slower here)
+//   parameter gradients   54.1 / 30.1 / 28.8 / 28.5    6 of 347, 1.40
+//   ... few channels      11.5 / 13.1 / 10.5 / 10.4    1 of 198, 1.32
+struct HereCost {
+    double fixed, block256, block128, block64, value, out, cut, weight;            // the last five per million
+};
+struct ThereCost {
+    double fixed, wave, block128, block64, block32, out, longest;
+};
+constexpr HereCost HERE_FORWARD{13.2, 0.97, 0.80, 0.51, 0.82, 1.25, 5.8, 12.7}, HERE_FEW{12.5, 0.30, 0.30, 0.15, 3.33, 1.67, 0.0, 137.0},
+    HERE_FEW_LARGE{13.3, 0.60, 0.60, 0.30, 2.28, 0.46, 4.5, 13.5}, HERE_STRIDED{15.2, 1.37, 0.79, 0.52, 0.51, 1.65, 5.5, 8.0};
+constexpr ThereCost THERE_FORWARD{9.2, 1.72, 1.35, 1.18, 1.0, 0.51, 0.0}, THERE_FEW{6.1, 0.0, 5.69, 4.20, 3.84, 0.45, 0.78},
+    THERE_FEW_LARGE{6.7, 2.87, 1.80, 1.37, 1.21, 0.79, 0.0}, THERE_STRIDED{4.2, 3.97, 1.97, 1.42, 1.20, 0.45, 0.44};
+constexpr double MARGIN = 1.05;
+
+static bool is_faster(const Plan &pl, int N, const HereCost &h, const ThereCost &t, double values, double out, double weights)
 {
-    if (g.kH * g.kW > 32) return true;                      // those sum fp32 blocks there: 2.2 us a k-block
     const Params &p = pl.p;
-    const int grid = sm_count(), tiles = p.full + (p.items - p.full) / p.splits, rest = tiles - p.full, blocks = p.ph[0].blocks;
-    const double in = (double)g.N * g.C * g.H * g.W / 1e6, out = (double)g.N * g.K * g.oH * g.oW / 1e6, weights = (double)g.K * g.C * g.kH * g.kW / 1e6;
-    const double waves = p.full / grid + (rest ? 1 : 0), longest = blocks * (p.full / grid + (rest ? 1.0 / p.splits : 0.0));
-    const double here = 12.2 + 2.4 * waves + (pl.bn == 256 ? 1.18 : 0.75) * longest + 2.0 * in + 1.34 * out + (p.splits > 1 ? 5.1 : 0.0) + 11.8 * weights;
-    const long long rows = (long long)g.N * g.oH * g.oW;
-    const int bn = element_copy_columns(g.K, rows);
-    const double there_waves = (double)ceil_div_ll(ceil_div_ll(rows, BM) * ceil_div(g.K, bn), grid);
-    const double there = 9.2 + there_waves * (0.84 + (bn == 128 ? 1.36 : bn == 64 ? 1.1 : 1.01) * ceil_div(g.C * g.kH * g.kW, BK)) + 1.12 * out;
-    return here < there;
+    const int grid = sm_count();
+    double blocks = 0, there_blocks = 0, rows = 0, longest = 0;
+    int tiles = 0;
+    for (int i = 0; i < p.n_phases; ++i) rows += (double)N * p.ph[i].HW;
+    const int bn = element_copy_columns(p.N_total, (long long)rows), there_cols = ceil_div(p.N_total, bn);
+    double there_tiles = 0;
+    for (int i = 0; i < p.n_phases; ++i) {
+        const Phase &f = p.ph[i];
+        const double m = std::ceil((double)N * f.HW / BM), k = ceil_div(f.taps * p.g_C, BK);
+        tiles += (int)m * p.n_tiles;
+        blocks += m * p.n_tiles * f.taps * p.groups;
+        there_tiles += m * there_cols;
+        there_blocks += m * there_cols * k;
+        longest = std::max(longest, k);
+    }
+    const double busiest = blocks / tiles * (tiles / grid + (tiles % grid ? 1.0 / p.splits : 0.0)), waves = std::ceil(there_tiles / grid);
+    const double here = h.fixed + (pl.bn == 256 ? h.block256 : pl.bn == 128 ? h.block128 : h.block64) * busiest + (h.value * values + h.out * out + h.weight * weights) / 1e6 +
+                        (p.splits > 1 ? h.cut : 0.0);
+    const double there = t.fixed + waves * (t.wave + (bn == 128 ? t.block128 : bn == 64 ? t.block64 : t.block32) * there_blocks / there_tiles) + t.out * out / 1e6 +
+                         (waves == 1.0 ? t.longest * longest : 0.0);
+    return here * MARGIN < there;
 }
 
-static bool plan_forward(Plan &pl, const Geometry &g)
+static bool plan_forward(Plan &pl, const Geometry &whole)
 {
     pl = Plan{};
-    if (g.C < 16 || g.K < 16 || g.kH * g.kW == 1 || (long long)g.C * g.kH * g.kW < 128) return false;
+    Geometry g;
+    if (whole.K < 16 || whole.kH * whole.kW == 1 || !windowed(whole, g, pl.win)) return false;
     Phase &f = pl.p.ph[0];
     f.HW = g.oH * g.oW; f.pix_W = g.oW; f.taps = g.kH * g.kW; f.kW = g.kW;
     f.lH = -g.padH; f.lW = -g.padW; f.stH = g.dH; f.stW = g.dW; f.dlH = g.dilH; f.dlW = g.dilW;
@@ -1019,11 +1244,15 @@ static bool plan_forward(Plan &pl, const Geometry &g)
     pl.p.n_phases = 1;
     pl.wh[0] = Walk{g.H, f.lH, g.oH, g.dH, g.kH, g.dilH};
     pl.ww[0] = Walk{g.W, f.lW, g.oW, g.dW, g.kW, g.dilW};
-    return finish_plan(pl, g.N, g.C, g.H, g.W, g.K, g.kH * g.kW, f.HW) && forward_is_faster(pl, g);
+    if (!finish_plan(pl, g.N, g.C, g.H, g.W, g.K, g.kH * g.kW, f.HW)) return false;
+    const double in = (double)whole.N * whole.C * whole.H * whole.W, split = (double)g.N * g.H * g.W * pl.Cp, out = (double)g.N * g.K * f.HW;
+    const double weights = (double)whole.K * whole.C * whole.kH * whole.kW;
+    const bool large = whole.kH * whole.kW > 32;               // of 16 channels and more: always faster here
+    if (!pl.win.C) return large || is_faster(pl, g.N, HERE_FORWARD, THERE_FORWARD, in + split, out, weights);
+    return is_faster(pl, g.N, large ? HERE_FEW_LARGE : HERE_FEW, large ? THERE_FEW_LARGE : THERE_FEW, in + split, out, weights);
 }
 
-// No rule on times: of 123 drawn layers one took longer than on the other kernels, by 4 %.  Residues of fewer than 48 products belong to
-// phase_fma_kernel, which loses no bits of them.
+// Residues of fewer than 48 products belong to phase_fma_kernel, which loses no bits of them.
 static bool plan_grad_input(Plan &pl, const Geometry &g)
 {
     pl = Plan{};
@@ -1050,7 +1279,10 @@ static bool plan_grad_input(Plan &pl, const Geometry &g)
         pl.wh[i] = Walk{g.oH, f.lH, a.n, 1, a.taps, a.ostep};
         pl.ww[i] = Walk{g.oW, f.lW, b.n, 1, b.taps, b.ostep};
     }
-    return finish_plan(pl, g.N, g.K, g.oH, g.oW, g.C, g.kH * g.kW, g.H * g.W);
+    if (!finish_plan(pl, g.N, g.K, g.oH, g.oW, g.C, g.kH * g.kW, g.H * g.W)) return false;
+    if (p.n_phases == 1 || g.kH * g.kW > 32) return true;
+    return is_faster(pl, g.N, HERE_STRIDED, THERE_STRIDED, (double)g.N * g.oH * g.oW * (g.K + pl.Cp), (double)g.N * g.C * g.H * g.W,
+                     (double)g.K * g.C * g.kH * g.kW);
 }
 
 // src: the gathered tensor; weights of (row, channel, tap) at row * w_row + channel * w_c + tap.
@@ -1068,7 +1300,7 @@ static int run_plan(Plan &pl, int N, const float *src, const float *weight, long
     for (int at = 0; at < N; at += pl.images) {
         const int n = std::min(pl.images, N - at);
         plan_tiles(p, n);
-        const float *from = src + (size_t)at * p.g_C * g_HW;
+        const float *from = src + (size_t)at * (pl.win.C ? (size_t)pl.win.C * p.g_H * pl.win.W : (size_t)p.g_C * g_HW);
         p.out = out + (size_t)at * p.N_total * p.o_HW;
         p.raw_a = redo_nan ? from : nullptr;
         p.raw_w = weight;
@@ -1077,13 +1309,15 @@ static int run_plan(Plan &pl, int N, const float *src, const float *weight, long
         PrepParams q{};
         Act &act = q.act[0];
         act.src = from; act.dst = a; act.exps = const_cast<int8_t *>(p.exps); act.C = p.g_C; act.Cp = pl.Cp; act.HW = g_HW;
-        act.groups = p.groups; act.pixels = (uint32_t)n * g_HW; act.blocks = (int)ceil_div_ll((long long)act.pixels, 64) * p.groups;
+        act.groups = p.groups; act.pixels = (uint32_t)n * g_HW; 
         act.vec = can_vec(from, g_HW);
-        q.n_act = 1;
+        act.win = pl.win;
         q.w = weight; q.w_dst = w; q.w_exp = const_cast<int *>(p.w_exp); q.rows = at ? 0 : pl.rows; q.w_C = p.g_C; q.w_Cp = pl.Cp; q.taps = pl.taps;
-        q.w_row = w_row; q.w_c = w_c; q.tickets = p.tickets; q.n_tickets = sm_count();
-        if (launch("convolution operand split", (const void *)prep_kernel<false>, q.rows + act.blocks, 256, 0, stream, false, q)) return 1;
-        const void *kern = pl.bn == 128 ? (const void *)split_gemm_kernel<128, false> : (const void *)split_gemm_kernel<256, false>;
+        q.w_row = w_row; q.w_c = w_c; q.win_C = pl.win.C; q.win_kW = pl.win.kW; q.tickets = p.tickets; q.n_tickets = sm_count();
+        if (launch("convolution operand split", pl.win.C ? (const void *)prep_kernel<false, true> : (const void *)prep_kernel<false, false>, prep_grid(q, 1), 256, 0, stream, false, q)) return 1;
+        const void *kern = pl.bn == 64    ? (const void *)split_gemm_kernel<64, false>
+                           : pl.bn == 128 ? (const void *)split_gemm_kernel<128, false>
+                                          : (const void *)split_gemm_kernel<256, false>;
         if (launch("convolution of split operands", kern, std::min(p.items, sm_count()), THREADS, SMEM, stream, true, p, maps)) return 1;
     }
     return 0;
@@ -1117,8 +1351,10 @@ int grad_input(const Geometry &g, const float *gy, const float *weight, const fl
 // ---- weight gradients ---------------------------------------------------------------------------------------------------------------
 struct WgradPlan {
     Params p;
+    Window win;
+    Geometry v;                                // the convolution, on row windows where the channels are few
     Walk wh, ww;
-    int images, Cp, Kp, bn;
+    int images, Cp, Kp, bn, bg;
     size_t off_gy, off_max, off_bias, off_partial, bytes;
 };
 static void plan_splits(WgradPlan &pl, int images)
@@ -1137,49 +1373,53 @@ static void plan_splits(WgradPlan &pl, int images)
     }
     p.items = p.tiles * p.splits;
 }
-// As forward_is_faster: the two passes over both tensors cost more than the gathering kernel where sums are many but products few.
-// Fitted to 221 layers: 37.6 ms on the gathering kernel, 26.3 ms here, 23.7 ms by the rule, 23.5 ms with the better one each time; 3 of
-// 221 lose, the worst 1.34 times.
+// As is_faster.
 static bool grad_weight_is_faster(const WgradPlan &pl, const Geometry &g)
 {
-    if (g.kH * g.kW > 32) return true;
+    if (!pl.win.C && g.kH * g.kW > 32) return true;
     const Params &p = pl.p;
+    const bool few = pl.win.C != 0;
     const int grid = sm_count();
-    const double weights = (double)g.K * g.C * g.kH * g.kW / 1e6, in = (double)g.N * g.H * g.W * p.groups * GROUP / 1e6;
-    const double out = (double)g.N * p.pix_HW * ceil_div(g.K, GROUP) * GROUP / 1e6;
-    const double here = 14.2 + 2.05 * ceil_div(p.items, grid) * p.per_split + 2.85 * (double)p.items * pl.bn * BM / 1e6 + 3.05 * (in + out) + 3.2 * weights;
+    const double weights = (double)g.K * g.C * g.kH * g.kW / 1e6, values = ((double)g.N * g.C * g.H * g.W + (double)g.N * g.K * p.pix_HW) / 1e6;
+    const double split = ((double)g.N * pl.v.H * pl.v.W * pl.Cp + (double)g.N * p.pix_HW * pl.Kp) / 1e6, partial = (double)p.items * pl.bn * BM / 1e6;
+    const double busiest = (double)ceil_div(p.items, grid) * p.per_split;
+    const double here = few ? 19.0 + 0.68 * busiest + 3.97 * partial + 2.04 * values + 2.41 * split
+                            : 17.8 + (pl.bn == 256 ? 1.38 : 1.07) * busiest + 2.60 * partial + 2.71 * split + 4.0 * weights;
     const double tiles = (double)ceil_div(g.K, BM) * ceil_div(g.C * g.kH * g.kW, BM), blocks = (double)ceil_div_ll((long long)g.N * p.pix_HW, BK);
-    const double there = 14.7 + 1.82 * tiles * blocks / grid + 6.85 * weights + (tiles * blocks > grid ? 1.16 : 0.0) +
-                         0.143 * std::min(blocks, std::ceil(tiles * blocks / grid));
-    return here < there;
+    const double there = few ? 16.1 + 1.26 * tiles * blocks / grid + 196.0 * weights + 0.47 * std::min(blocks, std::ceil(tiles * blocks / grid))
+                             : 16.3 + 1.97 * tiles * blocks / grid + 6.14 * weights;
+    return here * MARGIN < there;
 }
-static bool plan_grad_weight(WgradPlan &pl, const Geometry &g)
+static bool plan_grad_weight(WgradPlan &pl, const Geometry &whole)
 {
     pl = WgradPlan{};
     Params &p = pl.p;
-    if (g.C < 16 || g.K < 16 || g.kH * g.kW == 1) return false;
+    if (whole.K < 16 || whole.kH * whole.kW == 1 || !windowed(whole, pl.v, pl.win)) return false;
+    const Geometry &g = pl.v;
     const int kk = g.kH * g.kW;
-    p.groups = ceil_div(g.C, GROUP);
+    pl.bg = g.C <= 32 && kk > 2 ? 32 : GROUP;
+    p.groups = ceil_div(g.C, pl.bg);
     p.col_groups = kk * p.groups;
-    pl.bn = p.col_groups <= 2 ? 128 : 256;
-    p.n_tiles = ceil_div(p.col_groups, pl.bn / GROUP);
+    pl.bn = p.col_groups * pl.bg <= 128 ? 128 : 256;
+    p.n_tiles = ceil_div(p.col_groups, pl.bn / pl.bg);
     p.m_tiles = ceil_div(g.K, BM);
+    p.N_total = g.K;
     p.tiles = p.n_tiles * p.m_tiles;
     p.kW = g.kW; p.pix_HW = g.oH * g.oW; p.pix_W = g.oW;
     p.lH = -g.padH; p.lW = -g.padW; p.stH = g.dH; p.stW = g.dW; p.dlH = g.dilH; p.dlW = g.dilW;
     pl.wh = Walk{g.H, p.lH, g.oH, g.dH, g.kH, g.dilH};
     pl.ww = Walk{g.W, p.lW, g.oW, g.dW, g.kW, g.dilW};
     if (!pl.wh.fits() || !pl.ww.fits()) return false;
-    pl.Cp = round8(g.C); pl.Kp = round8(g.K);
+    pl.Cp = padded(g.C); pl.Kp = padded(g.K);
     const size_t x_bytes = (size_t)g.H * g.W * pl.Cp * 4, gy_bytes = (size_t)p.pix_HW * pl.Kp * 4;
     pl.images = images_per_round(g.N, std::max(x_bytes, gy_bytes));
     if (pl.images * x_bytes < MIN_MAP_BYTES) return false;
     plan_splits(pl, pl.images);
-    if (!grad_weight_is_faster(pl, g)) return false;
+    if (!grad_weight_is_faster(pl, whole)) return false;
     size_t at = round256(pl.images * x_bytes);
     pl.off_gy = at; at += round256(pl.images * gy_bytes);
-    pl.off_max = at; at += round256((size_t)(g.C + g.K) * 4);
-    pl.off_bias = at; at += round256((size_t)ceil_div_ll((long long)pl.images * p.pix_HW, 64) * g.K * 8);
+    pl.off_max = at; at += round256((size_t)(whole.C + g.K) * 4);
+    pl.off_bias = at; at += round256((size_t)ceil_div_ll((long long)pl.images * ceil_div(p.pix_HW, PIECE), 8) * g.K * 8);
     // a round of fewer images may be cut into a few more parts than a whole one
     pl.off_partial = at; at += round256((size_t)(p.splits + 1) * p.n_tiles * pl.bn * p.m_tiles * BM * 4);
     pl.bytes = at + 256;
@@ -1211,33 +1451,42 @@ int grad_weight(const Geometry &g, const float *x, const float *gy, float *grad_
         const float *xr = x + (size_t)at * g.C * x_HW, *gr = gy + (size_t)at * g.K * p.pix_HW;
         alignas(64) Maps maps;
         if (map_3d(&maps.a[0], gs, pl.Kp, (long long)n * p.pix_HW, 2, GROUP, BK, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
-        if (map_im2col(&maps.b, xs, pl.Cp, 2 * n, pl.wh, pl.ww, GROUP, BK, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
+        if (map_im2col(&maps.b, xs, pl.Cp, 2 * n, pl.wh, pl.ww, pl.bg, BK, pl.bg == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
         CUNN_CUDA(cudaMemsetAsync(gy_max, 0, (size_t)(g.C + g.K) * 4, stream));
         MaxParams m{};
         m.src[0] = gr; m.src[1] = xr; m.chmax[0] = gy_max; m.chmax[1] = x_max; m.C[0] = g.K; m.C[1] = g.C; m.HW[0] = p.pix_HW; m.HW[1] = x_HW;
         m.images = n;
+        m.sums = grad_bias ? bias_part : nullptr;
         for (int t = 0; t < 2; ++t) {
-            m.chunks[t] = std::max(1, std::min(ceil_div(n, 8), ceil_div(sm_count() * 8, m.C[t])));
+            // 32 pieces a block, so that a warp has four loads in flight, or 8 where that leaves SMs idle
+            m.pieces[t] = ceil_div(m.HW[t], PIECE);
+            const long long pieces = (long long)n * m.pieces[t];
+            m.chunks[t] = (int)std::max(ceil_div_ll(pieces, 32), std::min(ceil_div_ll(pieces, 8), (long long)ceil_div(2 * sm_count(), m.C[t])));
             m.vec[t] = can_vec(m.src[t], m.HW[t]);
         }
         if (launch("convolution channel maxima", (const void *)channel_max_kernel, m.C[0] * m.chunks[0] + m.C[1] * m.chunks[1], 256, 0, stream, false, m)) return 1;
         PrepParams q{};
         for (int t = 0; t < 2; ++t) {
             Act &act = q.act[t];
-            act.src = t ? xr : gr; act.dst = t ? xs : gs; act.chmax = t ? x_max : gy_max; act.bias_part = !t && grad_bias ? bias_part : nullptr;
-            act.C = t ? g.C : g.K; act.Cp = t ? pl.Cp : pl.Kp; act.HW = t ? x_HW : p.pix_HW; act.groups = ceil_div(act.C, GROUP);
+            act.src = t ? xr : gr; act.dst = t ? xs : gs; act.chmax = t ? x_max : gy_max;
+            act.C = t ? pl.v.C : g.K; act.Cp = t ? pl.Cp : pl.Kp; act.HW = t ? pl.v.H * pl.v.W : p.pix_HW; act.groups = ceil_div(act.C, GROUP);
+            if (t) act.win = pl.win;
             act.vec = can_vec(act.src, act.HW);
-            act.pixels = (uint32_t)n * act.HW; act.blocks = (int)ceil_div_ll((long long)act.pixels, 64) * act.groups;
-        }
-        q.n_act = 2;
-        if (launch("convolution operand split", (const void *)prep_kernel<true>, q.act[0].blocks + q.act[1].blocks, 256, 0, stream, true, q)) return 1;
-        const void *kern = pl.bn == 128 ? (const void *)split_gemm_kernel<128, true> : (const void *)split_gemm_kernel<256, true>;
+            act.pixels = (uint32_t)n * act.HW;
+            }
+        if (launch("convolution operand split", pl.win.C ? (const void *)prep_kernel<true, true> : (const void *)prep_kernel<true, false>, prep_grid(q, 2), 256, 0, stream, true, q)) return 1;
+        const void *kern = pl.bg == 32    ? pl.bn == 128 ? (const void *)split_gemm_kernel<128, true, 32> : (const void *)split_gemm_kernel<256, true, 32>
+                           : pl.bn == 128 ? (const void *)split_gemm_kernel<128, true>
+                                          : (const void *)split_gemm_kernel<256, true>;
         if (launch("convolution parameter gradient of split operands", kern, std::min(p.items, sm_count()), THREADS, SMEM, stream, true, p, maps)) return 1;
         ReduceParams r{};
         r.partial = p.partial; r.gw = grad_weight; r.gb = grad_bias; r.gy_max = gy_max; r.x_max = x_max; r.bias_part = bias_part;
-        r.K = g.K; r.C = g.C; r.kk = kk; r.groups = p.groups; r.splits = p.splits; r.cols = p.n_tiles * pl.bn; r.rows = p.m_tiles * BM;
-        r.gw_blocks = ceil_div(g.K, 32) * ceil_div(g.C * kk, 32);
-        r.bias_blocks = (int)ceil_div_ll((long long)n * p.pix_HW, 64);
+        r.K = g.K; r.C = g.C; r.kk = kk; r.groups = p.groups; r.bg = pl.bg; r.win_kW = pl.win.kW; r.splits = p.splits; r.cols = p.n_tiles * pl.bn; r.rows = p.m_tiles * BM;
+        // one warp per output leaves SMs idle where the outputs are few: 9,408 outputs of 146 splits took 36 us
+        r.shares = 1;
+        while (r.shares < 8 && r.shares * 8 <= p.splits && ceil_div(g.K, 32) * ceil_div(g.C * kk * r.shares, 32) < 4 * sm_count()) r.shares *= 2;
+        r.gw_blocks = ceil_div(g.K, 32) * ceil_div(g.C * kk, 32 / r.shares);
+        r.bias_blocks = m.chunks[0];
         r.scale = scale;
         if (launch("convolution parameter gradient sums", (const void *)reduce_kernel, r.gw_blocks + (grad_bias ? ceil_div(g.K, 8) : 0), 256, 0, stream,
                    true, r)) return 1;

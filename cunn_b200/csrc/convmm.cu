@@ -2070,6 +2070,7 @@ extern "C" CUNN_API size_t cunn_b200_conv_scratch(int pass, int N, int C, int H,
         clear_error();
         return 0;
     }
+    if (dilH == 1 && dilW == 1 && pass != PASS_GRAD_INPUT && stem::applies(C, K, kH, kW)) return 0;
     try {
         return split_scratch(pass, split::Geometry{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW});
     } catch (const std::bad_alloc &) {

@@ -48,6 +48,12 @@ SHAPES = [
     (9, 80, 33, 35, 64, 3, 5, 1, 1, 1, "fgw"),        # a kernel that is not square
     (3, 176, 12, 50, 96, 1, 7, 1, 3, 1, "fg"),        # one row of taps, padding beyond it
     (40, 256, 14, 14, 100, 7, 7, 1, 3, 1, "fgw"),     # 49 taps
+    (32, 3, 150, 141, 48, 7, 7, 2, 3, 1, "fw"),       # few channels: row windows of 21 values, an odd map
+    (64, 12, 60, 60, 64, 5, 5, 1, 2, 1, "fw"),        # ... of 60
+    (20, 3, 150, 161, 40, 11, 11, 4, 5, 1, "f"),      # ... of 33, parts of a row tile
+    (30, 3, 150, 161, 40, 11, 11, 2, 5, 1, "w"),      # ... in groups of 64 columns
+    (9, 5, 90, 97, 130, 3, 3, 1, 1, 1, "f"),          # ... and two columns past a tile
+    (12, 3, 40, 700, 64, 5, 5, 1, 2, 1, "f"),         # ... rows that share a block in twos
 ]
 
 
@@ -87,7 +93,7 @@ def test_all_passes(F, shape):
 @pytest.mark.parametrize("stride", [1, 2])
 def test_exponents_of_any_range(F, stride):
     """Images of sizes 1e-26 to 1e26 against filters of 1e-8 to 1e8: every plane is as exact as if it were alone."""
-    N, C, K, H = 8, 96, 72, 28
+    N, C, K, H = 40, 96, 72, 28
     o = out_size(H, 3, stride, 1, 1)
     g = torch.Generator(device="cuda").manual_seed(21)
     x, gy = torch.randn(N, C, H, H, device="cuda", generator=g), torch.randn(N, K, o, o, device="cuda", generator=g)
@@ -128,7 +134,8 @@ def test_parameter_gradient_of_any_range(F):
 @pytest.mark.parametrize("where", ["x", "w"])
 def test_what_is_not_finite(F, where, value):
     """A sum that reads it is not finite, every other one is what it was; a strided input gradient has the sign of its infinities."""
-    N, C, K, H = 16, 64, 64, 28
+    N, C, K, H = 96, 64, 64, 28
+    assert scratch(0, N, C, H, H, K, 3, 3, 1, 1, 1) and scratch(1, N, C, H, H, K, 3, 3, 2, 1, 1)
     g = torch.Generator(device="cuda").manual_seed(23)
     x, gy = torch.randn(N, C, H, H, device="cuda", generator=g), torch.randn(N, K, 14, 14, device="cuda", generator=g)
     w = torch.rand(K, C, 3, 3, device="cuda", generator=g) + 0.5
