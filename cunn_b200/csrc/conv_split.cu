@@ -1114,7 +1114,7 @@ static bool windowed(const Geometry &g, Geometry &v, Window &win)
     win = Window{};
     if (g.C >= 16) return true;
     win = Window{g.C, g.kW, g.dW, g.padW, g.W, g.oW};
-    if (g.C * g.kW > GROUP || g.dilW != 1 || win.row_values() > TILE_VALUES) return false;
+    if (g.kH * g.kW == 1 || g.C * g.kW > GROUP || g.dilW != 1 || win.row_values() > TILE_VALUES) return false;
     v.C = g.C * g.kW; v.W = g.oW; v.kW = v.dW = v.dilW = 1; v.padW = 0;
     return true;
 }
@@ -1194,25 +1194,34 @@ static int element_copy_columns(int columns, long long rows)
 //   strided gradients     22.3 / 9.06 / 9.02 / 9.00    1 of 129, 1.06   (stride 1: 29.3 / 8.0, never slower here)
 //   parameter gradients   54.1 / 30.1 / 28.8 / 28.5    6 of 347, 1.40
 //   ... few channels      11.5 / 13.1 / 10.5 / 10.4    1 of 198, 1.32
+// and of 330 1x1 layers, on whose planes tensor maps work / do not:
+//   forward               4.15 / 5.31 / 4.04 / 4.03    0 of 106        8.23 / 7.26 / 6.83 / 6.76    2 of 190, 1.27
+//   input gradients       3.51 / 4.91 / 3.39 / 3.37    0 of 86         4.79 / 4.07 / 3.90 / 3.88    4 of 101, 1.09
+//   parameter gradients   4.73 / 8.70 / 4.73 / 4.72    0 of 120        7.77 / 11.2 / 7.61 / 7.47    0 of 163
 struct HereCost {
-    double fixed, block256, block128, block64, value, out, cut, weight;            // the last five per million
+    double fixed, block256, block128, block64, value, out, cut, weight;            // the last five but cut per million
 };
 struct ThereCost {
-    double fixed, wave, block128, block64, block32, out, longest;
+    double fixed, wave, block128, block64, block32, out, longest, in = 0.0;
 };
 constexpr HereCost HERE_FORWARD{13.2, 0.97, 0.80, 0.51, 0.82, 1.25, 5.8, 12.7}, HERE_FEW{12.5, 0.30, 0.30, 0.15, 3.33, 1.67, 0.0, 137.0},
     HERE_FEW_LARGE{13.3, 0.60, 0.60, 0.30, 2.28, 0.46, 4.5, 13.5}, HERE_STRIDED{15.2, 1.37, 0.79, 0.52, 0.51, 1.65, 5.5, 8.0};
 constexpr ThereCost THERE_FORWARD{9.2, 1.72, 1.35, 1.18, 1.0, 0.51, 0.0}, THERE_FEW{6.1, 0.0, 5.69, 4.20, 3.84, 0.45, 0.78},
     THERE_FEW_LARGE{6.7, 2.87, 1.80, 1.37, 1.21, 0.79, 0.0}, THERE_STRIDED{4.2, 3.97, 1.97, 1.42, 1.20, 0.45, 0.44};
+// 1x1 layers of stride 1 on planes and channels that tensor maps take (multiples of four), and the others.
+constexpr HereCost HERE_POINT{14.7, 1.10, 0.57, 0.06, 0.71, 1.35, 5.6, 5.0}, HERE_POINT_GRAD{13.2, 1.30, 0.77, 0.30, 0.72, 1.09, 5.0, 6.5};
+constexpr ThereCost THERE_POINT{9.1, 0.26, 0.66, 0.53, 0.45, 0.76, 0.0, 0.06}, THERE_POINT_ODD{8.3, 0.71, 1.10, 0.85, 0.79, 2.19, 0.15, 0.09},
+    THERE_POINT_GRAD{7.6, 0.42, 0.74, 0.61, 0.52, 0.20, 0.0, 0.04}, THERE_POINT_GRAD_ODD{7.8, 0.10, 1.26, 1.15, 1.10, 1.18, 0.0};
 constexpr double MARGIN = 1.05;
 
-static bool is_faster(const Plan &pl, int N, const HereCost &h, const ThereCost &t, double values, double out, double weights)
+// `aligned`: the other kernel works on whole groups of 32 pixels of an image.
+static bool is_faster(const Plan &pl, int N, const HereCost &h, const ThereCost &t, double values, double out, double weights, bool aligned = false)
 {
     const Params &p = pl.p;
     const int grid = sm_count();
     double blocks = 0, there_blocks = 0, rows = 0, longest = 0;
     int tiles = 0;
-    for (int i = 0; i < p.n_phases; ++i) rows += (double)N * p.ph[i].HW;
+    for (int i = 0; i < p.n_phases; ++i) rows += (double)N * (aligned ? ceil_div(p.ph[i].HW, 32) * 32 : p.ph[i].HW);
     const int bn = element_copy_columns(p.N_total, (long long)rows), there_cols = ceil_div(p.N_total, bn);
     double there_tiles = 0;
     for (int i = 0; i < p.n_phases; ++i) {
@@ -1220,15 +1229,16 @@ static bool is_faster(const Plan &pl, int N, const HereCost &h, const ThereCost 
         const double m = std::ceil((double)N * f.HW / BM), k = ceil_div(f.taps * p.g_C, BK);
         tiles += (int)m * p.n_tiles;
         blocks += m * p.n_tiles * f.taps * p.groups;
-        there_tiles += m * there_cols;
-        there_blocks += m * there_cols * k;
+        const double there_m = aligned ? std::ceil(rows / BM) : m;
+        there_tiles += there_m * there_cols;
+        there_blocks += there_m * there_cols * k;
         longest = std::max(longest, k);
     }
     const double busiest = blocks / tiles * (tiles / grid + (tiles % grid ? 1.0 / p.splits : 0.0)), waves = std::ceil(there_tiles / grid);
     const double here = h.fixed + (pl.bn == 256 ? h.block256 : pl.bn == 128 ? h.block128 : h.block64) * busiest + (h.value * values + h.out * out + h.weight * weights) / 1e6 +
                         (p.splits > 1 ? h.cut : 0.0);
     const double there = t.fixed + waves * (t.wave + (bn == 128 ? t.block128 : bn == 64 ? t.block64 : t.block32) * there_blocks / there_tiles) + t.out * out / 1e6 +
-                         (waves == 1.0 ? t.longest * longest : 0.0);
+                         t.in * rows * p.g_C / 1e6 + (waves == 1.0 ? t.longest * longest : 0.0);
     return here * MARGIN < there;
 }
 
@@ -1236,7 +1246,7 @@ static bool plan_forward(Plan &pl, const Geometry &whole)
 {
     pl = Plan{};
     Geometry g;
-    if (whole.K < 16 || whole.kH * whole.kW == 1 || !windowed(whole, g, pl.win)) return false;
+    if (whole.K < 16 || !windowed(whole, g, pl.win)) return false;
     Phase &f = pl.p.ph[0];
     f.HW = g.oH * g.oW; f.pix_W = g.oW; f.taps = g.kH * g.kW; f.kW = g.kW;
     f.lH = -g.padH; f.lW = -g.padW; f.stH = g.dH; f.stW = g.dW; f.dlH = g.dilH; f.dlW = g.dilW;
@@ -1247,6 +1257,10 @@ static bool plan_forward(Plan &pl, const Geometry &whole)
     if (!finish_plan(pl, g.N, g.C, g.H, g.W, g.K, g.kH * g.kW, f.HW)) return false;
     const double in = (double)whole.N * whole.C * whole.H * whole.W, split = (double)g.N * g.H * g.W * pl.Cp, out = (double)g.N * g.K * f.HW;
     const double weights = (double)whole.K * whole.C * whole.kH * whole.kW;
+    if (whole.kH * whole.kW == 1) {
+        const bool aligned = whole.dH == 1 && whole.dW == 1 && whole.padH == 0 && whole.padW == 0 && f.HW % 4 == 0 && whole.C % 4 == 0;
+        return is_faster(pl, g.N, HERE_POINT, aligned ? THERE_POINT : THERE_POINT_ODD, in + split, out, weights, aligned);
+    }
     const bool large = whole.kH * whole.kW > 32;               // of 16 channels and more: always faster here
     if (!pl.win.C) return large || is_faster(pl, g.N, HERE_FORWARD, THERE_FORWARD, in + split, out, weights);
     return is_faster(pl, g.N, large ? HERE_FEW_LARGE : HERE_FEW, large ? THERE_FEW_LARGE : THERE_FEW, in + split, out, weights);
@@ -1256,7 +1270,7 @@ static bool plan_forward(Plan &pl, const Geometry &whole)
 static bool plan_grad_input(Plan &pl, const Geometry &g)
 {
     pl = Plan{};
-    if (g.C < 16 || g.K < 64 || g.kH * g.kW == 1 || g.dH > 2 || g.dW > 2) return false;
+    if (g.C < 16 || g.K < 64 || g.dH > 2 || g.dW > 2) return false;
     bool gaps = false;
     const std::vector<AxisPhase> ah = axis_phases(g.H, g.kH, g.dH, g.padH, g.dilH, false, &gaps), aw = axis_phases(g.W, g.kW, g.dW, g.padW, g.dilW, false, &gaps);
     if (gaps || ah.empty() || aw.empty()) return false;
@@ -1280,6 +1294,11 @@ static bool plan_grad_input(Plan &pl, const Geometry &g)
         pl.ww[i] = Walk{g.oW, f.lW, b.n, 1, b.taps, b.ostep};
     }
     if (!finish_plan(pl, g.N, g.K, g.oH, g.oW, g.C, g.kH * g.kW, g.H * g.W)) return false;
+    if (g.kH * g.kW == 1 && g.dH == 1 && g.dW == 1) {
+        const bool aligned = g.padH == 0 && g.padW == 0 && g.H * g.W % 4 == 0 && g.C % 4 == 0;
+        return is_faster(pl, g.N, HERE_POINT_GRAD, aligned ? THERE_POINT_GRAD : THERE_POINT_GRAD_ODD, (double)g.N * g.oH * g.oW * (g.K + pl.Cp),
+                         (double)g.N * g.C * g.H * g.W, (double)g.K * g.C, aligned);
+    }
     if (p.n_phases == 1 || g.kH * g.kW > 32) return true;
     return is_faster(pl, g.N, HERE_STRIDED, THERE_STRIDED, (double)g.N * g.oH * g.oW * (g.K + pl.Cp), (double)g.N * g.C * g.H * g.W,
                      (double)g.K * g.C * g.kH * g.kW);
@@ -1383,6 +1402,13 @@ static bool grad_weight_is_faster(const WgradPlan &pl, const Geometry &g)
     const double weights = (double)g.K * g.C * g.kH * g.kW / 1e6, values = ((double)g.N * g.C * g.H * g.W + (double)g.N * g.K * p.pix_HW) / 1e6;
     const double split = ((double)g.N * pl.v.H * pl.v.W * pl.Cp + (double)g.N * p.pix_HW * pl.Kp) / 1e6, partial = (double)p.items * pl.bn * BM / 1e6;
     const double busiest = (double)ceil_div(p.items, grid) * p.per_split;
+    if (g.kH * g.kW == 1) {
+        // 1x1: against the tensor-map kernel never; planes that it does not take
+        if (g.dH == 1 && g.dW == 1 && g.padH == 0 && g.padW == 0 && p.pix_HW % 4 == 0) return false;
+        const double t = (double)ceil_div(g.K, BM) * ceil_div(g.C, g.C <= 32 ? 32 : g.C <= 64 ? 64 : 128), b = (double)ceil_div_ll((long long)g.N * p.pix_HW, BK);
+        const double here = 17.6 + (pl.bn == 256 ? 1.27 : 1.91) * busiest + 3.98 * partial + 3.04 * split;
+        return here * MARGIN < 16.9 + 1.19 * t * b / grid + 18.0 * weights + (t * b > grid ? 0.72 : 0.0) + 0.19 * std::min(b, std::ceil(t * b / grid));
+    }
     const double here = few ? 19.0 + 0.68 * busiest + 3.97 * partial + 2.04 * values + 2.41 * split
                             : 17.8 + (pl.bn == 256 ? 1.38 : 1.07) * busiest + 2.60 * partial + 2.71 * split + 4.0 * weights;
     const double tiles = (double)ceil_div(g.K, BM) * ceil_div(g.C * g.kH * g.kW, BM), blocks = (double)ceil_div_ll((long long)g.N * p.pix_HW, BK);
@@ -1394,7 +1420,7 @@ static bool plan_grad_weight(WgradPlan &pl, const Geometry &whole)
 {
     pl = WgradPlan{};
     Params &p = pl.p;
-    if (whole.K < 16 || whole.kH * whole.kW == 1 || !windowed(whole, pl.v, pl.win)) return false;
+    if (whole.K < 16 || !windowed(whole, pl.v, pl.win)) return false;
     const Geometry &g = pl.v;
     const int kk = g.kH * g.kW;
     pl.bg = g.C <= 32 && kk > 2 ? 32 : GROUP;

@@ -1720,7 +1720,7 @@ using namespace cunn::mm;
 enum Pass : int { PASS_FORWARD = 0, PASS_GRAD_INPUT = 1, PASS_GRAD_WEIGHT = 2 };
 static size_t split_scratch(int pass, const split::Geometry &g)
 {
-    if (!g_use_tma || g.N == 0) return 0;
+    if (!g_use_tma || g.N == 0 || (g.H == 1 && g.W == 1)) return 0;
     return pass == PASS_FORWARD ? split::forward_scratch(g) : pass == PASS_GRAD_INPUT ? split::grad_input_scratch(g) : split::grad_weight_scratch(g);
 }
 static bool split_applies(int pass, const split::Geometry &g, const void *scratch, size_t scratch_bytes)
@@ -1742,6 +1742,8 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     const bool dilated = dilH != 1 || dilW != 1;
     CUNN_CHECK_ARG(!dilated || gather_applies(kH, kW), "dilated kernels of more than 32 taps are not supported");
     if (!dilated && stem::applies(C, K, kH, kW)) return stem::forward(x, weight, bias, y, N, H, W, oH, oW, dH, dW, padH, padW, stream);
+    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
+    if (split_applies(PASS_FORWARD, geo, scratch, scratch_bytes)) return split::forward(geo, x, weight, bias, y, scratch, stream);
     if (pw_applies(kH, kW, dH, dW, padH, padW) && H * W == 1 && K % 4 == 0 && tma_applies(x, weight, y, C, 4)) {
         // a fully connected layer: y[n][k] = sum_c x[n][c] W[k][c], two K-major matrices, i.e. the weight gradient's GEMM over one
         // "image" of C pixels (with element copies of single-pixel planes, 128 x 1024 -> 1000 took 129 us)
@@ -1780,8 +1782,6 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
         return pw_launch(pw_pick<OP_FWD>(bn), q, stream);
     }
-    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
-    if (split_applies(PASS_FORWARD, geo, scratch, scratch_bytes)) return split::forward(geo, x, weight, bias, y, scratch, stream);
     if (gather_applies(kH, kW)) {
         pw::Params q{};
         q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
@@ -1840,6 +1840,12 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
     CUNN_CHECK_ARG(gy && weight && gx, "null tensor pointer");
     const bool dilated = dilH != 1 || dilW != 1;
     CUNN_CHECK_ARG(!dilated || gather_applies(kH, kW), "dilated kernels of more than 32 taps are not supported");
+    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
+    try {
+        if (split_applies(PASS_GRAD_INPUT, geo, scratch, scratch_bytes)) return split::grad_input(geo, gy, weight, bias, gx, scratch, stream);
+    } catch (const std::bad_alloc &) {
+        return fail("convmm grad input: out of host memory");
+    }
     if (pw_applies(kH, kW, dH, dW, padH, padW) && H * W == 1 && K % 4 == 0 && K < (1 << 24) && (long long)K * C < (1LL << 31) &&
         tma_applies(gy, weight, gx, C, K))
         // a fully connected layer: gx[n][c] = sum_k gy[n][k] W[k][c] is the 1x1 convolution of the one "image" W (K channels of C
@@ -1867,12 +1873,6 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         q.bulk_out = (q.HW % 4 == 0) && q.HW >= 8 * BM && aligned16(gx);
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets);
         return add_bias(pw_launch(pw_pick<OP_DGRAD>(bn), q, stream));
-    }
-    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
-    try {
-        if (split_applies(PASS_GRAD_INPUT, geo, scratch, scratch_bytes)) return split::grad_input(geo, gy, weight, bias, gx, scratch, stream);
-    } catch (const std::bad_alloc &) {
-        return fail("convmm grad input: out of host memory");
     }
     if (dH == 1 && dW == 1 && padH <= dilH * (kH - 1) && padW <= dilW * (kW - 1) && (gather_applies(kH, kW) || !small_kernel(kH, kW))) {
         // stride 1: a convolution of gy with the kernel rotated by 180 degrees and padding dil (k - 1) - pad
@@ -1963,6 +1963,8 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         if (stem::weight_grad_partials(x, gy, partial, grad_bias ? bias_part : nullptr, N, H, W, oH, oW, dH, dW, padH, padW, stream)) return 1;
         return reduce_partials(partial, grad_weight, n, ctas, scale, grad_bias ? bias_part : nullptr, grad_bias, K, stream);
     }
+    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
+    if (split_applies(PASS_GRAD_WEIGHT, geo, workspace, workspace_bytes)) return split::grad_weight(geo, x, gy, grad_weight, grad_bias, scale, workspace, stream);
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         const bool tma = tma_applies(gy, x, workspace, H * W, 4);
         pw_wgrad_plan(C, K, 1, N, H * W, tma, &bn, &splits, &kb);
@@ -1987,8 +1989,6 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         }
         return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
     }
-    const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
-    if (split_applies(PASS_GRAD_WEIGHT, geo, workspace, workspace_bytes)) return split::grad_weight(geo, x, gy, grad_weight, grad_bias, scale, workspace, stream);
     if (gathered_wgrad(kH, kW)) {
         const int oHW = oH * oW;
         pw_wgrad_plan(C, K, kk, N, oHW, false, &bn, &splits, &kb);

@@ -98,10 +98,11 @@ static void plan(const Model &m, int B, Arena &a)
         bnwork = std::max(bnwork, cunn_b200_batchnorm_workspace(B, L.cout));
         if (L.kind == KIND_DW)
             dwwork = std::max(dwwork, cunn_b200_dwconv_acc_grad_workspace(B, L.cin, L.hin, L.hin, 1, 3, 3, L.stride, L.stride, 1, 1));
-        else if (L.kind == KIND_PW)
-            work = std::max(work, cunn_b200_convmm_acc_grad_workspace(B, L.cin, L.hin, L.hin, L.cout, 1, 1, 1, 1, 0, 0));
-        else
-            work = std::max(work, cunn_b200_convmm_acc_grad_workspace(B, L.cin, L.hin, L.hin, L.cout, 3, 3, L.stride, L.stride, 1, 1));
+        else {
+            const int k = L.kind == KIND_PW ? 1 : 3, d = L.kind == KIND_PW ? 1 : L.stride, pad = L.kind == KIND_PW ? 0 : 1;
+            work = std::max(work, cunn_b200_convmm_acc_grad_workspace(B, L.cin, L.hin, L.hin, L.cout, k, k, d, d, pad, pad));
+            for (int pass = 0; pass < 3; ++pass) work = std::max(work, cunn_b200_conv_scratch(pass, B, L.cin, L.hin, L.hin, L.cout, k, k, d, d, pad, pad, 1, 1));
+        }
     }
     work = std::max(work, cunn_b200_convmm_acc_grad_workspace(B, m.feat, 1, 1, m.classes, 1, 1, 1, 1, 0, 0));
     a.pooled = off; off = align_up(off + (size_t)B * m.feat * 4);
@@ -215,9 +216,9 @@ extern "C" CUNN_API int cunn_b200_mobilenet_step(const cunn_b200_mobilenet_confi
         if (L.kind == KIND_DW)
             STEP(cunn_b200_dwconv_forward(x, w, b, co, B, L.cin, L.hin, L.hin, 1, 3, 3, L.stride, L.stride, 1, 1, stream));
         else if (L.kind == KIND_PW)
-            STEP(cunn_b200_convmm_forward(x, w, b, co, B, L.cin, L.hin, L.hin, L.cout, 1, 1, 1, 1, 0, 0, stream));
+            STEP(cunn_b200_conv_forward_scratch(x, w, b, co, B, L.cin, L.hin, L.hin, L.cout, 1, 1, 1, 1, 0, 0, 1, 1, work, wbytes, stream));
         else
-            STEP(cunn_b200_convmm_forward(x, w, b, co, B, L.cin, L.hin, L.hin, L.cout, 3, 3, L.stride, L.stride, 1, 1, stream));
+            STEP(cunn_b200_conv_forward_scratch(x, w, b, co, B, L.cin, L.hin, L.hin, L.cout, 3, 3, L.stride, L.stride, 1, 1, 1, 1, work, wbytes, stream));
         // BN + ReLU in one pass (the caller-side fusion of nn.SpatialBatchNormalization + nn.ReLU)
         STEP(cunn_b200_batchnorm_relu_forward(co, ac, params + L.g_off, params + L.beta_off, bn_running + L.bn_off,
                                               bn_running + L.bn_off + L.cout, sv, sv + L.cout, B, L.cout, L.hout * L.hout,
@@ -264,8 +265,8 @@ extern "C" CUNN_API int cunn_b200_mobilenet_step(const cunn_b200_mobilenet_confi
             STEP(cunn_b200_convmm_acc_grad(xin, g2, grads + L.w_off, grads + L.b_off, B, L.cin, L.hin, L.hin, L.cout, k, k,
                                            L.stride, L.stride, pad, pad, 1.f, work, wbytes, stream));
             if (i > 0)   // the first layer has no input gradient
-                STEP(cunn_b200_convmm_grad_input(g2, params + L.w_off, g, B, L.cin, L.hin, L.hin, L.cout, k, k, L.stride,
-                                                 L.stride, pad, pad, stream));
+                STEP(cunn_b200_conv_grad_input_scratch(g2, params + L.w_off, g, B, L.cin, L.hin, L.hin, L.cout, k, k, L.stride,
+                                                       L.stride, pad, pad, 1, 1, work, wbytes, stream));
         }
     }
     return 0;

@@ -159,6 +159,7 @@ def batchnorm_backward(x, gy, weight, running_mean, running_var, save_mean, save
 
 
 _LARGE = 16 << 20
+_POINT = 1 << 20        # values of a 1x1 layer's tensor from which on it may be better off with scratch
 
 
 def _conv_scratch(size_fn, which, geo, device, least=0):
@@ -186,7 +187,7 @@ def convmm_forward(x, weight, bias, dH, dW, padH, padW, out=None):
     oH, oW = conv_out(H, kH, dH, padH), conv_out(W, kW, dW, padW)
     if out is None:
         out = torch.empty((N, K, max(oH, 0), max(oW, 0)), dtype=torch.float32, device=x.device)
-    if kH * kW > 1:
+    if kH * kW > 1 or x.numel() >= _POINT:
         geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
         ws = _conv_scratch(lib.cunn_b200_conv_scratch, 0, geo, x.device)
         check(lib.cunn_b200_conv_forward_scratch(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), *geo,
@@ -203,7 +204,7 @@ def convmm_grad_input(gy, weight, H, W, dH, dW, padH, padW, out=None):
     N = gy.shape[0]
     if out is None:
         out = torch.empty((N, C, H, W), dtype=torch.float32, device=gy.device)
-    if kH * kW > 1:
+    if kH * kW > 1 or gy.numel() >= _POINT:
         geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
         ws = _conv_scratch(lib.cunn_b200_conv_scratch, 1, geo, gy.device)
         check(lib.cunn_b200_conv_grad_input_scratch(_ptr(gy), _ptr(weight), _ptr(out), *geo,
@@ -220,7 +221,7 @@ def convmm_acc_grad(x, gy, grad_weight, grad_bias, dH, dW, padH, padW, scale=1.0
     N, C, H, W = x.shape
     K, _, kH, kW = grad_weight.shape
     need = lib.cunn_b200_convmm_acc_grad_workspace(N, C, H, W, K, kH, kW, dH, dW, padH, padW)
-    if kH * kW > 1 and need:
+    if need and (kH * kW > 1 or x.numel() >= _POINT):
         ws, at, size = _conv_scratch(lib.cunn_b200_conv_scratch, 2, (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1), x.device, need)
     else:
         ws = workspace(need, x.device)

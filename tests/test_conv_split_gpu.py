@@ -48,6 +48,8 @@ SHAPES = [
     (9, 80, 33, 35, 64, 3, 5, 1, 1, 1, "fgw"),        # a kernel that is not square
     (3, 176, 12, 50, 96, 1, 7, 1, 3, 1, "fg"),        # one row of taps, padding beyond it
     (40, 256, 14, 14, 100, 7, 7, 1, 3, 1, "fgw"),     # 49 taps
+    (128, 1024, 7, 7, 512, 1, 1, 1, 0, 1, "fgw"),     # 1x1 on planes of an odd size
+    (40, 512, 15, 15, 500, 1, 1, 1, 0, 1, "fg"),      # ... two column tiles, the second one ragged
     (32, 3, 150, 141, 48, 7, 7, 2, 3, 1, "fw"),       # few channels: row windows of 21 values, an odd map
     (64, 12, 60, 60, 64, 5, 5, 1, 2, 1, "fw"),        # ... of 60
     (20, 3, 150, 161, 40, 11, 11, 4, 5, 1, "f"),      # ... of 33, parts of a row tile
