@@ -11,14 +11,17 @@
 //   input grad   in padded coordinates h + pad = S q + a: gx[S q + a][S r + b] = sum_{t,u} w[a + S t][b + S u] gy[q - t][r - u];
 //                a thread takes TH consecutive q of one r and writes their S * S residues, so no product with a zero is formed
 //   param grad   a cluster of up to eight CTAs per filter shares the images; every thread keeps the k * k sums of its strips in
-//                registers for at most kChain terms, then they go through fp64: across the warp (WarpSums), the CTA, the cluster and
-//                onto the gradient; the bias sum is fp64 throughout.  The order is fixed, so results do not depend on timing.  Over 40 layers of
+//                registers for at most kChain terms, then they go through fp64: the thread (3x3) or the warp (WarpSums), the CTA, the
+//                cluster and onto the gradient; the bias sum is fp64 throughout.  The order is fixed, so results do not depend on timing.  Over 40 layers of
 //                16 to 600 channels the error is that of the kernel for any shape, which has fp64 across threads and images: 3.5e-8 to
 //                6e-8 against 3.5e-8 to 1.2e-7 (2-norm; chains of 32 terms: 4.3e-8 to 1.1e-7).
 //
-// Forward / input gradient / parameter gradient on a cold cache, in us: 32 x 96 x 57 x 43, 5x5 stride 2: 671 in all before,
-// 35 / 30 / 54 now (38 MB a pass: 6 us); 12 x 144 x 37 x 29, 3x3 stride 1 (rows of an odd length): 13 / 16 / 33.  What is left is
-// the 4-byte copies and the wait of a CTA for its only tile, which other CTAs of the SM fill.
+// Forward / input gradient / parameter gradient on a cold cache, in us: 32 x 96 x 57 x 43, 5x5 stride 2: 21 / 16 / 34 (38 MB a pass: 6 us;
+// 35 / 30 / 52 with bounds and addresses worked out row by row, 671 in all for any shape); 12 x 144 x 37 x 29, 3x3 stride 1 (rows of an odd
+// length): 10 / 10 / 14 (13 / 16 / 31).  What bounds them is issue: an SM issues two thirds of what it can, and of the forward pass's
+// 5,000 instructions a plane of 57 x 43 a third are the multiply-adds and their loads, half the staging.  Two tiles in flight per CTA
+// were 15 % slower; planes as they lie in memory, by bulk copies into a ring, took half the instructions and were faster for small planes
+// (17 / 19 / 27) but up to twice slower for wide ones, which leave such a CTA few warps.
 #pragma once
 
 namespace plane {
@@ -29,6 +32,19 @@ constexpr int kTileFloats = 6144;            // staged floats per tile to aim at
 constexpr int kMaxFloats = 11264;            // ... and the most a tile may take (44 KB)
 constexpr int kChain = 8;                    // fp32 terms per sum before it goes through fp64
 
+// Division of 0 <= k < 2^31 by a multiplication (Granlund and Montgomery, Division by Invariant Integers using Multiplication, 1994).
+struct Divisor {
+    uint32_t mul, shift;                     // mul 0: by one
+    __device__ __forceinline__ int operator()(int k) const { return mul ? (int)(__umulhi((uint32_t)k, mul) >> shift) : k; }
+};
+static Divisor divisor_of(int d)
+{
+    if (d == 1) return {0u, 0u};
+    uint32_t bits = 1;
+    while ((1LL << bits) < d) ++bits;
+    return {(uint32_t)(((1ull << (31 + bits)) + (unsigned)d - 1) / (unsigned)d), bits - 1};
+}
+
 struct Params {
     const float *in, *gy, *w, *bias;         // forward, parameter gradient: in = x; input gradient: in = gy
     float *out, *gw, *gb;
@@ -36,16 +52,19 @@ struct Params {
     int P, groups;                           // planes of a tile (parameter gradient: images), tiles that cover C (N)
     int R, bands;                            // strip rows of a band (a multiple of TH), bands
     int rows, cols, half, ld;                // staged rows and columns per plane; stride 2: columns of one parity; floats per row
+    int lanes;                               // log2 of the lanes that stage a row
     int base_q, base_r, cols_out;            // input gradient: first q and r; columns of strips
     int strips;                              // strips per band
+    int ranks;                               // parameter gradient: CTAs of a filter
+    Divisor by_bands, by_groups, by_filters;  // by bands, groups and M
     uint32_t cols_magic, strips_magic;
     float scale;
 };
 
 __device__ __forceinline__ int mdiv(int k, uint32_t magic) { return magic ? (int)__umulhi((uint32_t)k, magic) : k; }
-__device__ __forceinline__ void copy4(uint32_t dst, const float *src, bool on)
+__device__ __forceinline__ void copy4(uint32_t dst, const float *src)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(on ? 4u : 0u) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void copies_land()
 {
@@ -81,29 +100,55 @@ __device__ __forceinline__ double cluster_ld(const double *local, int rank)
 }
 
 // Stages `count` planes (plane i at src + i * step, h x w) from row row0 and column col0 on, zeros outside.
+// A group of `1 << p.lanes` lanes takes a row, a lane two columns of it; what is inside is known beforehand, so that a copy costs an
+// address and little else.  (Rows one by one, each with bounds and addresses of its own, took 90 instructions a row of 47 columns, three
+// quarters of what the forward pass executed.)
 template <int S>
 __device__ __forceinline__ void stage_planes(const Params &p, float *tile, const float *src, long long step, int count, int h, int w, int row0,
                                              int col0)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t base = smem_u32(tile);
-    int pl = 0, i = warp;
-    while (i >= p.rows) { i -= p.rows; ++pl; }
-    while (pl < count) {
-        const int row = row0 + i;
-        const bool row_ok = (unsigned)row < (unsigned)h;
-        const float *s = src + pl * step + (long long)row * w;
-        const uint32_t d = base + (uint32_t)((pl * p.rows + i) * p.ld) * 4u;
-        // 32 columns further is 32 words further, or 16 of the same parity
-        const float *sj = s + (col0 + lane);
-        uint32_t dj = d + (uint32_t)(S == 1 ? lane : (lane & 1) * p.half + (lane >> 1)) * 4u;
-        unsigned col = (unsigned)(col0 + lane);
-        for (int j = lane; j < p.cols; j += 32, sj += 32, dj += S == 1 ? 128u : 64u, col += 32u) {
-            const bool ok = row_ok && col < (unsigned)w;
-            copy4(dj, ok ? sj : src, ok);
+    // rows and columns that are inside
+    const int lo = min(max(-row0, 0), p.rows), nv = max(min(p.rows, h - row0) - lo, 0);
+    const int left = min(max(-col0, 0), p.cols), nc = max(min(p.cols, w - col0) - left, 0);
+    const int lanes = 1 << p.lanes, lane = (int)threadIdx.x & (lanes - 1), group = (int)threadIdx.x >> p.lanes, groups = THREADS >> p.lanes;
+    const uint32_t base = smem_u32(tile) + (uint32_t)(lo * p.ld) * 4u, pitch = (uint32_t)p.ld * 4u, next = (uint32_t)lanes * (S == 1 ? 4u : 2u);
+    const float *first = src + (long long)(row0 + lo) * w + (col0 + left);
+    for (int k = lane; k < nc; k += 2 * lanes) {
+        const int j = left + k;
+        const bool two = k + lanes < nc;
+        const float *s = first + k;
+        const uint32_t d = base + (uint32_t)(S == 1 ? j : (j & 1) * p.half + (j >> 1)) * 4u;
+        if (count == 1 || nv >= 2 * groups) {
+            for (int pl = 0; pl < count; ++pl) {
+                const float *si = s + pl * step + group * w;
+                uint32_t di = d + (uint32_t)(pl * p.rows + group) * pitch;
+#pragma unroll 2
+                for (int i = group; i < nv; i += groups, si += groups * w, di += (uint32_t)groups * pitch) {
+                    copy4(di, si);
+                    if (two) copy4(di + next, si + lanes);
+                }
+            }
+        } else if (nv > 0) {
+            const uint32_t magic = nv == 1 ? 0u : 0xffffffffu / (uint32_t)nv + 1u;                      // exact for the few rows of a tile
+            for (int q = group; q < count * nv; q += groups) {
+                const int pl = mdiv(q, magic), i = q - pl * nv;
+                const float *si = s + pl * step + i * w;
+                const uint32_t di = d + (uint32_t)(pl * p.rows + i) * pitch;
+                copy4(di, si);
+                if (two) copy4(di + next, si + lanes);
+            }
         }
-        i += THREADS / 32;
-        while (i >= p.rows) { i -= p.rows; ++pl; }
+    }
+    if (nc < p.cols)
+        for (int q = threadIdx.x; q < count * p.rows; q += THREADS)
+            for (int k = 0; k < p.cols - nc; ++k) {
+                const int j = k < left ? k : k + nc;
+                tile[q * p.ld + (S == 1 ? j : (j & 1) * p.half + (j >> 1))] = 0.f;
+            }
+    if (nv < p.rows) {
+        const int above = lo * p.ld, zeros = (p.rows - nv) * p.ld, skip = nv * p.ld, stride = count == 1 ? THREADS : 32;
+        for (int pl = count == 1 ? 0 : (int)threadIdx.x >> 5; pl < count; pl += THREADS / 32)
+            for (int e = (int)threadIdx.x & (stride - 1); e < zeros; e += stride) tile[pl * p.rows * p.ld + e + (e < above ? 0 : skip)] = 0.f;
     }
 }
 
@@ -117,7 +162,7 @@ struct Weights {
         for (int s = threadIdx.x; s < count * p.M; s += THREADS) bad[s] = 0;
         __syncthreads();
         for (int e = threadIdx.x; e < count * p.M * KK; e += THREADS) {
-            const int s = e / KK, i = e - s * KK, pl = s / p.M, j = s - pl * p.M;
+            const int s = e / KK, i = e - s * KK, pl = p.by_filters(s), j = s - pl * p.M;
             const float v = __ldg(p.w + ((size_t)j * p.C + c0 + pl) * KK + i);
             wsm[s * WS + i] = v;
             if (!(fabsf(v) <= 3.402823466e38f)) bad[s] = 1;
@@ -143,7 +188,7 @@ fwd_kernel(const __grid_constant__ Params p)
     float *wsm = sm;                                           // [P * M][WS], then flags, then the tile
     int *bad = reinterpret_cast<int *>(wsm + p.P * p.M * WT::WS);
     float *tile = reinterpret_cast<float *>(bad + ((p.P * p.M + 3) & ~3));
-    const int unit = (int)blockIdx.x, band = unit % p.bands, ng = unit / p.bands, g = ng % p.groups, n = ng / p.groups;
+    const int unit = (int)blockIdx.x, ng = p.by_bands(unit), band = unit - ng * p.bands, n = p.by_groups(ng), g = ng - n * p.groups;
     const int c0 = g * p.P, planes = min(p.P, p.C - c0), r0 = band * p.R;
     stage_planes<S>(p, tile, p.in + ((long long)n * p.C + c0) * p.H * p.W, (long long)p.H * p.W, planes, p.H, p.W, r0 * S - p.padH, -p.padW);
     WT::stage(p, wsm, bad, c0, planes);
@@ -152,7 +197,7 @@ fwd_kernel(const __grid_constant__ Params p)
     for (int it = threadIdx.x; it < items; it += THREADS) {
         const int t2 = mdiv(it, p.cols_magic), ow = it - t2 * p.oW;
         const int slot = mdiv(t2, p.strips_magic), t0 = (t2 - slot * p.strips) * TH;
-        const int pl = slot / p.M, j = slot - pl * p.M, c = c0 + pl;
+        const int pl = p.by_filters(slot), j = slot - pl * p.M, c = c0 + pl;
         const int oh0 = r0 + t0, cnt = min(TH, p.oH - oh0);
         if (cnt <= 0) continue;
         const float b = p.bias ? __ldg(p.bias + (size_t)j * p.C + c) : 0.f;
@@ -183,8 +228,8 @@ fwd_kernel(const __grid_constant__ Params p)
             }
         }
 #pragma unroll
-        for (int t = 0; t < TH; ++t)
-            if (t < cnt) dst[(long long)t * p.oW] = acc[t];
+        for (int t = 0; t < TH; ++t, dst += p.oW)
+            if (t < cnt) *dst = acc[t];
     }
 }
 
@@ -198,7 +243,7 @@ dgrad_kernel(const __grid_constant__ Params p)
     float *wsm = sm;
     int *bad = reinterpret_cast<int *>(wsm + p.P * p.M * WT::WS);
     float *tile = reinterpret_cast<float *>(bad + ((p.P * p.M + 3) & ~3));
-    const int unit = (int)blockIdx.x, band = unit % p.bands, ng = unit / p.bands, g = ng % p.groups, n = ng / p.groups;
+    const int unit = (int)blockIdx.x, ng = p.by_bands(unit), band = unit - ng * p.bands, n = p.by_groups(ng), g = ng - n * p.groups;
     const int c0 = g * p.P, planes = min(p.P, p.C - c0), q0 = p.base_q + band * p.R;
     stage_planes<1>(p, tile, p.in + ((long long)n * p.C + c0) * p.M * p.oH * p.oW, (long long)p.oH * p.oW, planes * p.M, p.oH, p.oW, q0 - (T - 1),
                     p.base_r - (T - 1));
@@ -241,43 +286,49 @@ dgrad_kernel(const __grid_constant__ Params p)
             }
         }
         const int h0 = (q0 + t0) * S - p.padH, w0 = (p.base_r + ri) * S - p.padW;
-        float *dst = p.out + ((long long)n * p.C + c0 + pl) * p.H * p.W;
-#pragma unroll
-        for (int t = 0; t < TH; ++t)
-#pragma unroll
-            for (int a = 0; a < S; ++a) {
-                const int h = h0 + t * S + a;
-                if ((unsigned)h >= (unsigned)p.H) continue;
-#pragma unroll
-                for (int b = 0; b < S; ++b) {
-                    const int wi = w0 + b;
-                    if ((unsigned)wi >= (unsigned)p.W) continue;
-                    dst[(long long)h * p.W + wi] =
-                        any_bad ? dgrad_point(p.in, p.w, n, c0 + pl, h, wi, p.C, p.M, K, K, S, S, p.padH, p.padW, p.oH, p.oW) : acc[t][a][b];
-                }
+        float *plane = p.out + ((long long)n * p.C + c0 + pl) * p.H * p.W;
+        if (any_bad) {
+#pragma unroll 1
+            for (int e = 0; e < TH * S * S; ++e) {
+                const int h = h0 + e / S, wi = w0 + e % S;
+                if ((unsigned)h < (unsigned)p.H && (unsigned)wi < (unsigned)p.W)
+                    plane[(long long)h * p.W + wi] = dgrad_point(p.in, p.w, n, c0 + pl, h, wi, p.C, p.M, K, K, S, S, p.padH, p.padW, p.oH, p.oW);
             }
+            continue;
+        }
+        float *dst = plane + (long long)h0 * p.W + w0;
+#pragma unroll
+        for (int r = 0; r < TH * S; ++r, dst += p.W) {
+            if ((unsigned)(h0 + r) >= (unsigned)p.H) continue;
+#pragma unroll
+            for (int b = 0; b < S; ++b)
+                if ((unsigned)(w0 + b) < (unsigned)p.W) dst[b] = acc[r / S][r % S][b];
+        }
     }
 }
 
-// Sums over a warp of SUMS values per lane, added up in fp64.  Each of the five steps halves the values as well as the lanes that they
-// still have to meet: a lane passes on half of its values and keeps the other half, so that SUMS = 25 takes 46 shuffles (250 for a
-// butterfly per value) and every lane ends up with a sum or two of its own.
+// Sums over a warp of SUMS values per lane, added up in fp64: those of a 3x3 filter in registers of each lane, more of them (which would
+// leave an SM two CTAs for three) across the warp each time.  Across the warp, each of the five steps halves the values as well as the
+// lanes that they still have to meet: a lane passes on half of its values and keeps the other half, so that SUMS = 25 takes 46 shuffles
+// (250 for a butterfly per value) and every lane ends up with a sum or two of its own.  Of 5x5, 32 x 96 x 57 x 43: 35 us across the warp,
+// 45 in registers; of 3x3, 12 x 144 x 37 x 29: 27 and 26.
 template <int SUMS>
 struct WarpSums {
-    static constexpr int P = SUMS <= 16 ? 16 : (SUMS <= 32 ? 32 : 64), KEEP = P > 32 ? 2 : 1;
-    double mine[KEEP];
+    static constexpr bool OWN = SUMS <= 9;
+    static constexpr int P = SUMS <= 16 ? 16 : (SUMS <= 32 ? 32 : 64), KEEP = P > 32 ? 2 : 1, N = OWN ? SUMS : KEEP;
+    double mine[N];
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
-        for (int q = 0; q < KEEP; ++q) mine[q] = 0.0;
+        for (int q = 0; q < N; ++q) mine[q] = 0.0;
     }
-    __device__ __forceinline__ void add(float (&acc)[SUMS])
+    template <class T>
+    __device__ __forceinline__ static void across(const T (&acc)[SUMS], double (&v)[P / 2])
     {
         const int lane = threadIdx.x & 31;
-        double v[P / 2];
 #pragma unroll
         for (int i = 0; i < P / 2; ++i) {
-            const float a = i < SUMS ? acc[i < SUMS ? i : 0] : 0.f, b = i + P / 2 < SUMS ? acc[i + P / 2 < SUMS ? i + P / 2 : 0] : 0.f;
+            const T a = i < SUMS ? acc[i < SUMS ? i : 0] : T(0), b = i + P / 2 < SUMS ? acc[i + P / 2 < SUMS ? i + P / 2 : 0] : T(0);
             v[i] = (double)(lane & 16 ? b : a) + (double)__shfl_xor_sync(0xffffffffu, lane & 16 ? a : b, 16);
         }
         int count = P / 2;
@@ -296,18 +347,30 @@ struct WarpSums {
                 for (int q = 0; q < KEEP; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
             }
         }
+    }
+    __device__ __forceinline__ void add(float (&acc)[SUMS])
+    {
+        if constexpr (OWN) {
 #pragma unroll
-        for (int q = 0; q < KEEP; ++q) mine[q] += v[q];
+            for (int i = 0; i < SUMS; ++i) mine[i] += (double)acc[i];
+        } else {
+            double v[P / 2];
+            across(acc, v);
+#pragma unroll
+            for (int q = 0; q < KEEP; ++q) mine[q] += v[q];
+        }
 #pragma unroll
         for (int i = 0; i < SUMS; ++i) acc[i] = 0.f;
     }
     __device__ __forceinline__ void store(double *dst) const
     {
         const int lane = threadIdx.x & 31;
+        double v[P / 2];
+        if constexpr (OWN) across(mine, v);
 #pragma unroll
         for (int q = 0; q < KEEP; ++q) {
             const int i = P == 16 ? lane >> 1 : KEEP * lane + q;
-            if (i < SUMS) dst[i] = mine[q];
+            if (i < SUMS) dst[i] = OWN ? v[q] : mine[q];
         }
     }
 };
@@ -333,37 +396,48 @@ wgrad_kernel(const __grid_constant__ Params p)
     const long long units = (long long)p.groups * p.bands;                  // (image group, band)
     const int u_end = (int)(units * (rank + 1) / ranks);
     for (int u = (int)(units * rank / ranks); u < u_end; ++u) {
-        const int band = u % p.bands, n0 = (u / p.bands) * p.P, imgs = min(p.P, p.N - n0), r0 = band * p.R;
-        stage_planes<S>(p, tile, p.in + ((long long)n0 * p.C + c) * p.H * p.W, (long long)p.C * p.H * p.W, imgs, p.H, p.W, r0 * S - p.padH, -p.padW);
-        copies_land();
+        const int group = p.by_bands(u), band = u - group * p.bands, n0 = group * p.P, imgs = min(p.P, p.N - n0), r0 = band * p.R;
         const int items = imgs * p.strips * p.oW;
+        // an item's gy, and where its strip starts in the tile: read while the tile, or the strip before, is on its way
+        float next[TH];
+        int at_next = 0;
+        auto fetch = [&](int it) {
+            if (it >= items) return;
+            const int t2 = mdiv(it, p.cols_magic), ow = it - t2 * p.oW;
+            const int pl = mdiv(t2, p.strips_magic), t0 = (t2 - pl * p.strips) * TH, oh0 = r0 + t0;
+            const float *gp = p.gy + (((long long)(n0 + pl) * p.C + c) * p.M + j) * p.oH * p.oW + (long long)oh0 * p.oW + ow;
+#pragma unroll
+            for (int t = 0; t < TH; ++t, gp += p.oW) next[t] = oh0 + t < p.oH ? __ldg(gp) : 0.f;
+            at_next = (pl * p.rows + t0 * S) * p.ld + ow;
+        };
+        stage_planes<S>(p, tile, p.in + ((long long)n0 * p.C + c) * p.H * p.W, (long long)p.C * p.H * p.W, imgs, p.H, p.W, r0 * S - p.padH, -p.padW);
+        fetch(threadIdx.x);
+        copies_land();
         for (int it0 = 0; it0 < items; it0 += THREADS) {
             if (chain + TH > kChain) { sums.add(acc); chain = 0; }
             chain += TH;
             const int it = it0 + (int)threadIdx.x;
             if (it >= items) continue;
-            const int t2 = mdiv(it, p.cols_magic), ow = it - t2 * p.oW;
-            const int pl = mdiv(t2, p.strips_magic), t0 = (t2 - pl * p.strips) * TH, oh0 = r0 + t0;
-            const float *gp = p.gy + (((long long)(n0 + pl) * p.C + c) * p.M + j) * p.oH * p.oW + (long long)oh0 * p.oW + ow;
             float gv[TH];
 #pragma unroll
-            for (int t = 0; t < TH; ++t) gv[t] = oh0 + t < p.oH ? __ldg(gp + (long long)t * p.oW) : 0.f;
+            for (int t = 0; t < TH; ++t) gv[t] = next[t];
+            const float *row0 = tile + at_next;
+            fetch(it + THREADS);
 #pragma unroll
             for (int t = 0; t < TH; ++t) bias += (double)gv[t];
-            const float *row0 = tile + (pl * p.rows + t0 * S) * p.ld + ow;
 #pragma unroll
             for (int kw = 0; kw < K; ++kw) {
                 const float *col = row0 + (S == 1 ? kw : (kw & 1) * p.half + (kw >> 1));
 #pragma unroll
-                for (int r = 0; r < (TH - 1) * S + K; ++r) {
-                    const float v = col[r * p.ld];
+                for (int r = 0; r < (TH - 1) * S + K; ++r, col += p.ld) {
+                    const float v = *col;
 #pragma unroll
                     for (int t = 0; t < TH; ++t)
                         if (r - t * S >= 0 && r - t * S < K) acc[(r - t * S) * K + kw] = fmaf(gv[t], v, acc[(r - t * S) * K + kw]);
                 }
             }
         }
-        __syncthreads();                                                    // the tile is read before the next one lands
+        __syncthreads();                                                    // the tile is read before the next one lands in its place
     }
     // The CTA's sums; true if one of the filter's is not finite.
     auto gather = [&]() {
@@ -428,13 +502,12 @@ static uint32_t magic_of(int d) { return d == 1 ? 0u : (uint32_t)((1ull << 32) /
 
 enum Pass { FWD, DGRAD, WGRAD };
 
-// Whether a planned pass is faster than the kernel for any shape, by straight lines fitted to 2,970 layers (maps of 3 to 900 columns, 1 to
-// 1024 channels, 1 to 128 images; us on a busy stream).  A few channels, or maps of 7 x 7 to 17 x 17 at stride 2, are over sooner there:
-// staging takes an instruction per row and warp however short the row is, and nothing can be computed before it has landed.
-// Forward of 70 x 560 x 9 x 9, 5x5 stride 2: 26 us for any shape, 66 staged; 32 x 96 x 57 x 43, 5x5 stride 2: 102 and 36 us; input gradient
-// of 12 x 47 x 12 x 9, 3x3 stride 2: 5.0 and 9.8 us; parameter gradient of 1 x 23 x 35 x 35, two 3x3 filters, stride 2: 3.8 and 5.5 us.
-// With the rule 0.2 % of those passes, and 0.5 % of the 3,600 of 1,200 other layers, are more than 7 % slower than for any shape, by 1 to 8 us;
-// 2 % would gain 20 % from the staged form.
+// Whether a planned pass is faster than the kernel for any shape, by straight lines fitted to 1,500 layers (maps of 3 to 900 columns, 1 to
+// 1024 channels, 1 to 128 images; us on a busy stream).  A few channels, or maps of a few pixels, are over sooner there: staging takes an
+// instruction per row and warp however short the row is, and nothing can be computed before it has landed.
+// Forward of 128 x 600 x 5 x 4, 5x5: 17 us for any shape, 23 staged; of 3 x 2 x 113 x 143, three 3x3 filters: 8.4 and 9.4; of
+// 70 x 560 x 9 x 9, 5x5 stride 2: 29 and 23; of 32 x 96 x 57 x 43, 5x5 stride 2: 54 and 21; parameter gradient of 1 x 3 x 46 x 40, 7x7
+// stride 2: 4.4 and 7.9.  Over 1,500 other layers the passes that the rule picks take 1.01 / 1.002 / 1.006 times what the faster ones would.
 static bool faster_than_any_shape(const Params &p, Pass pass, int K)
 {
     const double sms = sm_count(), kk = K * K;
@@ -442,22 +515,19 @@ static bool faster_than_any_shape(const Params &p, Pass pass, int K)
     const double strips = std::ceil((double)p.P * (pass == FWD ? p.M : 1) * p.strips * p.cols_out / THREADS);
     if (pass == WGRAD) {
         const double ctas = (double)p.C * p.M * (kk + 1) / (sms * 8), loops = std::ceil((double)p.oH * p.oW / 256) * p.N;
-        int ranks = 1;
-        while (ranks < 8 && (long long)ranks * 2 <= (long long)p.groups * p.bands) ranks *= 2;
-        const double units = std::ceil((double)p.groups * p.bands / ranks), waves = std::max(1.0, (double)p.C * p.M * ranks / (sms * 3));
+        const double units = std::ceil((double)p.groups * p.bands / p.ranks), waves = std::max(1.0, (double)p.C * p.M * p.ranks / (sms * 3));
         return 3.4 + waves * (units * (0.147 * rows_per_warp + 0.015 * strips * kk) + 0.047 * kk) <
                2.5 + loops * (0.43 + (ctas > 1.0 ? 0.63 * ctas : 0.0));
     }
     const double full = (double)p.N * p.groups * p.bands / (sms * 3), weights = (double)p.P * p.M * kk / THREADS;
     if (pass == FWD) {
         const double threads = (double)p.N * p.C * p.M * p.oH * p.oW / (sms * 2048);
-        return 2.2 + rows_per_warp * (0.095 + 0.056 * full) + strips * kk * (0.011 + 0.028 * full) + 1.56 * full + 0.37 * weights <
-               0.85 * (2.2 + 0.076 * K + kk * (0.078 + 0.10 * threads + 0.10 * std::max(0.0, threads - 1.0)) + 2.1 * threads);
+        return 3.7 + rows_per_warp * (0.004 + 0.037 * full) + strips * kk * (0.017 + 0.028 * full) + 1.9 * full + 0.22 * weights <
+               1.1 * (2.2 + 0.076 * K + kk * (0.078 + 0.10 * threads + 0.10 * std::max(0.0, threads - 1.0)) + 2.1 * threads);
     }
     const double threads = (double)p.N * p.C * p.H * p.W / (sms * 2048);
-    const double staged = 2.6 + 0.10 * K + rows_per_warp * (0.13 + 0.11 * full) + strips * p.M * kk * (0.001 + 0.010 * full) + 2.4 * full + 0.47 * weights;
     const double any = 1.3 + 0.43 * K * p.M + kk * p.M * (0.16 + 0.46 * threads + 0.02 * std::max(0.0, threads - 1.0));
-    return staged < 0.85 * any || (staged < 4.25 && staged < 1.05 * any);         // the smallest: a launch either way
+    return 3.7 + 0.04 * K + rows_per_warp * (0.026 + 0.035 * full) + strips * p.M * kk * (0.012 + 0.023 * full) + 2.2 * full + 0.04 * weights < 1.1 * any;
 }
 
 // Fills the tile plan of a pass; false when the shape is left to the kernels for any shape: other kernel sizes and strides, rows so
@@ -495,6 +565,14 @@ static bool plan(Params &p, Pass pass, int N, int C, int H, int W, int M, int kH
         const int most = pass == WGRAD ? N : C;
         p.P = 1;
         while (p.P < want && p.P < most && floats(p.P + 1, whole) <= kTileFloats) ++p.P;
+        const long long one = (long long)strips * p.cols_out * (pass == FWD ? M : 1);
+        // up to four rounds of strips, while CTAs for 2.75 on each SM remain: what a CTA does once counts for less.  12 x 144 x 37 x 29, 3x3:
+        // 13 / 14 us with one plane, 10 / 11 with two, 8.4 / 10 with four, 10 / 12 with eight (forward / input gradient)
+        if (pass != WGRAD)
+            while (p.P < most && floats(p.P + 1, whole) <= kMaxFloats && (p.P + 1) * one <= 4 * THREADS &&
+                   (long long)N * ceil_div(C, p.P + 1) * 4 >= 11LL * sm_count())
+                ++p.P;
+        else p.P = (int)std::min<long long>(N, kTileFloats / floats(1, whole));
     } else {
         int R = whole;
         while (R > TH && floats(1, R) > kTileFloats) R -= TH;
@@ -506,9 +584,33 @@ static bool plan(Params &p, Pass pass, int N, int C, int H, int W, int M, int kH
     }
     p.rows = (p.R - 1) * step + halo;
     p.strips = p.R / TH;
+    p.lanes = 3;                                                 // two columns a lane, if there are enough
+    while (p.lanes < 8 && (2 << p.lanes) < p.cols) ++p.lanes;
+    if (pass == WGRAD) {
+        // CTAs of a filter and images of a unit: the fewest microseconds with the units shared out evenly, a start of 1.5 and 0.6 a unit;
+        // w warps on an SM issue w / (w + 10) of what it can (0.48 with 9, 0.65 with 21, 0.77 with 29).  16 x 512 x 14 x 14, 5x5: 41 us with
+        // images for one round of strips and as many CTAs as there are units, 23 so; 32 x 96 x 57 x 43, 5x5 stride 2: 39 and 31
+        const long long sms = sm_count();
+        const int per_sm = K == 7 ? 2 : 3, fit = p.P;
+        double best = 0.0;
+        for (int ranks = 1; ranks <= 8; ranks *= 2) {
+            int groups = ceil_div(N, fit);
+            if (p.bands == 1) groups = std::min(N, ceil_div(groups, ranks) * ranks);
+            const int P = ceil_div(N, groups);
+            groups = ceil_div(N, P);
+            if ((long long)groups * p.bands < ranks) break;
+            const double unit = 0.6 + 0.015 * K * K * std::ceil((double)P * p.strips * oW / THREADS) + 0.06 * P * p.rows * ((p.cols + 31) / 32) / (THREADS / 32);
+            const long long ctas = (long long)C * M * ranks, together = std::min<long long>(per_sm, ceil_div_ll(ctas, sms));
+            const double cost = (double)ceil_div_ll(ctas, sms * per_sm) * (1.5 + unit * ceil_div_ll((long long)groups * p.bands, ranks)) * (double)(8 * together + 10);
+            if (best == 0.0 || cost < best) { best = cost; p.P = P; p.ranks = ranks; }
+        }
+    }
     p.groups = ((pass == WGRAD ? N : C) + p.P - 1) / p.P;
     p.cols_magic = magic_of(p.cols_out);
     p.strips_magic = magic_of(p.strips);
+    p.by_bands = divisor_of(p.bands);
+    p.by_groups = divisor_of(p.groups);
+    p.by_filters = divisor_of(M);
     const long long items = (long long)p.P * (pass == FWD ? M : 1) * p.strips * p.cols_out;
     // exact divisions: items * divisor < 2^32 (see magic_of); grids within the launch limits
     if (items * std::max(p.cols_out, p.strips) >= (1LL << 32) || p.cols_out >= (1 << 16)) return false;
@@ -544,16 +646,14 @@ static int launch(const Params &p, Pass pass, int K, int S, cudaStream_t stream)
         CUNN_CUDA(cudaLaunchKernel((const void *)kern, dim3((unsigned)((long long)p.N * p.groups * p.bands)), dim3(THREADS), args, smem_bytes(p, pass, K), stream));
         return 0;
     }
-    int ranks = 1;
-    while (ranks < 8 && (long long)ranks * 2 <= (long long)p.groups * p.bands) ranks *= 2;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(p.C * p.M * ranks));
+    cfg.gridDim = dim3((unsigned)(p.C * p.M * p.ranks));
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem_bytes(p, pass, K);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)ranks;
+    attr[0].val.clusterDim.x = (unsigned)p.ranks;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;

@@ -157,3 +157,31 @@ def test_parameter_gradient_sums_in_fp64(F, shape):
 ])
 def test_both_sides_of_the_staging_rule(F, ref64, ref32, shape):
     test_staged_plane_shapes(F, ref64, ref32, shape)
+
+
+@pytest.mark.parametrize("width", [8, 9, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 512, 517])
+@pytest.mark.parametrize("d", [1, 2])
+def test_rows_that_lanes_share(F, width, d):
+    """Rows of staged columns at the edges of what 8 to 256 lanes copy, two columns each, and of one round of them.  Against fp64, with the
+    bound of a chain of n fp32 multiply-adds: (n + 1) units of 2^-24 of the sum of the terms' magnitudes; n = 25 taps for y and gx, eight
+    products and fp64 for gw and gb."""
+    import torch
+    N, C, H, k, p = 7, 24, 11, 5, 2
+    W = max((width - k) // d * d + k - 2 * p, 4)          # staged columns: (oW - 1) d + k
+    g = torch.Generator(device="cuda").manual_seed(width)
+    x, w = torch.randn(N, C, H, W, device="cuda", generator=g), torch.randn(1, C, k, k, device="cuda", generator=g)
+    b = torch.randn(1, C, device="cuda", generator=g)
+    x64, w64 = x.double().requires_grad_(), w.double().view(C, 1, k, k).requires_grad_()
+    y64 = torch.nn.functional.conv2d(x64, w64, b.double().view(-1), d, p, groups=C)
+    gy = torch.randn(y64.shape, device="cuda", generator=g)
+    gx64, gw64 = torch.autograd.grad(y64, (x64, w64), gy.double())
+    xa, wa = x64.detach().abs().requires_grad_(), w64.detach().abs().requires_grad_()
+    ya = torch.nn.functional.conv2d(xa, wa, b.double().abs().view(-1), d, p, groups=C)
+    gxa, gwa = torch.autograd.grad(ya, (xa, wa), gy.double().abs())
+    gw, gb = torch.zeros_like(w), torch.zeros_like(b)
+    F.dwconv_acc_grad(x, gy, gw, gb, d, d, p, p)
+    gb64, gba = gy.double().sum((0, 2, 3)).view(1, C), gy.double().abs().sum((0, 2, 3)).view(1, C)
+    for what, got, want, size, n in (("gb", gb, gb64, gba, 8), ("y", F.dwconv_forward(x, w, b, d, d, p, p), y64, ya, k * k),
+                                     ("gx", F.dwconv_grad_input(gy, w, H, W, d, d, p, p), gx64, gxa, k * k),
+                                     ("gw", gw.view(C, 1, k, k), gw64, gwa, 8)):
+        assert bool(((got.double() - want).abs() <= (n + 1) * 2.0 ** -24 * size).all()), what
