@@ -1,4 +1,4 @@
-"""Builds libTHCUNN.so (the sm_100a kernels + C ABI) in-tree with nvcc.
+"""Builds libTHCUNN.so (the sm_100a kernels + C ABI) and _calls.so (the ABI as a Python module) in-tree.
 
     python -m cunn_b200.build [--force] [--verbose]
 
@@ -10,12 +10,14 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 SO = os.path.join(LIBDIR, "libTHCUNN.so")
+CALLS = os.path.join(LIBDIR, "_calls.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
@@ -83,7 +85,20 @@ def build(force=False, verbose=False):
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link of libTHCUNN.so failed")
+    _build_calls(force)
     return SO
+
+
+def _build_calls(force):
+    src = os.path.join(CSRC, "py", "calls.cpp")
+    if not force and os.path.exists(CALLS) and os.path.getmtime(CALLS) >= max(os.path.getmtime(src), _deps_mtime()):
+        return
+    cmd = ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall", "-shared", "-I", sysconfig.get_paths()["include"], src, "-o", CALLS,
+           "-L", LIBDIR, "-l:libTHCUNN.so", "-Wl,-rpath,$ORIGIN"] + LINK_EXTRA
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on " + src)
 
 
 if __name__ == "__main__":

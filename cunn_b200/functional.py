@@ -8,7 +8,7 @@ import math
 
 import torch
 
-from ._lib import lib, check
+from ._lib import calls as lib, check
 
 _workspaces = {}
 

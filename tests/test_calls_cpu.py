@@ -1,0 +1,44 @@
+"""The extension module's calls take and refuse what ctypes does, and reach the same library."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from cunn_b200._lib import calls, lib
+
+GEO = (64, 32, 112, 112, 1, 3, 3, 1, 1, 1, 1)
+
+
+def outcome(f, *args):
+    try:
+        return f(*args)
+    except (ctypes.ArgumentError, TypeError) as e:
+        return type(e)
+
+
+@pytest.mark.parametrize("arg", [64, True, np.int32(7), np.int64(3), -1, 2 ** 31, 2 ** 32 + 5, -2 ** 70, 1.0, "1", None, [1]])
+def test_integers(arg):
+    for name in ("cunn_b200_dwconv_acc_grad_workspace", "cunn_b200_convmm_acc_grad_workspace"):
+        assert outcome(getattr(calls, name), arg, *GEO[1:]) == outcome(getattr(lib, name), arg, *GEO[1:])
+    assert outcome(calls.cunn_b200_maxpool_out_size, arg, 3, 2, 1, 1, 1) == outcome(lib.cunn_b200_maxpool_out_size, arg, 3, 2, 1, 1, 1)
+
+
+@pytest.mark.parametrize("arg", [None, 0, 1.0, np.float32(1), True])
+def test_pointers_and_numbers(arg):
+    """n = 0 returns before anything is read."""
+    for L in (calls, lib):
+        assert outcome(L.cunn_b200_sgd_update, None, None, 0, 0.5, None) == 0
+    for at in (0, 3):
+        args = [None, None, 0, 0.5, None]
+        args[at] = arg
+        assert outcome(calls.cunn_b200_sgd_update, *args) == outcome(lib.cunn_b200_sgd_update, *args)
+
+
+def test_too_few_arguments():
+    assert outcome(calls.cunn_b200_dwconv_acc_grad_workspace, *GEO[1:]) is TypeError
+
+
+def test_errors_reach_the_caller():
+    """A call that is refused leaves its message for the thread that made it."""
+    assert calls.cunn_b200_dwconv_forward(None, None, None, None, *GEO, None) != 0
+    assert b"null" in lib.cunn_b200_last_error()
