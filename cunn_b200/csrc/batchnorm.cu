@@ -546,7 +546,8 @@ grad_apply_flat_kernel(const float *__restrict__ x, const float *__restrict__ gy
 // of the tensor out of the 126 MB L2.  Here the channels are taken in groups whose slabs (N planes per channel)
 // fit in a fraction of L2, and a persistent grid of co-resident CTAs (cooperative launch) walks the groups.
 //
-// Every CTA is two halves — four consumer warps and one copy-issuing warp each — with a stream of their own:
+// Every CTA is two halves — eight consumer warps and one copy-issuing warp each — with a stream of their own (with four consumer warps the
+// forward pass of 256 x 64 x 112 x 112 took 416 us, the backward pass 13 % more than two launches; now 378 and 6 %):
 //   * the statistics half reduces group after group (reads carry an L2 evict_last policy), hands in one partial
 //     per (CTA, channel) and takes a ticket; the CTA that draws a channel's last ticket merges the partials in fp64
 //     (in CTA order: results do not depend on timing), publishes mean / inverse std (or the gradient coefficients)
@@ -579,7 +580,7 @@ struct GroupPlan {
 
 constexpr int kStages = 3;              // per half
 constexpr int kStageBytes = 16384;      // per slot: 1024 items of one tensor (forward) or 512 items of two (backward)
-constexpr int kHalf = 128;              // consumer threads per half (4 warps); each half has a fifth warp that only issues copies
+constexpr int kHalfWarps = 8, kHalf = 32 * kHalfWarps;      // consumer threads per half; each half has one more warp that only issues copies
 constexpr int kGroupedThreads = 2 * (kHalf + 32);
 
 __device__ __forceinline__ unsigned long long l2_policy_evict_last()
@@ -609,22 +610,25 @@ __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-// Barrier among the 128 threads of one half (barrier 0 is __syncthreads).
+// Barrier among the consumer threads of one half (barrier 0 is __syncthreads).
 __device__ __forceinline__ void half_sync(int half)
 {
-    if (half == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
-    else asm volatile("bar.sync 2, 128;" ::: "memory");
+    if (half == 0) asm volatile("bar.sync 1, %0;" ::"n"(kHalf) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"n"(kHalf) : "memory");
 }
 
-// Sum over one half; sh: 4 floats of that half.
+// Sum over one half; sh: a float per warp of that half.
 __device__ __forceinline__ float half_sum(float v, float *sh, int half)
 {
     v = warp_sum(v);
-    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) & 3;
+    const int lane = threadIdx.x & 31, w = (int)(threadIdx.x >> 5) % (kHalfWarps + 1);
     half_sync(half);
     if (lane == 0) sh[w] = v;
     half_sync(half);
-    return (sh[0] + sh[1]) + (sh[2] + sh[3]);
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < kHalfWarps; ++i) t += sh[i];
+    return t;
 }
 
 // The CTAs whose shares touch channel cl (local index in the group) of a group of W items: first and last.
@@ -773,8 +777,8 @@ grouped_kernel(const GroupedArgs a)
     constexpr int P = kStageBytes / 16 / T;
     extern __shared__ __align__(128) unsigned char ring_raw[];
     __shared__ __align__(8) unsigned long long full_s[2][kStages];      // slot filled (transaction bytes)
-    __shared__ __align__(8) unsigned long long empty_s[2][kStages];     // slot read by the half's four consumer warps
-    __shared__ float sums_s[2][4];
+    __shared__ __align__(8) unsigned long long empty_s[2][kStages];     // slot read by the half's consumer warps
+    __shared__ float sums_s[2][kHalfWarps];
     __shared__ float k_s;
     __shared__ int flag_s[2];
     __shared__ volatile int applied_s;       // groups this CTA's apply half has finished
@@ -783,8 +787,8 @@ grouped_kernel(const GroupedArgs a)
     const GroupPlan gp = a.gp;
     const int grid = (int)gridDim.x, b = (int)blockIdx.x;
     const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
-    const int half = warp / 5, wi = warp % 5;                           // wi == 4: the half's producer warp
-    const int ht = wi * 32 + lane;                                      // consumer index inside the half, 0..127
+    const int half = warp / (kHalfWarps + 1), wi = warp % (kHalfWarps + 1);                           // wi == 4: the half's producer warp
+    const int ht = wi * 32 + lane;                                      // consumer index inside the half
     float4 *ring = reinterpret_cast<float4 *>(ring_raw) + (size_t)half * kStages * T * P;     // [kStages][T][P] of this half
     unsigned long long *bars = full_s[half], *empties = empty_s[half];
     float *sh = sums_s[half];
@@ -795,7 +799,7 @@ grouped_kernel(const GroupedArgs a)
         for (int h = 0; h < 2; ++h)
             for (int s = 0; s < kStages; ++s) {
                 mbar_init(smem_u32(&full_s[h][s]), 1);
-                mbar_init(smem_u32(&empty_s[h][s]), 4);
+                mbar_init(smem_u32(&empty_s[h][s]), kHalfWarps);
             }
         mbar_fence_init();
         applied_s = 0;
@@ -819,9 +823,9 @@ grouped_kernel(const GroupedArgs a)
         return true;
     };
 
-    if (wi == 4) {
+    if (wi == kHalfWarps) {
         // ------------------------------------------------ producer warp of this half -----------------------------------
-        // Issues every stage of the half's stream, kStages ahead of the consumers: a slot is refilled as soon as the four
+        // Issues every stage of the half's stream, kStages ahead of the consumers: a slot is refilled as soon as the
         // consumer warps have released it.  Before leaving it lets its last copies land (shared memory stays valid until
         // the whole CTA has exited, but nothing may still be in flight when it does).
         StageIter prod;
@@ -1102,11 +1106,13 @@ using namespace cunn;
 using namespace cunn::bn;
 
 // ---- grouped path: planning and launch ---------------------------------------------------------------------
-// Bytes of one group's slabs.  Two groups are in flight (one waiting to be normalised, one being reduced) beside
-// the output being written, and a B200's L2 serves each half of the chip from its own half of the 126 MB.
-static size_t g_group_bytes = (size_t)28 << 20;
-// Bytes of all the groups between the statistics half and the apply half (what has to stay in L2).
-static size_t g_window_bytes = (size_t)56 << 20;
+// Bytes of one group's slabs, and of the two groups that are in flight at most (one waiting to be normalised, one being reduced).  Whatever
+// the 126 MB of L2 keep of them is not read again; the ends of a group cost about 5 us, so that groups that fit with room to spare were
+// slower.  Forward / backward of 256 x 64 x 112 x 112, group and window in MB: 28 and 56 436 / 827 us, 40 and 80 404 / 862, 52 and 104
+// 384 / 641, 64 and 128 378 / 649, 78 and 156 374 / 613, 104 and 208 377 / 616; but 512 x 512 x 14 x 14: 131 / 198 with 64, 175 / 210 with 78.
+// Tensors of less than 128 MB take groups of 28 MB, to have a second one at all.
+static size_t g_group_bytes = (size_t)64 << 20;
+static size_t g_window_bytes = (size_t)128 << 20;
 #ifdef CUNN_B200_DEV_HOOKS
 // sweeps only: CUNN_B200_BN_GROUP_MB / CUNN_B200_BN_WINDOW_MB override the budgets (group 0 disables the grouped kernels)
 static const bool g_group_bytes_from_env = [] {
@@ -1116,13 +1122,25 @@ static const bool g_group_bytes_from_env = [] {
 }();
 #endif
 
-// 0: never use the grouped kernels; 1 (default): the training forward pass with channel slabs of at least 6 MB — two launches / grouped,
-// in us: 128 x 64 x 112 x 112 (6.4 MB) 221 / 212, 256 x 64 x 112 x 112 (12.8) 423 / 416, 1024 x 64 x 56 x 56 (12.8) 459 / 415, 1024 x 128 x
-// 56 x 56 (12.8) 895 / 825, 1024 x 32 x 112 x 112 (51.4) 831 / 833, but 512 x 32 x 112 x 112 (25.7) 419 / 450; below, the plan has too little
-// work per group.  The backward kernel moves the algorithmic 3 passes but is instruction-bound and 10-20 % slower than two launches;
-// 2: wherever they apply.
+// 0: never use the grouped kernels; 1 (default): where they are faster; 2: wherever they apply.
 static int g_grouped_mode = 1;
-static const size_t kGroupedMinSlab = (size_t)6 << 20;
+// Tensors of 128 MB or more with channel slabs of at least 1 MB, two launches / grouped in us.
+// Forward: 128 x 96 x 56 x 56 (154 MB) 94 / 80, 128 x 32 x 112 x 112 111 / 103, 256 x 64 x 112 x 112 420 / 378, 1024 x 64 x 56 x 56
+// 454 / 384, 512 x 32 x 112 x 112 (slabs of 26 MB) 424 / 391, 2 x 16 x 1024 x 1024 315 / 69; but 128 x 256 x 28 x 28 (103 MB) 58 / 62,
+// 256 x 256 x 28 x 28 (slabs of 0.8 MB) 112 / 113.
+// Backward, which is instruction-bound: planes of 1025 to 4000 elements, of which the other kernels' CTAs of 256 threads make poor use
+// (128 x 128 x 56 x 56 176 / 166, 1024 x 64 x 56 x 56 680 / 656, 1000 x 40 x 40 x 32 181 / 166), and few planes (16 x 64 x 256 x 256 224 / 205,
+// 2 x 16 x 1024 x 1024 393 / 108); but 256 x 64 x 112 x 112 612 / 649, 256 x 128 x 32 x 32 106 / 116.
+// Smaller tensors, forward, with slabs of at least 6 MB (few channels, to which the other kernels give few CTAs): 128 x 8 x 112 x 112 35 / 29,
+// 64 x 8 x 224 x 224 66 / 56, 16 x 3 x 500 x 500 91 / 35.
+constexpr size_t kGroupedMinBytes = (size_t)128 << 20;
+static bool grouped_is_faster(int N, int C, int S, bool backward)
+{
+    const size_t slab = (size_t)N * S * sizeof(float);
+    if (slab < ((size_t)1 << 20)) return false;
+    if (slab * C < kGroupedMinBytes) return !backward && slab >= ((size_t)6 << 20);
+    return !backward || (S > 1024 && S <= 4000) || (long long)N * C <= 1024;
+}
 
 static int grouped_grid_cap() { return sm_count() * 2; }
 
@@ -1137,24 +1155,29 @@ static size_t part_region_bytes(int N, int C)
 
 // Fills gp and returns true when the grouped kernels apply: 16-byte rows, channel slabs (tensors_per_item tensors
 // of N planes) that fit the group budget, enough items for every CTA in every group, partials that fit.
-static bool plan_groups(int N, int C, int S, int tensors, const void *a, const void *b, const void *c, int grid, GroupPlan *gp)
+static bool plan_groups(int N, int C, int S, int tensors, const void *a, const void *b, const void *c, int *grid_, GroupPlan *gp)
 {
+    int grid = *grid_;
     if (g_grouped_mode == 0) return false;
-    if (g_grouped_mode == 1 && (tensors != 1 || (size_t)N * S * sizeof(float) < kGroupedMinSlab)) return false;
+    if (g_grouped_mode == 1 && !grouped_is_faster(N, C, S, tensors == 2)) return false;
     if (S % 4 != 0 || ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) != 0) || C > kMaxCounterChannels || grid < 1) return false;
     const size_t slab = (size_t)N * S * sizeof(float) * tensors;
-    if (slab * 2 > g_window_bytes) return false;                 // two groups of one channel must fit the window
-    const int gmax = (int)std::min<size_t>(std::max<size_t>(g_group_bytes / slab, 1), (size_t)C);
+    const bool large = (size_t)N * S * sizeof(float) * C >= kGroupedMinBytes;
+    const size_t group = large ? g_group_bytes : std::min(g_group_bytes, (size_t)28 << 20), window = large ? g_window_bytes : 2 * group;
+    if (slab * 2 > window) return false;                         // two groups of one channel must fit the window
+    const int gmax = (int)std::min<size_t>(std::max<size_t>(group / slab, 1), (size_t)C);
     const int groups = ceil_div(C, gmax);
     const int G = ceil_div(C, groups);
+    if (G <= grid) grid = grid / G * G;                          // CTAs take whole shares of a channel
     const int glast = C - (ceil_div(C, G) - 1) * G;
     gp->N = N; gp->C = C; gp->S = S; gp->L = S / 4;
     gp->G = G; gp->groups = ceil_div(C, G);
     gp->NL = (long long)N * gp->L;
     gp->pstride = grid / glast + 2;
-    gp->lookahead = (int)std::max<size_t>(2, g_window_bytes / ((size_t)G * slab));
+    gp->lookahead = (int)std::max<size_t>(2, window / ((size_t)G * slab));
     if ((long long)glast * gp->NL < 8LL * grid) return false;                      // too little work per CTA and group
     if ((size_t)C * gp->pstride * sizeof(ChunkStat) > part_region_bytes(N, C)) return false;
+    *grid_ = grid;
     return true;
 }
 
@@ -1203,8 +1226,8 @@ static int bn_forward_impl(const float *x, float *y, const float *weight, const 
         {
             GroupedArgs ga{};
             const void *fn = relu ? (const void *)grouped_kernel<false, true> : (const void *)grouped_kernel<false, false>;
-            const int grid = grouped_grid(fn);
-            if (plan_groups(N, C, S, 1, x, y, y, grid, &ga.gp)) {
+            int grid = grouped_grid(fn);
+            if (plan_groups(N, C, S, 1, x, y, y, &grid, &ga.gp)) {
                 unsigned int *cw = (unsigned int *)workspace;
                 ga.x = x; ga.out = y; ga.weight = weight; ga.bias = bias; ga.part = part;
                 ga.cn = GroupCounters{cw, cw + 2 * kMaxCounterChannels, cw + 3 * kMaxCounterChannels};
@@ -1283,8 +1306,8 @@ static int bn_backward_impl(const float *x, const float *gy, bool relu, const fl
     if (gx && need_sums) {
         GroupedArgs ga{};
         const void *fn = relu ? (const void *)grouped_kernel<true, true> : (const void *)grouped_kernel<true, false>;
-        const int grid = grouped_grid(fn);
-        if (plan_groups(N, C, S, 2, x, gy, gx, grid, &ga.gp)) {
+        int grid = grouped_grid(fn);
+        if (plan_groups(N, C, S, 2, x, gy, gx, &grid, &ga.gp)) {
             unsigned int *cw = (unsigned int *)workspace;
             ga.x = x; ga.gy = gy; ga.out = gx; ga.weight = weight; ga.bias = bias; ga.part = part;
             ga.cn = GroupCounters{cw + kMaxCounterChannels, cw + 4 * kMaxCounterChannels, cw + 5 * kMaxCounterChannels};

@@ -279,3 +279,50 @@ def test_bn_full_size_properties(F):
     scale = float(gxd.abs().sum((0, 2, 3)).max())
     assert float(gxd.sum((0, 2, 3)).abs().max()) < 1e-5 * scale
     assert float((gxd * (xd - mean.view(1, C, 1, 1))).sum((0, 2, 3)).abs().max()) < 1e-5 * scale * 2
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, H, W: planes of 1025 to 4000 elements (backward too), larger ones, few of them; slabs of 28 MB groups
+    (96, 101, 60, 60),       # three groups of 34 channels, the last smaller: CTAs whose shares end inside a channel
+    (130, 67, 64, 68),       # two groups
+    (16, 70, 180, 172),      # backward on two launches
+    (2, 17, 1024, 1000),     # two planes a channel
+    (129, 9, 112, 112),      # less than 128 MB
+])
+@pytest.mark.parametrize("relu", [False, True])
+def test_batchnorm_groups_of_channels(F, shape, relu):
+    """Layers large enough for the kernels that walk groups of channels, against fp64."""
+    import torch
+    N, C, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(11)
+    x = torch.randn(shape, device="cuda", generator=g) * 2 + torch.arange(C, device="cuda").view(1, C, 1, 1) * 0.5
+    w, b = torch.rand(C, device="cuda", generator=g) + 0.5, torch.randn(C, device="cuda", generator=g)
+    gy = torch.randn(shape, device="cuda", generator=g)
+    rm, rv = torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+    gw, gb = torch.zeros(C, device="cuda"), torch.zeros(C, device="cuda")
+    forward = F.batchnorm_relu_forward if relu else F.batchnorm_forward
+    y, mean, std = forward(x, w, b, rm, rv, True)
+    if relu:
+        gx = F.batchnorm_relu_backward(x, gy, w, b, rm, rv, mean, std, True, 1.0, 1e-5, gw, gb)
+    else:
+        gx = F.batchnorm_backward(x, gy, w, rm, rv, mean, std, True, 1.0, 1e-5, gw, gb)
+    n, col = N * H * W, lambda t: t.double().view(1, C, 1, 1)
+    m64 = x.double().mean((0, 2, 3))
+    v64 = x.double().var((0, 2, 3), unbiased=False)
+    # the mean is rounded to fp32; a sum of n fp32 values in chains, then fp64, is far closer than 1e-6 of the deviation
+    assert float(((mean.double() - m64).abs() / (m64.abs() * 2.0 ** -24 + 1e-6 * v64.sqrt())).max()) <= 1
+    assert torch.allclose(std.double(), (v64 + 1e-5).rsqrt(), rtol=1e-6, atol=0)
+    assert torch.allclose(rv.double(), 0.9 + 0.1 * v64 * n / (n - 1), rtol=1e-6, atol=0)
+    xh = (x.double() - col(m64)) * (col(v64) + 1e-5).rsqrt()
+    t = xh * col(w) + col(b)
+    keep = (t > 0) if relu else torch.ones_like(t, dtype=torch.bool)
+    sure = t.abs() > 1e-4                                # beyond rounding from where the ReLU turns
+    # three roundings of values up to |x| / std and 8
+    bound = 4 * 2.0 ** -24 * (x.double().abs() * (col(v64) + 1e-5).rsqrt() * col(w) + 8)
+    assert bool(((y.double() - torch.where(keep, t, 0.0)).abs() <= bound + (0 if not relu else 1e-6)).all())
+    g64 = torch.where(y > 0, gy, torch.zeros_like(gy)).double() if relu else gy.double()
+    gb64, gw64 = g64.sum((0, 2, 3)), (g64 * xh).sum((0, 2, 3))
+    size = n ** 0.5
+    assert float((gb.double() - gb64).abs().max()) <= 1e-5 * size and float((gw.double() - gw64).abs().max()) <= 1e-5 * size
+    gx64 = (g64 - col(gb64) / n - xh * col(gw64) / n) * col(w) * (col(v64) + 1e-5).rsqrt()
+    assert float(((gx.double() - gx64).abs() * sure).max()) <= 1e-5
