@@ -547,7 +547,8 @@ grad_apply_flat_kernel(const float *__restrict__ x, const float *__restrict__ gy
 // fit in a fraction of L2, and a persistent grid of co-resident CTAs (cooperative launch) walks the groups.
 //
 // Every CTA is two halves — eight consumer warps and one copy-issuing warp each — with a stream of their own (with four consumer warps the
-// forward pass of 256 x 64 x 112 x 112 took 416 us, the backward pass 13 % more than two launches; now 378 and 6 %):
+// forward pass of 256 x 64 x 112 x 112 took 416 us, the backward pass 13 % more than two launches; now 378 and 6 %.  Less than 128 MB, where
+// a group's sums and flags weigh more, has four: 64 x 8 x 224 x 224 62 us with eight, 56 with four):
 //   * the statistics half reduces group after group (reads carry an L2 evict_last policy), hands in one partial
 //     per (CTA, channel) and takes a ticket; the CTA that draws a channel's last ticket merges the partials in fp64
 //     (in CTA order: results do not depend on timing), publishes mean / inverse std (or the gradient coefficients)
@@ -580,8 +581,8 @@ struct GroupPlan {
 
 constexpr int kStages = 3;              // per half
 constexpr int kStageBytes = 16384;      // per slot: 1024 items of one tensor (forward) or 512 items of two (backward)
-constexpr int kHalfWarps = 8, kHalf = 32 * kHalfWarps;      // consumer threads per half; each half has one more warp that only issues copies
-constexpr int kGroupedThreads = 2 * (kHalf + 32);
+// HW: warps of a half that consume; each half has one more that only issues copies.
+constexpr int grouped_threads(int hw) { return 2 * 32 * (hw + 1); }
 
 __device__ __forceinline__ unsigned long long l2_policy_evict_last()
 {
@@ -611,23 +612,25 @@ __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v)
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // Barrier among the consumer threads of one half (barrier 0 is __syncthreads).
+template <int HW>
 __device__ __forceinline__ void half_sync(int half)
 {
-    if (half == 0) asm volatile("bar.sync 1, %0;" ::"n"(kHalf) : "memory");
-    else asm volatile("bar.sync 2, %0;" ::"n"(kHalf) : "memory");
+    if (half == 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * HW) : "memory");
+    else asm volatile("bar.sync 2, %0;" ::"n"(32 * HW) : "memory");
 }
 
 // Sum over one half; sh: a float per warp of that half.
+template <int HW>
 __device__ __forceinline__ float half_sum(float v, float *sh, int half)
 {
     v = warp_sum(v);
-    const int lane = threadIdx.x & 31, w = (int)(threadIdx.x >> 5) % (kHalfWarps + 1);
-    half_sync(half);
+    const int lane = threadIdx.x & 31, w = (int)(threadIdx.x >> 5) % (HW + 1);
+    half_sync<HW>(half);
     if (lane == 0) sh[w] = v;
-    half_sync(half);
+    half_sync<HW>(half);
     float t = 0.f;
 #pragma unroll
-    for (int i = 0; i < kHalfWarps; ++i) t += sh[i];
+    for (int i = 0; i < HW; ++i) t += sh[i];
     return t;
 }
 
@@ -769,16 +772,16 @@ __device__ __forceinline__ void finish_stats_shifted_warp(const float2 *part, in
     running_var[c] = (float)((1.0 - momentum) * (double)running_var[c] + momentum * (double)unbiased);
 }
 
-template <bool BWD, bool RELU>
-__global__ void __launch_bounds__(kGroupedThreads, 2)
+template <bool BWD, bool RELU, int HW>
+__global__ void __launch_bounds__(grouped_threads(HW), 2)
 grouped_kernel(const GroupedArgs a)
 {
     constexpr int T = BWD ? 2 : 1;
-    constexpr int P = kStageBytes / 16 / T;
+    constexpr int P = kStageBytes / 16 / T, kHalf = 32 * HW;
     extern __shared__ __align__(128) unsigned char ring_raw[];
     __shared__ __align__(8) unsigned long long full_s[2][kStages];      // slot filled (transaction bytes)
     __shared__ __align__(8) unsigned long long empty_s[2][kStages];     // slot read by the half's consumer warps
-    __shared__ float sums_s[2][kHalfWarps];
+    __shared__ float sums_s[2][HW];
     __shared__ float k_s;
     __shared__ int flag_s[2];
     __shared__ volatile int applied_s;       // groups this CTA's apply half has finished
@@ -787,7 +790,7 @@ grouped_kernel(const GroupedArgs a)
     const GroupPlan gp = a.gp;
     const int grid = (int)gridDim.x, b = (int)blockIdx.x;
     const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
-    const int half = warp / (kHalfWarps + 1), wi = warp % (kHalfWarps + 1);                           // wi == 4: the half's producer warp
+    const int half = warp / (HW + 1), wi = warp % (HW + 1);                           // wi == HW: the half's producer warp
     const int ht = wi * 32 + lane;                                      // consumer index inside the half
     float4 *ring = reinterpret_cast<float4 *>(ring_raw) + (size_t)half * kStages * T * P;     // [kStages][T][P] of this half
     unsigned long long *bars = full_s[half], *empties = empty_s[half];
@@ -799,7 +802,7 @@ grouped_kernel(const GroupedArgs a)
         for (int h = 0; h < 2; ++h)
             for (int s = 0; s < kStages; ++s) {
                 mbar_init(smem_u32(&full_s[h][s]), 1);
-                mbar_init(smem_u32(&empty_s[h][s]), kHalfWarps);
+                mbar_init(smem_u32(&empty_s[h][s]), HW);
             }
         mbar_fence_init();
         applied_s = 0;
@@ -823,7 +826,7 @@ grouped_kernel(const GroupedArgs a)
         return true;
     };
 
-    if (wi == kHalfWarps) {
+    if (wi == HW) {
         // ------------------------------------------------ producer warp of this half -----------------------------------
         // Issues every stage of the half's stream, kStages ahead of the consumers: a slot is refilled as soon as the
         // consumer warps have released it.  Before leaving it lets its last copies land (shared memory stays valid until
@@ -868,9 +871,9 @@ grouped_kernel(const GroupedArgs a)
             }
             flag_s[half] = ok;
         }
-        half_sync(half);
+        half_sync<HW>(half);
         const bool ok = flag_s[half] != 0;
-        half_sync(half);
+        half_sync<HW>(half);
         return ok;
     };
     const int qstep = kHalf / gp.L, rstep = kHalf % gp.L;
@@ -896,7 +899,7 @@ grouped_kernel(const GroupedArgs a)
                         e = warp_sum(e);
                         if (ht == 0) k_s = e / (float)mm;
                     }
-                    half_sync(0);
+                    half_sync<HW>(0);
                     K = k_s;
                 } else {
                     mean = __ldg(a.mean_v + c);
@@ -931,8 +934,8 @@ grouped_kernel(const GroupedArgs a)
             release_slot(slot);
             if (st.seg_last) {
                 // hand in this segment's partial; the CTA with the channel's last ticket merges and raises the flag
-                a1 = half_sum(a1, sh, 0);
-                a2 = half_sum(a2, sh, 0);
+                a1 = half_sum<HW>(a1, sh, 0);
+                a2 = half_sum<HW>(a2, sh, 0);
                 int bf, bl;
                 channel_ctas((long long)min(gp.G, gp.C - st.g * gp.G) * gp.NL, gp.NL, st.cl, grid, &bf, &bl);
                 const int cnt = bl - bf + 1;
@@ -942,9 +945,9 @@ grouped_kernel(const GroupedArgs a)
                     __threadfence();                                  // the partial is visible before the ticket
                     flag_s[0] = atomicAdd(a.cn.tick + c, 1u) == (unsigned)(cnt - 1);
                 }
-                half_sync(0);
+                half_sync<HW>(0);
                 const bool last = flag_s[0] != 0;
-                half_sync(0);
+                half_sync<HW>(0);
                 if (last) {
                     __threadfence();                                  // the other CTAs' partials are visible after their tickets
                     if (ht < 32) {
@@ -1134,11 +1137,12 @@ static int g_grouped_mode = 1;
 // Smaller tensors, forward, with slabs of at least 6 MB (few channels, to which the other kernels give few CTAs): 128 x 8 x 112 x 112 35 / 29,
 // 64 x 8 x 224 x 224 66 / 56, 16 x 3 x 500 x 500 91 / 35.
 constexpr size_t kGroupedMinBytes = (size_t)128 << 20;
+static bool grouped_large(int N, int C, int S) { return (size_t)N * S * sizeof(float) * C >= kGroupedMinBytes; }
 static bool grouped_is_faster(int N, int C, int S, bool backward)
 {
     const size_t slab = (size_t)N * S * sizeof(float);
     if (slab < ((size_t)1 << 20)) return false;
-    if (slab * C < kGroupedMinBytes) return !backward && slab >= ((size_t)6 << 20);
+    if (!grouped_large(N, C, S)) return !backward && slab >= ((size_t)6 << 20);
     return !backward || (S > 1024 && S <= 4000) || (long long)N * C <= 1024;
 }
 
@@ -1162,7 +1166,7 @@ static bool plan_groups(int N, int C, int S, int tensors, const void *a, const v
     if (g_grouped_mode == 1 && !grouped_is_faster(N, C, S, tensors == 2)) return false;
     if (S % 4 != 0 || ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) != 0) || C > kMaxCounterChannels || grid < 1) return false;
     const size_t slab = (size_t)N * S * sizeof(float) * tensors;
-    const bool large = (size_t)N * S * sizeof(float) * C >= kGroupedMinBytes;
+    const bool large = grouped_large(N, C, S);
     const size_t group = large ? g_group_bytes : std::min(g_group_bytes, (size_t)28 << 20), window = large ? g_window_bytes : 2 * group;
     if (slab * 2 > window) return false;                         // two groups of one channel must fit the window
     const int gmax = (int)std::min<size_t>(std::max<size_t>(group / slab, 1), (size_t)C);
@@ -1182,12 +1186,12 @@ static bool plan_groups(int N, int C, int S, int tensors, const void *a, const v
 }
 
 // CTAs of a grouped launch: as many as are co-resident (the kernels wait on one another), two per SM at most.
-static int grouped_grid(const void *kernel)
+static int grouped_grid(const void *kernel, int threads)
 {
     const int smem = 2 * kStages * kStageBytes;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return 0;
     int occ = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kGroupedThreads, smem) != cudaSuccess || occ < 1) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) return 0;
     return sm_count() * std::min(occ, 2);
 }
 
@@ -1225,8 +1229,11 @@ static int bn_forward_impl(const float *x, float *y, const float *weight, const 
         ChunkStat *part = (ChunkStat *)((char *)workspace + kCounterBytes);
         {
             GroupedArgs ga{};
-            const void *fn = relu ? (const void *)grouped_kernel<false, true> : (const void *)grouped_kernel<false, false>;
-            int grid = grouped_grid(fn);
+            const bool large = grouped_large(N, C, S);
+            const void *fn = large ? (relu ? (const void *)grouped_kernel<false, true, 8> : (const void *)grouped_kernel<false, false, 8>)
+                                   : (relu ? (const void *)grouped_kernel<false, true, 4> : (const void *)grouped_kernel<false, false, 4>);
+            const int threads = grouped_threads(large ? 8 : 4);
+            int grid = grouped_grid(fn, threads);
             if (plan_groups(N, C, S, 1, x, y, y, &grid, &ga.gp)) {
                 unsigned int *cw = (unsigned int *)workspace;
                 ga.x = x; ga.out = y; ga.weight = weight; ga.bias = bias; ga.part = part;
@@ -1234,7 +1241,7 @@ static int bn_forward_impl(const float *x, float *y, const float *weight, const 
                 ga.running_mean = running_mean; ga.running_var = running_var; ga.save_mean = save_mean; ga.save_std = save_std;
                 ga.momentum = momentum; ga.eps = eps; ga.train = 1; ga.status = device_status_ptr();
                 void *args[] = {(void *)&ga};
-                CUNN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kGroupedThreads), args, (size_t)2 * kStages * kStageBytes, stream));
+                CUNN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, (size_t)2 * kStages * kStageBytes, stream));
                 return 0;
             }
         }
@@ -1305,8 +1312,9 @@ static int bn_backward_impl(const float *x, const float *gy, bool relu, const fl
     const bool need_sums = train || grad_weight || grad_bias;
     if (gx && need_sums) {
         GroupedArgs ga{};
-        const void *fn = relu ? (const void *)grouped_kernel<true, true> : (const void *)grouped_kernel<true, false>;
-        int grid = grouped_grid(fn);
+        const void *fn = relu ? (const void *)grouped_kernel<true, true, 8> : (const void *)grouped_kernel<true, false, 8>;
+        const int threads = grouped_threads(8);
+        int grid = grouped_grid(fn, threads);
         if (plan_groups(N, C, S, 2, x, gy, gx, &grid, &ga.gp)) {
             unsigned int *cw = (unsigned int *)workspace;
             ga.x = x; ga.gy = gy; ga.out = gx; ga.weight = weight; ga.bias = bias; ga.part = part;
@@ -1314,7 +1322,7 @@ static int bn_backward_impl(const float *x, const float *gy, bool relu, const fl
             ga.mean_v = mean_v; ga.std_or_var = sv; ga.grad_weight = grad_weight; ga.grad_bias = grad_bias; ga.coef = coef;
             ga.eps = eps; ga.scale = scale; ga.train = train; ga.status = device_status_ptr();
             void *args[] = {(void *)&ga};
-            CUNN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kGroupedThreads), args, (size_t)2 * kStages * kStageBytes, stream));
+            CUNN_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, (size_t)2 * kStages * kStageBytes, stream));
             return 0;
         }
     }
