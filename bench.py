@@ -335,7 +335,7 @@ def other_configs_bench(dev):
         for op, fn in ops.items():
             ms = timed(fn, nbuf)
             res["%s_%s" % (name, op)] = {"us": round(ms * 1e3, 1), "value": round(flop / (ms * 1e-3) / 1e12, 1),
-                                         "unit": "TFLOP/s fp32-equivalent (3xTF32 tcgen05)"}
+                                         "unit": "TFLOP/s fp32-equivalent (split operands, tcgen05)"}
         del xs, gys, ys, gxs
     # ---- BatchNormalization and SpatialMaxPooling --------------------------------------------
     N, C, HW = 256, 64, 112

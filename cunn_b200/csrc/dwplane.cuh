@@ -18,8 +18,8 @@
 //
 // Forward / input gradient / parameter gradient on a cold cache, in us: 32 x 96 x 57 x 43, 5x5 stride 2: 21 / 16 / 34 (38 MB a pass: 6 us;
 // 35 / 30 / 52 with bounds and addresses worked out row by row, 671 in all for any shape); 12 x 144 x 37 x 29, 3x3 stride 1 (rows of an odd
-// length): 10 / 10 / 14 (13 / 16 / 31).  What bounds them is issue: an SM issues two thirds of what it can, and of the forward pass's
-// 5,000 instructions a plane of 57 x 43 a third are the multiply-adds and their loads, half the staging.  Two tiles in flight per CTA
+// length): 10 / 10 / 14 (13 / 16 / 31).  What bounds them is issue and shared memory: 54 to 64 % of the issue slots, and forward 58 % of the
+// cycles of shared memory, for 3,500 / 3,000 / 6,400 warp instructions a plane of 57 x 43 (7,900 / 4,800 / 10,600 before).  Two tiles in flight per CTA
 // were 15 % slower; planes as they lie in memory, by bulk copies into a ring, took half the instructions and were faster for small planes
 // (17 / 19 / 27) but up to twice slower for wide ones, which leave such a CTA few warps.
 #pragma once
