@@ -1485,6 +1485,41 @@ static PwTmaKernel pw_tma_pick(int bn)
         default: return pwt::pw_tma_kernel<OP, 128, 4, 8, 4, 2>;
     }
 }
+// CTAs that share a tile of a launch whose tiles (of 32 columns) leave most SMs idle: four, where the reduction is ten k-blocks or longer, two
+// where four do not fit, eight for the longest.  A share's start, and adding up through the others' shared memory, cost what four k-blocks do.
+// Forward, one CTA / two / four / eight a tile, in us: 512 -> 512 on one 14 x 14 image (32 tiles, 16 k-blocks) 15.9 / 14.5 / 10.4 / -,
+// 1024 -> 1024 at 8 x 8 24.7 / 18.6 / 12.9 / 13.1, 512 -> 512 at 8 x 8 15.2 / 14.0 / 10.4 / 14.5, 768 -> 768 at 14 x 14 20.6 / 16.5 / - / -,
+// 4096 -> 64 at 4 x 4 (128 k-blocks) 80 / - / - / 17.6; but 256 -> 256 (8 k-blocks) on three 14 x 14 images 10.4 / 12.4 / - / -, 128 -> 128 at
+// 28 x 28 8.3 / 10.4 / - / -.  The sums are in the order of the ranks, whatever finishes first; shorter chains: errors 5.2e-7 -> 4.3e-7.
+static int pw_cluster(int bn, int tiles, int kblocks)
+{
+    const int sms = sm_count();
+    if (bn != 32 || kblocks < 10) return 1;
+    if (kblocks >= 64 && tiles * 8 <= sms) return 8;
+    if (tiles * 4 <= sms) return 4;
+    return kblocks >= 16 && tiles * 2 <= sms ? 2 : 1;
+}
+template <int OP>
+static int pw_cluster_launch(pw::Params &p, int ranks, CUtensorMap &ma, CUtensorMap &mb, cudaStream_t stream)
+{
+    const void *kern = (const void *)pwt::pw_tma_kernel<OP, 32, 4, 8, 4, 2, true>;
+    CUNN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pw::SMEM));
+    p.kblocks = ceil_div(p.kblocks, ranks);
+    void *args[] = {(void *)&p, (void *)&ma, (void *)&mb, (void *)&ma};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ranks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.total_tiles * ranks));
+    cfg.blockDim = dim3((unsigned)pwt::tma_threads(4, 8));
+    cfg.dynamicSmemBytes = pw::SMEM;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    CUNN_CUDA(cudaLaunchKernelExC(&cfg, kern, args));
+    return 0;
+}
 // `mo` is the map of the output tensor for the bulk-store epilogue (forward / input gradient); kernels that do not use
 // it get a copy of `ma`.
 static int pw_tma_launch(PwTmaKernel kern, pw::Params &p, CUtensorMap &ma, CUtensorMap &mb, CUtensorMap &mo, cudaStream_t stream)
@@ -1773,6 +1808,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
             tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, false, q.total_tiles);
             if (make_map(&ma, x, q.HW, C, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return 1;
             if (make_map(&mb, weight, C, K, 0, 32, bn, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
+            if (const int ranks = pw_cluster(bn, q.total_tiles, q.kblocks); ranks > 1) return pw_cluster_launch<OP_FWD>(q, ranks, ma, mb, stream);
             if (q.bulk_out) { if (make_map(&mo, y, q.HW, K, N, BM, pwt::HALF_STAGE_COLS, CU_TENSOR_MAP_SWIZZLE_NONE)) return 1; }
             else mo = ma;
             return pw_tma_launch(pw_tma_pick<OP_FWD>(bn), q, ma, mb, mo, stream);
@@ -1865,6 +1901,8 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
             tma_accumulators(bn, q.kblocks, &q.nacc, &q.sets, false, q.total_tiles);
             if (make_map(&ma, gy, q.HW, K, N, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return 1;
             if (make_map(&mb, weight, C, K, 0, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B)) return 1;
+            if (const int ranks = pw_cluster(bn, q.total_tiles, q.kblocks); ranks > 1)
+                return add_bias(pw_cluster_launch<OP_DGRAD>(q, ranks, ma, mb, stream));
             if (q.bulk_out) { if (make_map(&mo, gx, q.HW, C, N, BM, pwt::HALF_STAGE_COLS, CU_TENSOR_MAP_SWIZZLE_NONE)) return 1; }
             else mo = ma;
             return add_bias(pw_tma_launch(pw_tma_pick<OP_DGRAD>(bn), q, ma, mb, mo, stream));

@@ -73,23 +73,7 @@ __device__ __forceinline__ void copies_land()
     __syncthreads();
 }
 
-// Thread-block clusters: this CTA's rank, their number, a barrier of all their threads, a double in another CTA's shared memory.
-__device__ __forceinline__ int cluster_rank()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return (int)r;
-}
-__device__ __forceinline__ int cluster_size()
-{
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return (int)r;
-}
-__device__ __forceinline__ void cluster_sync()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// A double in another CTA's shared memory.
 __device__ __forceinline__ double cluster_ld(const double *local, int rank)
 {
     uint32_t a;

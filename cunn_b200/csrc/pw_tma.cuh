@@ -204,7 +204,10 @@ __device__ __forceinline__ void drain_tile(const Params &p, const CUtensorMap &m
     }
 }
 
-template <int OP, int BN, int SW, int EW, int NS, int NL>
+// CL: a cluster of CTAs shares a tile, each its run of p.kblocks k-blocks; every CTA then adds up its part of the columns, in the order of
+// the ranks, from the sums that the others leave in their shared memory.  For launches whose tiles would leave most SMs idle and take
+// a k-block after the other: one image through 512 -> 512 at 14 x 14 is 32 tiles of 16 k-blocks.
+template <int OP, int BN, int SW, int EW, int NS, int NL, bool CL = false>
 __global__ void __launch_bounds__(tma_threads(SW, EW), 1)
 pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
               const __grid_constant__ CUtensorMap map_out)
@@ -249,7 +252,8 @@ pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const _
     // NS raw stages and NL lo buffers of 32 KB (the library runs 4 + 2, which leaves room for the 32 KB output staging area;
     // 4 + 3 and 5 + 2 without the staging area measured within 3 % of it)
     static_assert(NS >= NL && NS <= MAX_STAGES && (size_t)(NS + NL) * 2 * TILE + 1024 <= SMEM, "one completion barrier per raw stage also guards the lo buffers");
-    const int my_tiles = ((int)blockIdx.x < p.total_tiles) ? (p.total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int ranks = CL ? cluster_size() : 1, rank = CL ? cluster_rank() : 0, tile0 = CL ? (int)blockIdx.x / ranks : (int)blockIdx.x;
+    const int my_tiles = CL ? 1 : ((int)blockIdx.x < p.total_tiles) ? (p.total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const int total_it = my_tiles * KB;
     // nacc == 1: all three products of every k-block go to one accumulator (tiles of one or two k-blocks, whose chains are
     // short anyway); otherwise the hi*hi products are dealt round-robin to nacc - 1 accumulators and the cross terms share the last
@@ -262,9 +266,9 @@ pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const _
     if (warp == TMA_WARP) {
         // ---- copy issue: k-block i goes to raw stage i % NS as soon as the MMAs that read it last are done ----
         if (lane == 0) {
-            int t = (int)blockIdx.x, kb = 0;
+            int t = tile0, kb = 0;
             for (int i = 0; i < total_it; ++i) {
-                const int rs = i % NS;
+                const int rs = i % NS, k0 = (rank * KB + kb) * BK;               // beyond the last value: zero fill
                 if (i >= NS && !mbar_wait(smem_u32(mmadone + rs), (uint32_t)((i / NS - 1) & 1), p.status)) break;
                 const uint32_t bar = smem_u32(rawfull + rs);
                 const uint32_t sa = smem_u32(smem + (size_t)rs * 2 * TILE), sb = sa + TILE;
@@ -274,13 +278,13 @@ pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const _
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int g = m_tile * 4 + j, im = g / p.gpi, p0 = (g - im * p.gpi) * 32;
-                        tma_load_3d(sa + (uint32_t)(j * GROUP_BYTES), &map_a, p0, kb * BK, im, bar);     // image >= n_img: zero fill
+                        tma_load_3d(sa + (uint32_t)(j * GROUP_BYTES), &map_a, p0, k0, im, bar);     // image >= n_img: zero fill
                     }
                     if (OP == OP_FWD) {
-                        tma_load_2d(sb, &map_b, kb * BK, n_tile * BN, bar);
+                        tma_load_2d(sb, &map_b, k0, n_tile * BN, bar);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < BN / 32; ++j) tma_load_2d(sb + (uint32_t)(j * GROUP_BYTES), &map_b, n_tile * BN + 32 * j, kb * BK, bar);
+                        for (int j = 0; j < BN / 32; ++j) tma_load_2d(sb + (uint32_t)(j * GROUP_BYTES), &map_b, n_tile * BN + 32 * j, k0, bar);
                     }
                 } else {
                     const int split = t / p.tiles_per_split, r = t - split * p.tiles_per_split;
@@ -364,6 +368,18 @@ pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const _
             const int set = count % p.sets;
             if (!mbar_wait(smem_u32(accready + set), (uint32_t)((count / p.sets) & 1), p.status)) { ok = false; break; }
             tc_fence_after();
+            if constexpr (CL) {
+                float *stage = reinterpret_cast<float *>(smem + (size_t)(NS + NL) * 2 * TILE) + quarter * 32 + lane;      // [column][row]
+                for (int c0 = half * (BN * 4 / EW); c0 < (half + 1) * (BN * 4 / EW); c0 += 16) {
+                    float acc[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[j] = 0.f;
+                    gather_acc16<EW == 8>(acc, tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, nhi_used, p.nacc, ACC_COLS);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) stage[(c0 + j) * BM] = acc[j];
+                }
+                continue;
+            }
             drain_tile<OP, BN, EW / 4>(p, map_out, reinterpret_cast<float *>(smem + (size_t)(NS + NL) * 2 * TILE), tmem_base + (uint32_t)set * set_cols, t,
                                nhi_used, quarter, half, lane, tid - (SW + 4 * half) * 32);
             tc_fence_before();                                       // the TMEM reads above are ordered before the arrival
@@ -438,6 +454,27 @@ pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const _
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
+    if constexpr (CL) {
+        static_assert(OP != OP_WGRAD && BN <= 64, "columns of 128 rows fit the output staging area");
+        cluster_sync();                                              // everybody's sums are in shared memory
+        const int m_tile = tile0 / p.n_tiles, n_tile0 = (tile0 - m_tile * p.n_tiles) * BN, columns = BN / ranks;
+        const uint32_t stage = smem_u32(smem + (size_t)(NS + NL) * 2 * TILE);
+        for (int e = tid; e < columns * BM; e += (int)blockDim.x) {
+            const int row = e % BM, col = rank * columns + e / BM, n = n_tile0 + col;
+            const int g = m_tile * 4 + row / 32, im = g / p.gpi, pix = (g - im * p.gpi) * 32 + row % 32;
+            if (im >= p.n_img || pix >= p.HW || n >= p.N_total) continue;
+            float sum = OP == OP_FWD && p.bias ? __ldg(p.bias + n) : 0.f;
+            for (int r = 0; r < ranks; ++r) {
+                uint32_t a;
+                float v;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(stage + (uint32_t)(col * BM + row) * 4u), "r"(r));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+                sum += v;
+            }
+            p.out[((size_t)im * p.N_total + n) * p.HW + pix] = sum;
+        }
+        cluster_sync();                                              // shared memory outlives the others' reads
+    }
 }
 
 }  // namespace pwt

@@ -278,3 +278,36 @@ def test_fully_connected_layers_of_one_or_two_k_blocks(F, shape):
     # truncated operands 3.5e-7; two chains of four and eight truncations, the longer one at 2^-10 of the sum: 2e-7
     for got, want in ((y, xd @ wd.t()), (gx, gd @ wd)):
         assert float((got.double() - want).norm() / want.norm()) <= 5.5e-7
+
+
+@pytest.mark.parametrize("shape", [
+    # N, C, K, H, W: clusters of four, two and eight CTAs a tile; reductions that do not divide by them; ragged tiles; two images in a tile
+    (1, 512, 512, 14, 14), (1, 320, 40, 8, 8), (1, 332, 36, 5, 4), (2, 484, 100, 6, 6), (1, 768, 768, 14, 14), (1, 4096, 64, 4, 4), (1, 2052, 32, 1, 4),
+    (3, 352, 200, 9, 4),
+])
+def test_pointwise_layers_of_few_tiles(shape):
+    """Few tiles and long reductions: CTAs of a cluster share a tile.  Against fp64, with the bound of the truncating accumulation: products
+    of 22 bits and chains of 12 additions a k-block of 32, at most KB k-blocks a CTA."""
+    import torch
+    from cunn_b200 import functional as F
+    N, C, K, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(C + K)
+    x, w = torch.randn(N, C, H, W, device="cuda", generator=g), torch.randn(K, C, 1, 1, device="cuda", generator=g)
+    b, gy = torch.randn(K, device="cuda", generator=g), torch.randn(N, K, H, W, device="cuda", generator=g)
+    wm = w.double().view(K, C)
+    for what, got, a, t, bias in (("y", F.convmm_forward(x, w, b, 1, 1, 0, 0), wm, x, b), ("gx", F.convmm_grad_input(gy, w, H, W, 1, 1, 0, 0), wm.t(), gy, None)):
+        want = torch.einsum("kc,nchw->nkhw", a, t.double())
+        size = torch.einsum("kc,nchw->nkhw", a.abs(), t.double().abs())
+        if bias is not None:
+            want, size = want + bias.double().view(1, -1, 1, 1), size + bias.double().abs().view(1, -1, 1, 1)
+        kb = -(-a.shape[1] // 32)
+        assert bool(((got.double() - want).abs() <= (4 + 12 * kb) * 2.0 ** -23 * size).all()), what
+        assert float((got.double() - want).norm() / want.norm()) <= 1e-6, what
+    y = F.convmm_forward(x, w, b, 1, 1, 0, 0)
+    assert torch.equal(y, F.convmm_forward(x, w, b, 1, 1, 0, 0))          # the same order of sums each time
+    # infinities and NaN reach the outputs that read them and no others
+    x[0, 1, 0, 0], x[-1, 0, -1, -1] = float("inf"), float("nan")
+    bad = ~torch.isfinite(F.convmm_forward(x, w, b, 1, 1, 0, 0))
+    hit = torch.zeros(N, 1, H, W, dtype=torch.bool, device="cuda")
+    hit[0, 0, 0, 0] = hit[-1, 0, -1, -1] = True
+    assert torch.equal(bad, hit.expand_as(bad))
