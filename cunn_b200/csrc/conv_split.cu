@@ -59,6 +59,9 @@ constexpr size_t SMEM = RING_BYTES + EPI_WARPS * STORE_BYTES;
 constexpr int SCALED_MAX = 14;           // the largest value of a group lies in [2^14, 2^15) after scaling
 
 
+// A pass is a few kernels, each launched while the one before still runs; it waits for it (pdl_wait) before it reads or writes.  What an
+// earlier kernel of the pass wrote is read by plain loads: the read-only path (__ldg) is for memory that nobody writes while a kernel exists.
+
 // ---- exponents ----------------------------------------------------------------------------------------------------------------
 // Exponent of a group from the bits of its largest finite magnitude; 2^(SCALED_MAX - e) is a normal number.
 __device__ __forceinline__ int group_exp(uint32_t max_bits) { return max((int)(max_bits >> 23) - 127, -112); }
@@ -203,7 +206,7 @@ __device__ __forceinline__ void prep_act(const Act &a, int block, float *tile_)
     float f[8];
     if (PER_CHANNEL) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = pow2(SCALED_MAX - group_exp(c0 + i < a.C ? __ldg(a.chmax + c0 + i) : 0u));
+        for (int i = 0; i < 8; ++i) f[i] = pow2(SCALED_MAX - group_exp(c0 + i < a.C ? a.chmax[c0 + i] : 0u));
     }
     __syncthreads();
     const size_t part = (size_t)a.pixels * a.Cp;
@@ -268,7 +271,7 @@ __device__ __forceinline__ void prep_window(const Act &a, int block, float *tile
             for (int i = tid; i < w.oW; i += T) a.exps[(size_t)row * w.oW + i] = (int8_t)e;
     }
     for (int c = 0; c < w.C; ++c) {
-        if (PER_CHANNEL) s = pow2(SCALED_MAX - group_exp(__ldg(a.chmax + c)));
+        if (PER_CHANNEL) s = pow2(SCALED_MAX - group_exp(a.chmax[c]));
 #pragma unroll 4
         for (int i = tid; i < cols; i += T) {
             const int at = i - w.padW;
@@ -794,7 +797,7 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
             auto exp_at = [&]() -> int {
                 const int ih = ih0 + th * f.dlH, iw = iw0 + tw * f.dlW;
                 return row_ok && (unsigned)ih < (unsigned)p.g_H && (unsigned)iw < (unsigned)p.g_W
-                           ? (int)__ldg(p.exps + (((size_t)im * p.g_H + ih) * p.g_W + iw) * p.groups + g) : NO_EXP;
+                           ? (int)p.exps[(((size_t)im * p.g_H + ih) * p.g_W + iw) * p.groups + g] : NO_EXP;
             };
             int next = WG ? 0 : exp_at(), top = NO_EXP;
             for (int q = it.begin; q < it.end; ++q) {
@@ -886,7 +889,7 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                 const int last = min(STORE_COLS, my_cols - c);
                 __syncwarp();
                 if (lane < STORE_COLS) {
-                    const int ec = lane < last ? __ldg(p.w_exp + n0 + c + lane) : 0, hc = ec / 2;
+                    const int ec = lane < last ? p.w_exp[n0 + c + lane] : 0, hc = ec / 2;
                     column[lane] = make_float4(pow2(hc), pow2(ec - hc), p.bias && lane < last ? __ldg(p.bias + n0 + c + lane) : 0.f, 0.f);
                 }
 #pragma unroll
@@ -987,12 +990,12 @@ reduce_kernel(const __grid_constant__ ReduceParams p)
     for (int k = share; k < p.splits; k += p.shares)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            sum[i] += __ldg(src[i]);
+            sum[i] += *src[i];
             src[i] += split_step;
         }
-    const int eg = ko < p.K ? group_exp(__ldg(p.gy_max + ko)) : 0;
+    const int eg = ko < p.K ? group_exp(p.gy_max[ko]) : 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) tile[warp][i][lane] = scale_by(sum[i], eg + group_exp(__ldg(p.x_max + c[i])) - 2 * SCALED_MAX);
+    for (int i = 0; i < 4; ++i) tile[warp][i][lane] = scale_by(sum[i], eg + group_exp(p.x_max[c[i]]) - 2 * SCALED_MAX);
     __syncthreads();
     for (int i = tid; i < 32 * per; i += 256) {
         const int k = i / per, o = i - k * per;
