@@ -128,6 +128,14 @@ __device__ __forceinline__ void bulk_g2s_hint(uint32_t dst_smem, const void *src
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Kernels that run only if an earlier one of the pass says so.  Called first, by all threads: such a kernel is launched programmatically.
+__device__ __forceinline__ bool gated_off(const int *gate)
+{
+    if (!gate) return false;
+    pdl_wait();
+    return *gate == 0;
+}
+
 // Thread-block clusters: this CTA's rank, their number, a barrier of all their threads.
 __device__ __forceinline__ int cluster_rank()
 {

@@ -53,6 +53,7 @@ struct GatherParams {
     const float *a, *b, *bias;    // gathered tensor, weights, bias or null
     float *out;
     int *status;
+    const int *gate;              // null, or see gated_off
     int g_C, g_H, g_W;            // channels, rows and columns of the gathered tensor
     int N_total, n_tiles, total_tiles, n_phases;
     int w_kk;                     // taps of the whole kernel
@@ -237,6 +238,7 @@ gather_gemm_kernel(const __grid_constant__ GatherParams p)
     constexpr int COLS = BN / 4;                                           // columns per producer warp
     constexpr uint32_t idesc = idesc_of(BN, true, B_MN);
 
+    if (gated_off(p.gate)) return;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t done[RAW_STAGES];     // the MMAs of this stage's k-block have finished
     __shared__ uint64_t full[RAW_STAGES];     // stage split and visible to the tensor core: one arrival per producer warp
@@ -430,6 +432,7 @@ constexpr int CH = 4, MAX_AXIS = 64;
 struct FmaParams {
     const float *gy, *w, *bias;
     float *gx;
+    const int *gate;
     int N, C, H, W, K, kW, kk, dH, dW, oH, oW, groups;
     int only_short;                                             // leave residues of SHORT_SUM products or more alone
     AxisPhase rows[MAX_AXIS], cols[MAX_AXIS];
@@ -437,6 +440,7 @@ struct FmaParams {
 __global__ void __launch_bounds__(256)
 phase_fma_kernel(const __grid_constant__ FmaParams p)
 {
+    if (gated_off(p.gate)) return;
     const AxisPhase &a = p.rows[blockIdx.y], &b = p.cols[blockIdx.z];
     if (p.only_short && (long long)p.K * a.taps * b.taps >= SHORT_SUM) return;
     const int part = (int)blockIdx.x / p.groups, n0 = ((int)blockIdx.x - part * p.groups) * CH;

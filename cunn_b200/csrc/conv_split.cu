@@ -1,4 +1,4 @@
-// Convolutions of more than one tap on operands that are split once.
+// Convolutions on operands that are split once.
 //
 // The kernels of convmm.cu gather every operand value for every tap and split it on the way: for a 3x3 layer each input value is
 // copied with 4-byte copies, and split, nine times per column tile, and the warps that do so are what the layer waits for.  Here a
@@ -6,9 +6,9 @@
 // kernel fetches its tiles with im2col tensor-map copies: 128 consecutive output pixels x 32 channels of one tap are one copy, zeros
 // outside the image included, in the layout that the tensor core reads.  No thread touches an operand again.
 //
-// Split.  v = (hi + lo) * 2^e with hi, lo of 11 bits each, products hi*hi + hi*lo + lo*hi: the same bits as the 3xTF32 split with
-// rounding (tf32 and fp16 have 11-bit significands), at twice the rate of tf32 and half its bytes.  fp16 has five exponent bits, so
-// values are scaled by powers of two, which is exact:
+// Split.  v = (hi + lo) * 2^e with hi, lo of 11 bits each, products hi*hi + hi*lo + lo*hi: as the 3xTF32 split with rounding (tf32 and
+// fp16 have 11-bit significands), at twice the rate of tf32 and half its bytes.  fp16 has five exponent bits, so values share exponents,
+// powers of two that scale them exactly:
 //   * activations of the forward pass and of input gradients: one exponent per pixel and group of 64 channels, that of its largest
 //     finite value.  It varies along the reduction, so the tensor core sums one block of 64 channels at a time and the block's sum
 //     is scaled when it is added to fp32 registers.
@@ -16,6 +16,14 @@
 //   * weight gradients reduce over pixels: one exponent per channel of x and of gy, found by a pass over both.
 // A value is kept to max(2^-23 |v|, 2^-40 of the largest in its group).  Infinities and NaN stay what they are (lo = 0) and do not
 // count for the exponent.
+//
+// Range.  Values below 2^-17 of their group's largest lose bits.  The sums do not show it where the largest is part of them, and it mostly is:
+// behind a batch normalisation whole channels are 1e-5 or 1e-7 of others.  But where it meets zeros the error is the sum's: a channel of 1e9
+// without weights among ordinary ones left 3 digits, one of 1e13 none.  So the sums are compared with what the exponents of their operands
+// allow for: SMALL_SUM and SMALL_GRAD say when they are too small for that, by more than chance, and the images of the round are done again by the
+// kernels of convmm.cu, whose tf32 operands have an exponent each.  Those are launched every time and leave at once if *gate says that
+// nothing was lost, which costs a pass 2 to 5 us.  (Looking at the operands instead cost the split as much, and sent the gradients of half of
+// MobileNetV1's pointwise layers there.)
 //
 // Accumulation: the tensor core truncates when it adds, so a chain is one block, 64 channels (or pixels) of 12 additions, the eight of
 // the cross terms first, while the accumulator is small; blocks are added in registers with rounding (two TMEM buffers in turn).
@@ -57,6 +65,16 @@ constexpr size_t RING_BYTES = 192 * 1024;
 constexpr int STORE_COLS = 16, STORE_BYTES = STORE_COLS * (128 + 16);     // columns that a summing warp stores at a time, and its room for them
 constexpr size_t SMEM = RING_BYTES + EPI_WARPS * STORE_BYTES;
 constexpr int SCALED_MAX = 14;           // the largest value of a group lies in [2^14, 2^15) after scaling
+// Values below 2^-2 after scaling are off by 2^-26.8 on average, 2^-25 at most.  A block's sum of 64 products is off by 2^-9.3 on average and 2^-3
+// at most if all its values are lost on both sides; a sum of less than 2^12 per block (2^(exponent of the block), ordinary ones are 2^26) can be
+// off by more than 5e-7 on average, which is what the gathering kernels' sums are off by.  Ordinary sums are that small one in 30,000 times.
+constexpr float SMALL_SUM = 4096.f;
+constexpr int MOST_SMALL = 8;            // ... of the 32 x 16 sums that a warp writes at a time; a lost row makes 16, a lost column 32
+// The same of a parameter gradient's sum of n products, beside sqrt(n): 2^25 ordinary, off by 2^-12 on average if all values are lost.  Sums of
+// mostly zeros are small without that: only those count one of whose channels has a WIDE range, shares of it (a warp's of channel_max_kernel)
+// being below 2^-16 of its largest.
+constexpr float SMALL_GRAD = 512.f;
+constexpr int WIDE = 16, MOST_SMALL_GRADS = 2;             // threads of a block of 32 x 4 to 32 gradients
 
 
 // A pass is a few kernels, each launched while the one before still runs; it waits for it (pdl_wait) before it reads or writes.  What an
@@ -64,7 +82,8 @@ constexpr int SCALED_MAX = 14;           // the largest value of a group lies in
 
 // ---- exponents ----------------------------------------------------------------------------------------------------------------
 // Exponent of a group from the bits of its largest finite magnitude; 2^(SCALED_MAX - e) is a normal number.
-__device__ __forceinline__ int group_exp(uint32_t max_bits) { return max((int)(max_bits >> 23) - 127, -112); }
+constexpr int ZERO_EXP = -112;           // of zeros, or the next thing to them
+__device__ __forceinline__ int group_exp(uint32_t max_bits) { return max((int)(max_bits >> 23) - 127, ZERO_EXP); }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }      // -126 <= e <= 127
 // s * 2^e, |e| <= 252, in two steps that neither overflow nor lose bits unless the result does
 __device__ __forceinline__ float scale_by(float s, int e)
@@ -81,6 +100,31 @@ __device__ __forceinline__ void parts(float v, float s, __half &hi, __half &lo)
     hi = __float2half_rn(t);
     lo = finite(v) ? __float2half_rn(t - __half2float(hi)) : __float2half_rn(0.f);
 }
+
+// Row windows: an image has zeros around it or in it, whose sums are small without loss.  Here the values are looked at: 32 consecutive ones of a
+// row and channel that are lost, fewer than 19 bits left, beside the row's largest; most of a row; a quarter of a filter.  Fewer than four of 32 are
+// chance.
+__device__ __forceinline__ bool is_lost(float v, float s) { return fabsf(v * s) < 0x1p-5f && v != 0.f; }
+struct Lost {
+    uint32_t values = 0, lost = 0;
+    __device__ __forceinline__ void take(float v, float s)
+    {
+        values += v != 0.f;
+        lost += is_lost(v, s);
+    }
+    // One in `share` of all threads' values of a block of 256, by all of them.
+    __device__ __forceinline__ bool too_many(uint32_t share) const
+    {
+        __shared__ uint32_t sums[2][8];
+        const uint32_t v = __reduce_add_sync(0xffffffffu, values), l = __reduce_add_sync(0xffffffffu, lost);
+        if ((threadIdx.x & 31) == 0) { sums[0][threadIdx.x >> 5] = v; sums[1][threadIdx.x >> 5] = l; }
+        __syncthreads();
+        uint32_t all = 0, n = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { all += sums[0][i]; n += sums[1][i]; }
+        return n > 1 && n * share > all;
+    }
+};
 
 // ---- splitting --------------------------------------------------------------------------------------------------------------------
 constexpr int TILE_PITCH = 65, TILE_VALUES = GROUP * TILE_PITCH;          // shared memory of a splitting block, in fp32 values
@@ -114,9 +158,13 @@ struct PrepParams {
     int win_C, win_kW;           // Window's: value (row, kw * C + c, th) at row * w_row + c * w_c + th * kW + kw; 0: none
     int *tickets;
     int n_tickets;
+    int *gate;                   // zero for the matrix kernel to set; weight gradient: it is zero already
+    uint8_t *wide;               // row windows: per block, whether values were lost
 };
 
-__device__ __forceinline__ void prep_weights(const PrepParams &p, int row, float *tile)
+// COUNT: returns whether values were lost.
+template <bool COUNT>
+__device__ __forceinline__ bool prep_weights(const PrepParams &p, int row, float *tile)
 {
     __shared__ uint32_t red[8];
     const float *w = p.w + (long long)row * p.w_row;
@@ -139,6 +187,7 @@ __device__ __forceinline__ void prep_weights(const PrepParams &p, int row, float
     if (threadIdx.x == 0) p.w_exp[row] = e;
     const float s = pow2(SCALED_MAX - e);
     const size_t part = (size_t)p.taps * p.rows * p.w_Cp;
+    Lost filter;
 #pragma unroll 4
     for (int i = threadIdx.x; i < p.w_Cp * p.taps; i += 256) {
         const int t = i / p.w_Cp, c = i - t * p.w_Cp;
@@ -152,7 +201,9 @@ __device__ __forceinline__ void prep_weights(const PrepParams &p, int row, float
         __half *d = p.w_dst + ((size_t)t * p.rows + row) * p.w_Cp + c;
         d[0] = hi;
         d[part] = lo;
+        if (COUNT) filter.take(v, s);
     }
+    return COUNT && filter.too_many(4);
 }
 
 // One block: 64 pixels (of the flat pixel sequence) x 64 channels, through shared memory: read along the pixels, written along the
@@ -240,10 +291,10 @@ __device__ __forceinline__ void prep_act(const Act &a, int block, float *tile_)
 }
 
 // Row windows: a block takes up to four rows of the images.  A row's values are split once, into shared memory in pixel-major order; a
-// window is a run of them.  (Split where they are written, 3.5 times each for 7x7 stride 2, 32 x 3 x 224 x 224 took 59 us; with a block
+// window is a run of them.  Returns whether values were lost (PER_CHANNEL: false).  (Split where they are written, 3.5 times each for 7x7 stride 2, 32 x 3 x 224 x 224 took 59 us; with a block
 // per row 45.)  One exponent per row.
 template <bool PER_CHANNEL>
-__device__ __forceinline__ void prep_window(const Act &a, int block, float *tile)
+__device__ __forceinline__ bool prep_window(const Act &a, int block, float *tile)
 {
     __shared__ uint32_t red[8];
     const Window &w = a.win;
@@ -270,16 +321,36 @@ __device__ __forceinline__ void prep_window(const Act &a, int block, float *tile
         if (ok)
             for (int i = tid; i < w.oW; i += T) a.exps[(size_t)row * w.oW + i] = (int8_t)e;
     }
+    bool some = false, wide = false;
     for (int c = 0; c < w.C; ++c) {
         if (PER_CHANNEL) s = pow2(SCALED_MAX - group_exp(a.chmax[c]));
 #pragma unroll 4
         for (int i = tid; i < cols; i += T) {
             const int at = i - w.padW;
-            parts((unsigned)at < (unsigned)w.W ? __ldg(src + c * plane + at) : 0.f, s, hi[i * w.C + c], lo[i * w.C + c]);
+            const float v = (unsigned)at < (unsigned)w.W ? __ldg(src + c * plane + at) : 0.f;
+            parts(v, s, hi[i * w.C + c], lo[i * w.C + c]);
+            if (!PER_CHANNEL) some |= is_lost(v, s);
         }
     }
-    __syncthreads();
-    if (!ok) return;
+    if (PER_CHANNEL) {
+        __syncthreads();
+    } else if (__syncthreads_or(some)) {
+        Lost rows;
+#pragma unroll 1
+        for (int c = 0; ok && c < w.C; ++c) {
+#pragma unroll 1
+            for (int i0 = tid & ~31; i0 < w.W; i0 += T) {                  // T is a multiple of 32
+                const int i = i0 + (tid & 31);
+                const float v = i < w.W ? __ldg(src + c * plane + i) : 0.f;
+                const uint32_t values = __ballot_sync(0xffffffffu, v != 0.f), kept = __ballot_sync(0xffffffffu, v != 0.f && !is_lost(v, s));
+                wide |= __popc(values) >= 4 && !kept;
+                rows.take(v, s);
+            }
+        }
+        wide = __syncthreads_or(wide);
+        wide |= rows.too_many(8);                                          // most of one row of four
+    }
+    if (!ok) return wide;
     // 16-byte pieces of the windows; those past a window's last value are zeros
     const int pieces = a.Cp / 8, step = w.dW * w.C;
     const size_t part = (size_t)a.pixels * a.Cp;
@@ -296,6 +367,7 @@ __device__ __forceinline__ void prep_window(const Act &a, int block, float *tile
         *reinterpret_cast<uint4 *>(dst + (size_t)i * 8) = *reinterpret_cast<const uint4 *>(ph);
         *reinterpret_cast<uint4 *>(dst + part + (size_t)i * 8) = *reinterpret_cast<const uint4 *>(pl);
     }
+    return wide;
 }
 
 // WINDOW: the last tensor is one of row windows.
@@ -307,25 +379,29 @@ prep_kernel(const __grid_constant__ PrepParams p)
     pdl_wait();
     pdl_launch_dependents();
     int b = (int)blockIdx.x;
-    if (b == 0)
+    if (!PER_CHANNEL && b == 0) {
         for (int i = threadIdx.x; i < p.n_tickets; i += 256) p.tickets[i] = 0;
-    if (b < p.rows) {
-        prep_weights(p, b, tile);
-        return;
+        if (threadIdx.x == 0) *p.gate = 0;
     }
-    b -= p.rows;
-    const Act &act = p.act[PER_CHANNEL && b >= p.act[0].ctas ? 1 : 0];
-    if (PER_CHANNEL && b >= p.act[0].ctas) b -= p.act[0].ctas;
-    if (WINDOW && act.win.C) prep_window<PER_CHANNEL>(act, b, tile);
-    else prep_act<PER_CHANNEL>(act, b, tile);
+    bool wide = false;
+    if (b < p.rows) {
+        wide = prep_weights<WINDOW>(p, b, tile);
+    } else {
+        b -= p.rows;
+        const Act &act = p.act[PER_CHANNEL && b >= p.act[0].ctas ? 1 : 0];
+        if (PER_CHANNEL && b >= p.act[0].ctas) b -= p.act[0].ctas;
+        if (WINDOW && act.win.C) wide = prep_window<PER_CHANNEL>(act, b, tile);
+        else prep_act<PER_CHANNEL>(act, b, tile);
+    }
+    if (WINDOW && !PER_CHANNEL && threadIdx.x == 0) p.wide[blockIdx.x] = wide;
 }
 
-// Largest finite magnitude of every channel, and the sums of the first tensor's channels (the bias gradient): block = (channel, chunk of
+// Largest finite magnitude of every channel and the smallest of its shares' largest, and the sums of the first tensor's channels (the bias gradient): block = (channel, chunk of
 // the channel's pieces), a warp per piece of a plane.
 constexpr int PIECE = 2048;              // values of a plane that a warp takes, at most
 struct MaxParams {
     const float *src[2];
-    uint32_t *chmax[2];
+    uint32_t *chmax[2], *chlow[2];                               // chlow: the complement of the smallest share's largest, 0: no share has values
     double *sums;                                                // [chunks][C] of the first tensor, or null
     int C[2], HW[2], pieces[2], chunks[2], vec[2], images;       // pieces of a plane; vec: planes of a multiple of four values, 16-byte aligned
 };
@@ -384,6 +460,7 @@ channel_max_kernel(const __grid_constant__ MaxParams p)
     }
     uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
     if (lane == 0) red[warp] = bits;
+    uint32_t low = bits ? ~bits : 0u;                                      // a warp's share of the channel
     if (add) {
         sum = warp_sum(sum);
         if (lane == 0) part[warp] = sum;
@@ -391,8 +468,12 @@ channel_max_kernel(const __grid_constant__ MaxParams p)
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int i = 1; i < 8; ++i) bits = max(bits, red[i]);
+        for (int i = 1; i < 8; ++i) {
+            bits = max(bits, red[i]);
+            low = max(low, red[i] ? ~red[i] : 0u);
+        }
         atomicMax(p.chmax[t] + c, bits);
+        atomicMax(p.chlow[t] + c, low);
         if (add) {
 #pragma unroll
             for (int i = 1; i < 8; ++i) sum += part[i];
@@ -417,7 +498,9 @@ struct Params {
     const int *w_exp;                        // ... per column
     const float *bias;                       // or null
     float *out, *partial;
-    int *tickets, *status;
+    int *tickets, *status, *gate;
+    const uint8_t *wide;                     // row windows: the splitting blocks' verdicts
+    int n_wide;                              // ... and their number; otherwise the sums are looked at
     const float *raw_a, *raw_w;              // the operands in fp32, for sums that came out as NaN; null: left as they are
     int images, g_C, g_H, g_W, groups;
     int w_kk, o_HW, N_total, n_tiles, width; // columns in all, column tiles and a tile's columns
@@ -581,9 +664,10 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
     return d;
 }
 template <int N>
-__device__ __forceinline__ void raise(uint64_t (&acc2)[N], int &top, int to)
+__device__ __forceinline__ void raise(uint64_t (&acc2)[N], float &blocks, int &top, int to)
 {
     const float f = step(top, to);
+    blocks *= f;
     const uint64_t f2 = pack2(f, f);
 #pragma unroll
     for (int j = 0; j < N; ++j) acc2[j] = mul2(acc2[j], f2);
@@ -605,7 +689,7 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
     constexpr bool ALT = !WG && BN <= 128;
     constexpr int HALF_COLS = ALT ? BN : BN / 2, SETS = ALT ? 2 : 1, BUFS = 512 / BN / SETS;      // TMEM buffers per set
     constexpr int RING = NS / SETS;                                                                // stages per set
-    constexpr size_t PART = BN * BM + BM;             // partial sums of a cut tile and their rows' exponents
+    constexpr size_t PART = BN * BM + 2 * BM;         // partial sums of a cut tile, their rows' exponents and sizes of blocks
 
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t full[NS], empty[NS];          // stage landed; its MMAs are done
@@ -770,6 +854,12 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
         int buf = 0;
         uint32_t parity = 0;
         bool ok = true, nan_seen = false, tail_done = false;
+        if (!WG && p.n_wide) {
+            // this CTA's share of the verdicts, while the first block is on its way
+            bool wide = false;
+            for (int i = (int)blockIdx.x * (EPI_WARPS * 32) + tid; i < p.n_wide; i += (int)gridDim.x * (EPI_WARPS * 32)) wide |= p.wide[i] != 0;
+            if (wide) *p.gate = 1;
+        }
         // this lane's pixel of a tile
         auto locate = [&](const Item &it, const Phase &f, int &im, int &row, int &col) {
             const int m = it.m_tile * BM + row_in;
@@ -800,6 +890,7 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                            ? (int)p.exps[(((size_t)im * p.g_H + ih) * p.g_W + iw) * p.groups + g] : NO_EXP;
             };
             int next = WG ? 0 : exp_at(), top = NO_EXP;
+            float blocks = 0.f;                                                    // the sum of the blocks' 2^(e - top)
             for (int q = it.begin; q < it.end; ++q) {
                 const int e = next;
                 if (!WG && q + 1 < it.end) {
@@ -808,8 +899,9 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                 }
                 float s = 1.f;
                 if (!WG) {
-                    if (__any_sync(0xffffffffu, e > top)) raise(acc2, top, max(e + 4, top));
+                    if (__any_sync(0xffffffffu, e > top)) raise(acc2, blocks, top, max(e + 4, top));
                     s = step(e, top);
+                    if (e > ZERO_EXP) blocks += s;
                 }
                 if (!mbar_wait(smem_u32(my_ready + buf), parity, p.status)) { ok = false; break; }
                 tc_fence_after();
@@ -851,7 +943,10 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
             if (it.tail >= 0) {
                 float *mine = p.partial + (size_t)(it.tail * p.splits + it.part) * PART + (size_t)col0 * BM + row_in;
                 int *my_top = reinterpret_cast<int *>(p.partial + (size_t)(it.tail * p.splits + it.part) * PART + BN * BM) + row_in;
-                if (ALT || half == 0) __stcg(my_top, top);
+                if (ALT || half == 0) {
+                    __stcg(my_top, top);
+                    __stcg(reinterpret_cast<float *>(my_top + BM), blocks);
+                }
 #pragma unroll
                 for (int j = 0; j < HALF_COLS; ++j) __stcg(mine + j * BM, acc[j]);
                 __threadfence();
@@ -863,12 +958,14 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                 const float *first = p.partial + (size_t)it.tail * p.splits * PART + row_in;
                 auto top_of = [&](int s) { return __ldcg(reinterpret_cast<const int *>(first + (size_t)s * PART + BN * BM)); };
                 top = NO_EXP;
+                blocks = 0.f;
                 for (int s = 0; s < p.splits; ++s) top = max(top, top_of(s));
 #pragma unroll
                 for (int j = 0; j < HALF_COLS; ++j) acc[j] = 0.f;
 #pragma unroll 1
                 for (int s = 0; s < p.splits; ++s) {
                     const float w = step(top_of(s), top);
+                    blocks = fmaf(__ldcg(first + (size_t)s * PART + BN * BM + BM), w, blocks);
                     const float *src = first + (size_t)s * PART + (size_t)col0 * BM;
 #pragma unroll
                     for (int j = 0; j < HALF_COLS; ++j) acc[j] = fmaf(__ldcg(src + j * BM), w, acc[j]);
@@ -879,7 +976,7 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
             // tile, it is fetched from memory and took 20 us of a layer.  2^(row + column exponent) goes on in two halves, see scale_by;
             // a lane fetches a column's halves and bias for all (from memory in the loop: 160 clocks a column; by shuffles 90).
             const int n0 = it.n_tile * p.width + col0, he = (top - 2 * SCALED_MAX) / 2;
-            const float ra = pow2(he), rb = pow2(top - 2 * SCALED_MAX - he);
+            const float ra = pow2(he), rb = pow2(top - 2 * SCALED_MAX - he), small_sum = p.n_wide ? 0.f : blocks * SMALL_SUM;
             float *dst = p.out + ((size_t)im * p.N_total + n0) * p.o_HW + (f.o_off + row * f.o_sH + col * f.o_sW);
             float *stage = reinterpret_cast<float *>(smem + RING_BYTES + warp * STORE_BYTES) + lane;        // a lane reads what it wrote itself
             float4 *column = reinterpret_cast<float4 *>(smem + RING_BYTES + warp * STORE_BYTES + STORE_COLS * 128);
@@ -890,12 +987,14 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
                 __syncwarp();
                 if (lane < STORE_COLS) {
                     const int ec = lane < last ? p.w_exp[n0 + c + lane] : 0, hc = ec / 2;
-                    column[lane] = make_float4(pow2(hc), pow2(ec - hc), p.bias && lane < last ? __ldg(p.bias + n0 + c + lane) : 0.f, 0.f);
+                    // a filter of zeros loses nothing
+                    column[lane] = make_float4(pow2(hc), pow2(ec - hc), p.bias && lane < last ? __ldg(p.bias + n0 + c + lane) : 0.f, ec > ZERO_EXP ? 1.f : 0.f);
                 }
 #pragma unroll
                 for (int j = 0; j < STORE_COLS; ++j) stage[j * 32] = acc[c + j];
                 __syncwarp();
                 const int count = row_ok ? last : 0;
+                int small = 0;
                 float *to = dst + (size_t)c * p.o_HW;
 #pragma unroll 1
                 for (int j = 0; j < last; j += 8) {                // eight columns in step: one after the other they take 130 clocks each
@@ -906,12 +1005,14 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         nan_seen |= v[i] != v[i];
+                        small += fabsf(v[i]) < small_sum * k[i].w && j + i < count;
                         v[i] = v[i] * (ra * k[i].x) * (rb * k[i].y) + k[i].z;
                     }
 #pragma unroll
                     for (int i = 0; i < 8; ++i, to += p.o_HW)
                         if (j + i < count) *to = v[i];
                 }
+                if (__reduce_add_sync(0xffffffffu, (unsigned)small) > MOST_SMALL && lane == 0) *p.gate = 1;
             }
         }
         if (!WG && p.raw_a && __any_sync(0xffffffffu, ok && nan_seen)) {          // rows past the last may have seen some: they write nothing
@@ -938,18 +1039,21 @@ split_gemm_kernel(const __grid_constant__ Params p, const __grid_constant__ Maps
     if (warp == 0) tmem_dealloc(tmem_base, 512);
 }
 
-// gw[ko][c][tap] += scale * the sum of the splits in their order, scaled back; further blocks: the bias gradient from its partial sums.
-// Partial sums are contiguous along the output channels, gw along (c, tap).
+// The sum of the splits of gw[ko][c][tap] in their order, scaled back, to `sums`; further blocks: the bias gradient from its partial sums.
+// Partial sums are contiguous along the output channels, the sums along (c, tap).  They are added to the gradient by the next kernel, which
+// knows all blocks' verdicts.
 struct ReduceParams {
     const float *partial;
-    float *gw, *gb;
-    const uint32_t *gy_max, *x_max;
+    float *sums, *gb;
+    int *gate;
+    const uint32_t *gy_max, *x_max, *gy_low, *x_low;
     const double *bias_part;
     int K, C, kk, groups, bg, splits, cols, rows, gw_blocks, bias_blocks;
     int shares;                              // warps that share an output's splits: 1, 2, 4 or 8
     int win_kW;                              // Window's kernel columns, or 0
-    float scale;
+    float scale, small_sum;                  // SMALL_GRAD of all products
 };
+__device__ __forceinline__ bool wide_range(uint32_t most, uint32_t low) { return low && (int)(most >> 23) - (int)(~low >> 23) > WIDE; }
 __global__ void __launch_bounds__(256)
 reduce_kernel(const __grid_constant__ ReduceParams p)
 {
@@ -997,13 +1101,19 @@ reduce_kernel(const __grid_constant__ ReduceParams p)
 #pragma unroll
     for (int i = 0; i < 4; ++i) tile[warp][i][lane] = scale_by(sum[i], eg + group_exp(p.x_max[c[i]]) - 2 * SCALED_MAX);
     __syncthreads();
+    bool small = false;
     for (int i = tid; i < 32 * per; i += 256) {
-        const int k = i / per, o = i - k * per;
-        if (kb * 32 + k >= p.K || ob * per + o >= n) continue;
+        const int k = i / per, o = i - k * per, row = kb * 32 + k, col = ob * per + o;
+        if (row >= p.K || col >= n) continue;
         float s = 0.f;
         for (int j = 0; j < p.shares; ++j) s += tile[(o >> 2) * p.shares + j][o & 3][k];
-        p.gw[(size_t)(kb * 32 + k) * n + ob * per + o] += p.scale * s;
+        p.sums[(size_t)row * n + col] = s;
+        const int ch = col / p.kk;
+        const uint32_t gm = p.gy_max[row], xm = p.x_max[ch];
+        if (gm && xm && (wide_range(gm, p.gy_low[row]) || wide_range(xm, p.x_low[ch])))
+            small |= fabsf(s) < scale_by(p.small_sum, group_exp(gm) + group_exp(xm) - 2 * SCALED_MAX);
     }
+    if (__syncthreads_count(small) > MOST_SMALL_GRADS && tid == 0) *p.gate = 1;
 }
 
 // ---- host ---------------------------------------------------------------------------------------------------------------------------
@@ -1126,9 +1236,9 @@ struct Plan {
     Params p;
     Window win;
     Walk wh[MAX_PHASES], ww[MAX_PHASES];
-    int images, Cp, bn;                    // images per round, channels of the gathered tensor padded to 8, column tile of the kernel
+    int images, Cp, bn;                    // images per round, padded() channels of the gathered tensor, column tile of the kernel
     int rows, taps;                        // weight rows (columns of the product) and taps
-    size_t off_w, off_exps, off_exp, off_tickets, off_partial, bytes;
+    size_t off_w, off_exps, off_exp, off_tickets, off_partial, off_gate, off_wide, bytes;
 };
 
 // The tiles of `images` images: their number, which of them are cut, and into how many parts.
@@ -1173,7 +1283,9 @@ static bool finish_plan(Plan &pl, int N, int gC, int gH, int gW, int columns, in
     pl.off_exps = at; at += round256((size_t)pl.images * gH * gW * p.groups);
     pl.off_exp = at; at += round256((size_t)columns * 4);
     pl.off_tickets = at; at += round256((size_t)sm_count() * 4);
-    pl.off_partial = at; at += round256((size_t)sm_count() * (pl.bn + 1) * BM * 4);
+    pl.off_partial = at; at += round256((size_t)sm_count() * (pl.bn + 2) * BM * 4);
+    pl.off_gate = at; at += 256;
+    if (pl.win.C) { pl.off_wide = at; at += round256((size_t)columns + (size_t)pl.images * gH); }         // a block has a row or more
     pl.bytes = at + 256;
     return true;
 }
@@ -1309,13 +1421,14 @@ static bool plan_grad_input(Plan &pl, const Geometry &g)
 
 // src: the gathered tensor; weights of (row, channel, tap) at row * w_row + channel * w_c + tap.
 static int run_plan(Plan &pl, int N, const float *src, const float *weight, long long w_row, long long w_c, const float *bias, float *out, bool redo_nan,
-                    void *scratch, cudaStream_t stream)
+                    const Fallback &again, void *scratch, cudaStream_t stream)
 {
     Params &p = pl.p;
     char *ws = (char *)scratch;
     __half *a = (__half *)ws, *w = (__half *)(ws + pl.off_w);
     p.exps = (const int8_t *)(ws + pl.off_exps); p.w_exp = (int *)(ws + pl.off_exp); p.tickets = (int *)(ws + pl.off_tickets);
     p.partial = (float *)(ws + pl.off_partial); p.bias = bias; p.status = device_status_ptr();
+    p.gate = (int *)(ws + pl.off_gate); p.wide = (const uint8_t *)(ws + pl.off_wide);
     const int g_HW = p.g_H * p.g_W;
     alignas(64) Maps maps;
     if (map_3d(&maps.b, w, pl.Cp, pl.rows, 2 * pl.taps, BK, pl.bn, CU_TENSOR_MAP_SWIZZLE_64B)) return 1;
@@ -1336,11 +1449,15 @@ static int run_plan(Plan &pl, int N, const float *src, const float *weight, long
         act.win = pl.win;
         q.w = weight; q.w_dst = w; q.w_exp = const_cast<int *>(p.w_exp); q.rows = at ? 0 : pl.rows; q.w_C = p.g_C; q.w_Cp = pl.Cp; q.taps = pl.taps;
         q.w_row = w_row; q.w_c = w_c; q.win_C = pl.win.C; q.win_kW = pl.win.kW; q.tickets = p.tickets; q.n_tickets = sm_count();
-        if (launch("convolution operand split", pl.win.C ? (const void *)prep_kernel<false, true> : (const void *)prep_kernel<false, false>, prep_grid(q, 1), 256, 0, stream, false, q)) return 1;
+        q.gate = p.gate; q.wide = const_cast<uint8_t *>(p.wide) + (at ? pl.rows : 0);        // the weights' verdicts count for all rounds
+        const int blocks = prep_grid(q, 1);
+        p.n_wide = pl.win.C ? pl.rows + act.ctas : 0;
+        if (launch("convolution operand split", pl.win.C ? (const void *)prep_kernel<false, true> : (const void *)prep_kernel<false, false>, blocks, 256, 0, stream, true, q)) return 1;
         const void *kern = pl.bn == 64    ? (const void *)split_gemm_kernel<64, false>
                            : pl.bn == 128 ? (const void *)split_gemm_kernel<128, false>
                                           : (const void *)split_gemm_kernel<256, false>;
         if (launch("convolution of split operands", kern, std::min(p.items, sm_count()), THREADS, SMEM, stream, true, p, maps)) return 1;
+        if (again(at, n, p.gate)) return 1;
     }
     return 0;
 }
@@ -1355,19 +1472,21 @@ size_t grad_input_scratch(const Geometry &g)
     Plan pl;
     return plan_grad_input(pl, g) ? pl.bytes : 0;
 }
-int forward(const Geometry &g, const float *x, const float *weight, const float *bias, float *y, void *scratch, cudaStream_t stream)
+int forward(const Geometry &g, const float *x, const float *weight, const float *bias, float *y, const Fallback &again, void *scratch,
+            cudaStream_t stream)
 {
     Plan pl;
     if (!plan_forward(pl, g)) return fail("convolution forward: no plan for split operands");
     const int kk = g.kH * g.kW;
-    return run_plan(pl, g.N, x, weight, (long long)g.C * kk, kk, bias, y, false, scratch, stream);
+    return run_plan(pl, g.N, x, weight, (long long)g.C * kk, kk, bias, y, false, again, scratch, stream);
 }
-int grad_input(const Geometry &g, const float *gy, const float *weight, const float *bias, float *gx, void *scratch, cudaStream_t stream)
+int grad_input(const Geometry &g, const float *gy, const float *weight, const float *bias, float *gx, const Fallback &again, void *scratch,
+               cudaStream_t stream)
 {
     Plan pl;
     if (!plan_grad_input(pl, g)) return fail("convolution input gradient: no plan for split operands");
     const int kk = g.kH * g.kW;
-    return run_plan(pl, g.N, gy, weight, kk, (long long)g.C * kk, bias, gx, g.dH > 1 || g.dW > 1, scratch, stream);
+    return run_plan(pl, g.N, gy, weight, kk, (long long)g.C * kk, bias, gx, g.dH > 1 || g.dW > 1, again, scratch, stream);
 }
 
 // ---- weight gradients ---------------------------------------------------------------------------------------------------------------
@@ -1377,7 +1496,7 @@ struct WgradPlan {
     Geometry v;                                // the convolution, on row windows where the channels are few
     Walk wh, ww;
     int images, Cp, Kp, bn, bg;
-    size_t off_gy, off_max, off_bias, off_partial, bytes;
+    size_t off_x, off_gy, off_bias, off_partial, bytes;
 };
 static void plan_splits(WgradPlan &pl, int images)
 {
@@ -1445,29 +1564,37 @@ static bool plan_grad_weight(WgradPlan &pl, const Geometry &whole)
     if (pl.images * x_bytes < MIN_MAP_BYTES) return false;
     plan_splits(pl, pl.images);
     if (!grad_weight_is_faster(pl, whole)) return false;
-    size_t at = round256(pl.images * x_bytes);
+    size_t at = grad_weight_head(whole);
+    pl.off_x = at; at += round256(pl.images * x_bytes);
     pl.off_gy = at; at += round256(pl.images * gy_bytes);
-    pl.off_max = at; at += round256((size_t)(whole.C + g.K) * 4);
     pl.off_bias = at; at += round256((size_t)ceil_div_ll((long long)pl.images * ceil_div(p.pix_HW, PIECE), 8) * g.K * 8);
     // a round of fewer images may be cut into a few more parts than a whole one
     pl.off_partial = at; at += round256((size_t)(p.splits + 1) * p.n_tiles * pl.bn * p.m_tiles * BM * 4);
     pl.bytes = at + 256;
     return true;
 }
-size_t grad_weight_scratch(const Geometry &g)
+size_t grad_weight_scratch(const Geometry &g, size_t (*again_bytes)(const Geometry &))
 {
     WgradPlan pl;
-    return plan_grad_weight(pl, g) ? pl.bytes : 0;
+    if (!plan_grad_weight(pl, g)) return 0;
+    size_t bytes = pl.bytes;
+    Geometry round = g;
+    for (int images : {pl.images, (g.N - 1) % pl.images + 1}) {
+        round.N = images;
+        bytes = std::max(bytes, grad_weight_head(g) + again_bytes(round));
+    }
+    return bytes;
 }
-int grad_weight(const Geometry &g, const float *x, const float *gy, float *grad_weight, float *grad_bias, float scale, void *scratch,
+int grad_weight(const Geometry &g, const float *x, const float *gy, float *grad_bias, float scale, const Fallback &again, void *scratch,
                 cudaStream_t stream)
 {
     WgradPlan pl;
     if (!plan_grad_weight(pl, g)) return fail("convolution parameter gradient: no plan for split operands");
     Params &p = pl.p;
     char *ws = (char *)scratch;
-    __half *xs = (__half *)ws, *gs = (__half *)(ws + pl.off_gy);
-    uint32_t *gy_max = (uint32_t *)(ws + pl.off_max), *x_max = gy_max + g.K;
+    p.gate = (int *)ws;
+    __half *xs = (__half *)(ws + pl.off_x), *gs = (__half *)(ws + pl.off_gy);
+    uint32_t *gy_max = (uint32_t *)(ws + GATE_BYTES), *x_max = gy_max + g.K, *gy_low = x_max + g.C, *x_low = gy_low + g.K;
     double *bias_part = (double *)(ws + pl.off_bias);
     p.partial = (float *)(ws + pl.off_partial);
     p.status = device_status_ptr();
@@ -1481,9 +1608,9 @@ int grad_weight(const Geometry &g, const float *x, const float *gy, float *grad_
         alignas(64) Maps maps;
         if (map_3d(&maps.a[0], gs, pl.Kp, (long long)n * p.pix_HW, 2, GROUP, BK, CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
         if (map_im2col(&maps.b, xs, pl.Cp, 2 * n, pl.wh, pl.ww, pl.bg, BK, pl.bg == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B)) return 1;
-        CUNN_CUDA(cudaMemsetAsync(gy_max, 0, (size_t)(g.C + g.K) * 4, stream));
+        CUNN_CUDA(cudaMemsetAsync(ws, 0, GATE_BYTES + max_bytes(g), stream));
         MaxParams m{};
-        m.src[0] = gr; m.src[1] = xr; m.chmax[0] = gy_max; m.chmax[1] = x_max; m.C[0] = g.K; m.C[1] = g.C; m.HW[0] = p.pix_HW; m.HW[1] = x_HW;
+        m.src[0] = gr; m.src[1] = xr; m.chmax[0] = gy_max; m.chmax[1] = x_max; m.chlow[0] = gy_low; m.chlow[1] = x_low; m.C[0] = g.K; m.C[1] = g.C; m.HW[0] = p.pix_HW; m.HW[1] = x_HW;
         m.images = n;
         m.sums = grad_bias ? bias_part : nullptr;
         for (int t = 0; t < 2; ++t) {
@@ -1502,14 +1629,15 @@ int grad_weight(const Geometry &g, const float *x, const float *gy, float *grad_
             if (t) act.win = pl.win;
             act.vec = can_vec(act.src, act.HW);
             act.pixels = (uint32_t)n * act.HW;
-            }
+        }
         if (launch("convolution operand split", pl.win.C ? (const void *)prep_kernel<true, true> : (const void *)prep_kernel<true, false>, prep_grid(q, 2), 256, 0, stream, true, q)) return 1;
         const void *kern = pl.bg == 32    ? pl.bn == 128 ? (const void *)split_gemm_kernel<128, true, 32> : (const void *)split_gemm_kernel<256, true, 32>
                            : pl.bn == 128 ? (const void *)split_gemm_kernel<128, true>
                                           : (const void *)split_gemm_kernel<256, true>;
         if (launch("convolution parameter gradient of split operands", kern, std::min(p.items, sm_count()), THREADS, SMEM, stream, true, p, maps)) return 1;
         ReduceParams r{};
-        r.partial = p.partial; r.gw = grad_weight; r.gb = grad_bias; r.gy_max = gy_max; r.x_max = x_max; r.bias_part = bias_part;
+        r.partial = p.partial; r.sums = grad_weight_sums(g, scratch); r.gate = p.gate; r.gb = grad_bias; r.gy_max = gy_max; r.x_max = x_max; r.gy_low = gy_low;
+        r.x_low = x_low; r.bias_part = bias_part; r.small_sum = SMALL_GRAD * std::sqrt((float)n * (float)p.pix_HW);
         r.K = g.K; r.C = g.C; r.kk = kk; r.groups = p.groups; r.bg = pl.bg; r.win_kW = pl.win.kW; r.splits = p.splits; r.cols = p.n_tiles * pl.bn; r.rows = p.m_tiles * BM;
         // one warp per output leaves SMs idle where the outputs are few: 9,408 outputs of 146 splits took 36 us
         r.shares = 1;
@@ -1519,6 +1647,7 @@ int grad_weight(const Geometry &g, const float *x, const float *gy, float *grad_
         r.scale = scale;
         if (launch("convolution parameter gradient sums", (const void *)reduce_kernel, r.gw_blocks + (grad_bias ? ceil_div(g.K, 8) : 0), 256, 0, stream,
                    true, r)) return 1;
+        if (again(at, n, p.gate)) return 1;
     }
     return 0;
 }

@@ -52,6 +52,7 @@ struct GemmParams {
     const float *bias;    // FWD only, may be null
     float *out;           // FWD: y; DGRAD: gx; WGRAD: partial sums [splits][M_total][N_total]
     int *status;
+    const int *gate;      // null, or see gated_off
     // geometry of the gathered image operand (FWD: x; DGRAD: gy; WGRAD: x)
     int g_C, g_H, g_W;            // channels, rows, cols of that tensor
     int g_padH, g_padW, g_dH, g_dW;
@@ -156,6 +157,7 @@ template <int OP, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 conv_gemm_kernel(const GemmParams p)
 {
+    if (gated_off(p.gate)) return;
     constexpr int A_TILE = BM * BK * 4;             // bytes of one hi (or lo) A tile
     constexpr int B_TILE = BN * BK * 4;
     constexpr int STAGE = 2 * (A_TILE + B_TILE);
@@ -415,10 +417,20 @@ conv_gemm_kernel(const GemmParams p)
     if (warp == 0) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
+// The end of a parameter gradient that may have been done already (conv_split.h): adds those sums where the gate says so.
+__device__ __forceinline__ bool add_sums(const int *gate, const float *sums, float *gw, long long n, float scale)
+{
+    if (!gated_off(gate)) return false;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) gw[i] = fmaf(scale, sums[i], gw[i]);
+    return true;
+}
+
 // gW[i] += scale * sum_s partial[s][i], in split order.
 __global__ void __launch_bounds__(256)
-wgrad_reduce_kernel(const float *__restrict__ partial, float *__restrict__ gw, long long n, int splits, float scale)
+wgrad_reduce_kernel(const float *__restrict__ partial, float *__restrict__ gw, long long n, int splits, float scale, const int *gate,
+                    const float *__restrict__ sums)
 {
+    if (add_sums(gate, sums, gw, n, scale)) return;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         float s = 0.f;
         for (int k = 0; k < splits; ++k) s += __ldg(partial + (size_t)k * n + i);
@@ -462,8 +474,9 @@ bias_finish_kernel(const float *__restrict__ part, float *__restrict__ gb, int K
 // gb[k] += scale * sum_j bias_part[k][j] for the K threads after them (bias_part may be null).
 __global__ void __launch_bounds__(256)
 wgrad_bias_reduce_kernel(const float *__restrict__ partial, float *__restrict__ gw, long long n, int splits, float scale,
-                         const float *__restrict__ bias_part, float *__restrict__ gb, int K)
+                         const float *__restrict__ bias_part, float *__restrict__ gb, int K, const int *gate, const float *__restrict__ sums)
 {
+    if (add_sums(gate, sums, gw, n, scale)) return;
     const long long total = n + (bias_part ? K : 0);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         if (i < n) {
@@ -482,8 +495,9 @@ wgrad_bias_reduce_kernel(const float *__restrict__ partial, float *__restrict__ 
 // The same for many splits: eight threads share an output, each adds every eighth split, and their sums are added in order.
 __global__ void __launch_bounds__(256)
 wgrad_bias_reduce_wide_kernel(const float *__restrict__ partial, float *__restrict__ gw, long long n, int splits, float scale,
-                              const float *__restrict__ bias_part, float *__restrict__ gb, int K)
+                              const float *__restrict__ bias_part, float *__restrict__ gb, int K, const int *gate, const float *__restrict__ sums)
 {
+    if (add_sums(gate, sums, gw, n, scale)) return;
     __shared__ float part_s[8][32];
     __shared__ double bias_s[8][32];
     const long long total = n + (bias_part ? K : 0);
@@ -520,8 +534,9 @@ wgrad_bias_reduce_wide_kernel(const float *__restrict__ partial, float *__restri
 
 // y[img][q][pix] += bias[q]: the bias of a transposed convolution, whose product comes out of the input-gradient kernels.
 __global__ void __launch_bounds__(256)
-add_plane_bias_kernel(float *__restrict__ y, const float *__restrict__ bias, int Q, int HW, long long total)
+add_plane_bias_kernel(float *__restrict__ y, const float *__restrict__ bias, int Q, int HW, long long total, const int *gate)
 {
+    if (gated_off(gate)) return;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
         y[i] += __ldg(bias + (int)((i / HW) % Q));
 }
@@ -565,6 +580,7 @@ struct Params {
     float *out;        // FWD: y; DGRAD: gx; WGRAD: partial sums [splits][M_total][N_total]
     float *bias_part;  // WGRAD: [M_total][splits] row sums of gy, or null
     int *status;
+    const int *gate;   // null, or see gated_off
     int HW;            // pixels per image plane
     int M_total, N_total, Kd;
     int n_tiles, tiles_per_split, total_tiles;   // tile = (split * m_tiles + m_tile) * n_tiles + n_tile
@@ -932,6 +948,7 @@ template <int OP, int BN, int KS, bool ROUND = false>
 __global__ void __launch_bounds__(THREADS, 1)
 pw_gemm_kernel(const Params p)
 {
+    if (gated_off(p.gate)) return;
     using BiasSum = typename std::conditional<ROUND, double, float>::type;
     constexpr bool A_MN = OP != OP_WGRAD;     // A is M-major (forward, input gradient)
     constexpr bool B_MN = OP == OP_DGRAD;     // B is N-major (input gradient)
@@ -1297,12 +1314,27 @@ static size_t smem_bytes(int bn)
 
 static int pick_bn_for(int n_total) { return n_total <= 32 ? 32 : (n_total <= 64 ? 64 : 128); }
 
+// With a gate (see gated_off) the launch does not wait for the kernel before.
+static cudaError_t launch_gated(const void *kern, dim3 grid, dim3 threads, void **args, size_t smem, cudaStream_t stream, const int *gate)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = threads;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = gate ? 1 : 0;
+    return cudaLaunchKernelExC(&cfg, kern, args);
+}
 static int launch(GemmKernel kern, const GemmParams &p, dim3 grid, int bn, cudaStream_t stream)
 {
     const size_t smem = smem_bytes(bn);
     CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void *args[] = {(void *)&p};
-    CUNN_CUDA(cudaLaunchKernel((const void *)kern, grid, dim3(THREADS), args, smem, stream));
+    CUNN_CUDA(launch_gated((const void *)kern, grid, dim3(THREADS), args, smem, stream, p.gate));
     return 0;
 }
 
@@ -1421,7 +1453,7 @@ static int pw_launch(PwKernel kern, pw::Params &p, cudaStream_t stream)
     const int grid = std::min(p.total_tiles, sm_count());
     CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pw::SMEM));
     void *args[] = {(void *)&p};
-    CUNN_CUDA(cudaLaunchKernel((const void *)kern, dim3(grid), dim3(pw::THREADS), args, pw::SMEM, stream));
+    CUNN_CUDA(launch_gated((const void *)kern, dim3(grid), dim3(pw::THREADS), args, pw::SMEM, stream, p.gate));
     return 0;
 }
 
@@ -1529,7 +1561,7 @@ static int pw_tma_launch(PwTmaKernel kern, pw::Params &p, CUtensorMap &ma, CUten
     const int threads = pwt::tma_threads(4, 8);          // every configuration has 14 warps
     CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
     void *args[] = {(void *)&p, (void *)&ma, (void *)&mb, (void *)&mo};
-    CUNN_CUDA(cudaLaunchKernel((const void *)kern, dim3(grid), dim3(threads), args, smem_bytes, stream));
+    CUNN_CUDA(launch_gated((const void *)kern, dim3(grid), dim3(threads), args, smem_bytes, stream, p.gate));
     return 0;
 }
 
@@ -1627,7 +1659,7 @@ static int launch_gather(pwg::GatherParams &p, int bn, cudaStream_t stream)
     const GatherKernel kern = gather_pick<OP>(bn);
     CUNN_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pwg::GSMEM));
     void *args[] = {(void *)&p};
-    CUNN_CUDA(cudaLaunchKernel((const void *)kern, dim3(std::min(p.total_tiles, sm_count())), dim3(pwg::GTHREADS), args, pwg::GSMEM, stream));
+    CUNN_CUDA(launch_gated((const void *)kern, dim3(std::min(p.total_tiles, sm_count())), dim3(pwg::GTHREADS), args, pwg::GSMEM, stream, p.gate));
     return 0;
 }
 
@@ -1687,7 +1719,8 @@ static bool fp32_residues_are_faster(int N, int C, int K, const std::vector<Axis
 // Input gradient of a convolution with any stride, padding and dilation, plus `bias` per input channel (null: none): the
 // forward pass of a transposed convolution has one.
 static int phased_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
-                             int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, int oH, int oW, cudaStream_t stream)
+                             int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, int oH, int oW, const int *gate,
+                             cudaStream_t stream)
 {
     bool gaps = false;
     std::vector<AxisPhase> ah = axis_phases(H, kH, dH, padH, dilH, false, &gaps), aw = axis_phases(W, kW, dW, padW, dilW, false, &gaps);
@@ -1711,7 +1744,7 @@ static int phased_grad_input(const float *gy, const float *weight, const float *
     }
     if (any_fma) {
         pwg::FmaParams q{};
-        q.gy = gy; q.w = weight; q.bias = bias; q.gx = gx;
+        q.gy = gy; q.w = weight; q.bias = bias; q.gx = gx; q.gate = gate;
         q.N = N; q.C = C; q.H = H; q.W = W; q.K = K; q.kW = kW; q.kk = kH * kW; q.dH = dH; q.dW = dW; q.oH = oH; q.oW = oW;
         q.only_short = !all_fma;
         const int rc = launch_phase_fma(q, ah, aw, stream);
@@ -1734,7 +1767,7 @@ static int phased_grad_input(const float *gy, const float *weight, const float *
     std::stable_sort(ph.begin(), ph.end(), [](const pwg::Phase &a, const pwg::Phase &b) { return a.taps > b.taps; });
     for (size_t at = 0; at < ph.size(); at += pwg::MAX_PHASES) {
         pwg::GatherParams q{};
-        q.a = gy; q.b = weight; q.bias = bias; q.out = gx; q.status = device_status_ptr();
+        q.a = gy; q.b = weight; q.bias = bias; q.out = gx; q.status = device_status_ptr(); q.gate = gate;
         q.g_C = K; q.g_H = oH; q.g_W = oW; q.N_total = C; q.w_kk = kH * kW; q.o_HW = H * W;
         q.n_phases = (int)std::min<size_t>(pwg::MAX_PHASES, ph.size() - at);
         for (int i = 0; i < q.n_phases; ++i) q.ph[i] = ph[at + i];
@@ -1753,10 +1786,17 @@ using namespace cunn::mm;
 
 // Scratch memory of the kernels in conv_split.cu, or 0 where they do not take the pass.
 enum Pass : int { PASS_FORWARD = 0, PASS_GRAD_INPUT = 1, PASS_GRAD_WEIGHT = 2 };
+static size_t conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW, int padH, int padW,
+                                      int dilH, int dilW);
+static size_t gathered_workspace(const split::Geometry &g)
+{
+    return conv_acc_grad_workspace(g.N, g.C, g.H, g.W, g.K, g.kH, g.kW, g.dH, g.dW, g.padH, g.padW, g.dilH, g.dilW);
+}
 static size_t split_scratch(int pass, const split::Geometry &g)
 {
     if (!g_use_tma || g.N == 0 || (g.H == 1 && g.W == 1)) return 0;
-    return pass == PASS_FORWARD ? split::forward_scratch(g) : pass == PASS_GRAD_INPUT ? split::grad_input_scratch(g) : split::grad_weight_scratch(g);
+    return pass == PASS_FORWARD ? split::forward_scratch(g) : pass == PASS_GRAD_INPUT ? split::grad_input_scratch(g)
+                                                                                      : split::grad_weight_scratch(g, gathered_workspace);
 }
 static bool split_applies(int pass, const split::Geometry &g, const void *scratch, size_t scratch_bytes)
 {
@@ -1764,9 +1804,10 @@ static bool split_applies(int pass, const split::Geometry &g, const void *scratc
     return need && scratch_bytes >= need;
 }
 
+// `gate`: null, or the kernels do nothing where it is 0 (no scratch memory then).
 static int conv_forward(const float *x, const float *weight, const float *bias, float *y, int N, int C, int H, int W, int K,
                         int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_,
-                        void *scratch = nullptr, size_t scratch_bytes = 0)
+                        void *scratch = nullptr, size_t scratch_bytes = 0, const int *gate = nullptr)
 {
     clear_error();
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -1778,12 +1819,18 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     CUNN_CHECK_ARG(!dilated || gather_applies(kH, kW), "dilated kernels of more than 32 taps are not supported");
     if (!dilated && stem::applies(C, K, kH, kW)) return stem::forward(x, weight, bias, y, N, H, W, oH, oW, dH, dW, padH, padW, stream);
     const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
-    if (split_applies(PASS_FORWARD, geo, scratch, scratch_bytes)) return split::forward(geo, x, weight, bias, y, scratch, stream);
+    if (split_applies(PASS_FORWARD, geo, scratch, scratch_bytes)) {
+        auto again = [&](int first, int n, const int *wide) {
+            return conv_forward(x + (size_t)first * C * H * W, weight, bias, y + (size_t)first * K * oH * oW, n, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH,
+                                dilW, stream_, nullptr, 0, wide);
+        };
+        return split::forward(geo, x, weight, bias, y, split::fallback_of(again), scratch, stream);
+    }
     if (pw_applies(kH, kW, dH, dW, padH, padW) && H * W == 1 && K % 4 == 0 && tma_applies(x, weight, y, C, 4)) {
         // a fully connected layer: y[n][k] = sum_c x[n][c] W[k][c], two K-major matrices, i.e. the weight gradient's GEMM over one
         // "image" of C pixels (with element copies of single-pixel planes, 128 x 1024 -> 1000 took 129 us)
         pw::Params q{};
-        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
+        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr(); q.gate = gate;
         q.HW = C; q.gpi = ceil_div(C, 32); q.M_total = N; q.N_total = K; q.kblocks = q.gpi;
         const int bn = pw_bn_for(K, N);
         q.n_tiles = ceil_div(K, bn); q.tiles_per_split = q.total_tiles = ceil_div(N, BM) * q.n_tiles;
@@ -1796,7 +1843,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     }
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         pw::Params q{};
-        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
+        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr(); q.gate = gate;
         q.HW = H * W; q.M_total = N * H * W; q.N_total = K; q.Kd = C; q.kblocks = ceil_div(C, BK);
         const int bn = pw_bn_for(K, q.M_total);
         q.n_tiles = ceil_div(K, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
@@ -1820,7 +1867,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     }
     if (gather_applies(kH, kW)) {
         pw::Params q{};
-        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
+        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr(); q.gate = gate;
         q.HW = oH * oW; q.M_total = N * oH * oW; q.N_total = K; q.Kd = C * kH * kW; q.kblocks = ceil_div(q.Kd, BK);
         set_geometry(q, C, H, W, kH, kW, dH, dW, padH, padW, oW, dilH, dilW);
         const int bn = pw_bn_for(K, q.M_total);
@@ -1833,7 +1880,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
     }
     if (small_kernel(kH, kW)) {
         pwg::GatherParams q{};
-        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr();
+        q.a = x; q.b = weight; q.bias = bias; q.out = y; q.status = device_status_ptr(); q.gate = gate;
         q.g_C = C; q.g_H = H; q.g_W = W; q.N_total = K; q.w_kk = kH * kW; q.o_HW = oH * oW;
         q.vec_b = (C * kH * kW) % 4 == 0 && aligned16(weight);
         q.n_phases = 1;
@@ -1845,7 +1892,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
         return launch_gather<OP_FWD>(q, pw_bn_for(K, f.M_total), stream);
     }
     GemmParams p{};
-    p.a_src = x; p.b_src = weight; p.bias = bias; p.out = y; p.status = device_status_ptr();
+    p.a_src = x; p.b_src = weight; p.bias = bias; p.out = y; p.status = device_status_ptr(); p.gate = gate;
     p.g_C = C; p.g_H = H; p.g_W = W; p.g_padH = padH; p.g_padW = padW; p.g_dH = dH; p.g_dW = dW; p.kH = kH; p.kW = kW;
     p.pix_W = oW; p.pix_HW = oH * oW; p.C = C; p.K = K; p.n_img = N;
     p.M_total = N * oH * oW; p.N_total = K; p.Kd = C * kH * kW; p.kblocks = ceil_div(p.Kd, BK); p.out_HW = oH * oW;
@@ -1857,7 +1904,7 @@ static int conv_forward(const float *x, const float *weight, const float *bias, 
 // `bias` (null: none) is added to every plane of gx: a transposed convolution's forward pass is this one plus its bias.
 static int conv_grad_input(const float *gy, const float *weight, const float *bias, float *gx, int N, int C, int H, int W, int K,
                            int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, cunn_stream_t stream_,
-                           void *scratch = nullptr, size_t scratch_bytes = 0)
+                           void *scratch = nullptr, size_t scratch_bytes = 0, const int *gate = nullptr)
 {
     clear_error();
     // the stride-1 kernels leave the bias to a pass of its own
@@ -1865,7 +1912,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         if (rc || !bias) return rc;
         const long long total = (long long)N * C * H * W;
         const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 16));
-        add_plane_bias_kernel<<<blocks, 256, 0, (cudaStream_t)stream_>>>(gx, bias, C, H * W, total);
+        add_plane_bias_kernel<<<blocks, 256, 0, (cudaStream_t)stream_>>>(gx, bias, C, H * W, total, gate);
         CUNN_LAUNCH_CHECK("full convolution bias");
         return 0;
     };
@@ -1878,7 +1925,13 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
     CUNN_CHECK_ARG(!dilated || gather_applies(kH, kW), "dilated kernels of more than 32 taps are not supported");
     const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
     try {
-        if (split_applies(PASS_GRAD_INPUT, geo, scratch, scratch_bytes)) return split::grad_input(geo, gy, weight, bias, gx, scratch, stream);
+        if (split_applies(PASS_GRAD_INPUT, geo, scratch, scratch_bytes)) {
+            auto again = [&](int first, int n, const int *wide) {
+                return conv_grad_input(gy + (size_t)first * K * oH * oW, weight, bias, gx + (size_t)first * C * H * W, n, C, H, W, K, kH, kW, dH, dW, padH,
+                                       padW, dilH, dilW, stream_, nullptr, 0, wide);
+            };
+            return split::grad_input(geo, gy, weight, bias, gx, split::fallback_of(again), scratch, stream);
+        }
     } catch (const std::bad_alloc &) {
         return fail("convmm grad input: out of host memory");
     }
@@ -1889,7 +1942,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         return add_bias(conv_forward(weight, gy, nullptr, gx, 1, K, 1, C, N, 1, 1, 1, 1, 0, 0, 1, 1, stream_));
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         pw::Params q{};
-        q.a = gy; q.b = weight; q.bias = nullptr; q.out = gx; q.status = device_status_ptr();
+        q.a = gy; q.b = weight; q.bias = nullptr; q.out = gx; q.status = device_status_ptr(); q.gate = gate;
         q.HW = H * W; q.M_total = N * H * W; q.N_total = C; q.Kd = K; q.kblocks = ceil_div(K, BK);
         const int bn = pw_bn_for(C, q.M_total);
         q.n_tiles = ceil_div(C, bn); q.tiles_per_split = 0; q.total_tiles = ceil_div(q.M_total, BM) * q.n_tiles;
@@ -1916,7 +1969,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         // stride 1: a convolution of gy with the kernel rotated by 180 degrees and padding dil (k - 1) - pad
         if (gather_applies(kH, kW)) {
             pw::Params q{};
-            q.a = gy; q.b = weight; q.bias = nullptr; q.out = gx; q.status = device_status_ptr();
+            q.a = gy; q.b = weight; q.bias = nullptr; q.out = gx; q.status = device_status_ptr(); q.gate = gate;
             q.HW = H * W; q.M_total = N * H * W; q.N_total = C; q.Kd = K * kH * kW; q.kblocks = ceil_div(q.Kd, BK);
             set_geometry(q, K, oH, oW, kH, kW, 1, 1, dilH * (kH - 1) - padH, dilW * (kW - 1) - padW, W, dilH, dilW);
             const int bn = pw_bn_for(C, q.M_total);
@@ -1928,7 +1981,7 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
             return add_bias(pw_launch(pw_pick<OP_DGRAD>(bn, gather_ks(kH, kW)), q, stream));
         }
         GemmParams p{};
-        p.a_src = gy; p.b_src = weight; p.bias = nullptr; p.out = gx; p.status = device_status_ptr();
+        p.a_src = gy; p.b_src = weight; p.bias = nullptr; p.out = gx; p.status = device_status_ptr(); p.gate = gate;
         p.g_C = K; p.g_H = oH; p.g_W = oW; p.g_padH = kH - 1 - padH; p.g_padW = kW - 1 - padW; p.g_dH = 1; p.g_dW = 1;
         p.kH = kH; p.kW = kW; p.pix_W = W; p.pix_HW = H * W; p.C = C; p.K = K; p.n_img = N;
         p.M_total = N * H * W; p.N_total = C; p.Kd = K * kH * kW; p.kblocks = ceil_div(p.Kd, BK); p.out_HW = H * W;
@@ -1937,26 +1990,23 @@ static int conv_grad_input(const float *gy, const float *weight, const float *bi
         return add_bias(launch(pick_kernel<OP_DGRAD>(bn), p, grid, bn, stream));
     }
     try {
-        return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW, stream);
+        return phased_grad_input(gy, weight, bias, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW, gate, stream);
     } catch (const std::bad_alloc &) {
         return fail("convmm grad input: out of host memory");
     }
 }
 
 static int reduce_partials(const float *partial, float *gw, long long n, int splits, float scale, const float *bias_part, float *gb, int K,
-                           cudaStream_t stream)
+                           const int *gate, const float *sums, cudaStream_t stream)
 {
     const long long total = n + (bias_part ? K : 0);
     // eight threads per output where one per output would leave SMs short of warps: 9,408 outputs of 148 splits 6.8 us; 295,000 outputs
     // of 37 splits take 18 us that way and 7 us with a thread each
-    if (splits >= 16 && total < 128LL * 1024) {
-        const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 32), (long long)sm_count() * 8));
-        wgrad_bias_reduce_wide_kernel<<<blocks, 256, 0, stream>>>(partial, gw, n, splits, scale, bias_part, gb, K);
-    } else {
-        const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, 256), (long long)sm_count() * 8));
-        wgrad_bias_reduce_kernel<<<blocks, 256, 0, stream>>>(partial, gw, n, splits, scale, bias_part, gb, K);
-    }
-    CUNN_LAUNCH_CHECK("convmm acc grad reduce");
+    const bool wide = splits >= 16 && total < 128LL * 1024;
+    const int blocks = (int)std::max(1LL, std::min(ceil_div_ll(total, wide ? 32 : 256), (long long)sm_count() * 8));
+    void *args[] = {&partial, &gw, &n, &splits, &scale, &bias_part, &gb, &K, &gate, &sums};
+    CUNN_CUDA(launch_gated(wide ? (const void *)wgrad_bias_reduce_wide_kernel : (const void *)wgrad_bias_reduce_kernel, dim3(blocks), dim3(256), args, 0, stream,
+                           gate));
     return 0;
 }
 
@@ -1978,7 +2028,7 @@ static size_t conv_acc_grad_workspace(int N, int C, int H, int W, int K, int kH,
 
 static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, float *grad_bias, int N, int C, int H, int W, int K,
                          int kH, int kW, int dH, int dW, int padH, int padW, int dilH, int dilW, float scale, void *workspace,
-                         size_t workspace_bytes, cunn_stream_t stream_)
+                         size_t workspace_bytes, cunn_stream_t stream_, const int *gate = nullptr, const float *sums = nullptr)
 {
     clear_error();
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -1999,16 +2049,23 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         const long long n = (long long)K * C * kk;
         float *partial = (float *)workspace, *bias_part = partial + (size_t)ctas * n;
         if (stem::weight_grad_partials(x, gy, partial, grad_bias ? bias_part : nullptr, N, H, W, oH, oW, dH, dW, padH, padW, stream)) return 1;
-        return reduce_partials(partial, grad_weight, n, ctas, scale, grad_bias ? bias_part : nullptr, grad_bias, K, stream);
+        return reduce_partials(partial, grad_weight, n, ctas, scale, grad_bias ? bias_part : nullptr, grad_bias, K, gate, sums, stream);
     }
     const split::Geometry geo{N, C, H, W, K, kH, kW, dH, dW, padH, padW, dilH, dilW, oH, oW};
-    if (split_applies(PASS_GRAD_WEIGHT, geo, workspace, workspace_bytes)) return split::grad_weight(geo, x, gy, grad_weight, grad_bias, scale, workspace, stream);
+    if (!gate && split_applies(PASS_GRAD_WEIGHT, geo, workspace, workspace_bytes)) {
+        auto again = [&](int first, int n, const int *wide) {
+            const size_t head = split::grad_weight_head(geo);
+            return conv_acc_grad(x + (size_t)first * C * H * W, gy + (size_t)first * K * oH * oW, grad_weight, nullptr, n, C, H, W, K, kH, kW, dH, dW, padH, padW,
+                                 dilH, dilW, scale, (char *)workspace + head, workspace_bytes - head, stream_, wide, split::grad_weight_sums(geo, workspace));
+        };
+        return split::grad_weight(geo, x, gy, grad_bias, scale, split::fallback_of(again), workspace, stream);
+    }
     if (pw_applies(kH, kW, dH, dW, padH, padW)) {
         const bool tma = tma_applies(gy, x, workspace, H * W, 4);
         pw_wgrad_plan(C, K, 1, N, H * W, tma, &bn, &splits, &kb);
         const long long n = (long long)K * C;
         pw::Params q{};
-        q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr();
+        q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr(); q.gate = gate;
         q.bias_part = grad_bias ? (float *)workspace + (size_t)splits * n : nullptr;
         q.HW = H * W; q.M_total = K; q.N_total = C; q.Kd = 0; q.kblocks = kb;
         q.n_tiles = ceil_div(C, bn); q.tiles_per_split = ceil_div(K, BM) * q.n_tiles; q.total_tiles = q.tiles_per_split * splits;
@@ -2025,14 +2082,14 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
             pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
             if (pw_launch(rounds_wgrad(1, N, H * W) ? pw_pick_rounded(bn, 1) : pw_pick<OP_WGRAD>(bn), q, stream)) return 1;
         }
-        return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
+        return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, gate, sums, stream);
     }
     if (gathered_wgrad(kH, kW)) {
         const int oHW = oH * oW;
         pw_wgrad_plan(C, K, kk, N, oHW, false, &bn, &splits, &kb);
         const long long n = (long long)K * C * kk;
         pw::Params q{};
-        q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr();
+        q.a = gy; q.b = x; q.bias = nullptr; q.out = (float *)workspace; q.status = device_status_ptr(); q.gate = gate;
         q.bias_part = grad_bias ? (float *)workspace + (size_t)splits * n : nullptr;
         q.HW = oHW; q.M_total = K; q.N_total = C * kk; q.Kd = 0; q.kblocks = kb;
         set_geometry(q, C, H, W, kH, kW, dH, dW, padH, padW, oW, dilH, dilW);
@@ -2042,11 +2099,11 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
         pw_accumulators(bn, q.kblocks, &q.nacc, &q.sets, true, q.total_tiles);
         const int ks = gather_ks(kH, kW);
         if (pw_launch(rounds_wgrad(kk, N, oHW) ? pw_pick_rounded(bn, ks) : pw_pick<OP_WGRAD>(bn, ks), q, stream)) return 1;
-        return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, stream);
+        return reduce_partials((const float *)workspace, grad_weight, n, splits, scale, q.bias_part, grad_bias, K, gate, sums, stream);
     }
     wgrad_plan(N, C, K, kk, oH * oW, &bn, &splits, &ips, &pb);
     GemmParams p{};
-    p.a_src = gy; p.b_src = x; p.bias = nullptr; p.out = (float *)workspace; p.status = device_status_ptr();
+    p.a_src = gy; p.b_src = x; p.bias = nullptr; p.out = (float *)workspace; p.status = device_status_ptr(); p.gate = gate;
     p.g_C = C; p.g_H = H; p.g_W = W; p.g_padH = padH; p.g_padW = padW; p.g_dH = dH; p.g_dW = dW; p.kH = kH; p.kW = kW;
     p.pix_W = oW; p.pix_HW = oH * oW; p.C = C; p.K = K; p.n_img = N;
     p.M_total = K; p.N_total = C * kk; p.Kd = 0; p.kblocks = ips * pb; p.out_HW = 0;
@@ -2055,7 +2112,7 @@ static int conv_acc_grad(const float *x, const float *gy, float *grad_weight, fl
     if (launch(pick_kernel<OP_WGRAD>(bn), p, grid, bn, stream)) return 1;
     const long long n = (long long)K * C * kk;
     const int rblocks = (int)std::max(1LL, std::min(ceil_div_ll(n, 256), (long long)sm_count() * 8));
-    wgrad_reduce_kernel<<<rblocks, 256, 0, stream>>>((const float *)workspace, grad_weight, n, splits, scale);
+    wgrad_reduce_kernel<<<rblocks, 256, 0, stream>>>((const float *)workspace, grad_weight, n, splits, scale, gate, sums);
     CUNN_LAUNCH_CHECK("convmm acc grad reduce");
     if (grad_bias) {
         const int chunks = std::max(1, std::min(N, ceil_div(sm_count() * 4, K)));

@@ -224,6 +224,7 @@ pw_tma_kernel(const Params p, const __grid_constant__ CUtensorMap map_a, const _
     constexpr int SPLIT_PIECES = TILE / 16 / SPLITTERS;          // 16-byte pieces of a tile per splitter thread
     static_assert(SW % 4 == 0 && (EW == 4 || EW == 8) && (SPLIT_PIECES % 4 == 0 || SPLIT_PIECES == 2), "warp roles");
 
+    if (gated_off(p.gate)) return;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t mmadone[MAX_STAGES];    // the MMAs that read this raw stage (and the lo buffer of the same k-block) have finished
     __shared__ uint64_t accready[MAX_SETS];     // all MMAs of a tile have finished: its accumulator set can be read

@@ -237,3 +237,125 @@ def test_thnn_layer(F):
         F.convmm_acc_grad(x, gy, *want, 1, 1, 1, 1, 0.5)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     nnb.close()
+
+
+# ---- values of very different sizes that share an exponent ------------------------------------------------------------------------
+def wide_cases():
+    """(name, shape, what is scaled): a group with one large value whose partner is zero, so that it adds nothing to any sum."""
+    layer, strided = (32, 128, 28, 28, 128, 3, 3, 1, 1, 1), (20, 37, 40, 40, 320, 4, 4, 2, 1, 1)
+    first, point = (32, 3, 150, 141, 48, 7, 7, 2, 3, 1), (64, 512, 15, 15, 256, 1, 1, 1, 0, 1)
+    return [(what, shape) for shape in (layer, strided, first, point) for what in ("channel", "channels", "pixel", "weight")]
+
+
+def gather_bound(products):
+    """The gathering kernels' own error: operands of 22 bits without lo * lo 1.2e-7, chains that truncate at the size of the sum so far,
+    2^-24 an addition and 1.8e-8 sqrt(n) for what they round."""
+    return 1.2e-7 + 2.0 ** -24 * 40 + 1.8e-8 * products ** 0.5
+
+
+@pytest.mark.parametrize("size", [1e5, 1e6, 1e9, 1e13, 1e25])
+@pytest.mark.parametrize("what,shape", wide_cases())
+def test_large_values_opposite_zeros(F, what, shape, size):
+    """A channel, most channels, a pixel or a weight that is `size` times what shares its exponent, and adds nothing: the other values keep their bits."""
+    N, C, H, W, K, kH, kW, d, p, dil = shape
+    oH, oW = out_size(H, kH, d, p, dil), out_size(W, kW, d, p, dil)
+    g = torch.Generator(device="cuda").manual_seed(30)
+    x, gy = (torch.randn(*s, device="cuda", generator=g) for s in ((N, C, H, W), (N, K, oH, oW)))
+    w = torch.rand(K, C, kH, kW, device="cuda", generator=g) * 2 - 1
+    geo = (d, d, p, p, dil, dil)
+    takes = [scratch(i, N, C, H, W, K, kH, kW, d, p, dil) for i in range(3)]
+    assert any(takes)
+    if takes[0]:
+        xf, wf = x.clone(), w.clone()
+        if what in ("channel", "channels"):
+            n = slice(1, 2) if what == "channel" else slice(0, C * 4 // 5)
+            xf[:, n] *= size
+            wf[:, n] = 0
+        elif what == "pixel":
+            xf[3, 1, H // 2, W // 2] = size
+            wf[:, 1] = 0
+        else:
+            wf[5, 1, kH // 2, 0] = size
+            xf[:, 1] = 0
+        want = torch.nn.functional.conv2d(xf.double(), wf.double(), None, d, p, dil)
+        assert off(F.dilated_conv_forward(xf, wf, None, *geo), want) <= gather_bound(C * kH * kW)
+    if takes[1]:
+        gf, wf = gy.clone(), w.clone()
+        if what in ("channel", "channels"):
+            n = slice(1, 2) if what == "channel" else slice(0, K * 4 // 5)
+            gf[:, n] *= size
+            wf[n] = 0
+        elif what == "pixel":
+            gf[3, 1, oH // 2, oW // 2] = size
+            wf[1] = 0
+        else:
+            wf[1, 5, kH // 2, 0] = size
+            gf[:, 1] = 0
+        want = torch.nn.grad.conv2d_input(x.shape, wf.double(), gf.double(), d, p, dil)
+        assert off(F.dilated_conv_grad_input(gf, wf, H, W, *geo), want) <= gather_bound(K * kH * kW)
+    if takes[2] and what == "pixel":
+        # an outlier on one side, zeros where its sums read the other: every filter and channel for itself
+        for outlier in ("gy", "x"):
+            xw, gg, gw, gb = x.clone(), gy.clone(), torch.zeros_like(w), torch.zeros(K, device="cuda")
+            if outlier == "gy":
+                gg[3, 7, oH // 2, oW // 2] = size
+                xw[3] = 0
+            else:
+                xw[3, 1, H // 2, W // 2] = size
+                gg[3] = 0
+            F.dilated_conv_acc_grad(xw, gg, gw, gb, *geo)
+            want = torch.nn.grad.conv2d_weight(xw.double(), w.shape, gg.double(), d, p, dil)
+            rows = (gw.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
+            cols = (gw.double() - want).transpose(0, 1).flatten(1).norm(dim=1) / want.transpose(0, 1).flatten(1).norm(dim=1)
+            assert max(float(rows.max()), float(cols.max())) <= 2 * gather_bound(N * oH * oW)
+
+
+@pytest.mark.parametrize("kind", ["normal", "sparse", "gradient"])
+def test_ordinary_values_stay_here(F, kind):
+    """What a network's layers hold has values close to zero by chance: not a reason to leave the kernels of split operands."""
+    from cunn_b200._lib import lib, check
+    N, C, H, K = 64, 64, 28, 64
+    g = torch.Generator(device="cuda").manual_seed(32)
+    x, w = torch.randn(N, C, H, H, device="cuda", generator=g), torch.rand(K, C, 3, 3, device="cuda", generator=g) * 2 - 1
+    if kind == "sparse":                                # a ReLU with few active units
+        x = (x - torch.linspace(0, 4, C, device="cuda").view(1, -1, 1, 1)).relu()
+    elif kind == "gradient":                            # behind a ReLU and a batch normalisation of a million values
+        x = torch.where(torch.rand(x.shape, device="cuda", generator=g) < 0.5, x, x * 1e-3)
+    geo = (N, C, H, H, K, 3, 3, 1, 1, 1, 1)
+    stream = torch.cuda.current_stream().cuda_stream
+    y, gx = F.convmm_forward(x, w, None, 1, 1, 1, 1), F.convmm_grad_input(x, w, H, H, 1, 1, 1, 1)
+    y0, gx0 = torch.empty_like(y), torch.empty_like(gx)
+    check(lib.cunn_b200_convmm_forward(x.data_ptr(), w.data_ptr(), None, y0.data_ptr(), *geo, stream))
+    check(lib.cunn_b200_convmm_grad_input(x.data_ptr(), w.data_ptr(), gx0.data_ptr(), *geo, stream))
+    assert scratch(0, *geo[:8], 1, 1) and not torch.equal(y, y0) and not torch.equal(gx, gx0)
+    gws = [torch.zeros_like(w) for _ in range(2)]
+    assert scratch(2, *geo[:8], 1, 1)
+    F.convmm_acc_grad(x, x, gws[0], None, 1, 1, 1, 1)
+    ws = torch.empty(lib.cunn_b200_convmm_acc_grad_workspace(*geo), dtype=torch.uint8, device="cuda")
+    check(lib.cunn_b200_convmm_acc_grad(x.data_ptr(), x.data_ptr(), gws[1].data_ptr(), None, *geo, 1.0, ws.data_ptr(), ws.numel(), stream))
+    assert not torch.equal(*gws)
+    for got, want in ((y, y0), (gx, gx0), (gws[0], gws[1])):
+        assert off(got, want.double()) <= 6e-6
+
+
+def test_large_values_in_a_later_round(F):
+    """Scratch holds 512 MB of split values: a later part of the batch is judged, and taken, for itself; what the call adds to, it adds once."""
+    N, C, H, K = 44, 64, 240, 16
+    assert scratch(0, N, C, H, H, K, 3, 3, 1, 1, 1) and N * C * H * H * 4 > 512 << 20
+    g = torch.Generator(device="cuda").manual_seed(31)
+    x, w = torch.randn(N, C, H, H, device="cuda", generator=g), torch.rand(K, C, 3, 3, device="cuda", generator=g) * 2 - 1
+    w[:, 1] = 0
+    plain = F.convmm_forward(x, w, None, 1, 1, 1, 1)
+    x[N - 1, 1] = 1e13
+    y = F.convmm_forward(x, w, None, 1, 1, 1, 1)
+    assert torch.equal(y[:N // 2], plain[:N // 2])
+    for i in (0, N - 1):
+        assert off(y[i], torch.nn.functional.conv2d(x[i].double(), w.double(), None, 1, 1)) <= gather_bound(C * 9)
+    del y, plain
+    assert scratch(2, N, C, H, H, K, 3, 3, 1, 1, 1)
+    gy = torch.randn(N, K, H, H, device="cuda", generator=g)
+    gy[N - 1] = 0
+    gw, gb = torch.ones(K, C, 3, 3, device="cuda"), torch.ones(K, device="cuda")
+    F.convmm_acc_grad(x, gy, gw, gb, 1, 1, 1, 1)
+    want = sum(torch.nn.grad.conv2d_weight(x[i:i + 4].double(), w.shape, gy[i:i + 4].double(), 1, 1) for i in range(0, N, 4))
+    assert off(gw.double() - 1, want) <= 4e-6 and off(gb.double() - 1, gy.double().sum((0, 2, 3))) <= 1e-6
