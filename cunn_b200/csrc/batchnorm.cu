@@ -568,9 +568,9 @@ grad_apply_flat_kernel(const float *__restrict__ x, const float *__restrict__ gy
 // Work split: inside a group, the float4 items of its channels form one sequence (channel-major, N*L items per
 // channel); CTA b takes the b-th of `grid` equal shares, which may span channel boundaries ("segments").
 //
-// Forward statistics use one shift K per channel (the mean of the first 32 elements of the channel's first plane,
-// read by every CTA): sums of (x - K) and (x - K)^2 keep their fp32 accuracy when |mean| >> std, and partials with
-// a common shift merge by plain fp64 addition.
+// Forward statistics are shifted, share by share, by the mean of the share's first stage (which takes 1 % of the time): sums of (x - K) and (x - K)^2 keep their fp32 accuracy
+// when |mean| >> std and when an image has a border.  (With one shift per channel, from the first 32 elements of its first image, channels
+// of mean / std 100 whose first 32 were zero had variances off by 6e-4.)  The partials merge in fp64 as those of the two-launch path.
 struct GroupPlan {
     int N, C, S, L;         // L = S / 4: float4 items per plane
     int G, groups;          // channels per group (the last group may be smaller), number of groups
@@ -619,19 +619,50 @@ __device__ __forceinline__ void half_sync(int half)
     else asm volatile("bar.sync 2, %0;" ::"n"(32 * HW) : "memory");
 }
 
-// Sum over one half; sh: a float per warp of that half.
+// Sum over one half, in fp64; sh: a double per warp of that half.
 template <int HW>
-__device__ __forceinline__ float half_sum(float v, float *sh, int half)
+__device__ __forceinline__ float half_sum(float v, double *sh, int half)
 {
-    v = warp_sum(v);
+    const double d = warp_sum((double)v);
     const int lane = threadIdx.x & 31, w = (int)(threadIdx.x >> 5) % (HW + 1);
     half_sync<HW>(half);
-    if (lane == 0) sh[w] = v;
+    if (lane == 0) sh[w] = d;
     half_sync<HW>(half);
-    float t = 0.f;
+    double t = 0.0;
 #pragma unroll
     for (int i = 0; i < HW; ++i) t += sh[i];
-    return t;
+    return (float)t;
+}
+
+// The shift of a segment, by all consumers of the half: the mean of as many of the `len` items that begin it as are a power of two.  Equal values
+// add up without rounding, so that a constant channel has a variance of exactly zero.  No shift where they hold an infinity or a NaN, or
+// add up to one: x - K would be NaN for values that are neither.
+template <int HW>
+__device__ __forceinline__ float segment_shift(const float4 *items, int len, int ht, double *sh)
+{
+    constexpr int kHalf = 32 * HW;
+    const int n = 1 << (31 - __clz(len));
+    auto at = [&](int j) {
+        if (j >= n) return 0.f;
+        const float4 q = items[j];
+        return ((q.x + q.y) + (q.z + q.w)) * 0.25f;
+    };
+    float v = 0.f;
+#pragma unroll
+    for (int j = 0; j < kStageBytes / 16; j += 4 * kHalf) v += (at(ht + j) + at(ht + j + kHalf)) + (at(ht + j + 2 * kHalf) + at(ht + j + 3 * kHalf));
+    v = warp_sum(v);
+    half_sync<HW>(0);
+    if ((ht & 31) == 0) sh[ht >> 5] = (double)v;
+    half_sync<HW>(0);
+    double t[HW];
+#pragma unroll
+    for (int i = 0; i < HW; ++i) t[i] = sh[i];
+#pragma unroll
+    for (int h = HW / 2; h > 0; h /= 2)
+#pragma unroll
+        for (int i = 0; i < h; ++i) t[i] += t[i + h];
+    const float k = (float)t[0] / (float)n;
+    return fabsf(k) < INFINITY ? k : 0.f;
 }
 
 // The CTAs whose shares touch channel cl (local index in the group) of a group of W items: first and last.
@@ -727,7 +758,7 @@ struct GroupedArgs {
     const float *x, *gy;             // gy: backward only
     float *out;                      // y (forward) or gx (backward)
     const float *weight, *bias;
-    void *part;                      // float2 partials, pstride per channel
+    void *part;                      // ChunkStat (forward) or float2 partials, pstride per channel
     GroupCounters cn;
     float *running_mean, *running_var, *save_mean, *save_std;     // forward: written
     const float *mean_v, *std_or_var;                              // backward: saved or running statistics
@@ -739,39 +770,6 @@ struct GroupedArgs {
     int *status;
 };
 
-// Forward merge for channel c by one warp: partials (sum (x - K), sum (x - K)^2) share the shift K.
-__device__ __forceinline__ void finish_stats_shifted_warp(const float2 *part, int c, int cnt, float K, long long count,
-                                                          float *running_mean, float *running_var, float *save_mean,
-                                                          float *save_std, double momentum, double eps)
-{
-    const int lane = threadIdx.x & 31;
-    double s1 = 0.0, s2 = 0.0;
-    for (int j = lane; j < cnt; j += 32) {
-        const float2 p = __ldcg(part + j);
-        s1 += (double)p.x;
-        s2 += (double)p.y;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s1 += __shfl_down_sync(0xffffffffu, s1, o);
-        s2 += __shfl_down_sync(0xffffffffu, s2, o);
-    }
-    if (lane != 0) return;
-    const double n = (double)count;
-    const double mean = (double)K + s1 / n;
-    double m2 = s2 - s1 * s1 / n;
-    if (m2 < 0.0) m2 = 0.0;
-    const float meanf = (float)mean;
-    const float varN = (float)m2;
-    float invstd = 0.f;
-    if (varN != 0.f || (float)eps != 0.f) invstd = 1.f / sqrtf((float)(m2 / n) + (float)eps);
-    const float unbiased = (float)(m2 / (n - 1.0));
-    save_mean[c] = meanf;
-    save_std[c] = invstd;
-    running_mean[c] = (float)((1.0 - momentum) * (double)running_mean[c] + momentum * (double)meanf);
-    running_var[c] = (float)((1.0 - momentum) * (double)running_var[c] + momentum * (double)unbiased);
-}
-
 template <bool BWD, bool RELU, int HW>
 __global__ void __launch_bounds__(grouped_threads(HW), 2)
 grouped_kernel(const GroupedArgs a)
@@ -781,8 +779,7 @@ grouped_kernel(const GroupedArgs a)
     extern __shared__ __align__(128) unsigned char ring_raw[];
     __shared__ __align__(8) unsigned long long full_s[2][kStages];      // slot filled (transaction bytes)
     __shared__ __align__(8) unsigned long long empty_s[2][kStages];     // slot read by the half's consumer warps
-    __shared__ float sums_s[2][HW];
-    __shared__ float k_s;
+    __shared__ double sums_s[2][HW];
     __shared__ int flag_s[2];
     __shared__ volatile int applied_s;       // groups this CTA's apply half has finished
     __shared__ volatile int abort_s;         // a wait ran out somewhere in the CTA: everybody leaves
@@ -794,7 +791,7 @@ grouped_kernel(const GroupedArgs a)
     const int ht = wi * 32 + lane;                                      // consumer index inside the half
     float4 *ring = reinterpret_cast<float4 *>(ring_raw) + (size_t)half * kStages * T * P;     // [kStages][T][P] of this half
     unsigned long long *bars = full_s[half], *empties = empty_s[half];
-    float *sh = sums_s[half];
+    double *sh = sums_s[half];
     const float4 *x4 = reinterpret_cast<const float4 *>(a.x), *g4 = reinterpret_cast<const float4 *>(a.gy);
     const unsigned long long pol = half == 0 ? l2_policy_evict_last() : l2_policy_evict_first();
 
@@ -881,7 +878,9 @@ grouped_kernel(const GroupedArgs a)
 
     if (half == 0) {
         // ------------------------------------------------ statistics half ------------------------------------------------
-        float K = 0.f, a1 = 0.f, a2 = 0.f;             // forward: shift, sum (x - K), sum (x - K)^2; backward: a1 = sum gy, a2 = sum gy (x - mean)
+        // forward: shift, sum (x - K), sum (x - K)^2; backward: a1 = sum gy, a2 + b2 = sum gy (x - mean), in two halves, so that a thread's chains are
+        // as short as those of the two-launch path (one chain had up to twice its error)
+        float K = 0.f, a1 = 0.f, a2 = 0.f, b2 = 0.f;
         float mean = 0.f, invstd = 0.f, gam = 1.f, bet = 0.f;
         for (int it = 0; cons.next(st); ++it) {
             const int slot = it % kStages;
@@ -890,18 +889,8 @@ grouped_kernel(const GroupedArgs a)
             if (st.seg_first) {
                 // stay at most `lookahead` groups ahead of this CTA's apply half
                 if (st.g >= gp.lookahead && !bounded([&] { return applied_s >= st.g - gp.lookahead + 1; })) return;
-                a1 = 0.f; a2 = 0.f;
-                if (!BWD) {
-                    // the channel's shift: mean of the first 32 elements of its first plane (the same value in every CTA)
-                    if (ht < 32) {
-                        const int mm = min(32, gp.S);
-                        float e = ht < mm ? __ldg(a.x + (long long)c * gp.S + ht) : 0.f;
-                        e = warp_sum(e);
-                        if (ht == 0) k_s = e / (float)mm;
-                    }
-                    half_sync<HW>(0);
-                    K = k_s;
-                } else {
+                a1 = 0.f; a2 = 0.f; b2 = 0.f;
+                if (BWD) {
                     mean = __ldg(a.mean_v + c);
                     if (RELU) {
                         invstd = a.train ? __ldg(a.std_or_var + c) : 1.f / sqrtf(__ldg(a.std_or_var + c) + (float)a.eps);
@@ -912,6 +901,7 @@ grouped_kernel(const GroupedArgs a)
             }
             if (!wait_phase(bars + slot, (uint32_t)((it / kStages) & 1))) return;
             if (!BWD) {
+                if (st.seg_first) K = segment_shift<HW>(sx, st.len, ht, sh);
 #pragma unroll 4
                 for (int j = ht; j < st.len; j += kHalf) {
                     const float4 q = sx[j];
@@ -927,21 +917,23 @@ grouped_kernel(const GroupedArgs a)
                     float4 gv = sg[j];
                     gv.x = one(xv.x, gv.x); gv.y = one(xv.y, gv.y); gv.z = one(xv.z, gv.z); gv.w = one(xv.w, gv.w);
                     a1 += (gv.x + gv.y) + (gv.z + gv.w);
-                    a2 = fmaf(gv.x, xv.x - mean, a2); a2 = fmaf(gv.y, xv.y - mean, a2);
-                    a2 = fmaf(gv.z, xv.z - mean, a2); a2 = fmaf(gv.w, xv.w - mean, a2);
+                    a2 = fmaf(gv.x, xv.x - mean, a2); b2 = fmaf(gv.y, xv.y - mean, b2);
+                    a2 = fmaf(gv.z, xv.z - mean, a2); b2 = fmaf(gv.w, xv.w - mean, b2);
                 }
             }
             release_slot(slot);
             if (st.seg_last) {
                 // hand in this segment's partial; the CTA with the channel's last ticket merges and raises the flag
                 a1 = half_sum<HW>(a1, sh, 0);
-                a2 = half_sum<HW>(a2, sh, 0);
+                a2 = half_sum<HW>(a2 + b2, sh, 0);
                 int bf, bl;
                 channel_ctas((long long)min(gp.G, gp.C - st.g * gp.G) * gp.NL, gp.NL, st.cl, grid, &bf, &bl);
                 const int cnt = bl - bf + 1;
-                float2 *pc = reinterpret_cast<float2 *>(a.part) + (size_t)c * gp.pstride;
+                ChunkStat *stats = reinterpret_cast<ChunkStat *>(a.part) + (size_t)c * gp.pstride;
+                float2 *sums = reinterpret_cast<float2 *>(a.part) + (size_t)c * gp.pstride;
                 if (ht == 0) {
-                    pc[b - bf] = make_float2(a1, a2);
+                    if (BWD) sums[b - bf] = make_float2(a1, a2);
+                    else stats[b - bf] = ChunkStat{K, a1, a2, (float)(st.seg_items * 4)};
                     __threadfence();                                  // the partial is visible before the ticket
                     flag_s[0] = atomicAdd(a.cn.tick + c, 1u) == (unsigned)(cnt - 1);
                 }
@@ -952,10 +944,9 @@ grouped_kernel(const GroupedArgs a)
                     __threadfence();                                  // the other CTAs' partials are visible after their tickets
                     if (ht < 32) {
                         if (!BWD)
-                            finish_stats_shifted_warp(pc, c, cnt, K, (long long)gp.N * gp.S, a.running_mean, a.running_var, a.save_mean,
-                                                      a.save_std, a.momentum, a.eps);
+                            finish_stats_channel_warp(stats, c, cnt, a.running_mean, a.running_var, a.save_mean, a.save_std, a.momentum, a.eps);
                         else
-                            finish_grad_channel_warp(pc, c, cnt, (long long)gp.N * gp.S, a.weight, a.bias, a.mean_v, a.std_or_var, a.train,
+                            finish_grad_channel_warp(sums, c, cnt, (long long)gp.N * gp.S, a.weight, a.bias, a.mean_v, a.std_or_var, a.train,
                                                      a.eps, a.scale, a.grad_weight, a.grad_bias, a.coef);
                         if (ht == 0) {
                             a.cn.tick[c] = 0u;

@@ -326,3 +326,64 @@ def test_batchnorm_groups_of_channels(F, shape, relu):
     assert float((gb.double() - gb64).abs().max()) <= 1e-5 * size and float((gw.double() - gw64).abs().max()) <= 1e-5 * size
     gx64 = (g64 - col(gb64) / n - xh * col(gw64) / n) * col(w) * (col(v64) + 1e-5).rsqrt()
     assert float(((gx.double() - gx64).abs() * sure).max()) <= 1e-5
+
+
+@pytest.mark.parametrize("mean", [10.0, 100.0, 1000.0])
+@pytest.mark.parametrize("shape", [(128, 96, 56, 56), (2, 17, 1024, 1000), (129, 9, 112, 112)])
+def test_batchnorm_groups_shift_by_typical_values(F, shape, mean):
+    """Channels whose first values are none of the others' size (a border of zeros): the squares about the shift stay small beside what they are
+    summed to.  A CTA's shift is off by at most 32 / 1024 of the mean in the share with the border, where its fp32 chains of 256 squares round by
+    2^-24 of them; the other shares' shift is within a tenth of the deviation."""
+    import torch
+    N, C, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(12)
+    x = torch.randn(shape, device="cuda", generator=g) + mean
+    x.view(N, C, -1)[0, :, :32] = 0
+    rm, rv = torch.zeros(C, device="cuda"), torch.zeros(C, device="cuda")
+    _, m, _ = F.batchnorm_forward(x, None, None, rm, rv, True)
+    n = N * H * W
+    m64, v64 = x.double().mean((0, 2, 3)), x.double().var((0, 2, 3))
+    share = 4096.0 * 16 / n                                    # of the channel's values that are in the share with the border, or more
+    bound = 1e-6 + 2.0 ** -24 * 16 * share * (mean / 32) ** 2
+    assert float(((rv.double() * 10 - v64) / v64).abs().max()) <= bound
+    assert float(((m.double() - m64).abs() / (m64.abs() * 2.0 ** -24 + 1e-6 * v64.sqrt())).max()) <= 1
+
+
+@pytest.mark.parametrize("shape", [(128, 96, 56, 56), (129, 9, 112, 112)])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_batchnorm_groups_of_what_is_not_finite(F, shape, value):
+    """An infinity is the mean's, wherever it is; the other channels are what they were.  A constant channel has no variance at all."""
+    import torch
+    N, C, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(13)
+    x = torch.randn(shape, device="cuda", generator=g)
+    x[:, 5] = 0.1
+    want = F.batchnorm_forward(x, None, None, torch.zeros(C, device="cuda"), torch.zeros(C, device="cuda"), True)
+    assert float(want[1][5]) == float(torch.tensor(0.1))
+    rv0 = torch.zeros(C, device="cuda")
+    F.batchnorm_forward(x, None, None, torch.zeros(C, device="cuda"), rv0, True)
+    assert float(rv0[5]) == 0
+    for at in ((0, 2, 0, 3), (N // 2, 2, 5, 7), (N - 1, 2, H - 1, W - 1)):
+        z = x.clone()
+        z[at] = value
+        y, m, s = F.batchnorm_forward(z, None, None, torch.zeros(C, device="cuda"), torch.zeros(C, device="cuda"), True)
+        assert m[2].isnan() if value != value else float(m[2]) == value
+        others = [c for c in range(C) if c != 2]
+        assert torch.equal(m[others], want[1][others]) and torch.equal(s[others], want[2][others]) and torch.equal(y[:, others], want[0][:, others])
+
+
+@pytest.mark.parametrize("shape", [(128, 128, 56, 56), (2, 16, 1024, 1024)])
+def test_batchnorm_groups_gradient_sums(F, shape):
+    """The weight's gradient of layers on the one-launch backward kernel.  A chain of 42 fp32 multiply-adds is off by 2^-25.8 (42 / 2^0.5) of a
+    term, 7.8e-8 of its own size sqrt(42); so are their sums, with a largest of 4 times that among the channels and twice for the products."""
+    import torch
+    N, C, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, gy = torch.randn(shape, device="cuda", generator=g) + 30, torch.randn(shape, device="cuda", generator=g) + 0.5
+    w, rm, rv = torch.ones(C, device="cuda"), torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+    _, mean, std = F.batchnorm_forward(x, w, None, rm, rv, True)
+    gw, gb = torch.zeros(C, device="cuda"), torch.zeros(C, device="cuda")
+    F.batchnorm_backward(x, gy, w, rm, rv, mean, std, True, 1.0, 1e-5, gw, gb)
+    col = lambda t: t.double().view(1, C, 1, 1)
+    want = (gy.double() * (x.double() - col(mean)) * col(std)).sum((0, 2, 3))
+    assert float((gw.double() - want).abs().max()) <= 6e-7 * (N * H * W) ** 0.5
