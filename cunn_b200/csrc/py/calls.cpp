@@ -128,5 +128,7 @@ PyMODINIT_FUNC PyInit__calls()
     if (!ctypes) return nullptr;
     g_argument_error = PyObject_GetAttrString(ctypes, "ArgumentError");
     Py_DECREF(ctypes);
-    return g_argument_error ? PyModule_Create(&g_module) : nullptr;
+    PyObject *m = g_argument_error ? PyModule_Create(&g_module) : nullptr;
+    if (m && PyModule_AddIntConstant(m, "CONV_POINT_VALUES", CUNN_B200_CONV_POINT_VALUES)) Py_CLEAR(m);
+    return m;
 }

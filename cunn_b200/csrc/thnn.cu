@@ -54,7 +54,7 @@ struct ConvScratch {
         if (want > least && take(state_stream(s), want)) return;
         if (!least) return;
         ptr = state_scratch(s, 0, least);
-        bytes = ptr ? state_scratch_bytes(s, 0) : 0;
+        bytes = ptr ? least : 0;                     // not what the state has: which kernels run must not depend on earlier calls
     }
     ConvScratch(const ConvScratch &) = delete;
     ConvScratch &operator=(const ConvScratch &) = delete;
@@ -130,18 +130,18 @@ struct RealFloat {
     static int convmm_forward(THCState *s, const float *x, const float *w, const float *b, float *y, int N, int C, int H, int W, int K, int kH,
                               int kW, int dH, int dW, int padH, int padW)
     {
-        const ConvScratch ws(s, (kH * kW > 1 || (long long)N * C * H * W >= 1 << 20) ? cunn_b200_conv_scratch(0, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1) : 0);
+        const ConvScratch ws(s, cunn_b200_conv_scratch(0, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1));
         return cunn_b200_conv_forward_scratch(x, w, b, y, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1, ws.ptr, ws.bytes, state_stream(s));
     }
     static int convmm_grad_input(THCState *s, const float *gy, const float *w, float *gx, int N, int C, int H, int W, int K, int kH, int kW,
                                  int dH, int dW, int padH, int padW)
     {
-        const ConvScratch ws(s, (kH * kW > 1 || (long long)N * C * H * W >= 1 << 20) ? cunn_b200_conv_scratch(1, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1) : 0);
+        const ConvScratch ws(s, cunn_b200_conv_scratch(1, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1));
         return cunn_b200_conv_grad_input_scratch(gy, w, gx, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1, ws.ptr, ws.bytes, state_stream(s));
     }
     static size_t convmm_acc_grad_scratch(int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW, int padH, int padW)
     {
-        return (kH * kW > 1 || (long long)N * C * H * W >= 1 << 20) ? cunn_b200_conv_scratch(2, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1) : 0;
+        return cunn_b200_conv_scratch(2, N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1);
     }
     static constexpr auto convmm_acc_grad_workspace = &cunn_b200_convmm_acc_grad_workspace;
     static constexpr auto convmm_acc_grad = &cunn_b200_convmm_acc_grad;

@@ -159,13 +159,14 @@ def batchnorm_backward(x, gy, weight, running_mean, running_var, save_mean, save
 
 
 _LARGE = 16 << 20
-_POINT = 1 << 20        # values of a 1x1 layer's tensor from which on it may be better off with scratch
+_POINT = lib.CONV_POINT_VALUES          # of a 1x1 layer: cunn_b200_conv_scratch is 0 below, and asking takes a microsecond of a small layer's 7
 
 
 def _conv_scratch(size_fn, which, geo, device, least=0):
     """(tensor, pointer, bytes) of the scratch memory that a pass of a convolution takes: 0 forward, 1 input gradient, 2 parameter
     gradient, which cannot do without `least` bytes.  Large buffers are the allocator's again when the call has been queued; none are
-    shared between streams or with a graph under capture."""
+    shared between streams or with a graph under capture.  The bytes are those that were asked for, not those that a kept buffer has: they
+    decide which kernels run."""
     need = size_fn(which, *geo)
     if need > least:
         try:
@@ -176,7 +177,7 @@ def _conv_scratch(size_fn, which, geo, device, least=0):
     if not least:
         return None, None, 0
     ws = workspace(least, device) if least <= _LARGE else torch.empty(least, dtype=torch.uint8, device=device)
-    return ws, _ptr(ws), ws.numel()
+    return ws, _ptr(ws), least
 
 
 def convmm_forward(x, weight, bias, dH, dW, padH, padW, out=None):
@@ -187,14 +188,14 @@ def convmm_forward(x, weight, bias, dH, dW, padH, padW, out=None):
     oH, oW = conv_out(H, kH, dH, padH), conv_out(W, kW, dW, padW)
     if out is None:
         out = torch.empty((N, K, max(oH, 0), max(oW, 0)), dtype=torch.float32, device=x.device)
-    if kH * kW > 1 or x.numel() >= _POINT:
-        geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
-        ws = _conv_scratch(lib.cunn_b200_conv_scratch, 0, geo, x.device)
-        check(lib.cunn_b200_conv_forward_scratch(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), *geo,
-                                                 ws[1], ws[2], _stream()))
+    if kH * kW == 1 and x.numel() < _POINT:
+        check(lib.cunn_b200_convmm_forward(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), N, C, H, W, K, kH, kW,
+                                           dH, dW, padH, padW, _stream()))
         return out
-    check(lib.cunn_b200_convmm_forward(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), N, C, H, W, K, kH, kW,
-                                       dH, dW, padH, padW, _stream()))
+    geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
+    ws = _conv_scratch(lib.cunn_b200_conv_scratch, 0, geo, x.device)
+    check(lib.cunn_b200_conv_forward_scratch(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), *geo,
+                                             ws[1], ws[2], _stream()))
     return out
 
 
@@ -204,14 +205,14 @@ def convmm_grad_input(gy, weight, H, W, dH, dW, padH, padW, out=None):
     N = gy.shape[0]
     if out is None:
         out = torch.empty((N, C, H, W), dtype=torch.float32, device=gy.device)
-    if kH * kW > 1 or gy.numel() >= _POINT:
-        geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
-        ws = _conv_scratch(lib.cunn_b200_conv_scratch, 1, geo, gy.device)
-        check(lib.cunn_b200_conv_grad_input_scratch(_ptr(gy), _ptr(weight), _ptr(out), *geo,
-                                                    ws[1], ws[2], _stream()))
+    if kH * kW == 1 and gy.numel() < _POINT:
+        check(lib.cunn_b200_convmm_grad_input(_ptr(gy), _ptr(weight), _ptr(out), N, C, H, W, K, kH, kW,
+                                              dH, dW, padH, padW, _stream()))
         return out
-    check(lib.cunn_b200_convmm_grad_input(_ptr(gy), _ptr(weight), _ptr(out), N, C, H, W, K, kH, kW,
-                                          dH, dW, padH, padW, _stream()))
+    geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1)
+    ws = _conv_scratch(lib.cunn_b200_conv_scratch, 1, geo, gy.device)
+    check(lib.cunn_b200_conv_grad_input_scratch(_ptr(gy), _ptr(weight), _ptr(out), *geo,
+                                                ws[1], ws[2], _stream()))
     return out
 
 
@@ -220,14 +221,14 @@ def convmm_acc_grad(x, gy, grad_weight, grad_bias, dH, dW, padH, padW, scale=1.0
     _chk(x, gy, grad_weight, grad_bias)
     N, C, H, W = x.shape
     K, _, kH, kW = grad_weight.shape
-    need = lib.cunn_b200_convmm_acc_grad_workspace(N, C, H, W, K, kH, kW, dH, dW, padH, padW)
-    if need and (kH * kW > 1 or x.numel() >= _POINT):
-        ws, at, size = _conv_scratch(lib.cunn_b200_conv_scratch, 2, (N, C, H, W, K, kH, kW, dH, dW, padH, padW, 1, 1), x.device, need)
-    else:
+    geo = (N, C, H, W, K, kH, kW, dH, dW, padH, padW)
+    need = max(lib.cunn_b200_convmm_acc_grad_workspace(*geo), 1)
+    if kH * kW == 1 and x.numel() < _POINT:
         ws = workspace(need, x.device)
-        at, size = _ptr(ws), ws.numel()
-    check(lib.cunn_b200_convmm_acc_grad(_ptr(x), _ptr(gy), _ptr(grad_weight), _ptr(grad_bias), N, C, H, W, K, kH, kW,
-                                        dH, dW, padH, padW, scale, at, size, _stream()))
+        ws = ws, _ptr(ws), need
+    else:
+        ws = _conv_scratch(lib.cunn_b200_conv_scratch, 2, geo + (1, 1), x.device, need)
+    check(lib.cunn_b200_convmm_acc_grad(_ptr(x), _ptr(gy), _ptr(grad_weight), _ptr(grad_bias), *geo, scale, ws[1], ws[2], _stream()))
     return grad_weight, grad_bias
 
 

@@ -135,6 +135,7 @@ CUNN_API int cunn_b200_convmm_get_tma(void);
  * (16-byte aligned, contents arbitrary, at most about the size of the tensor that the pass reads, bounded by 0.5 GiB
  * and one image's, plus that of the weights); 0: the pass has no use for scratch.  With less, or NULL, the calls are those
  * without scratch.  No reference counterpart: the reference's `columns` buffer is scratch of the same kind. */
+#define CUNN_B200_CONV_POINT_VALUES (1 << 20) /* 1x1 layers that read fewer values have no use for scratch */
 CUNN_API size_t cunn_b200_conv_scratch(int pass, int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW,
                                        int padH, int padW, int dilH, int dilW);
 CUNN_API int cunn_b200_conv_forward_scratch(const float *x, const float *weight, const float *bias, float *y,

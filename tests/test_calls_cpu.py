@@ -42,3 +42,17 @@ def test_errors_reach_the_caller():
     """A call that is refused leaves its message for the thread that made it."""
     assert calls.cunn_b200_dwconv_forward(None, None, None, None, *GEO, None) != 0
     assert b"null" in lib.cunn_b200_last_error()
+
+
+def test_small_pointwise_layers_have_no_use_for_scratch():
+    """What functional.py does not ask for is 0: both sides of the limit, by the tensor that the pass reads."""
+    limit = calls.CONV_POINT_VALUES
+    N, H, W = 8, 7, 9
+    for which in range(3):
+        sizes = []
+        for C in range(limit // (N * H * W) - 300, limit // (N * H * W) + 300, 50):
+            cin, cout = (64, C) if which == 1 else (C, 512)
+            need = calls.cunn_b200_conv_scratch(which, N, cin, H, W, cout, 1, 1, 1, 1, 0, 0, 1, 1)
+            assert need == 0 or N * C * H * W >= limit
+            sizes.append(need)
+        assert which == 2 or any(sizes)

@@ -359,3 +359,29 @@ def test_large_values_in_a_later_round(F):
     F.convmm_acc_grad(x, gy, gw, gb, 1, 1, 1, 1)
     want = sum(torch.nn.grad.conv2d_weight(x[i:i + 4].double(), w.shape, gy[i:i + 4].double(), 1, 1) for i in range(0, N, 4))
     assert off(gw.double() - 1, want) <= 4e-6 and off(gb.double() - 1, gy.double().sum((0, 2, 3))) <= 1e-6
+
+
+@pytest.mark.parametrize("front", ["functional", "thnn"])
+def test_kernel_does_not_depend_on_earlier_calls(F, front):
+    """The parameter gradient of a layer that is better off without scratch, before and after another layer has made the shared buffers grow."""
+    from cunn_b200 import thnn
+    N, C, H, K = 16, 1024, 7, 2048
+    g = torch.Generator(device="cuda").manual_seed(33)
+    x, gy = torch.randn(N, C, H, H, device="cuda", generator=g), torch.randn(N, K, H, H, device="cuda", generator=g)
+    state = thnn.THNN()
+
+    def grad(x, gy):
+        w = torch.zeros(gy.shape[1], x.shape[1], 1, 1, device="cuda")
+        if front == "thnn":
+            state.SpatialConvolutionMM_accGradParameters(x, gy, w.view(w.shape[0], -1), None, 1, 1, 1, 1, 0, 0, 1.0)
+        else:
+            F.convmm_acc_grad(x, gy, w, None, 1, 1, 0, 0)
+        return w
+
+    first = grad(x, gy)
+    big = torch.randn(64, 1024, 20, 20, device="cuda", generator=g)
+    grad(big, torch.randn(64, 2048, 20, 20, device="cuda", generator=g))
+    if front == "functional":
+        F.workspace(64 << 20, x.device)
+    assert torch.equal(grad(x, gy), first)
+    state.close()
