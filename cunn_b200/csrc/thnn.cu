@@ -6,13 +6,52 @@
 #include "common.cuh"
 #include "../../include/THCUNN_b200.h"   // with CUNN_B200_USE_REAL_THC this pulls in cutorch's <THC/THC.h>
 
-#include <list>
 #include <mutex>
-#include <new>
 #include <stdlib.h>
 #include <string.h>
 #include <string>
 #include <vector>
+
+// ---- scratch of the convolutions -------------------------------------------------------------------------
+// The fast kernels of a convolution want scratch memory, which the passes did without before: what goes wrong with it must not
+// show.  It comes from a memory pool per device and is stream-ordered: a call's memory is its stream's from before its kernels to after them, the
+// pool passes it on when they have run, nothing waits and no stream waits for another one's work, destroyed streams included.  The pool
+// keeps up to 1 GiB (a pass takes 0.8 at most) and gives all of it back when a state is freed.
+namespace {
+constexpr int POOL_DEVICES = 64;
+std::mutex g_pool_mutex;
+cudaMemPool_t g_pool[POOL_DEVICES];
+bool g_pool_failed[POOL_DEVICES];
+
+cudaMemPool_t scratch_pool(int dev)
+{
+    if (dev < 0 || dev >= POOL_DEVICES) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (g_pool[dev] || g_pool_failed[dev]) return g_pool[dev];
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = (uint64_t)1 << 30;
+    int wait_for_others = 0;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess || cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &wait_for_others) != cudaSuccess) {
+        cudaGetLastError();
+        if (pool) cudaMemPoolDestroy(pool);
+        g_pool_failed[dev] = true;
+        return nullptr;
+    }
+    return g_pool[dev] = pool;
+}
+// What no call uses.
+void scratch_pools_release()
+{
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    for (cudaMemPool_t pool : g_pool)
+        if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess) cudaGetLastError();
+}
+}  // namespace
 
 // Tensor and state access goes through one of two back-ends with the same helper names:
 //   thc_backend_builtin.inc  the library's own state and tensor struct (default; what the tests drive);
@@ -30,28 +69,14 @@ extern "C" void thcunn_b200_not_implemented(THCState *state, const char *name)
     else fprintf(stderr, "THCUNN error: %s is not implemented in this build\n", name);
 }
 
-// ---- scratch of the convolutions -------------------------------------------------------------------------
-// The fast kernels of a convolution want scratch memory, which the passes did without before: what goes wrong with it must not
-// show.  A call has its buffer to itself until its kernels are queued, and gets one that only its own stream has used, so calls of
-// several threads and streams stay independent; where none can be had (no memory; a stream under capture, whose graph would keep the
-// address) it gets `least` bytes as ever, or none, and the other kernels.
-struct ScratchBuffer {
-    int device;
-    cudaStream_t stream;
-    void *ptr;
-    size_t bytes;
-    bool busy;
-};
-static std::mutex g_conv_scratch_mutex;
-static std::list<ScratchBuffer> g_conv_scratch;                            // used longest ago first
-
+// The scratch of one call: `want` bytes or, where they cannot be had (no memory; a stream under capture, whose graph would keep the address),
+// `least` bytes as ever, or none, and the other kernels.
 struct ConvScratch {
     void *ptr = nullptr;
     size_t bytes = 0;
-    ScratchBuffer *owner = nullptr;
-    ConvScratch(THCState *s, size_t want, size_t least = 0)
+    ConvScratch(THCState *s, size_t want, size_t least = 0) : stream(state_stream(s))
     {
-        if (want > least && take(state_stream(s), want)) return;
+        if (want > least && take(want)) return;
         if (!least) return;
         ptr = state_scratch(s, 0, least);
         bytes = ptr ? least : 0;                     // not what the state has: which kernels run must not depend on earlier calls
@@ -60,58 +85,28 @@ struct ConvScratch {
     ConvScratch &operator=(const ConvScratch &) = delete;
     ~ConvScratch()
     {
-        if (!owner) return;
-        std::lock_guard<std::mutex> lock(g_conv_scratch_mutex);
-        owner->busy = false;
+        if (pooled && cudaFreeAsync(ptr, stream) != cudaSuccess) cudaGetLastError();
     }
 
 private:
-    bool take(cudaStream_t stream, size_t want)
+    cudaStream_t stream;
+    bool pooled = false;
+    bool take(size_t want)
     {
-        constexpr size_t KEPT = 4;
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         int dev = 0;
         if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
-        std::lock_guard<std::mutex> lock(g_conv_scratch_mutex);
-        auto &pool = g_conv_scratch;
-        auto it = pool.begin();
-        while (it != pool.end() && (it->busy || it->device != dev || it->stream != stream)) ++it;
-        if (it != pool.end() && it->bytes >= want) {
-            pool.splice(pool.end(), pool, it);
-        } else {
-            // a larger one in its place, or in that of the one used longest ago when enough are kept; cudaFree waits for the device,
-            // so no kernel reads what goes
-            if (it == pool.end() && pool.size() >= KEPT) {
-                it = pool.begin();
-                while (it != pool.end() && it->busy) ++it;
-            }
-            if (it != pool.end()) {
-                if (cudaFree(it->ptr) != cudaSuccess) {
-                    cudaGetLastError();
-                    return false;
-                }
-                pool.erase(it);
-            }
-            void *p = nullptr;
-            if (cudaMalloc(&p, want) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
-            try {
-                pool.push_back(ScratchBuffer{dev, stream, p, want, false});
-            } catch (const std::bad_alloc &) {
-                cudaFree(p);
-                return false;
-            }
+        const cudaMemPool_t pool = scratch_pool(dev);
+        if (!pool || cudaMallocFromPoolAsync(&ptr, want, pool, stream) != cudaSuccess) {
+            cudaGetLastError();
+            ptr = nullptr;
+            return false;
         }
-        owner = &pool.back();
-        owner->busy = true;
-        ptr = owner->ptr;
-        bytes = owner->bytes;
-        return true;
+        bytes = want;
+        return pooled = true;
     }
 };
 

@@ -385,3 +385,50 @@ def test_kernel_does_not_depend_on_earlier_calls(F, front):
         F.workspace(64 << 20, x.device)
     assert torch.equal(grad(x, gy), first)
     state.close()
+
+
+def test_thnn_scratch_of_many_streams(F):
+    """More streams than buffers were once kept: calls do not wait for what other streams run, give the same results from several threads,
+    and the memory is given back with the state."""
+    import gc, threading, time
+    from cunn_b200 import thnn
+    N, C, H, K = 32, 128, 28, 128
+    g = torch.Generator(device="cuda").manual_seed(34)
+    xs = [torch.randn(N, C, H, H, device="cuda", generator=g) for _ in range(7)]
+    w = torch.randn(K, C * 9, device="cuda", generator=g)
+    want = [F.convmm_forward(x, w.view(K, C, 3, 3), None, 1, 1, 1, 1) for x in xs]
+    streams, states, got = [torch.cuda.Stream() for _ in xs], [thnn.THNN() for _ in xs], [None] * len(xs)
+    torch.cuda.synchronize()
+
+    def call(i):
+        with torch.cuda.stream(streams[i]):
+            got[i] = states[i].SpatialConvolutionMM_updateOutput(xs[i], w, None, 3, 3, 1, 1, 1, 1)
+
+    def everywhere(threads):
+        jobs = [threading.Thread(target=call, args=(i,)) for i in range(1, len(xs))] if threads else []
+        for t in jobs:
+            t.start()
+        for t in jobs:
+            t.join()
+        if not threads:
+            for i in range(1, len(xs)):
+                call(i)
+
+    for threads in (False, False, True):
+        everywhere(threads)
+        torch.cuda.synchronize()
+    for threads in (False, True):
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(400_000_000)                    # a fifth of a second
+        begin = time.perf_counter()
+        everywhere(threads)
+        assert time.perf_counter() - begin < 0.1
+        assert not streams[0].query()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got[1:], want[1:]))
+    gc.collect()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    for s in states:
+        s.close()
+    assert torch.cuda.mem_get_info()[0] - before >= (scratch(0, N, C, H, H, K, 3, 3, 1, 1, 1) >> 21) << 21
