@@ -6,10 +6,11 @@ There is no fallback: if the library has not been built, importing raises.
 import ctypes
 import importlib.util
 import os
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 SO_PATH = os.path.join(_HERE, "lib", "libTHCUNN.so")
-_CALLS_PATH = os.path.join(_HERE, "lib", "_calls.so")
+_CALLS_PATH = os.path.join(_HERE, "lib", "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 for _path in (SO_PATH, _CALLS_PATH):
     if not os.path.exists(_path):

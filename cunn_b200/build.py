@@ -1,4 +1,4 @@
-"""Builds libTHCUNN.so (the sm_100a kernels + C ABI) and _calls.so (the ABI as a Python module) in-tree.
+"""Builds libTHCUNN.so (the sm_100a kernels + C ABI) and _calls.<python version>.so (the ABI as a Python module) in-tree.
 
     python -m cunn_b200.build [--force] [--verbose]
 
@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 SO = os.path.join(LIBDIR, "libTHCUNN.so")
-CALLS = os.path.join(LIBDIR, "_calls.so")
+CALLS = os.path.join(LIBDIR, "_calls" + sysconfig.get_config_var("EXT_SUFFIX"))          # one per Python version
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [

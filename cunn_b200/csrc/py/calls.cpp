@@ -3,7 +3,8 @@
 // A small layer is over on the GPU before its call is: through ctypes, which looks up a converter for each of 14 arguments, a call takes
 // 5 us (2.4 us for a size with 11 integers), here 0.5.  The arguments' types come from include/cunn_b200.h; integers, numbers and addresses
 // are taken and refused as ctypes does with those types: an int or what has an __index__ for an integer, an int or None for a pointer, what
-// converts to float for a float, ctypes.ArgumentError otherwise.  Like ctypes, a call runs without the interpreter's lock.
+// converts to float for a float, ctypes.ArgumentError otherwise.  What ctypes takes beside them, instances of its own types and, as pointers,
+// bytes, is refused.  Like ctypes, a call runs without the interpreter's lock.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 

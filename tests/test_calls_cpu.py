@@ -56,3 +56,11 @@ def test_small_pointwise_layers_have_no_use_for_scratch():
             assert need == 0 or N * C * H * W >= limit
             sizes.append(need)
         assert which == 2 or any(sizes)
+
+
+def test_module_of_this_python():
+    """A module built for another version of Python is another file: it is neither loaded nor taken for one that is up to date."""
+    import os
+    import sysconfig
+    from cunn_b200 import build
+    assert os.path.basename(calls.__spec__.origin) == os.path.basename(build.CALLS) == "_calls" + sysconfig.get_config_var("EXT_SUFFIX")
