@@ -547,7 +547,7 @@ grad_apply_flat_kernel(const float *__restrict__ x, const float *__restrict__ gy
 // fit in a fraction of L2, and a persistent grid of co-resident CTAs (cooperative launch) walks the groups.
 //
 // Every CTA is two halves — eight consumer warps and one copy-issuing warp each — with a stream of their own (with four consumer warps the
-// forward pass of 256 x 64 x 112 x 112 took 416 us, the backward pass 13 % more than two launches; now 378 and 6 %.  Less than 128 MB, where
+// forward pass of 256 x 64 x 112 x 112 took 416 us, the backward pass 13 % more than two launches; now 382 and 6 %.  Less than 128 MB, where
 // a group's sums and flags weigh more, has four: 64 x 8 x 224 x 224 62 us with eight, 56 with four):
 //   * the statistics half reduces group after group (reads carry an L2 evict_last policy), hands in one partial
 //     per (CTA, channel) and takes a ticket; the CTA that draws a channel's last ticket merges the partials in fp64
@@ -1119,8 +1119,8 @@ static const bool g_group_bytes_from_env = [] {
 // 0: never use the grouped kernels; 1 (default): where they are faster; 2: wherever they apply.
 static int g_grouped_mode = 1;
 // Tensors of 128 MB or more with channel slabs of at least 1 MB, two launches / grouped in us.
-// Forward: 128 x 96 x 56 x 56 (154 MB) 94 / 80, 128 x 32 x 112 x 112 111 / 103, 256 x 64 x 112 x 112 420 / 378, 1024 x 64 x 56 x 56
-// 454 / 384, 512 x 32 x 112 x 112 (slabs of 26 MB) 424 / 391, 2 x 16 x 1024 x 1024 315 / 69; but 128 x 256 x 28 x 28 (103 MB) 58 / 62,
+// Forward: 128 x 96 x 56 x 56 (154 MB) 94 / 82, 128 x 32 x 112 x 112 111 / 103, 256 x 64 x 112 x 112 420 / 382, 1024 x 64 x 56 x 56
+// 454 / 387, 512 x 32 x 112 x 112 (slabs of 26 MB) 424 / 391, 2 x 16 x 1024 x 1024 315 / 69; but 128 x 256 x 28 x 28 (103 MB) 58 / 62,
 // 256 x 256 x 28 x 28 (slabs of 0.8 MB) 112 / 113.
 // Backward, which is instruction-bound: planes of 1025 to 4000 elements, of which the other kernels' CTAs of 256 threads make poor use
 // (128 x 128 x 56 x 56 176 / 166, 1024 x 64 x 56 x 56 680 / 656, 1000 x 40 x 40 x 32 181 / 166), and few planes (16 x 64 x 256 x 256 224 / 205,

@@ -29,10 +29,10 @@
 // the cross terms first, while the accumulator is small; blocks are added in registers with rounding (two TMEM buffers in turn).
 //
 // Forward / input gradient / parameter gradient in us, gathering kernels and here: 3x3 256 -> 256 on 128 x 14 x 14 270 / 313 / 354 and
-// 101 / 99 / 124; 3x3 stride 2 128 -> 256 on 64 x 56 x 56 312 / 427 / 360 and 134 / 172 / 189; 4x4 stride 2 transposed 256 -> 128 on
-// 64 x 14 x 14 240 / 193 / 172 and 72 / 61 / 80; 7x7 stride 2, 3 -> 64 on 32 x 224 x 224 234 / - / 316 and 130 / - / 196.  2-norm errors of the
-// first 9.7e-7 / 2.1e-6 / 2.7e-6 and 0.8e-7 / 1.6e-7 / 1.9e-7.  The split takes 14 of the 101 us, in a parameter gradient the maxima 18 and
-// the split 19 of 124.  The matrix kernel needs 1,100 to 1,200 clocks per 128 x 256 x 32 values, where the tensor pipe needs 768 and reading
+// 106 / 106 / 129; 3x3 stride 2 128 -> 256 on 64 x 56 x 56 312 / 427 / 360 and 139 / 174 / 185; 4x4 stride 2 transposed 256 -> 128 on
+// 64 x 14 x 14 240 / 193 / 172 and 69 / 61 / 84; 7x7 stride 2, 3 -> 64 on 32 x 224 x 224 234 / - / 316 and 131 / - / 189.  2-norm errors of the
+// first 9.7e-7 / 2.1e-6 / 2.7e-6 and 0.8e-7 / 1.6e-7 / 1.9e-7.  The split takes 14 of the 106 us, looking at the sums 3, the idle launch after the
+// kernel 5; in a parameter gradient the maxima take 18 and the split 20 of 129.  The matrix kernel needs 1,100 to 1,200 clocks per 128 x 256 x 32 values, where the tensor pipe needs 768 and reading
 // its operands from shared memory, and filling them, 940.
 //
 // Work: 128 x BN tiles of the persistent grid; the tiles of a last wave that would leave SMs idle are cut along the reduction, and the
@@ -1216,7 +1216,9 @@ static int images_per_round(int N, size_t image_bytes)
     const int most = (int)std::max<size_t>(1, std::min<size_t>((size_t)N, ROUND_BYTES / std::max<size_t>(1, image_bytes)));
     return ceil_div(N, ceil_div(N, most));             // rounds of one size
 }
-// Tensor maps of less memory than this are left alone: some drivers encode smaller im2col maps for walks that they do not do.
+// Smaller im2col tensor maps are left alone, as a precaution: public code for them works around what drivers encode for tensors below 128 KiB.
+// Not seen here, and not to be tried: a wrong walk may read out of bounds.  It keeps layers of up to 32,768 values away, of a pass's fixed
+// 12 us the smallest.
 constexpr size_t MIN_MAP_BYTES = 131072;
 
 // ---- forward pass and input gradients -------------------------------------------------------------------------------------------

@@ -114,7 +114,7 @@ CUNN_API int cunn_b200_convmm_grad_input(const float *gy, const float *weight, f
 
 /* grad_weight [K, C*kH*kW] += scale * dL/dW, grad_bias [K] += scale * sum gy (may be NULL).  `workspace`:
  * caller-owned scratch of at least cunn_b200_convmm_acc_grad_workspace(...) bytes, 16-byte aligned,
- * contents irrelevant.  Replaces ..._accGradParameters
+ * contents irrelevant; cunn_b200_conv_scratch(2, ...) bytes, where that is not 0, get faster kernels.  Replaces ..._accGradParameters
  * (lib/THCUNN/generic/SpatialConvolutionMM.cu:327-486). */
 CUNN_API size_t cunn_b200_convmm_acc_grad_workspace(int N, int C, int H, int W, int K, int kH, int kW,
                                                     int dH, int dW, int padH, int padW);
@@ -130,11 +130,20 @@ CUNN_API int cunn_b200_convmm_acc_grad(const float *x, const float *gy, float *g
 CUNN_API void cunn_b200_convmm_set_tma(int on);
 CUNN_API int cunn_b200_convmm_get_tma(void);
 
-/* Forward pass (pass 0) and input gradient (pass 1) of a convolution with scratch memory: kernels of more than one tap then
- * run on operands that a first pass splits once, two to five times faster.  cunn_b200_conv_scratch(...) gives the bytes
- * (16-byte aligned, contents arbitrary, at most about the size of the tensor that the pass reads, bounded by 0.5 GiB
- * and one image's, plus that of the weights); 0: the pass has no use for scratch.  With less, or NULL, the calls are those
- * without scratch.  No reference counterpart: the reference's `columns` buffer is scratch of the same kind. */
+/* Convolutions with scratch memory: most kernels of more than one tap, and the larger 1x1 layers, then run on operands that a
+ * first pass splits once, two to five times faster.  cunn_b200_conv_scratch(pass, ...) gives the bytes (16-byte aligned,
+ * contents arbitrary); 0: the pass has no use for scratch, or is faster without.
+ *   pass 0, 1  forward pass and input gradient: the scratch of the two calls below.  4 bytes a value of the tensor that is
+ *              read, channels padded to 16 or 32 (of fewer than 16 channels: every value as often as a row's windows
+ *              overlap), at most 512 MiB or one image at a time, the same of the weights, and up to 20 MiB.
+ *   pass 2     parameter gradient: the workspace of cunn_b200_convmm_acc_grad and cunn_b200_dilated_conv_acc_grad.  Both
+ *              tensors as above, and several times the weights' size for partial sums.
+ * With less, or NULL, the calls are those without scratch: other kernels, results that agree to rounding.  What decides is
+ * the size that a call is given, so a caller that keeps a larger buffer passes the size it asked for, lest its
+ * kernels depend on its history.
+ * Values of a tensor may differ in size as floats do: sums that the shared exponents of the split operands would cost
+ * digits are taken again by the kernels without scratch, within the call and at their speed.
+ * No reference counterpart: the reference's `columns` buffer is scratch of the same kind. */
 #define CUNN_B200_CONV_POINT_VALUES (1 << 20) /* 1x1 layers that read fewer values have no use for scratch */
 CUNN_API size_t cunn_b200_conv_scratch(int pass, int N, int C, int H, int W, int K, int kH, int kW, int dH, int dW,
                                        int padH, int padW, int dilH, int dilW);
@@ -184,7 +193,7 @@ CUNN_API int cunn_b200_full_conv_grad_input(const float *gy, const float *weight
                                             int N, int P, int H, int W, int Q, int kH, int kW, int dH, int dW,
                                             int padH, int padW, int dilH, int dilW, int adjH, int adjW,
                                             cunn_stream_t stream);
-/* The first two with scratch memory, as for cunn_b200_conv_forward_scratch. */
+/* The first two with scratch memory, as for cunn_b200_conv_forward_scratch; pass 2: cunn_b200_full_conv_acc_grad's workspace. */
 CUNN_API size_t cunn_b200_full_conv_scratch(int pass, int N, int P, int H, int W, int Q, int kH, int kW, int dH, int dW,
                                             int padH, int padW, int dilH, int dilW, int adjH, int adjW);
 CUNN_API int cunn_b200_full_conv_forward_scratch(const float *x, const float *weight, const float *bias, float *y,
