@@ -71,8 +71,8 @@ constexpr int SCALED_MAX = 14;           // the largest value of a group lies in
 constexpr float SMALL_SUM = 4096.f;
 constexpr int MOST_SMALL = 8;            // ... of the 32 x 16 sums that a warp writes at a time; a lost row makes 16, a lost column 32
 // The same of a parameter gradient's sum of n products, beside sqrt(n): 2^25 ordinary, off by 2^-12 on average if all values are lost.  Sums of
-// mostly zeros are small without that: only those count one of whose channels has a WIDE range, shares of it (a warp's of channel_max_kernel)
-// being below 2^-16 of its largest.
+// mostly zeros are small without that: only those count one of whose channels has a WIDE range, pieces of it (channel_max_kernel's, planes of up to 2048
+// values) being below 2^-16 of its largest.
 constexpr float SMALL_GRAD = 512.f;
 constexpr int WIDE = 16, MOST_SMALL_GRADS = 2;             // threads of a block of 32 x 4 to 32 gradients
 
@@ -396,21 +396,21 @@ prep_kernel(const __grid_constant__ PrepParams p)
     if (WINDOW && !PER_CHANNEL && threadIdx.x == 0) p.wide[blockIdx.x] = wide;
 }
 
-// Largest finite magnitude of every channel and the smallest of its shares' largest, and the sums of the first tensor's channels (the bias gradient): block = (channel, chunk of
-// the channel's pieces), a warp per piece of a plane.
+// Largest finite magnitude of every channel and the smallest of its pieces' largest, and the sums of the first tensor's channels (the bias
+// gradient): block = (channel, chunk of the channel's pieces), a warp per piece of a plane.
 constexpr int PIECE = 2048;              // values of a plane that a warp takes, at most
 struct MaxParams {
     const float *src[2];
-    uint32_t *chmax[2], *chlow[2];                               // chlow: the complement of the smallest share's largest, 0: no share has values
+    uint32_t *chmax[2], *chlow[2];                               // chlow: the complement of the smallest piece's largest, 0: no piece has values
     double *sums;                                                // [chunks][C] of the first tensor, or null
     int C[2], HW[2], pieces[2], chunks[2], vec[2], images;       // pieces of a plane; vec: planes of a multiple of four values, 16-byte aligned
 };
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 5)
 channel_max_kernel(const __grid_constant__ MaxParams p)
 {
     pdl_launch_dependents();
     __shared__ double part[8];
-    __shared__ uint32_t red[8];
+    __shared__ uint32_t red[8], red_low[8];
     int b = (int)blockIdx.x, t = 0;
     if (b >= p.C[0] * p.chunks[0]) { b -= p.C[0] * p.chunks[0]; t = 1; }
     const int chunk = b / p.C[t], c = b - chunk * p.C[t], HW = p.HW[t], per = p.pieces[t], warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -419,9 +419,10 @@ channel_max_kernel(const __grid_constant__ MaxParams p)
     const int unit = p.vec[t] ? HW / 4 : HW, len = (unit + per - 1) / per;           // (per - 1) * len < unit
     const float *src = p.src[t] + (size_t)c * HW;
     const bool add = p.sums && t == 0;
-    float m = 0.f;
+    uint32_t bits = 0, low = 0;
     double sum = 0.0;
     for (int n = n0 + warp; n < n1; n += 32) {                             // four pieces at a time
+        float m[4] = {0.f, 0.f, 0.f, 0.f};
         const float *s[4];
         int left[4];
 #pragma unroll
@@ -439,7 +440,7 @@ channel_max_kernel(const __grid_constant__ MaxParams p)
                 for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const float4 *>(s[j]) + min(i, left[j]));
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    m = fmaxf(m, fmaxf(fmaxf(finite_abs(v[j].x), finite_abs(v[j].y)), fmaxf(finite_abs(v[j].z), finite_abs(v[j].w))));
+                    m[j] = fmaxf(m[j], fmaxf(fmaxf(finite_abs(v[j].x), finite_abs(v[j].y)), fmaxf(finite_abs(v[j].z), finite_abs(v[j].w))));
                 if (add) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
@@ -452,15 +453,19 @@ channel_max_kernel(const __grid_constant__ MaxParams p)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float v = __ldg(s[j] + min(i, left[j]));
-                    m = fmaxf(m, finite_abs(v));
+                    m[j] = fmaxf(m[j], finite_abs(v));
                     if (add && i <= left[j] && n + 8 * j < n1) sum += (double)v;
                 }
             }
         }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t piece = __reduce_max_sync(0xffffffffu, __float_as_uint(m[j]));
+            bits = max(bits, piece);
+            low = max(low, piece ? ~piece : 0u);
+        }
     }
-    uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-    if (lane == 0) red[warp] = bits;
-    uint32_t low = bits ? ~bits : 0u;                                      // a warp's share of the channel
+    if (lane == 0) { red[warp] = bits; red_low[warp] = low; }
     if (add) {
         sum = warp_sum(sum);
         if (lane == 0) part[warp] = sum;
@@ -470,7 +475,7 @@ channel_max_kernel(const __grid_constant__ MaxParams p)
 #pragma unroll
         for (int i = 1; i < 8; ++i) {
             bits = max(bits, red[i]);
-            low = max(low, red[i] ? ~red[i] : 0u);
+            low = max(low, red_low[i]);
         }
         atomicMax(p.chmax[t] + c, bits);
         atomicMax(p.chlow[t] + c, low);

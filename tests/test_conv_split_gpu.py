@@ -338,6 +338,25 @@ def test_ordinary_values_stay_here(F, kind):
         assert off(got, want.double()) <= 6e-6
 
 
+@pytest.mark.parametrize("outlier", ["gy", "x"])
+@pytest.mark.parametrize("size", [1e7, 1e12])
+def test_large_images_opposite_zeros(F, outlier, size):
+    """A parameter gradient of images of two sizes, the large ones opposite zeros and among every eight images in turn."""
+    N, C, H, K, k = 20, 37, 40, 320, 4
+    assert scratch(2, N, C, H, H, K, k, k, 2, 1, 1)
+    g = torch.Generator(device="cuda").manual_seed(35)
+    x, gy = torch.randn(N, C, H, H, device="cuda", generator=g), torch.randn(N, K, 20, 20, device="cuda", generator=g)
+    large = torch.arange(N, device="cuda") // 8 % 2 == 0
+    a, b = (gy, x) if outlier == "gy" else (x, gy)
+    a[large] *= size
+    b[large] = 0
+    gw = torch.zeros(K, C, k, k, device="cuda")
+    F.convmm_acc_grad(x, gy, gw, None, 2, 2, 1, 1)
+    want = torch.nn.grad.conv2d_weight(x.double(), gw.shape, gy.double(), 2, 1)
+    rows = (gw.double() - want).flatten(1).norm(dim=1) / want.flatten(1).norm(dim=1)
+    assert float(rows.max()) <= 2 * gather_bound(N * 400)
+
+
 def test_large_values_in_a_later_round(F):
     """Scratch holds 512 MB of split values: a later part of the batch is judged, and taken, for itself; what the call adds to, it adds once."""
     N, C, H, K = 44, 64, 240, 16
