@@ -32,7 +32,7 @@
 // 106 / 106 / 129; 3x3 stride 2 128 -> 256 on 64 x 56 x 56 312 / 427 / 360 and 139 / 174 / 185; 4x4 stride 2 transposed 256 -> 128 on
 // 64 x 14 x 14 240 / 193 / 172 and 69 / 61 / 84; 7x7 stride 2, 3 -> 64 on 32 x 224 x 224 234 / - / 316 and 131 / - / 189.  2-norm errors of the
 // first 9.7e-7 / 2.1e-6 / 2.7e-6 and 0.8e-7 / 1.6e-7 / 1.9e-7.  The split takes 14 of the 106 us, looking at the sums 3, the idle launch after the
-// kernel 5; in a parameter gradient the maxima take 18 and the split 20 of 129.  The matrix kernel needs 1,100 to 1,200 clocks per 128 x 256 x 32 values, where the tensor pipe needs 768 and reading
+// kernel 5; in a parameter gradient the maxima take 19 and the split 20 of 130.  The matrix kernel needs 1,100 to 1,200 clocks per 128 x 256 x 32 values, where the tensor pipe needs 768 and reading
 // its operands from shared memory, and filling them, 940.
 //
 // Work: 128 x BN tiles of the persistent grid; the tiles of a last wave that would leave SMs idle are cut along the reduction, and the
