@@ -22,7 +22,7 @@
 // without weights among ordinary ones left 3 digits, one of 1e13 none.  So the sums are compared with what the exponents of their operands
 // allow for: SMALL_SUM and SMALL_GRAD say when they are too small for that, by more than chance, and the images of the round are done again by the
 // kernels of convmm.cu, whose tf32 operands have an exponent each.  Those are launched every time and leave at once if *gate says that
-// nothing was lost, which costs a pass 2 to 5 us.  (Looking at the operands instead cost the split as much, and sent the gradients of half of
+// nothing was lost, which costs a pass 2 to 8 us with looking at the sums.  (Looking at the operands instead cost the split as much, and sent the gradients of half of
 // MobileNetV1's pointwise layers there.)
 //
 // Accumulation: the tensor core truncates when it adds, so a chain is one block, 64 channels (or pixels) of 12 additions, the eight of
